@@ -563,6 +563,23 @@ int steps_grid(int consumer, int walk, bool pk, uint64_t nlocal, int* grid);
 cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, int consumer, int walk, bool pk,
                          int grid);
 
+// ---- light steps without a consumer (k_flight.cu) -----------------------------
+constexpr uint32_t kFlightMaxSteps = 4096;  // one launch stays short when nothing trips
+struct FlightArgs {
+    AtomCols c;
+    uint64_t nlocal;
+    double dt;
+    int first_fused;     // the first step's pass also applies the pending final half-kick
+    CheckArgs ck;        // the displacement check (every step)
+    FwdArgs fw;          // forward comm after the last step
+    uint32_t max_steps;
+    uint32_t* late;       // zero at launch
+    uint32_t* next_late;  // cleared for the next flight
+    uint32_t* out;        // host memory mapped for the device: steps completed; 1 if the
+                          // next step's check tripped
+};
+void launch_flight(cudaStream_t st, const FlightArgs& a);
+
 void launch_harmonic(cudaStream_t st, uint64_t nlocal, uint64_t ntotal, const AtomCols& c,
                      const double* radius, double k, int newton, const uint32_t* offsets,
                      const uint32_t* indices, const uint32_t* in_start, const uint32_t* in_list);

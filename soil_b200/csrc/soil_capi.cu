@@ -1716,6 +1716,7 @@ struct StepPlan {
     // pbc (and, when the sort is due, its binning) ran in the integration
     // pass of a step that rebuilds for certain; sort_plan's answers
     bool pbc_done = false, sort_due = false, periodic_sort = false;
+    bool tripped = false;  // the check is known to have tripped (light steps read it)
 };
 
 StepPlan plan_step(const soil_sys* s) {
@@ -1802,7 +1803,9 @@ int step_rest(soil_sys* s, const StepPlan& p, bool last) {
     // decide_rebuild
     if (s->state == COMMUNICATE_ONLY) {
         bool disp = false;
-        if (p.check) {
+        if (p.tripped) {
+            disp = true;
+        } else if (p.check) {
             TRY(read_flags(s));
             disp = s->hflags->rebuild != 0;
         }
@@ -1908,7 +1911,7 @@ uint64_t resident_limit(const soil_sys* s, uint64_t want) {
     const char* env = std::getenv("SOIL_RESIDENT_STEPS");
     const int mode = env ? std::atoi(env) : 2;  // 0 off, 1 always, 2 auto
     if (mode == 0) return 0;
-    if (mode == 2 && s->nlocal > kResidentAutoMaxAtoms) return 0;
+    if (mode == 2 && builtin_consumer(s) && s->nlocal > kResidentAutoMaxAtoms) return 0;
     if (s->hook || s->timing_mask || !s->check || s->every != 0) return 0;
     if (s->state != COMMUNICATE_ONLY || !displacement_needed(s) || needs_rebuild_with(s, false))
         return 0;
@@ -1925,6 +1928,59 @@ uint64_t resident_limit(const soil_sys* s, uint64_t want) {
         lim = std::min<uint64_t>(lim, s->sort_every - s->sort_counter - 1);
     }
     return lim;
+}
+
+// Room for the words of the light-step kernels, zero when first used.
+int light_words(soil_sys* s) {
+    const uint32_t* old = s->rstate.p;
+    TRY(ensure(s, s->rstate, 16));
+    if (s->rstate.p != old) CK(cudaMemsetAsync(s->rstate.p, 0, s->rstate.cap * 4, s->st));
+    return SOIL_OK;
+}
+
+// Bookkeeping of `done` completed light steps, the next one integrated too
+// when tripped.
+void light_steps_done(soil_sys* s, uint64_t done, bool tripped) {
+    s->steps_done += done;
+    s->steps_since_build += done;
+    if (s->sort_every > 0) s->sort_counter += done;
+    // every completed step leaves its final half-kick pending; a tripped
+    // step's integration pass applied the last one
+    s->pending_final = !tripped;
+}
+
+// Up to `max` communicate-only steps of a system without a consumer
+// (k_flight.cu); answers as resident_steps.
+int flight_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, StepPlan* plan) {
+    *plan = plan_step(s);
+    max = std::min<uint64_t>(max, kFlightMaxSteps);
+    s->pk_valid = false;
+    TRY(light_words(s));
+    FlightArgs a;
+    a.c = s->A;
+    a.nlocal = s->nlocal;
+    a.dt = s->dt;
+    a.first_fused = s->pending_final ? 1 : 0;
+    a.ck = make_check(s->lbx.p, s->lby.p, s->lbz.p, s->nlocal, displacement_threshold_sq(s),
+                      s->pbc_box, s->dflags, pbc_mask(s));
+    a.fw = fwd_args(s, true);
+    a.max_steps = (uint32_t)max;
+    a.late = s->rstate.p + 8 + s->flights % 2;
+    a.next_late = s->rstate.p + 8 + (s->flights + 1) % 2;
+    a.out = s->hword_dev;
+    s->flights += 1;
+    launch_flight(s->st, a);
+    TRY(check_launch(s));
+    TRY(sync(s));
+    *done = s->hword[0];
+    *tripped = s->hword[1] != 0;
+    if (*done > max || *tripped != (*done < max))
+        return fail(s->ctx, SOIL_ERR_CUDA, "light steps: inconsistent step count");
+    light_steps_done(s, *done, *tripped);
+    plan->check = true;
+    plan->fwd_fused = true;
+    plan->tripped = true;
+    return SOIL_OK;
 }
 
 // Up to `max` communicate-only steps in one launch; *done of them complete.
@@ -1962,7 +2018,7 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, Ste
         }
     }
     a.max_steps = max;
-    TRY(ensure(s, s->rstate, 8));
+    TRY(light_words(s));
     a.bar = reinterpret_cast<GridBar*>(s->rstate.p);
     a.out = s->rstate.p + 2;
     a.trip = s->rstate.p + 4;
@@ -1983,12 +2039,7 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, Ste
     *tripped = s->hword[1] != 0;
     if (*done > max || (!*tripped && *done != max))
         return fail(s->ctx, SOIL_ERR_CUDA, "resident steps: inconsistent step count");
-    s->steps_done += *done;
-    s->steps_since_build += *done;
-    if (s->sort_every > 0) s->sort_counter += *done;
-    // every completed step leaves its final half-kick pending; a tripped
-    // step's integration pass applied the last one
-    s->pending_final = !*tripped;
+    light_steps_done(s, *done, *tripped);
     *plan = p;
     plan->check = true;
     plan->fwd_fused = true;
@@ -2006,7 +2057,8 @@ int step_many(soil_sys* s, uint64_t n) {
             uint64_t done = 0;
             bool tripped = false;
             StepPlan p;
-            TRY(resident_steps(s, lim, &done, &tripped, &p));
+            TRY(builtin_consumer(s) ? resident_steps(s, lim, &done, &tripped, &p)
+                                    : flight_steps(s, lim, &done, &tripped, &p));
             k += done;
             if (tripped) {  // step k + 1: integrated, its check tripped
                 TRY(step_rest(s, p, k + 1 == n));

@@ -165,7 +165,10 @@ struct soil_sys {
     DArr<uint8_t> seq_owner;
     bool seq_valid = false;
     bool few_images = false;  // no local has images on both sides of a dim (<= 7 images)
-    DArr<uint32_t> rstate;    // resident steps: grid barrier words, step count, trip flag
+    // light steps: grid barrier words, step count and trip flag of the resident
+    // launch (0-7), the end-step words of the flights (8, 9, used in turn)
+    DArr<uint32_t> rstate;
+    uint64_t flights = 0;
     DArr<uint32_t> scan1p;    // single-pass scan: tile counter and descriptors (zeroed at growth)
     DArr<uint32_t> root_order;  // CSR-walk consumer: roots by work per block (rebuilt with the lists)
     bool order_valid = false;
