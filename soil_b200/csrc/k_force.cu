@@ -111,8 +111,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_walk(ForceArgs p) {
 }
 
 template <bool FOLD, bool PK>
-__global__ void __launch_bounds__(kBlock, 4) k_force_csr(ForceCsr q, AtomCols c, PlaneList rev) {
+__global__ void __launch_bounds__(kBlock, 4) k_force_csr(ForceCsr q, AtomCols c, PlaneList rev,
+                                                         const uint32_t* trip) {
     pdl_wait();  // launched with pdl_launch
+    if (trip && *trip) return;  // the step rebuilds: its forces come later
     // grid-stride over whole blocks of kBlock roots, so a block's order
     // permutes its own roots
     for (uint64_t b = (uint64_t)blockIdx.x * kBlock; b < q.nlocal; b += (uint64_t)gridDim.x * kBlock) {
@@ -165,7 +167,7 @@ void launch_root_order(cudaStream_t st, const ForceCsr& q, uint32_t* order) {
 }
 
 void launch_force_csr(cudaStream_t st, const ForceCsr& q, const AtomCols& c, const PlaneList& rev,
-                      bool fold) {
+                      bool fold, const uint32_t* trip) {
     if (q.nlocal == 0) return;
     note_launch();
     // one resident wave at <= 64 registers, striding over blocks of roots
@@ -177,11 +179,11 @@ void launch_force_csr(cudaStream_t st, const ForceCsr& q, const AtomCols& c, con
     const unsigned need = (unsigned)((q.nlocal + kBlock - 1) / kBlock);
     const unsigned grid = need < full ? need : full;
     if (q.pk) {
-        if (fold) pdl_launch(k_force_csr<true, true>, grid, kBlock, 0, st, q, c, rev);
-        else pdl_launch(k_force_csr<false, true>, grid, kBlock, 0, st, q, c, rev);
+        if (fold) pdl_launch(k_force_csr<true, true>, grid, kBlock, 0, st, q, c, rev, trip);
+        else pdl_launch(k_force_csr<false, true>, grid, kBlock, 0, st, q, c, rev, trip);
     } else {
-        if (fold) pdl_launch(k_force_csr<true, false>, grid, kBlock, 0, st, q, c, rev);
-        else pdl_launch(k_force_csr<false, false>, grid, kBlock, 0, st, q, c, rev);
+        if (fold) pdl_launch(k_force_csr<true, false>, grid, kBlock, 0, st, q, c, rev, trip);
+        else pdl_launch(k_force_csr<false, false>, grid, kBlock, 0, st, q, c, rev, trip);
     }
 }
 

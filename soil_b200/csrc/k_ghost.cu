@@ -235,8 +235,15 @@ void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCo
 
 __global__ void __launch_bounds__(kBlock) k_forward(uint64_t nlocal, uint64_t nghost, AtomCols c,
                                                     const uint32_t* root, const uint32_t* chain,
-                                                    SwapConst sc, PlaneList fwd, int zero_force) {
+                                                    SwapConst sc, PlaneList fwd, int zero_force,
+                                                    LightStep light) {
     pdl_wait();  // launched with pdl_launch
+    if (light.trip) {
+        const uint32_t tripped = *light.trip;
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            *(volatile uint32_t*)light.answer = light.tag | tripped;
+        if (tripped) return;
+    }
     for (uint64_t gi = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; gi < nghost;
          gi += (uint64_t)gridDim.x * blockDim.x)
         forward_ghost(c, nlocal, gi, root, chain, sc, fwd, zero_force != 0);
@@ -244,14 +251,14 @@ __global__ void __launch_bounds__(kBlock) k_forward(uint64_t nlocal, uint64_t ng
 
 void launch_forward(cudaStream_t st, uint64_t nlocal, uint64_t nghost, const AtomCols& c,
                     const uint32_t* ghost_root, const uint32_t* ghost_chain, const SwapConst& sc,
-                    const int* fwd_planes, int nfwd, bool zero_force) {
+                    const int* fwd_planes, int nfwd, bool zero_force, const LightStep* light) {
     if (nghost == 0) return;
     PlaneList pl;
     pl.n = nfwd;
     for (int k = 0; k < nfwd; ++k) pl.idx[k] = fwd_planes[k];
     note_launch();
     pdl_launch(k_forward, grid_wave<k_forward>(nghost), kBlock, 0, st, nlocal, nghost, c, ghost_root, ghost_chain, sc,
-                                                   pl, zero_force ? 1 : 0);
+                                                   pl, zero_force ? 1 : 0, light ? *light : LightStep{});
 }
 
 // ---- reverse comm as one fold per image tree ------------------------------

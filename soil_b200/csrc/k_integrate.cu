@@ -55,9 +55,10 @@ __global__ void __launch_bounds__(kBlock, 5) k_initial(uint64_t n, AtomCols c, d
             forward_images(c, n, i, x, y, z, vx, vy, vz, fw.fold_start, fw.fold_list, fw.chain,
                            fw.sc, fw.fwd, fw.zero_ghost_force != 0);
     }
-    if (ck.flags) {
+    if (ck.trip) {
         unsigned any = __ballot_sync(0xffffffffu, hit);
-        if (any && (threadIdx.x & 31) == 0) atomicOr(&ck.flags->rebuild, 1u);
+        if (any && (threadIdx.x & 31) == 0) atomicOr(ck.trip, 1u);
+        if (ck.next && blockIdx.x == 0 && threadIdx.x == 0) *ck.next = 0u;
     }
 }
 
@@ -75,8 +76,15 @@ CheckArgs make_check(const double* lbx, const double* lby, const double* lbz,
         ck.box[d] = box ? box[d] : 1.0;
         ck.ibox[d] = 1.0 / ck.box[d];  // ibx = 1.0 / bx (neighbor.rs:716-718)
     }
-    ck.flags = lbx ? flags : nullptr;
+    ck.trip = lbx ? &flags->rebuild : nullptr;
+    ck.next = nullptr;
     return ck;
+}
+
+static void light_check(CheckArgs& ck, const LightStep* light) {
+    if (!light) return;
+    ck.trip = light->trip;
+    ck.next = light->next;
 }
 
 template <bool FUSE_FINAL>
@@ -96,18 +104,21 @@ static void initial_kernel(cudaStream_t st, uint64_t n, const AtomCols& c, doubl
 void launch_initial(cudaStream_t st, uint64_t n, const AtomCols& c, double dt, bool zero_force,
                     const double* lbx, const double* lby, const double* lbz, uint64_t n_check,
                     double thr_sq, const double box[3], DevFlags* flags, int pbc_mask,
-                    const FwdArgs* fw) {
+                    const FwdArgs* fw, const LightStep* light) {
     if (n == 0) return;
     CheckArgs ck = make_check(lbx, lby, lbz, n_check, thr_sq, box, flags, pbc_mask);
+    light_check(ck, light);
     initial_kernel<false>(st, n, c, dt, zero_force, ck, fw);
 }
 
 void launch_final_initial(cudaStream_t st, uint64_t n, const AtomCols& c, double dt,
                           bool zero_force, const double* lbx, const double* lby,
                           const double* lbz, uint64_t n_check, double thr_sq,
-                          const double box[3], DevFlags* flags, int pbc_mask, const FwdArgs* fw) {
+                          const double box[3], DevFlags* flags, int pbc_mask, const FwdArgs* fw,
+                          const LightStep* light) {
     if (n == 0) return;
     CheckArgs ck = make_check(lbx, lby, lbz, n_check, thr_sq, box, flags, pbc_mask);
+    light_check(ck, light);
     initial_kernel<true>(st, n, c, dt, zero_force, ck, fw);
 }
 
@@ -203,7 +214,7 @@ __global__ void __launch_bounds__(kBlock) k_disp_check(uint64_t n, AtomCols c, C
          i += (uint64_t)gridDim.x * blockDim.x)
         hit |= check_moved(ck, c.x[i], c.y[i], c.z[i], i);
     if (__ballot_sync(0xffffffffu, hit) && (threadIdx.x & 31) == 0)
-        atomicOr(&ck.flags->rebuild, 1u);
+        atomicOr(ck.trip, 1u);
 }
 
 void launch_disp_check(cudaStream_t st, uint64_t n, const AtomCols& c, const double* lbx,

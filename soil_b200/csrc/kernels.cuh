@@ -80,8 +80,20 @@ struct CheckArgs {
     double thr_sq;
     double box[3];
     double ibox[3];
-    DevFlags* flags;
+    uint32_t* trip;  // set to 1 when an atom moved too far
+    uint32_t* next;  // when given, cleared by the pass (the next step's trip word)
     int mask;  // periodic axes (7: fully periodic fast path)
+};
+// A step's words when its forward comm and consumer go in before the host has
+// its check's answer: the pass sets *trip, clears *next, and the later
+// launches of the step do nothing when *trip is set.  The forward pass hands
+// the host the answer: *answer = tag, plus 1 when tripped (host memory mapped
+// for the device).
+struct LightStep {
+    uint32_t* trip = nullptr;
+    uint32_t* next = nullptr;
+    uint32_t* answer = nullptr;
+    uint32_t tag = 0;
 };
 CheckArgs make_check(const double* lbx, const double* lby, const double* lbz, uint64_t n_check,
                      double thr_sq, const double box[3], DevFlags* flags, int mask);
@@ -102,7 +114,7 @@ struct FwdArgs {
 void launch_initial(cudaStream_t st, uint64_t n, const AtomCols& c, double dt, bool zero_force,
                     const double* lbx, const double* lby, const double* lbz, uint64_t n_check,
                     double thr_sq, const double box[3], DevFlags* flags, int pbc_mask = 7,
-                    const FwdArgs* fw = nullptr);
+                    const FwdArgs* fw = nullptr, const LightStep* light = nullptr);
 // final_integration
 void launch_final(cudaStream_t st, uint64_t n, const AtomCols& c, double dt);
 // final_integration of step t fused with initial_integration of step t+1
@@ -110,7 +122,7 @@ void launch_final_initial(cudaStream_t st, uint64_t n, const AtomCols& c, double
                           bool zero_force, const double* lbx, const double* lby,
                           const double* lbz, uint64_t n_check, double thr_sq,
                           const double box[3], DevFlags* flags, int pbc_mask = 7,
-                          const FwdArgs* fw = nullptr);
+                          const FwdArgs* fw = nullptr, const LightStep* light = nullptr);
 // zero_all_forces over [0, n) + the #[zero] planes
 void launch_zero_forces(cudaStream_t st, uint64_t n, const AtomCols& c, const int* zero_planes,
                         int nzero);
@@ -341,7 +353,8 @@ void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCo
 // forward_comm: every ghost from its root local atom through its swap chain
 void launch_forward(cudaStream_t st, uint64_t nlocal, uint64_t nghost, const AtomCols& c,
                     const uint32_t* ghost_root, const uint32_t* ghost_chain, const SwapConst& sc,
-                    const int* fwd_planes, int nfwd, bool zero_force);
+                    const int* fwd_planes, int nfwd, bool zero_force,
+                    const LightStep* light = nullptr);
 // reverse_send_force: F[origin[g]] += F[g] (+ #[reverse] planes) over every
 // root's image tree in fold order
 void launch_reverse_fold(cudaStream_t st, uint64_t nlocal, const uint32_t* start,
@@ -522,8 +535,9 @@ struct ForceCsr {
     const uint32_t* order;
     const double* pk;  // packed (x, y, z, r) records, current; NULL: the columns
 };
+// trip: the launch does nothing when *trip is set (LightStep).
 void launch_force_csr(cudaStream_t st, const ForceCsr& q, const AtomCols& c, const PlaneList& rev,
-                      bool fold);
+                      bool fold, const uint32_t* trip = nullptr);
 // order[b + k] for every block of kBlock roots: the block's roots sorted by
 // their entry count (their own and their images' in-list and row lengths),
 // ties in index order.
@@ -535,33 +549,37 @@ int force_variant();  // from SOIL_FORCE (default chosen by measurement)
 void launch_force_seq(cudaStream_t st, const ForceArgs& p, bool fold, int variant);
 
 // ---- device-resident steps (k_steps.cu) --------------------------------------
-// Grid barrier words (count must be 0 when a launch starts).
-struct GridBar {
-    unsigned count;
-    unsigned gen;
-};
-constexpr uint32_t SOIL_STEPS_ERR_BARRIER = 4u;  // flags->error: a barrier wait ran out
+constexpr uint32_t SOIL_STEPS_ERR_BARRIER = 4u;  // out[2], out[3]: a barrier wait ran out
+constexpr uint32_t SOIL_STEPS_OVERFLOW = 32u;    // out[2]: the lists did not fit; nothing was written
 struct StepsArgs {
     AtomCols c;
     uint64_t nlocal;
     double dt;
-    int zero_force;    // zero the locals' forces in the integration pass
     int first_fused;   // the first step's pass also applies the pending final half-kick
     CheckArgs ck;      // the displacement check (every step)
     FwdArgs fw;        // forward comm of every step
-    ForceArgs fa;      // the grouped consumer (consumer != 0, mode 0 / 1)
-    ForceCsr fc;       // the CSR walk (consumer != 0, mode 2)
-    int walk;          // consumer mode: 0 warp tiles, 1 grouped walk, 2 CSR walk
+    ForceCsr fc;       // the lists
+    PlaneList rev;     // #[reverse] planes folded with the forces (newton)
+    double* rec[2];    // packed (x, y, z, r) records of locals and ghosts, 32-byte aligned
+    uint32_t ent_cap, img_cap;  // entries and images a CTA has shared memory for
     uint64_t max_steps;
-    GridBar* bar;
-    DevFlags* flags;   // flags->rebuild is set when a check trips
-    uint32_t* out;     // out[0]: steps completed; out[1]: 1 if the next step's check tripped
-    uint32_t* trip;    // 3 check-flag slots, zero at launch
+    unsigned long long* bar;  // 3 barrier words; the one of barrier `epoch` is zero at launch
+    uint64_t epoch;           // grid barriers passed by earlier launches
+    uint32_t* out;  // host memory mapped for the device: steps completed; 1 if the next
+                    // step's check tripped; status; status of any CTA's wait
 };
-// Cooperative grid for k_steps (consumer: 0 none, 1 grouped, 2 grouped + fold).
-int steps_grid(int consumer, int walk, bool pk, uint64_t nlocal, int* grid);
-cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, int consumer, int walk, bool pk,
-                         int grid);
+// Launch shape of k_steps: lanes per root, threads per CTA, CTAs (one per SM),
+// and the shared memory for ent_cap entries and img_cap images.
+struct StepsShape {
+    int group, threads, grid;
+    uint32_t ent_cap, img_cap;
+    size_t smem;
+};
+// The shape for a system on `sms` SMs (roomy: with all the shared memory);
+// false when it has too many atoms for one resident launch.
+bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, StepsShape* p);
+// fold: newton.
+cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold);
 
 // ---- light steps without a consumer (k_flight.cu) -----------------------------
 constexpr uint32_t kFlightMaxSteps = 4096;  // one launch stays short when nothing trips

@@ -1114,11 +1114,11 @@ SwapConst swap_const(const soil_sys* s) {
     return sc;
 }
 
-int forward_comm(soil_sys* s, bool zero_ghost_force) {
+int forward_comm(soil_sys* s, bool zero_ghost_force, const LightStep* light = nullptr) {
     int fp[kMaxPlanes], nf;
     zero_planes_of(s, SOIL_COL_FORWARD, fp, &nf);
     launch_forward(s->st, s->nlocal, s->nghost, s->A, s->ghost_root.p, s->ghost_chain.p,
-                   swap_const(s), fp, nf, zero_ghost_force);
+                   swap_const(s), fp, nf, zero_ghost_force, light);
     return check_launch(s);
 }
 
@@ -1290,8 +1290,9 @@ bool consumer_folds(const soil_sys* s) {
 }
 
 // The built-in consumer; with fold (newton), reverse comm of the forces and
-// #[reverse] planes is done in the same kernel.
-int launch_consumer(soil_sys* s, bool fold) {
+// #[reverse] planes is done in the same kernel.  trip (CSR walk only): the
+// kernel does nothing when *trip is set.
+int launch_consumer(soil_sys* s, bool fold, const uint32_t* trip = nullptr) {
     if (!s->in_lists_valid) TRY(build_in_lists(s));
     const int variant = force_variant();
     if (variant != SOIL_FORCE_GATHER) TRY(pk_ready(s));
@@ -1300,7 +1301,7 @@ int launch_consumer(soil_sys* s, bool fold) {
         zero_planes_of(s, SOIL_COL_REVERSE, rev.idx, &rev.n);
         ForceCsr q;
         TRY(csr_with_order(s, &q));
-        launch_force_csr(s->st, q, s->A, rev, fold);
+        launch_force_csr(s->st, q, s->A, rev, fold, trip);
         return check_launch(s);
     }
     if (!seq_consumer(s) || variant == SOIL_FORCE_GATHER) {
@@ -1901,33 +1902,43 @@ int full_step(soil_sys* s, bool last) {
 
 // ---- device-resident steps -------------------------------------------------
 
-// Steps that may run inside one k_steps launch from the current state: the
-// step keeps its lists exactly when its displacement check passes (every = 0
-// with the check on), nothing else a step does needs the host (no hook, no
-// deform, shear or shrink-wrap, no #[zero] planes, #[reverse] planes only
-// with the folding consumer, no phase timers), the built-in consumer (if
-// any) runs on grouped sequences, and no periodic sort falls due.  0: none.
-uint64_t resident_limit(const soil_sys* s, uint64_t want) {
+// Steps from the current state that keep their lists exactly when their
+// displacement check passes (every = 0 with the check on) and need nothing
+// else of the host: no hook, no deform, shear or shrink-wrap, no #[zero]
+// planes, #[reverse] planes only with the folding consumer, and no periodic
+// sort before their end.  0: none.
+uint64_t light_limit(const soil_sys* s, uint64_t want) {
     const char* env = std::getenv("SOIL_RESIDENT_STEPS");
-    const int mode = env ? std::atoi(env) : 2;  // 0 off, 1 always, 2 auto
-    if (mode == 0) return 0;
-    if (mode == 2 && builtin_consumer(s) && s->nlocal > kResidentAutoMaxAtoms) return 0;
-    if (s->hook || s->timing_mask || !s->check || s->every != 0) return 0;
+    if (env && std::atoi(env) == 0) return 0;
+    if (s->hook || !s->check || s->every != 0) return 0;
     if (s->state != COMMUNICATE_ONLY || !displacement_needed(s) || needs_rebuild_with(s, false))
         return 0;
     if (!fused_forward_allowed(s)) return 0;
-    const bool consumer = builtin_consumer(s);
-    if (consumer && force_variant() != SOIL_FORCE_CSR && !seq_consumer(s)) return 0;
     int idx[kMaxPlanes], nz, nr;
     zero_planes_of(s, SOIL_COL_ZERO, idx, &nz);
     zero_planes_of(s, SOIL_COL_REVERSE, idx, &nr);
-    if (nz > 0 || (nr > 0 && !(consumer && s->newton))) return 0;
+    if (nz > 0 || (nr > 0 && !(builtin_consumer(s) && s->newton))) return 0;
     uint64_t lim = want;
     if (s->sort_every > 0) {
         if (s->sort_counter + 1 >= s->sort_every) return 0;
         lim = std::min<uint64_t>(lim, s->sort_every - s->sort_counter - 1);
     }
     return lim;
+}
+
+// Those that may run as one stretch on the device (k_steps, k_flight): no
+// phase timers, and a system with a consumer fits one resident launch and has
+// no radii that change with every fold.
+uint64_t resident_limit(const soil_sys* s, uint64_t want) {
+    if (s->timing_mask) return 0;
+    if (builtin_consumer(s)) {
+        if (s->nlocal > kStepsMaxRoots || s->steps_refused_gen == s->border_gen) return 0;
+        int idx[kMaxPlanes], nr;
+        zero_planes_of(s, SOIL_COL_REVERSE, idx, &nr);
+        for (int k = 0; k < nr; ++k)
+            if (idx[k] == s->cols[s->radius_col].plane0) return 0;
+    }
+    return light_limit(s, want);
 }
 
 // Room for the words of the light-step kernels, zero when first used.
@@ -1983,66 +1994,169 @@ int flight_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, StepP
     return SOIL_OK;
 }
 
+// The two record buffers of the resident steps, for every local and ghost:
+// scratch of the neighbor build where it is large enough (the sorted records;
+// the row slots, 64 bytes per local), so that stepping allocates nothing.
+int steps_records(soil_sys* s, double* rec[2]) {
+    const uint64_t total = s->nlocal + s->nghost;
+    TRY(ensure(s, s->sp, total));
+    rec[0] = reinterpret_cast<double*>(s->sp.p);
+    if (s->row_slots.cap >= 8 * total) {
+        rec[1] = reinterpret_cast<double*>(s->row_slots.p);
+        return SOIL_OK;
+    }
+    TRY(ensure(s, s->rec, total, 0, s->acap));
+    rec[1] = reinterpret_cast<double*>(s->rec.p);
+    return SOIL_OK;
+}
+
 // Up to `max` communicate-only steps in one launch; *done of them complete.
 // *tripped: the next step's integration pass also ran and its displacement
 // check tripped (that step continues on the host from decide_rebuild, with
-// *plan).
-int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, StepPlan* plan) {
-    const StepPlan p = plan_step(s);
-    const bool consumer = builtin_consumer(s);
-    if (consumer && force_variant() != SOIL_FORCE_GATHER) TRY(pk_ready(s));
+// *plan).  *refused: nothing ran, the lists do not fit the launch (or there
+// is no memory for its records); resident_limit says so until they change.
+int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, bool* refused,
+                   StepPlan* plan) {
+    *done = 0;
+    *tripped = *refused = false;
+    *plan = plan_step(s);
+    if (!s->in_lists_valid) TRY(build_in_lists(s));
     StepsArgs a;
     std::memset(&a, 0, sizeof(a));
+    TRY(csr_with_order(s, &a.fc));
+    TRY(light_words(s));
+    if (steps_records(s, a.rec) != SOIL_OK) {
+        s->steps_refused_gen = s->border_gen;
+        *refused = true;
+        return SOIL_OK;
+    }
+    s->pk_valid = false;  // the columns move without the packed records
     a.c = s->A;
     a.nlocal = s->nlocal;
     a.dt = s->dt;
-    a.zero_force = p.fused_zero ? 1 : 0;
     a.first_fused = s->pending_final ? 1 : 0;
     a.ck = make_check(s->lbx.p, s->lby.p, s->lbz.p, s->nlocal, displacement_threshold_sq(s),
                       s->pbc_box, s->dflags, pbc_mask(s));
-    a.fw = fwd_args(s, p.fused_zero);
-    a.walk = 0;
-    int kind = 0;
-    if (consumer) {
-        if (!s->in_lists_valid) TRY(build_in_lists(s));
-        kind = s->newton ? 2 : 1;
-        const int v = force_variant();
-        if (v == SOIL_FORCE_CSR) {
-            TRY(csr_with_order(s, &a.fc));
-            zero_planes_of(s, SOIL_COL_REVERSE, a.fa.rev.idx, &a.fa.rev.n);
-            a.walk = 2;
-        } else {
-            if (!s->seq_valid) TRY(build_seq(s));
-            a.fa = consumer_args(s);
-            a.walk = (v == SOIL_FORCE_TILES4 || v == SOIL_FORCE_TILES2) ? 0 : 1;
+    a.fw = fwd_args(s, false);
+    if (s->newton) zero_planes_of(s, SOIL_COL_REVERSE, a.rev.idx, &a.rev.n);
+    a.max_steps = std::min<uint64_t>(max, 0x7fffffffull);
+    a.bar = reinterpret_cast<unsigned long long*>(s->rstate.p);
+    a.out = s->hword_dev;
+    for (;;) {
+        StepsShape shape;
+        if (!steps_shape(s->nlocal, s->npairs, kStepsSms, s->steps_roomy, &shape))
+            return fail(s->ctx, SOIL_ERR_STATE, "resident steps: too many atoms");
+        a.ent_cap = shape.ent_cap;
+        a.img_cap = shape.img_cap;
+        a.epoch = s->steps_epoch;
+        s->hword[2] = s->hword[3] = 0;
+        CK(launch_steps(s->st, a, shape, s->newton));
+        TRY(sync(s));
+        if (s->hword[2] == SOIL_STEPS_OVERFLOW) {
+            s->steps_epoch += 1;
+            if (s->steps_roomy) {
+                s->steps_refused_gen = s->border_gen;
+                *refused = true;
+                return SOIL_OK;
+            }
+            s->steps_roomy = true;  // from now on, for this system
+            continue;
         }
+        break;
     }
-    a.max_steps = max;
-    TRY(light_words(s));
-    a.bar = reinterpret_cast<GridBar*>(s->rstate.p);
-    a.out = s->rstate.p + 2;
-    a.trip = s->rstate.p + 4;
-    a.flags = s->dflags;
-    int grid = 0;
-    const bool pk = a.walk == 2 ? a.fc.pk != nullptr : a.fa.q.pk != nullptr;
-    if (steps_grid(kind, a.walk, pk, s->nlocal, &grid))
-        return fail(s->ctx, SOIL_ERR_CUDA, "no cooperative occupancy for the resident steps");
-    CK(cudaMemsetAsync(s->rstate.p, 0, 8 * 4, s->st));
-    CK(cudaMemsetAsync(&s->dflags->rebuild, 0, 4, s->st));
-    CK(cudaMemsetAsync(&s->dflags->error, 0, 4, s->st));
-    CK(launch_steps(s->st, a, kind, a.walk, pk, grid));
-    CK(cudaMemcpyAsync(s->hword, a.out, 8, cudaMemcpyDeviceToHost, s->st));
-    TRY(read_flags(s));
-    if (s->hflags->error & SOIL_STEPS_ERR_BARRIER)
+    if (s->hword[2] || s->hword[3]) {
+        CK(cudaMemsetAsync(s->rstate.p, 0, s->rstate.cap * 4, s->st));
+        s->steps_epoch = 0;
         return fail(s->ctx, SOIL_ERR_CUDA, "resident steps: a grid barrier wait ran out");
+    }
     *done = s->hword[0];
     *tripped = s->hword[1] != 0;
-    if (*done > max || (!*tripped && *done != max))
+    if (*done > a.max_steps || (!*tripped && *done != a.max_steps))
         return fail(s->ctx, SOIL_ERR_CUDA, "resident steps: inconsistent step count");
+    s->steps_epoch += *done + (*tripped ? 1 : 0);
     light_steps_done(s, *done, *tripped);
-    *plan = p;
     plan->check = true;
     plan->fwd_fused = true;
+    plan->tripped = true;
+    return SOIL_OK;
+}
+
+// The host's copy of a light step's answer, once the device has written it.
+int light_answer(soil_sys* s, uint32_t tag, bool* tripped) {
+    const volatile uint32_t* w = s->hword + kHostAnswer;
+    for (uint64_t k = 0;; ++k) {
+        uint32_t v = *w;
+        if ((v & ~1u) != tag && k % 4096 == 4095) {
+            const cudaError_t e = cudaStreamQuery(s->st);
+            if (e != cudaErrorNotReady) {  // nothing is left to write it: look once more
+                CK(e);
+                v = *w;
+                if ((v & ~1u) != tag)
+                    return fail(s->ctx, SOIL_ERR_CUDA, "light step: no answer to its check");
+            }
+        }
+        if ((v & ~1u) == tag) {
+            *tripped = (v & 1u) != 0;
+            return SOIL_OK;
+        }
+    }
+}
+
+// One light step (light_limit >= 1) of a system with the CSR consumer, phase
+// by phase: forward comm and the consumer go in behind the integration pass
+// and do nothing if its check tripped; the host reads the answer while they
+// run, so the stream never waits for it.
+int light_step(soil_sys* s, bool last) {
+    StepPlan p = plan_step(s);
+    TRY(light_words(s));
+    if (!s->in_lists_valid) TRY(build_in_lists(s));
+    TRY(pk_ready(s));  // before the pass moves the atoms
+    LightStep w;
+    w.trip = s->rstate.p + 10 + s->light_gen % 2;
+    w.next = s->rstate.p + 10 + (s->light_gen + 1) % 2;
+    w.answer = s->hword_dev + kHostAnswer;
+    s->light_gen += 1;
+    w.tag = 2u * s->light_gen;
+    s->hword[kHostAnswer] = w.tag - 2u;
+    timer_begin(s, T_INTEGRATE);
+    if (s->pending_final)
+        launch_final_initial(s->st, s->nlocal, s->A, s->dt, p.fused_zero, s->lbx.p, s->lby.p,
+                             s->lbz.p, s->nlocal, displacement_threshold_sq(s), s->pbc_box,
+                             s->dflags, pbc_mask(s), nullptr, &w);
+    else
+        launch_initial(s->st, s->nlocal, s->A, s->dt, p.fused_zero, s->lbx.p, s->lby.p, s->lbz.p,
+                       s->nlocal, displacement_threshold_sq(s), s->pbc_box, s->dflags, pbc_mask(s),
+                       nullptr, &w);
+    s->pending_final = false;
+    TRY(check_launch(s));
+    timer_end(s, T_INTEGRATE);
+    const size_t spans = s->spans.size();
+    timer_begin(s, T_FORWARD);
+    TRY(forward_comm(s, p.fused_zero, &w));
+    timer_end(s, T_FORWARD);
+    timer_begin(s, T_FORCE);
+    TRY(launch_consumer(s, s->newton, w.trip));
+    timer_end(s, T_FORCE);
+    bool tripped = false;
+    TRY(light_answer(s, w.tag, &tripped));
+    if (tripped) {
+        while (s->spans.size() > spans) {  // the empty launches are no phase
+            s->ev_pool.push_back(s->spans.back().a);
+            s->ev_pool.push_back(s->spans.back().b);
+            s->spans.pop_back();
+        }
+        p.tripped = true;
+        return step_rest(s, p, last);
+    }
+    if (s->newton) s->reverse_gen = s->border_gen;
+    light_steps_done(s, 1, false);
+    if (last) {
+        timer_begin(s, T_FINAL);
+        launch_final(s->st, s->nlocal, s->A, s->dt);
+        s->pending_final = false;
+        TRY(check_launch(s));
+        timer_end(s, T_FINAL);
+    }
     return SOIL_OK;
 }
 
@@ -2055,10 +2169,11 @@ int step_many(soil_sys* s, uint64_t n) {
         const uint64_t lim = resident_limit(s, n - k);
         if (lim >= 2) {
             uint64_t done = 0;
-            bool tripped = false;
+            bool tripped = false, refused = false;
             StepPlan p;
-            TRY(builtin_consumer(s) ? resident_steps(s, lim, &done, &tripped, &p)
+            TRY(builtin_consumer(s) ? resident_steps(s, lim, &done, &tripped, &refused, &p)
                                     : flight_steps(s, lim, &done, &tripped, &p));
+            if (refused) continue;  // resident_limit is 0 now
             k += done;
             if (tripped) {  // step k + 1: integrated, its check tripped
                 TRY(step_rest(s, p, k + 1 == n));
@@ -2070,7 +2185,10 @@ int step_many(soil_sys* s, uint64_t n) {
             }
             continue;
         }
-        TRY(full_step(s, k + 1 == n));
+        if (builtin_consumer(s) && force_variant() == SOIL_FORCE_CSR && light_limit(s, 1) >= 1)
+            TRY(light_step(s, k + 1 == n));
+        else
+            TRY(full_step(s, k + 1 == n));
         k += 1;
     }
     return SOIL_OK;
@@ -2201,7 +2319,7 @@ int soil_sys_create(soil_ctx* ctx, const soil_box* box, const soil_neigh_cfg* cf
     int r;
     if ((r = dev_alloc(s, (void**)&s->dflags, sizeof(DevFlags))) != SOIL_OK ||
         cudaHostAlloc((void**)&s->hflags, sizeof(DevFlags), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostAlloc((void**)&s->hword, 2 * kBorderStateWords * 4, cudaHostAllocMapped) !=
+        cudaHostAlloc((void**)&s->hword, kHostWords * 4, cudaHostAllocMapped) !=
             cudaSuccess ||
         cudaHostGetDevicePointer((void**)&s->hflags_dev, s->hflags, 0) != cudaSuccess ||
         cudaHostGetDevicePointer((void**)&s->hword_dev, s->hword, 0) != cudaSuccess) {
@@ -2235,7 +2353,7 @@ int soil_sys_destroy(soil_sys* s) {
     for (int k = 0; k < 2; ++k) { fr(s->slot_tag[k]); fr(s->slot_val[k]); }
     fr(s->in_count); fr(s->in_start); fr(s->in_cursor); fr(s->in_list); fr(s->in_split);
     fr(s->seq_cnt); fr(s->grp_cnt); fr(s->grp_start); fr(s->seq); fr(s->seq_owner);
-    fr(s->rstate); fr(s->scan1p); fr(s->root_order); fr(s->pk);
+    fr(s->rstate); fr(s->rec); fr(s->scan1p); fr(s->root_order); fr(s->pk);
     fr(s->ghost_root); fr(s->ghost_chain);
     fr(s->fold_start); fr(s->fold_list);
     for (auto& a : s->send) fr(a);

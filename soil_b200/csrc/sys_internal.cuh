@@ -165,10 +165,16 @@ struct soil_sys {
     DArr<uint8_t> seq_owner;
     bool seq_valid = false;
     bool few_images = false;  // no local has images on both sides of a dim (<= 7 images)
-    // light steps: grid barrier words, step count and trip flag of the resident
-    // launch (0-7), the end-step words of the flights (8, 9, used in turn)
+    // light steps: the resident launch's three barrier words (u32 0-5), the
+    // end-step words of the flights (8, 9, used in turn) and the trip words of
+    // the light steps launched phase by phase (10, 11, used in turn)
     DArr<uint32_t> rstate;
     uint64_t flights = 0;
+    uint32_t light_gen = 0;  // light steps launched phase by phase so far
+    uint64_t steps_epoch = 0;    // grid barriers of the resident launches so far
+    bool steps_roomy = false;    // a resident launch needed all the shared memory
+    uint64_t steps_refused_gen = ~0ull;  // border pass whose lists did not fit one
+    DArr<double4> rec;  // their second record buffer, where the row slots are too small
     DArr<uint32_t> scan1p;    // single-pass scan: tile counter and descriptors (zeroed at growth)
     DArr<uint32_t> root_order;  // CSR-walk consumer: roots by work per block (rebuilt with the lists)
     bool order_valid = false;
@@ -300,10 +306,15 @@ bool builtin_consumer(const soil_sys* s);
 bool needs_rebuild_with(const soil_sys* s, bool disp);
 bool displacement_needed(const soil_sys* s);
 SwapConst swap_const(const soil_sys* s);
+// Words of a system's mapped host buffer: two border states, then the answer of
+// a light step's displacement check.
+constexpr int kHostAnswer = 2 * kBorderStateWords;
+constexpr int kHostWords = kHostAnswer + 8;
 constexpr int kRowSlotsPerAtom = 16;
-// Largest system that takes the device-resident light steps by default
-// (SOIL_RESIDENT_STEPS=1 forces them on at any size, 0 off).
-constexpr uint64_t kResidentAutoMaxAtoms = 1ull << 20;
+// Systems with a consumer take the resident light steps (SOIL_RESIDENT_STEPS=0:
+// never) up to one root per thread of one CTA of 1,024 per SM.
+constexpr uint64_t kStepsSms = 148;
+constexpr uint64_t kStepsMaxRoots = kStepsSms * 1024;
 // largest count the single-pass scan serves (scan_1p)
 constexpr uint64_t kScan1pMaxCounts = 64ull * 2048ull;
 

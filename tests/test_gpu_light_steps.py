@@ -72,3 +72,47 @@ def test_free_flight_takes_up_the_forces_of_a_removed_consumer(ctx):
     assert a.counts().comm_state == abi.SOIL_COMMUNICATE_ONLY
     a.close()
     b.close()
+
+
+# Atom counts on both sides of every launch shape: the lanes per root (8 up to
+# 18,944 atoms, 4 to 37,888, 2 to 75,776, 1 to 151,552), full and ragged CTAs,
+# and the first size past one launch.
+@pytest.mark.parametrize("n", [40, 333, 4737, 18944, 18945, 37889, 75777, 151552, 151553])
+@pytest.mark.parametrize("newton", [1, 0])
+def test_resident_steps_match_oracle(ctx, n, newton):
+    w = W.poly("resident", 160 + n % 5, n, 0.45, 1e-4, 0, harmonic_k=1e3, newton=newton)
+    w.vel *= 6.0
+    calls = [1, 2, 17, 1, 9] if n < 30000 else [1, 11]
+    g = _stepped(ctx, w, "2", calls)
+    o = oracle.from_workload(w)
+    o.step(sum(calls))
+    assert_same_state(g, o, f"n={n}")
+    assert_same_lists(g, o)
+    g.close()
+
+
+@pytest.mark.parametrize("phi,n", [(0.45, 30), (0.45, 120), (2.5, 700), (6.0, 300)])
+def test_resident_steps_many_images_and_entries(ctx, phi, n):
+    """Boxes so small that a root has images on both sides of an axis (up to
+    26), and packings so dense that rows hold dozens of entries."""
+    w = W.poly("resident-dense", 171, n, phi, 1e-5, 0, harmonic_k=1e2)
+    g = _stepped(ctx, w, "2", [1, 25])
+    o = oracle.from_workload(w)
+    o.step(26)
+    assert_same_state(g, o, f"phi={phi} n={n}")
+    assert_same_lists(g, o)
+    g.close()
+
+
+def test_resident_steps_crowded_corner(ctx):
+    """One CTA's roots hold far more entries than the mean: the launch says so
+    with nothing written, and the run goes on (more shared memory, then one
+    launch per phase) with the same results."""
+    w = W.poly("resident-crowd", 172, 9000, 0.30, 1e-6, 0, harmonic_k=1e1)
+    w.pos[:1500] = 1.0 + w.pos[:1500] / w.L * 2.0
+    g = _stepped(ctx, w, "2", [1, 6, 5])
+    o = oracle.from_workload(w)
+    o.step(12)
+    assert_same_state(g, o)
+    assert_same_lists(g, o)
+    g.close()
