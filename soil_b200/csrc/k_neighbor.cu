@@ -26,30 +26,16 @@
 
 namespace soil {
 
-// Pass 1: one thread per local row (rows of a warp are neighbours in space, so
-// their candidate records are shared through L1); the first K entries go to
-// the row's slots, the length to rowcount.
-template <bool UNIFORM, bool FP32>
-__global__ void __launch_bounds__(kBlock) k_pairs_rows(PairParams p, uint32_t* rowcount,
-                                                       uint32_t* slots, DevFlags* flags) {
-    pdl_wait();  // launched with pdl_launch
-    const Filter<UNIFORM, FP32> test(p);
-    const uint32_t K = (uint32_t)p.row_slots;
-    uint32_t n_rechk = 0, n_cand32 = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < p.nlocal;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        rowcount[i] = row_scan<UNIFORM, FP32, true>(p, test, i, slots + i * K, K, &n_rechk,
-                                                    &n_cand32, flags, p.in_count);
-    // the block's totals, then one atomic per counter and block (the FP64
-    // filter rechecks nothing)
+// The block's filter statistics, then one atomic per counter and block (the
+// FP64 filter rechecks nothing).
+template <bool FP32>
+__device__ __forceinline__ void add_block_stats(DevFlags* flags, uint64_t n_cand, uint64_t r) {
     __shared__ unsigned long long s_cand, s_rechk;
     if (threadIdx.x == 0) {
         s_cand = 0;
         s_rechk = 0;
     }
     __syncthreads();
-    uint64_t n_cand = n_cand32;
-    uint64_t r = n_rechk;
     for (int o = 16; o > 0; o >>= 1) {
         n_cand += __shfl_down_sync(0xffffffffu, n_cand, o);
         r += __shfl_down_sync(0xffffffffu, r, o);
@@ -63,6 +49,43 @@ __global__ void __launch_bounds__(kBlock) k_pairs_rows(PairParams p, uint32_t* r
         atomicAdd((unsigned long long*)&flags->candidates, s_cand);
         if (FP32) atomicAdd((unsigned long long*)&flags->rechecked, s_rechk);
     }
+}
+
+// Pass 1: one thread per local row (rows of a warp are neighbours in space, so
+// their candidate records are shared through L1); the first K entries go to
+// the row's slots, the length to rowcount.
+template <bool UNIFORM, bool FP32, int U, int NR>
+__global__ void __launch_bounds__(kBlock) k_pairs_rows(PairParams p, uint32_t* rowcount,
+                                                       uint32_t* slots, DevFlags* flags) {
+    pdl_wait();  // launched with pdl_launch
+    const Filter<UNIFORM, FP32> test(p);
+    const uint32_t K = (uint32_t)p.row_slots;
+    uint32_t n_rechk = 0, n_cand32 = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < p.nlocal;
+         i += (uint64_t)gridDim.x * blockDim.x)
+        rowcount[i] = row_scan<UNIFORM, FP32, true, U, NR>(p, test, i, slots + i * K, K, &n_rechk,
+                                                           &n_cand32, flags, p.in_count);
+    add_block_stats<FP32>(flags, n_cand32, n_rechk);
+}
+
+// Pass 1 of a system with too few rows to fill the chip with one thread each:
+// G lanes per row.  What bounds it is the chain of a row's candidates through
+// L2, G times shorter here.
+template <int G, bool UNIFORM, bool FP32, int NR>
+__global__ void __launch_bounds__(kBlock) k_pairs_group(PairParams p, uint32_t* rowcount,
+                                                        uint32_t* slots, DevFlags* flags) {
+    pdl_wait();  // launched with pdl_launch
+    const Filter<UNIFORM, FP32> test(p);
+    const uint32_t K = (uint32_t)p.row_slots;
+    const uint32_t g = threadIdx.x & (G - 1);
+    uint32_t n_rechk = 0, n_cand32 = 0;
+    const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / G;
+    const bool valid = i < p.nlocal;
+    const uint32_t cnt = row_scan_group<G, UNIFORM, FP32, NR>(p, test, i, valid, g, slots + i * K,
+                                                              K, &n_rechk, &n_cand32, flags,
+                                                              p.in_count);
+    if (valid && g == 0) rowcount[i] = cnt;
+    add_block_stats<FP32>(flags, n_cand32, n_rechk);
 }
 
 // Pass 2: rows into their CSR place; rows longer than K are re-derived.
@@ -121,14 +144,40 @@ __global__ void __launch_bounds__(kBlock) k_pairs_fill(PairParams p, const uint3
     }
 }
 
+// Pass 1's form.  8 lanes per row up to 12,288 rows, 4 up to 36,864 (measured
+// with 1 / 4 / 8 lanes: 12.2 / 7.1 / 5.8 us on 8,009 rows, 13.4 / 8.3 / 11.5 on
+// 24,001, 13.9 / 14.5 / 16.7 on 50,021).  Above, one thread per row: two
+// candidates at a time where the cells hold enough atoms (row_scan_pre gives
+// both sides), else one.
+constexpr uint64_t kRows8Lanes = 12288, kRows4Lanes = 36864;
+constexpr double kTwoAtATime = 1.25;  // mean atoms per cell
+
+template <bool UNIFORM, bool FP32, int NR>
+static void launch_rows_t(cudaStream_t st, const PairParams& p, uint32_t* rowcount,
+                          uint32_t* slots, DevFlags* flags) {
+    const bool pre = p.pre_ranges && p.nstencil < NR;
+    const int g = !pre ? 1 : p.nlocal <= kRows8Lanes ? 8 : p.nlocal <= kRows4Lanes ? 4 : 1;
+    const unsigned blocks = (unsigned)((p.nlocal * (uint64_t)g + kBlock - 1) / kBlock);
+    auto launch = [&](auto k, unsigned grid) {
+        pdl_launch(k, grid, kBlock, 0, st, p, rowcount, slots, flags);
+    };
+    if (g == 8) launch(k_pairs_group<8, UNIFORM, FP32, NR>, blocks);
+    else if (g == 4) launch(k_pairs_group<4, UNIFORM, FP32, NR>, blocks);
+    else if (p.cell_atoms >= kTwoAtATime)
+        launch(k_pairs_rows<UNIFORM, FP32, 2, NR>, grid_wave<k_pairs_rows<UNIFORM, FP32, 2, NR>>(p.nlocal));
+    else
+        launch(k_pairs_rows<UNIFORM, FP32, 1, NR>, grid_wave<k_pairs_rows<UNIFORM, FP32, 1, NR>>(p.nlocal));
+}
+
 template <bool UNIFORM, bool FP32>
 static void launch_pairs_t(cudaStream_t st, const PairParams& p, uint32_t* rowcount,
                            uint32_t* slots, const uint32_t* offsets, uint32_t* indices,
                            DevFlags* flags, const FillGuard* g) {
     note_launch();
-    if (!g)
-        pdl_launch(k_pairs_rows<UNIFORM, FP32>, grid_wave<k_pairs_rows<UNIFORM, FP32>>(p.nlocal), kBlock, 0, st, p, rowcount, slots,
-                                                                            flags);
+    if (!g && p.nstencil < kPreRanges)
+        launch_rows_t<UNIFORM, FP32, kPreRanges>(st, p, rowcount, slots, flags);
+    else if (!g)
+        launch_rows_t<UNIFORM, FP32, kPreRangesFull>(st, p, rowcount, slots, flags);
     else
         pdl_launch(k_pairs_fill<UNIFORM, FP32>, grid_wave<k_pairs_fill<UNIFORM, FP32>>(p.nlocal), kBlock, 0, st, p, rowcount, slots,
                                                                             offsets, indices, *g);

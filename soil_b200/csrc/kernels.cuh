@@ -396,6 +396,7 @@ struct PairParams {
     uint32_t* in_count;
     const uint32_t* in_start;
     uint32_t* in_list;
+    double cell_atoms = 0.0;  // mean locals per interior cell (one system's pass 1)
     int pre_ranges;  // row_scan_pre for stencils of few runs (SOIL_PAIRS_PRE, default on)
 };
 // Pass 1: row lengths into rowcount[], the first K entries of each row into

@@ -1495,6 +1495,8 @@ int phase_neighbor(soil_sys* s) {
     p.in_start = nullptr;
     p.in_list = nullptr;
     p.pre_ranges = pairs_pre_ranges();
+    p.cell_atoms = (double)nl;  // times a cell's share of the box (bin_size in lamda when triclinic)
+    for (int d = 0; d < 3; ++d) p.cell_atoms *= s->triclinic ? s->bin_size[d] : s->bin_size[d] / s->size[d];
     uint64_t in_zero = 0;  // in_count[0, in_zero) is zero already
     const uint64_t in_range = total;  // the counts pass 1 may write and the scan reads
     if (with_in) {
