@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(kBlock) k_cells(uint64_t first, uint64_t n, At
 __global__ void __launch_bounds__(kBlock) k_pbc_cells(uint64_t n, AtomCols c, Geom g, double bv0,
                                                       double bv1, double bv2, Grid gr,
                                                       uint32_t* cell_out, uint32_t* counts) {
+    pdl_wait();  // launched with pdl_launch
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
         const uint64_t i = i0 + threadIdx.x;
@@ -133,8 +134,8 @@ void launch_pbc_cells(cudaStream_t st, uint64_t n, const AtomCols& c, const Geom
                       const double bvel[3], const Grid& gr, uint32_t* cell_out, uint32_t* counts) {
     if (n == 0) return;
     note_launch();
-    k_pbc_cells<<<grid_wave<k_pbc_cells>(n), kBlock, 0, st>>>(n, c, g, bvel[0], bvel[1], bvel[2],
-                                                              gr, cell_out, counts);
+    pdl_launch(k_pbc_cells, grid_wave<k_pbc_cells>(n), kBlock, 0, st, n, c, g, bvel[0], bvel[1],
+               bvel[2], gr, cell_out, counts);
 }
 
 void launch_cells(cudaStream_t st, uint64_t first, uint64_t n, const AtomCols& c, const Grid& gr,

@@ -124,6 +124,7 @@ void launch_final_initial(cudaStream_t st, uint64_t n, const AtomCols& c, double
 
 // final_integration, soil_verlet/src/lib.rs:175-194: v += h*F
 __global__ void __launch_bounds__(kBlock) k_final(uint64_t n, AtomCols c, double dt) {
+    pdl_wait();  // launched with pdl_launch
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x)
         final_atom(c, i, dt);
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kBlock) k_final(uint64_t n, AtomCols c, double
 void launch_final(cudaStream_t st, uint64_t n, const AtomCols& c, double dt) {
     if (n == 0) return;
     note_launch();
-    k_final<<<grid_wave<k_final>(n), kBlock, 0, st>>>(n, c, dt);
+    pdl_launch(k_final, grid_wave<k_final>(n), kBlock, 0, st, n, c, dt);
 }
 
 __global__ void __launch_bounds__(kBlock) k_zero(uint64_t n, AtomCols c, PlaneList zp) {

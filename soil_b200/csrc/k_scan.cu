@@ -1,10 +1,10 @@
 // k_scan.cu — device-wide exclusive scan of u32 counts (bin counts, row
-// counts, ghost tile counts).  Three passes over tiles of 2048 items:
-// tile sums -> one-CTA scan of the sums -> tile scans with the carry-in.
-// 256 threads x 8 consecutive items per thread; warp shuffles inside a warp,
-// shared memory across the 8 warps.
-#include <atomic>
-#include <cuda/atomic>
+// counts, ghost tile counts), 8 consecutive items per thread, warp shuffles
+// inside a warp, shared memory across warps.  By size:
+//   up to kScanDirectMax counts  one launch (k_scan_direct);
+//   up to kScanCarryTiles tiles of 2,048  two: tile sums, then tile scans that
+//                                add up the sums before them;
+//   above                        three, the sums scanned by one CTA between.
 
 #include "block_scan.cuh"
 #include "kernels.cuh"
@@ -162,23 +162,92 @@ __global__ void __launch_bounds__(kBlock) k_scan_down_carry(ScanJobs J) {
     if (t + 1 == q.ntiles && threadIdx.x == 0) q.out[n] = carry + tot;
 }
 
+// One launch without any wait between CTAs: a CTA of 1,024 threads takes a
+// tile of 8,192 counts and adds up every count before it itself, by 16-byte
+// loads that are all in flight at once.  The last of 16 tiles reads 480 KB
+// from L2 that way, which takes less time than a look-back chain (an atomic
+// ticket, the publication of the tile's sum and the wait for the
+// predecessor's, each a trip through L2): 3.0 against 4.1 us on 13,000 counts,
+// 4.5 against 4.9 on 70,000, and one launch for two scans.
+constexpr int kDirectThreads = 1024;
+constexpr uint64_t kDirectTile = (uint64_t)kDirectThreads * kScanItems;
+
+__device__ __forceinline__ uint32_t cta_exclusive_1024(uint32_t v, uint32_t* total) {
+    __shared__ uint32_t w[32];
+    static_assert(kDirectThreads == 32 * 32, "one warp scans the warps' sums");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) w[warp] = inc;
+    __syncthreads();
+    uint32_t x = w[lane], xi = x;  // every warp scans the sums: one barrier fewer
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, xi, o);
+        if (lane >= o) xi += t;
+    }
+    *total = __shfl_sync(0xffffffffu, xi, 31);
+    return __shfl_sync(0xffffffffu, xi - x, warp) + inc - v;
+}
+
+__global__ void __launch_bounds__(kDirectThreads) k_scan_direct(ScanJobs J) {
+    pdl_wait();  // launched with pdl_launch
+    __shared__ uint32_t before[32];
+    const ScanJob q = scan_job(J);
+    const uint64_t base = q.tile * kDirectTile + (uint64_t)threadIdx.x * kScanItems;
+    uint32_t v[kScanItems];
+    load8(q.in, base, q.n, v);
+    uint32_t c = 0;  // this thread's share of the counts before the tile
+    const uint64_t first = q.tile * kDirectTile;
+    if ((reinterpret_cast<uintptr_t>(q.in) & 15u) == 0) {
+        const uint4* in4 = reinterpret_cast<const uint4*>(q.in);
+#pragma unroll 8
+        for (uint64_t k = threadIdx.x; k < first / 4; k += kDirectThreads) {
+            const uint4 a = in4[k];
+            c += a.x + a.y + a.z + a.w;
+        }
+    } else {
+        for (uint64_t k = threadIdx.x; k < first; k += kDirectThreads) c += q.in[k];
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) before[threadIdx.x >> 5] = c;
+    uint32_t s = 0, tot;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) s += v[k];
+    const uint32_t in_tile = cta_exclusive_1024(s, &tot);  // its barrier covers `before`
+    const uint32_t carry = __reduce_add_sync(0xffffffffu, before[threadIdx.x & 31]);
+    store8_scan(q.out, base, q.n, v, carry + in_tile);
+    if (q.tile + 1 == q.ntiles && threadIdx.x == 0) q.out[q.n] = carry + tot;
+}
+
 uint64_t scan_temp_words(uint64_t n) { return (n + kScanTile - 1) / kScanTile + 2; }
 
-static ScanJobs one_job(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* temp) {
+static ScanJobs one_job(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* temp,
+                        uint64_t tile = kScanTile) {
     ScanJobs J{};
     J.in[0] = in;
     J.out[0] = out;
     J.n[0] = n;
     J.partial[0] = temp;
-    J.ntiles[0] = (n + kScanTile - 1) / kScanTile;
+    J.ntiles[0] = (n + tile - 1) / tile;
     return J;
 }
 
 void exclusive_scan_u32(cudaStream_t st, const uint32_t* in, uint32_t* out, uint64_t n,
-                        uint32_t* temp) {
+                        uint32_t* temp, uint64_t direct_max) {
     const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
     if (ntiles == 0) {
         cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
+        return;
+    }
+    if (n <= direct_max) {
+        const ScanJobs J = one_job(in, out, n, nullptr, kDirectTile);
+        note_launch();
+        pdl_launch(k_scan_direct, (unsigned)J.ntiles[0], kDirectThreads, 0, st, J);
         return;
     }
     const ScanJobs J = one_job(in, out, n, temp);
@@ -196,11 +265,23 @@ void exclusive_scan_u32(cudaStream_t st, const uint32_t* in, uint32_t* out, uint
 }
 
 void exclusive_scan_u32_pair(cudaStream_t st, const uint32_t* in0, uint32_t* out0, uint64_t n0,
-                             const uint32_t* in1, uint32_t* out1, uint64_t n1, uint32_t* temp) {
+                             const uint32_t* in1, uint32_t* out1, uint64_t n1, uint32_t* temp,
+                             uint64_t direct_max) {
+    if (n0 && n1 && n0 <= direct_max && n1 <= direct_max) {
+        ScanJobs J = one_job(in0, out0, n0, nullptr, kDirectTile);
+        J.in[1] = in1;
+        J.out[1] = out1;
+        J.n[1] = n1;
+        J.ntiles[1] = (n1 + kDirectTile - 1) / kDirectTile;
+        note_launch();
+        pdl_launch(k_scan_direct, (unsigned)(J.ntiles[0] + J.ntiles[1]), kDirectThreads, 0, st, J);
+        return;
+    }
     const uint64_t t0 = (n0 + kScanTile - 1) / kScanTile, t1 = (n1 + kScanTile - 1) / kScanTile;
-    if (t0 == 0 || t1 == 0 || t0 > kScanCarryTiles || t1 > kScanCarryTiles) {
-        exclusive_scan_u32(st, in0, out0, n0, temp);
-        exclusive_scan_u32(st, in1, out1, n1, temp + scan_temp_words(n0));
+    if (t0 == 0 || t1 == 0 || t0 > kScanCarryTiles || t1 > kScanCarryTiles || n0 <= direct_max ||
+        n1 <= direct_max) {
+        exclusive_scan_u32(st, in0, out0, n0, temp, direct_max);
+        exclusive_scan_u32(st, in1, out1, n1, temp + scan_temp_words(n0), direct_max);
         return;
     }
     ScanJobs J = one_job(in0, out0, n0, temp);
@@ -213,119 +294,6 @@ void exclusive_scan_u32_pair(cudaStream_t st, const uint32_t* in0, uint32_t* out
     pdl_launch(k_scan_reduce, (unsigned)(t0 + t1), kBlock, 0, st, J);
     note_launch();
     pdl_launch(k_scan_down_carry, (unsigned)(t0 + t1), kBlock, 0, st, J);
-}
-
-// ---- single-pass scan (decoupled look-back) ---------------------------------
-//
-// One launch of ntiles CTAs.  Each CTA claims the next tile from an atomic
-// counter (so every tile with a smaller number is held by a CTA that already
-// runs), publishes its tile's sum, looks back over its predecessors'
-// descriptors until it meets an inclusive prefix, publishes its own inclusive
-// prefix and writes its tile.  A descriptor is 64 bits: the call's epoch (30
-// bits), a status (1: tile sum, 2: inclusive prefix) and the value; the epoch
-// makes descriptors of earlier calls read as not yet published, so nothing is
-// cleared between calls.  The CTA that claims the last tile puts the counter
-// back to zero.  Waits are bounded; one that runs out sets SOIL_SCAN_ERR in
-// *err (when given) and counts the missing tiles as zero.
-
-constexpr uint64_t kLookbackSpinLimit = 1ull << 22;
-constexpr uint64_t kDescAgg = 1, kDescInc = 2;
-
-__device__ __forceinline__ uint64_t desc_pack(uint32_t epoch, uint64_t status, uint32_t v) {
-    return ((uint64_t)(epoch & 0x3fffffffu) << 34) | (status << 32) | v;
-}
-
-__global__ void __launch_bounds__(kBlock) k_scan_1p(const uint32_t* in, uint32_t* out, uint64_t n,
-                                                    uint32_t* counter, uint64_t* desc,
-                                                    uint32_t epoch, uint32_t* err) {
-    __shared__ uint32_t s_tile, s_prefix, tot;
-    if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    if (threadIdx.x == 0 && tile == ntiles - 1) atomicExch(counter, 0u);  // the last claim
-    const uint64_t base = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    load8(in, base, n, v);
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) s += v[k];
-    uint32_t pre = block_exclusive_scan(s, &tot);
-    const uint32_t agg = tot;
-    const uint32_t ep = epoch & 0x3fffffffu;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        uint32_t prefix = 0;
-        if (tile == 0) {
-            if (lane == 0)
-                cuda::atomic_ref<uint64_t, cuda::thread_scope_device>(desc[0]).store(
-                    desc_pack(ep, kDescInc, agg), cuda::memory_order_release);
-        } else {
-            if (lane == 0)
-                cuda::atomic_ref<uint64_t, cuda::thread_scope_device>(desc[tile]).store(
-                    desc_pack(ep, kDescAgg, agg), cuda::memory_order_release);
-            int64_t look = (int64_t)tile - 1;
-            for (;;) {
-                const int64_t idx = look - lane;  // lane 0: the nearest predecessor
-                uint64_t st = kDescInc;  // lanes past tile 0 take no part
-                uint32_t val = 0;
-                if (idx >= 0) {
-                    cuda::atomic_ref<uint64_t, cuda::thread_scope_device> d(desc[idx]);
-                    st = 0;
-                    for (uint64_t spin = 0; spin < kLookbackSpinLimit; ++spin) {
-                        const uint64_t x = d.load(cuda::memory_order_acquire);
-                        if ((uint32_t)(x >> 34) == ep && ((x >> 32) & 3u)) {
-                            st = (x >> 32) & 3u;
-                            val = (uint32_t)x;
-                            break;
-                        }
-                    }
-                    if (st == 0) {
-                        if (err) atomicOr(err, SOIL_SCAN_ERR);
-                        st = kDescAgg;  // counted as zero
-                    }
-                }
-                const unsigned inc = __ballot_sync(0xffffffffu, idx >= 0 && st == kDescInc);
-                const int stop = inc ? __ffs(inc) - 1 : 31;
-                uint32_t part = (lane <= stop && idx >= 0) ? val : 0u;
-                for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-                prefix += part;
-                if (inc || look - 32 < 0) break;
-                look -= 32;
-            }
-            if (lane == 0)
-                cuda::atomic_ref<uint64_t, cuda::thread_scope_device>(desc[tile]).store(
-                    desc_pack(ep, kDescInc, prefix + agg), cuda::memory_order_release);
-        }
-        if (lane == 0) s_prefix = prefix;
-    }
-    __syncthreads();
-    pre += s_prefix;
-    store8_scan(out, base, n, v, pre);
-    if (tile == ntiles - 1 && threadIdx.x == kBlock - 1) {
-        uint32_t last = pre;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) last += v[k];
-        out[n] = last;
-    }
-}
-
-uint64_t scan1p_words(uint64_t n) { return 2 * ((n + kScanTile - 1) / kScanTile) + 4; }
-
-static std::atomic<uint32_t> g_scan_epoch{1};
-
-void exclusive_scan_1p(cudaStream_t st, const uint32_t* in, uint32_t* out, uint64_t n,
-                       uint32_t* temp, uint32_t* err) {
-    const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    if (ntiles == 0) {
-        cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
-        return;
-    }
-    const uint32_t epoch = g_scan_epoch.fetch_add(1, std::memory_order_relaxed);
-    note_launch();
-    k_scan_1p<<<(unsigned)ntiles, kBlock, 0, st>>>(in, out, n, temp,
-                                                  reinterpret_cast<uint64_t*>(temp + 2), epoch,
-                                                  err);
 }
 
 }  // namespace soil

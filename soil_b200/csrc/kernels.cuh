@@ -185,23 +185,20 @@ void launch_interleave_w(cudaStream_t st, uint64_t n, int w, double* dst, const 
 
 // ---- scan (k_scan.cu) -----------------------------------------------------
 // Exclusive scan: out[0..n] with out[n] = total.  `temp` holds
-// scan_temp_words(n) u32.
+// scan_temp_words(n) u32.  Up to direct_max counts take one launch, whose last
+// CTA reads all of them: 16 tiles of 8,192 counts, where it meets the
+// two-launch scan (3.0 us against 4.2 plus a launch on 13,000 counts, 4.8
+// against 4.7 plus a launch on 100,000).
+constexpr uint64_t kScanDirectMax = 16ull * 8192ull;
 uint64_t scan_temp_words(uint64_t n);
 void exclusive_scan_u32(cudaStream_t st, const uint32_t* in, uint32_t* out, uint64_t n,
-                        uint32_t* temp);
-// Two independent scans in the same two launches (when each fits the
-// two-launch form; else one after the other).  temp holds
-// scan_temp_words(n0) + scan_temp_words(n1) u32.
+                        uint32_t* temp, uint64_t direct_max = kScanDirectMax);
+// Two independent scans in the same launches (when both are of the same
+// form; else one after the other).  temp holds scan_temp_words(n0) +
+// scan_temp_words(n1) u32.
 void exclusive_scan_u32_pair(cudaStream_t st, const uint32_t* in0, uint32_t* out0, uint64_t n0,
-                             const uint32_t* in1, uint32_t* out1, uint64_t n1, uint32_t* temp);
-// The same scan in one launch (decoupled look-back, k_scan.cu).  temp holds
-// scan1p_words(n) u32, 8-byte aligned, and must be zero when first used (its
-// words are left ready for the next call).  err: optional flag word that gets
-// SOIL_SCAN_ERR if a look-back wait runs out.
-constexpr uint32_t SOIL_SCAN_ERR = 16u;
-uint64_t scan1p_words(uint64_t n);
-void exclusive_scan_1p(cudaStream_t st, const uint32_t* in, uint32_t* out, uint64_t n,
-                       uint32_t* temp, uint32_t* err);
+                             const uint32_t* in1, uint32_t* out1, uint64_t n1, uint32_t* temp,
+                             uint64_t direct_max = kScanDirectMax);
 
 // ---- bins (k_bins.cu) -----------------------------------------------------
 // cell[i] = cell_of(pos[first+i]) and counts[cell]++ for i in [0, n)
@@ -427,8 +424,7 @@ void launch_pair_count_staged(cudaStream_t st, const PairParams& p, const PairSe
                               uint32_t* rowcount, uint32_t* slots, DevFlags* flags);
 constexpr uint32_t SOIL_PAIRS_ERR_STAGING = 8u;
 // A pass launched before the host has read the pair total runs only when the
-// total fits its arrays: *total + 1 <= cap, and err[0] (DevFlags::error) and
-// err[1] (DevFlags::fault) are clear.  Every thread reads the same words, so
+// total fits its arrays: *total + 1 <= cap, and *err (DevFlags::error) is clear.  Every thread reads the same words, so
 // a launch runs whole or not at all.  A default guard (null total) is open.
 // Pass 2 can also hand the host what it waits for (pub_total != null): the
 // first thread copies *total to *pub_total and *flags to *pub_flags (host
@@ -443,7 +439,7 @@ struct FillGuard {
 };
 __device__ __forceinline__ bool guard_open(const FillGuard& g) {
     if (!g.total) return true;
-    return (uint64_t)*g.total + 1 <= g.cap && g.err[0] == 0u && g.err[1] == 0u;
+    return (uint64_t)*g.total + 1 <= g.cap && *g.err == 0u;
 }
 __device__ __forceinline__ void guard_publish(const FillGuard& g) {
     if (g.pub_total && blockIdx.x == 0 && threadIdx.x == 0) {

@@ -310,43 +310,25 @@ int sync(soil_sys* s) {
     return SOIL_OK;
 }
 
-// Largest count the single-pass scan takes (SOIL_SCAN1P_MAX overrides, for
+// Largest count the one-launch scan takes (SOIL_SCAN1P_MAX overrides, for
 // A/B runs; read at each call).
-uint64_t scan1p_max() {
+uint64_t scan_direct_max() {
     const char* env = std::getenv("SOIL_SCAN1P_MAX");
-    return env ? std::strtoull(env, nullptr, 10) : kScan1pMaxCounts;
+    return env ? std::strtoull(env, nullptr, 10) : kScanDirectMax;
 }
 
-int scan_1p(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n) {
-    // Up to 64 tiles of 2,048 counts the single launch saves launch latency;
-    // above it the three-kernel scan is faster (the look-back of a thousand
-    // resident CTAs contends).
-    if (n > scan1p_max()) {
-        TRY(ensure(s, s->scan_tmp, scan_temp_words(n + 2)));
-        exclusive_scan_u32(s->st, in, out, n, s->scan_tmp.p);
-        return SOIL_OK;
-    }
-    const uint64_t need = scan1p_words(n);
-    if (!s->scan1p.p || s->scan1p.cap < need) {
-        TRY(ensure(s, s->scan1p, need, 0, scan1p_words(2 * n + 4096)));
-        CK(cudaMemsetAsync(s->scan1p.p, 0, s->scan1p.cap * 4, s->st));
-    }
-    exclusive_scan_1p(s->st, in, out, n, s->scan1p.p, &s->dflags->fault);
+int scan_counts(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n) {
+    TRY(ensure(s, s->scan_tmp, scan_temp_words(n + 2)));
+    exclusive_scan_u32(s->st, in, out, n, s->scan_tmp.p, scan_direct_max());
     return SOIL_OK;
 }
 
-// Two independent scans; above the single-pass size both go in the same two
-// launches.
+// Two independent scans, in the same launches when they are of the same form.
 int scan_pair(soil_sys* s, const uint32_t* in0, uint32_t* out0, uint64_t n0, const uint32_t* in1,
               uint32_t* out1, uint64_t n1) {
-    const uint64_t lim = scan1p_max();
-    if (n0 > lim && n1 > lim) {
-        TRY(ensure(s, s->scan_tmp, scan_temp_words(n0 + 2) + scan_temp_words(n1 + 2)));
-        exclusive_scan_u32_pair(s->st, in0, out0, n0, in1, out1, n1, s->scan_tmp.p);
-        return SOIL_OK;
-    }
-    TRY(scan_1p(s, in0, out0, n0));
-    return scan_1p(s, in1, out1, n1);
+    TRY(ensure(s, s->scan_tmp, scan_temp_words(n0 + 2) + scan_temp_words(n1 + 2)));
+    exclusive_scan_u32_pair(s->st, in0, out0, n0, in1, out1, n1, s->scan_tmp.p, scan_direct_max());
+    return SOIL_OK;
 }
 
 int pairs_pre_ranges() {
@@ -657,10 +639,7 @@ bool displacement_needed(const soil_sys* s) {
 
 int read_flags(soil_sys* s) {
     CK(cudaMemcpyAsync(s->hflags, s->dflags, sizeof(DevFlags), cudaMemcpyDeviceToHost, s->st));
-    TRY(sync(s));
-    if (s->hflags->fault & SOIL_SCAN_ERR)
-        return fail(s->ctx, SOIL_ERR_CUDA, "a single-pass scan's look-back wait ran out");
-    return SOIL_OK;
+    return sync(s);
 }
 
 int phase_decide_rebuild(soil_sys* s) {
@@ -893,7 +872,7 @@ int sort_run(soil_sys* s, bool periodic_sort, bool cells_done) {
         TRY(counts_zero(s, nc));
         launch_cells(s->st, 0, nl, s->A, grid_of(s), s->sort_cell.p, s->cell_counts.p);
     }
-    TRY(scan_1p(s, s->cell_counts.p, s->sort_start.p, nc));
+    TRY(scan_counts(s, s->cell_counts.p, s->sort_start.p, nc));
     launch_scatter_consume(s->st, nl, s->sort_cell.p, s->sort_start.p, s->cell_counts.p,
                            s->sort_perm.p);
     counts_consumed(s);
@@ -1137,7 +1116,7 @@ int build_in_lists(soil_sys* s) {
     CK(cudaMemsetAsync(s->in_count.p, 0, total * 4, s->st));
     s->in_zero = 0;  // left holding the counts
     launch_in_count(s->st, s->nlocal, s->offsets.p, s->indices.p, s->in_count.p);
-    TRY(scan_1p(s, s->in_count.p, s->in_start.p, total));
+    TRY(scan_counts(s, s->in_count.p, s->in_start.p, total));
     CK(cudaMemcpyAsync(s->in_cursor.p, s->in_start.p, total * 4, cudaMemcpyDeviceToDevice, s->st));
     launch_in_scatter(s->st, s->nlocal, s->offsets.p, s->indices.p, s->in_cursor.p, s->in_list.p);
     TRY(ensure(s, s->in_split, total + 1, 0, s->acap + 1));
@@ -1171,7 +1150,7 @@ int build_seq(soil_sys* s) {
     q.fold_start = s->fold_start.p;
     q.fold_list = s->fold_list.p;
     launch_seq_count(s->st, q, s->seq_cnt.p, s->grp_cnt.p);
-    TRY(scan_1p(s, s->grp_cnt.p, s->grp_start.p, nl));
+    TRY(scan_counts(s, s->grp_cnt.p, s->grp_start.p, nl));
     launch_seq_fill(s->st, q, s->grp_start.p, s->seq.p, s->seq_owner.p);
     TRY(check_launch(s));
     s->seq_valid = true;
@@ -1428,7 +1407,7 @@ int phase_neighbor(soil_sys* s) {
     else
         launch_cells(s->st, 0, total, s->A, gr, s->atom_cell.p, s->cell_counts.p, n_dev);
     s->local_cells_valid = false;
-    TRY(scan_1p(s, s->cell_counts.p, s->cell_start.p, nc));
+    TRY(scan_counts(s, s->cell_counts.p, s->cell_start.p, nc));
     if (after_sort) {
         // the locals are in bin order already: only the ghosts are sorted
         const bool zeroed =
@@ -1515,7 +1494,7 @@ int phase_neighbor(soil_sys* s) {
     else
         launch_pair_count(s->st, p, s->rowcount.p, s->row_slots.p, s->dflags);
     if (with_in) TRY(scan_pair(s, s->rowcount.p, s->offsets.p, nl, s->in_count.p, s->in_start.p, total));
-    else TRY(scan_1p(s, s->rowcount.p, s->offsets.p, nl));
+    else TRY(scan_counts(s, s->rowcount.p, s->offsets.p, nl));
     if (!s->ev_counts) CK(cudaEventCreateWithFlags(&s->ev_counts, cudaEventDisableTiming));
     // Pass 2 goes in before the host reads the pair total, into the arrays it
     // has: the stream stays busy while the host waits for the counts, which
@@ -1550,8 +1529,6 @@ int phase_neighbor(soil_sys* s) {
     }
     TRY(check_launch(s));
     CK(cudaEventSynchronize(s->ev_counts));
-    if (s->hflags->fault & SOIL_SCAN_ERR)
-        return fail(s->ctx, SOIL_ERR_CUDA, "a single-pass scan's look-back wait ran out");
     if (pend) {  // the deferred border pass, now read back
         s->borders_pending = false;
         const uint32_t* hb = s->hword + kBorderStateWords;
@@ -2355,7 +2332,7 @@ int soil_sys_destroy(soil_sys* s) {
     for (int k = 0; k < 2; ++k) { fr(s->slot_tag[k]); fr(s->slot_val[k]); }
     fr(s->in_count); fr(s->in_start); fr(s->in_cursor); fr(s->in_list); fr(s->in_split);
     fr(s->seq_cnt); fr(s->grp_cnt); fr(s->grp_start); fr(s->seq); fr(s->seq_owner);
-    fr(s->rstate); fr(s->rec); fr(s->scan1p); fr(s->root_order); fr(s->pk);
+    fr(s->rstate); fr(s->rec); fr(s->root_order); fr(s->pk);
     fr(s->ghost_root); fr(s->ghost_chain);
     fr(s->fold_start); fr(s->fold_list);
     for (auto& a : s->send) fr(a);

@@ -175,7 +175,6 @@ struct soil_sys {
     bool steps_roomy = false;    // a resident launch needed all the shared memory
     uint64_t steps_refused_gen = ~0ull;  // border pass whose lists did not fit one
     DArr<double4> rec;  // their second record buffer, where the row slots are too small
-    DArr<uint32_t> scan1p;    // single-pass scan: tile counter and descriptors (zeroed at growth)
     DArr<uint32_t> root_order;  // CSR-walk consumer: roots by work per block (rebuilt with the lists)
     bool order_valid = false;
     DArr<uint32_t> ghost_root, ghost_chain;
@@ -294,9 +293,8 @@ int counts_zero(soil_sys* s, uint64_t nc);
 std::vector<int32_t> stencil_runs(const std::vector<int32_t>& sten, bool newton);
 // Whether the pair scan preloads its ranges (SOIL_PAIRS_PRE=0: off; read at each call).
 int pairs_pre_ranges();
-// exclusive scan of in[0, n) into out[0, n] in one launch, errors into the
-// system's device flags
-int scan_1p(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n);
+// exclusive scan of in[0, n) into out[0, n]
+int scan_counts(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n);
 Geom geom_of(const soil_sys* s);
 Grid grid_of(const soil_sys* s);
 void compute_bin_grid(soil_sys* s);
@@ -315,7 +313,5 @@ constexpr int kRowSlotsPerAtom = 16;
 // never) up to one root per thread of one CTA of 1,024 per SM.
 constexpr uint64_t kStepsSms = 148;
 constexpr uint64_t kStepsMaxRoots = kStepsSms * 1024;
-// largest count the single-pass scan serves (scan_1p)
-constexpr uint64_t kScan1pMaxCounts = 64ull * 2048ull;
 
 }  // namespace soil_host

@@ -49,3 +49,24 @@ def test_rows_match_oracle(ctx, n, phi, newton, kind):
     assert_same_lists(g, o)
     g.close()
     assert _stats(ctx, w, "1") == _stats(ctx, w, "0")
+
+
+@pytest.mark.parametrize("n", [700, 2500, 9000, 60000, 110000])
+@pytest.mark.parametrize("limit", [None, "8192"])
+def test_scans_of_every_form(ctx, n, limit):
+    """Count scans of one tile, of several tiles in one launch, of two
+    launches, and pairs of scans on either side of the line."""
+    old = os.environ.get("SOIL_SCAN1P_MAX")
+    if limit:
+        os.environ["SOIL_SCAN1P_MAX"] = limit
+    try:
+        w = W.poly("scans", 190, n, 0.4, 1e-4, 0, harmonic_k=1e3)
+        g, o = system.from_workload(ctx, w), oracle.from_workload(w)
+        g.step(2)
+        o.step(2)
+        assert_same_state(g, o, f"n={n}")
+        assert_same_lists(g, o)
+        g.close()
+    finally:
+        if limit:
+            os.environ.pop("SOIL_SCAN1P_MAX") if old is None else os.environ.update(SOIL_SCAN1P_MAX=old)
