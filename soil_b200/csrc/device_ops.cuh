@@ -771,12 +771,12 @@ __device__ __forceinline__ void fold_root(const AtomCols& c, uint64_t nlocal, ui
     }
 }
 
-// one sorted slot of the neighbor build's bin order (neighbor.rs:1101-1125)
-__device__ __forceinline__ void sorted_view(const AtomCols& c, uint64_t m, const uint32_t* sorted,
+// sorted slot m of the neighbor build's bin order, holding atom a
+// (neighbor.rs:1101-1125)
+__device__ __forceinline__ void sorted_view(const AtomCols& c, uint64_t m, uint32_t a,
                                             uint32_t* asi, double4* sp, float4* spf, double o0,
                                             double o1, double o2, const BuildPos& bp = BuildPos{},
                                             bool atom_in_w = false) {
-    const uint32_t a = sorted[m];
     asi[a] = (uint32_t)m;
     const double x = c.x[a], y = c.y[a], z = c.z[a], cut = c.cut[a];
     // with a uniform cutoff the pair test reads no radius: the fourth word

@@ -231,16 +231,36 @@ void launch_scatter_consume(cudaStream_t st, uint64_t n, const uint32_t* cell,
 void launch_cells_reuse(cudaStream_t st, uint64_t nlocal, uint64_t n, const AtomCols& c,
                         const Grid& gr, const uint32_t* local_cell, uint32_t* cell_out,
                         uint32_t* counts, const uint32_t* n_dev = nullptr);
-// The neighbor build's bin order (out = sorted atoms) just after a spatial
-// sort on the same grid: local i of cell c at start[c] + i - sort_start[c],
-// then c's ghosts [nl, n) in ascending order after its locals.  counts: the
-// cells' local + ghost counts (the ghosts' part is consumed); tmp: scratch of
-// the atoms' size.  Returns true when counts[0, nc) were put back to zero
-// (there were ghost slots to rank).
+// What the neighbor build's bin order carries per sorted slot: the atom, its
+// inverse asi[atom], the record sp = {x, y, z, cutoff} (plus the FP32
+// grid-relative copy spf when spf != nullptr) and the build positions of the
+// locals (bp).  atom_in_w (for a uniform cutoff, whose test reads no radius)
+// stores the atom's bits in place of the cutoff; clear (when given) gets its
+// candidates, rechecked and error words zeroed by the pass.
+struct SortedViews {
+    AtomCols c;
+    uint32_t* sorted;
+    uint32_t* asi;
+    double4* sp;
+    float4* spf;
+    double origin[3];
+    BuildPos bp;
+    int atom_in_w;
+    DevFlags* clear;
+};
+// The neighbor build's bins and views just after a spatial sort on the same
+// grid: local i of cell c at start[c] + i - sort_start[c], then c's ghosts
+// [nl, n) in ascending order after its locals.  counts: the cells' local +
+// ghost counts (the ghosts' part is consumed); tmp: scratch of the atoms'
+// size.  Returns true when counts[0, nc) were put back to zero (there were
+// ghost slots to rank).
 bool launch_place_bins(cudaStream_t st, uint64_t nl, uint64_t n, uint64_t nc,
                        const uint32_t* n_dev, const uint32_t* cell, const uint32_t* start,
                        const uint32_t* sort_start, uint32_t* counts, uint32_t* tmp,
-                       uint32_t* out);
+                       const SortedViews& v);
+// The views alone, of sorted slots [0, n)
+void launch_sorted_views(cudaStream_t st, uint64_t n, const SortedViews& v,
+                         const uint32_t* n_dev = nullptr);
 // sort every segment [start[s], start[s+1]) ascending -> stable counting sort
 void launch_segsort(cudaStream_t st, uint64_t nseg, const uint32_t* start, uint32_t* items);
 // the same, and split[s] = entries of segment s below s (transposed lists)
@@ -255,6 +275,12 @@ void launch_in_split(cudaStream_t st, uint64_t nseg, const uint32_t* start, cons
 void launch_perm_gather(cudaStream_t st, uint64_t n, const uint32_t* perm, const AtomCols& src,
                         const AtomCols& dst, bool forces = true, const uint32_t* cell_in = nullptr,
                         uint32_t* cell_out = nullptr);
+// bins[0, n): the atoms in cell order (cell starts in start), unordered inside
+// a cell.  perm = the stable order; dst[k] = src[perm[k]] for every column and
+// cell_out[k] = cell[perm[k]].
+void launch_sort_gather(cudaStream_t st, uint64_t n, const uint32_t* bins, const uint32_t* cell,
+                        const uint32_t* start, const AtomCols& src, const AtomCols& dst,
+                        bool forces, uint32_t* perm, uint32_t* cell_out);
 // flags->not_identity |= any perm[k] != k
 void launch_identity_check(cudaStream_t st, uint64_t n, const uint32_t* perm, DevFlags* flags);
 // out[k] = cell[perm[k]]
@@ -265,17 +291,6 @@ void launch_slot_gather(cudaStream_t st, uint64_t n, const uint32_t* perm, uint3
                         uint32_t* dst_tag, double* dst_val);
 void launch_permute_u32(cudaStream_t st, uint64_t n, const uint32_t* perm, const uint32_t* in,
                         uint32_t* out);
-// inverse[sorted[m]] = m and the sorted records sp[m] = {x, y, z, cutoff}
-// (plus the FP32 grid-relative copy spf when spf != nullptr); atom_in_w (for
-// a uniform cutoff, whose test reads no radius) stores sorted[m]'s bits in
-// place of the cutoff; clear (when given, and n > 0) gets its candidates,
-// rechecked and error words zeroed
-void launch_sorted_views(cudaStream_t st, uint64_t n, const uint32_t* sorted, const AtomCols& c,
-                         uint32_t* atom_sorted_idx, double4* sp, float4* spf,
-                         const double origin[3], const BuildPos& bp = BuildPos{},
-                         const uint32_t* n_dev = nullptr, bool atom_in_w = false,
-                         DevFlags* clear = nullptr);
-
 // ---- ghosts (k_ghost.cu) --------------------------------------------------
 struct BorderDim {
     int dim;

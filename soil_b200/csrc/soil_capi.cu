@@ -827,6 +827,7 @@ int sort_plan(soil_sys* s, bool* run, bool* periodic) {
     TRY(ensure(s, s->sort_cell, s->acap));
     TRY(ensure(s, s->sort_perm, s->acap));
     TRY(ensure(s, s->sorted_local_cell, s->acap));
+    TRY(ensure(s, s->ghost_tmp, s->acap));
     TRY(ensure(s, s->cell_counts, nc + 1, 0, 2 * nc + 64));
     TRY(ensure(s, s->cell_start, nc + 2, 0, 2 * nc + 64));
     TRY(ensure(s, s->cell_cursor, nc + 1, 0, 2 * nc + 64));
@@ -873,35 +874,38 @@ int sort_run(soil_sys* s, bool periodic_sort, bool cells_done) {
         launch_cells(s->st, 0, nl, s->A, grid_of(s), s->sort_cell.p, s->cell_counts.p);
     }
     TRY(scan_counts(s, s->cell_counts.p, s->sort_start.p, nc));
-    launch_scatter_consume(s->st, nl, s->sort_cell.p, s->sort_start.p, s->cell_counts.p,
-                           s->sort_perm.p);
+    const bool ranked = !periodic_sort && nl <= kSortGatherMax;
+    uint32_t* bins = ranked ? s->ghost_tmp.p : s->sort_perm.p;
+    launch_scatter_consume(s->st, nl, s->sort_cell.p, s->sort_start.p, s->cell_counts.p, bins);
     counts_consumed(s);
-    launch_segsort(s->st, nc, s->sort_start.p, s->sort_perm.p);
-    TRY(check_launch(s));
-
+    // every column gathered through perm; ghosts (if any) are discarded by the
+    // borders that always follows a permutation
     bool apply = true;
-    if (periodic_sort) {
-        CK(cudaMemsetAsync(&s->dflags->not_identity, 0, 4, s->st));
-        launch_identity_check(s->st, nl, s->sort_perm.p, s->dflags);
-        TRY(check_launch(s));
-        TRY(read_flags(s));
-        apply = s->hflags->not_identity != 0;
-    }
-    if (apply) {
-        // every column gathered through perm; ghosts (if any) are discarded by
-        // the borders that always follows a permutation
-        launch_perm_gather(s->st, nl, s->sort_perm.p, s->A, s->B, !s->forces_dead,
-                           s->sort_cell.p, s->sorted_local_cell.p);
-        if (s->slot_max) {  // slots move with their atoms
-            const int o = s->slot_old;
-            launch_slot_gather(s->st, nl, s->sort_perm.p, s->slot_max, s->slot_width,
-                               s->slot_tag[o].p, s->slot_val[o].p, s->slot_tag[1 - o].p,
-                               s->slot_val[1 - o].p);
-            s->slot_old = 1 - o;
-        }
+    if (ranked) {
+        launch_sort_gather(s->st, nl, bins, s->sort_cell.p, s->sort_start.p, s->A, s->B,
+                           !s->forces_dead, s->sort_perm.p, s->sorted_local_cell.p);
         TRY(check_launch(s));
     } else {
-        launch_permute_u32(s->st, nl, s->sort_perm.p, s->sort_cell.p, s->sorted_local_cell.p);
+        launch_segsort(s->st, nc, s->sort_start.p, s->sort_perm.p);
+        if (periodic_sort) {  // applied only if it moves an atom: the host asks first
+            CK(cudaMemsetAsync(&s->dflags->not_identity, 0, 4, s->st));
+            launch_identity_check(s->st, nl, s->sort_perm.p, s->dflags);
+            TRY(check_launch(s));
+            TRY(read_flags(s));
+            apply = s->hflags->not_identity != 0;
+        }
+        if (apply)
+            launch_perm_gather(s->st, nl, s->sort_perm.p, s->A, s->B, !s->forces_dead,
+                               s->sort_cell.p, s->sorted_local_cell.p);
+        else
+            launch_permute_u32(s->st, nl, s->sort_perm.p, s->sort_cell.p, s->sorted_local_cell.p);
+        TRY(check_launch(s));
+    }
+    if (apply && s->slot_max) {  // slots move with their atoms
+        const int o = s->slot_old;
+        launch_slot_gather(s->st, nl, s->sort_perm.p, s->slot_max, s->slot_width, s->slot_tag[o].p,
+                           s->slot_val[o].p, s->slot_tag[1 - o].p, s->slot_val[1 - o].p);
+        s->slot_old = 1 - o;
         TRY(check_launch(s));
     }
     sort_done(s, apply, periodic_sort);
@@ -1408,27 +1412,32 @@ int phase_neighbor(soil_sys* s) {
         launch_cells(s->st, 0, total, s->A, gr, s->atom_cell.p, s->cell_counts.p, n_dev);
     s->local_cells_valid = false;
     TRY(scan_counts(s, s->cell_counts.p, s->cell_start.p, nc));
+    SortedViews views;
+    views.c = s->A;
+    views.sorted = s->sorted_atoms.p;
+    views.asi = s->asi.p;
+    views.sp = s->sp.p;
+    views.spf = fp32 ? s->spf.p : nullptr;
+    for (int d = 0; d < 3; ++d) views.origin[d] = s->blo[d];
+    views.bp.x = s->lbx.p;  // save_build_positions (neighbor.rs:669-690) in the same pass
+    views.bp.y = s->lby.p;
+    views.bp.z = s->lbz.p;
+    views.bp.nlocal = nl;
+    views.atom_in_w = s->has_uniform ? 1 : 0;
+    views.clear = s->dflags;  // the counters of the pair passes
     if (after_sort) {
         // the locals are in bin order already: only the ghosts are sorted
         const bool zeroed =
             launch_place_bins(s->st, nl, total, nc, n_dev, s->atom_cell.p, s->cell_start.p,
-                              s->sort_start.p, s->cell_counts.p, s->ghost_tmp.p,
-                              s->sorted_atoms.p);
+                              s->sort_start.p, s->cell_counts.p, s->ghost_tmp.p, views);
         s->counts_clean = zeroed ? nc : 0;  // else the locals' counts remain
     } else {
         launch_scatter_consume(s->st, total, s->atom_cell.p, s->cell_start.p, s->cell_counts.p,
                                s->sorted_atoms.p, n_dev);
         counts_consumed(s);
         launch_segsort(s->st, nc, s->cell_start.p, s->sorted_atoms.p);
+        launch_sorted_views(s->st, total, views, n_dev);
     }
-    BuildPos bpos;  // save_build_positions (neighbor.rs:669-690) in the same pass
-    bpos.x = s->lbx.p;
-    bpos.y = s->lby.p;
-    bpos.z = s->lbz.p;
-    bpos.nlocal = nl;
-    launch_sorted_views(s->st, total, s->sorted_atoms.p, s->A, s->asi.p, s->sp.p,
-                        fp32 ? s->spf.p : nullptr, s->blo, bpos, n_dev, s->has_uniform,
-                        s->dflags);  // also clears the counters of the pair passes
     const std::vector<int32_t>& sten = s->newton ? s->stencil_fwd : s->stencil;
     const std::vector<int32_t> runs = stencil_runs(sten, s->newton);
     const int32_t* old_stencil = s->d_stencil.p;

@@ -308,6 +308,11 @@ SwapConst swap_const(const soil_sys* s);
 // a light step's displacement check.
 constexpr int kHostAnswer = 2 * kBorderStateWords;
 constexpr int kHostWords = kHostAnswer + 8;
+// Largest system whose spatial sort ranks and gathers in one pass; above, a
+// segment sort and a gather are faster (46.9 against 49.5 us on 1,048,576
+// atoms, 176 against 167 on 4,194,304, where the rank's loads come on top of a
+// pass bound by HBM).
+constexpr uint64_t kSortGatherMax = 2000000;
 constexpr int kRowSlotsPerAtom = 16;
 // Systems with a consumer take the resident light steps (SOIL_RESIDENT_STEPS=0:
 // never) up to one root per thread of one CTA of 1,024 per SM.
