@@ -5,8 +5,10 @@
 // bits and, per category, the tile's member count (counts[k * nw + w]; row
 // kBorderCats holds all images of the tile).  After a per-category scan
 // (offs, same layout), pass 2 ranks each member inside its tile with a ballot
-// and writes its image, its send entry, its ghost root/chain and its root's
-// fold program.  Every routine is called by all 32 lanes of a warp.
+// and writes its image's root, chain and origin, its send entry and its root's
+// fold program; the images' columns follow with one thread per ghost
+// (make_ghost), whose writes are coalesced whatever the number of images per
+// root.  Every routine is called by all 32 lanes of a warp.
 #pragma once
 
 #include "block_scan.cuh"
@@ -77,13 +79,24 @@ __device__ __forceinline__ void border_state_words(const BorderCats& cats, uint6
 // chunk); chunk prefixes (cpre[k * nchunks + chunk]) are added back here.
 constexpr uint64_t kScanChunk = 8192;
 
-// Shared-memory scratch of one warp in pass 2: every lane's ghost index per
-// category (indexed by category, so it must not live in registers) and the
-// first ghost index of each swap.
+// Shared-memory scratch of one warp in pass 2: per category its members among
+// the tile's lanes and the ghost index of the first, and the first ghost index
+// of each swap.  Kept this small on purpose: with dependent launches an SM is
+// never idle between the kernels of a step, so it keeps the split of L1 and
+// shared memory of the kernel that needed most.  With every lane's index per
+// category here (27 KB a CTA, 6 CTAs) the pair count and the consumer that
+// follow ran on a third of the L1: k_force_csr 339 against 208 us on 4,194,304
+// atoms.
 struct BorderWarpSmem {
-    uint32_t idx[kBorderCats][32];
+    uint32_t members[kBorderCats];
+    uint32_t first[kBorderCats];
     uint32_t recv[kNumSwaps];
 };
+
+// Ghost index of a member lane's image of category k (below: the lanes before it).
+__device__ __forceinline__ uint32_t image_index(const BorderWarpSmem& sm, int k, unsigned below) {
+    return sm.first[k] + __popc(sm.members[k] & below);
+}
 
 // Pass 2 for warp tile w.  base_lane: on lane k < 26 the first ghost index of
 // category k (nlocal + the totals of the categories before it).  offs holds
@@ -91,9 +104,8 @@ struct BorderWarpSmem {
 // chunks' prefixes.  sm: this warp's scratch.  host_bs (optional): the host's
 // copy of bs, which gets the capacity word too.
 __device__ __forceinline__ void border_warp_images(
-    const AtomCols& c, uint64_t nlocal, uint64_t cap, const double (*shift)[3],
-    const double (*vshift)[3], const BorderCats& cats, const uint8_t* face, const uint32_t* offs,
-    const uint32_t* cpre, uint64_t nchunks, uint64_t nw, uint64_t w, uint32_t lane,
+    const AtomCols& c, uint64_t nlocal, uint64_t cap, const BorderCats& cats, const uint8_t* face,
+    const uint32_t* offs, const uint32_t* cpre, uint64_t nchunks, uint64_t nw, uint64_t w, uint32_t lane,
     uint32_t base_lane, uint32_t* bs, uint32_t* root, uint32_t* chain, uint32_t* const* send,
     uint32_t* fold_start, uint32_t* fold_list, BorderWarpSmem& sm, uint32_t* host_bs = nullptr) {
     const unsigned below = (1u << lane) - 1u;
@@ -120,13 +132,16 @@ __device__ __forceinline__ void border_warp_images(
     const uint32_t mine_cats = cats.member[bits];
     const uint32_t own = __popc(mine_cats);  // images of this lane's root
     // only categories the tile's faces cover can have members (uniform over
-    // the warp); only members read idx, and a member's parent category has
-    // it as a member too
+    // the warp); only members read their category, and a member's parent
+    // category has it as a member too
     for (uint32_t cand = cats.member[any]; cand; cand &= cand - 1) {
         const int k = __ffs(cand) - 1;
         const unsigned bal = __ballot_sync(0xffffffffu, (mine_cats >> k) & 1u);
         const uint32_t base = __shfl_sync(0xffffffffu, base_lane + off_lane, k);
-        sm.idx[k][lane] = base + __popc(bal & below);
+        if (lane == 0) {
+            sm.members[k] = bal;
+            sm.first[k] = base;
+        }
     }
     __syncwarp();
     const uint32_t fs = fold0 + warp_exclusive_sum(own, lane);
@@ -135,22 +150,24 @@ __device__ __forceinline__ void border_warp_images(
     if (bits) {
         for (uint32_t mk = mine_cats; mk; mk &= mk - 1) {
             const int k = __ffs(mk) - 1;
-            const uint32_t g = sm.idx[k][lane];
+            const uint32_t g = image_index(sm, k, below);
             if (g >= cap) {
                 bs[10] = 1u;  // out of capacity: the host grows the arrays and repeats
                 if (host_bs) host_bs[10] = 1u;
                 continue;
             }
             const uint32_t parent =
-                cats.parent[k] < 0 ? (uint32_t)r : sm.idx[cats.parent[k]][lane];
-            write_image(c, shift, vshift, cats, k, g, r, parent, nlocal, root, chain);
+                cats.parent[k] < 0 ? (uint32_t)r : image_index(sm, cats.parent[k], below);
+            root[g - nlocal] = (uint32_t)r;
+            chain[g - nlocal] = cats.code[k];
+            c.origin[g] = (int32_t)parent;
             const int s = cats.swap_of[k];
             send[s][g - sm.recv[s]] = parent;
         }
         uint32_t j = fs;
         for (uint32_t mf = cats.member_fold[bits]; mf; mf &= mf - 1) {
             const int k = cats.fold[__ffs(mf) - 1];
-            const uint32_t g = sm.idx[k][lane];
+            const uint32_t g = image_index(sm, k, below);
             if (g < cap && j < cap) fold_list[j] = g - (uint32_t)nlocal;
             ++j;
         }

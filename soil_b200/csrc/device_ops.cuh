@@ -108,43 +108,49 @@ __device__ __forceinline__ uint32_t face_bits(const AtomCols& c, const Geom& geo
     return b;
 }
 
-// Ghost g = image of root r through the swaps of chain category k
+// Ghost gi (index nlocal + gi) = image of its root through its swap chain
 // (pack_border + unpack_atom, atom.rs:520-553, applied swap by swap: the
-// shifts are added in chain order exactly as the reference's ghost of a
-// ghost does); its source (origin) is `parent`.
-__device__ __forceinline__ void write_image(const AtomCols& c, const double (*shift)[3],
-                                            const double (*vshift)[3], const BorderCats& cats,
-                                            int k, uint64_t g, uint64_t r, uint32_t parent,
-                                            uint64_t nlocal, uint32_t* root, uint32_t* chain) {
-    const uint64_t cap = c.cap;
+// shifts are added in chain order exactly as the reference's ghost of a ghost
+// does); its origin is the border pass's.  forces: false when the consumer
+// overwrites every force before anything reads one.  Returns the position.
+__device__ __forceinline__ double3 make_ghost(const AtomCols& c, uint64_t nlocal, uint64_t gi,
+                                              const uint32_t* root, const uint32_t* chain,
+                                              const SwapConst& sc, bool forces) {
+    const uint64_t cap = c.cap, g = nlocal + gi;
+    const uint32_t r = root[gi], code = chain[gi];
+    // every load before any store (see perm_gather_atom)
     double x = c.x[r], y = c.y[r], z = c.z[r];
     double vx = c.vx[r], vy = c.vy[r], vz = c.vz[r];
-    uint32_t code = 0;
-    for (int t = 0; t < cats.len[k]; ++t) {
-        const int s = cats.sw[k][t];
-        x = x + shift[s][0];
-        y = y + shift[s][1];
-        z = z + shift[s][2];
-        vx = vx + vshift[s][0];
-        vy = vy + vshift[s][1];
-        vz = vz + vshift[s][2];
-        code |= (uint32_t)s << (3 * t);
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    if (forces) {
+        fx = c.fx[r];
+        fy = c.fy[r];
+        fz = c.fz[r];
     }
-    code |= (uint32_t)cats.len[k] << 12;
-    // the root's other fields loaded before any store (see perm_gather_atom)
-    const double fx = c.fx[r], fy = c.fy[r], fz = c.fz[r];
     const double m = c.mass[r], cu = c.cut[r];
     const uint32_t tg = c.tag[r], ty = c.type[r];
     const int32_t i0 = c.img[r], i1 = c.img[cap + r], i2 = c.img[2 * cap + r];
+    const uint32_t len = code >> 12;
+    for (uint32_t k = 0; k < len; ++k) {
+        const int s = (code >> (3 * k)) & 7;
+        x = x + sc.off[s][0];
+        y = y + sc.off[s][1];
+        z = z + sc.off[s][2];
+        vx = vx + sc.voff[s][0];
+        vy = vy + sc.voff[s][1];
+        vz = vz + sc.voff[s][2];
+    }
     c.x[g] = x;
     c.y[g] = y;
     c.z[g] = z;
     c.vx[g] = vx;
     c.vy[g] = vy;
     c.vz[g] = vz;
-    c.fx[g] = fx;
-    c.fy[g] = fy;
-    c.fz[g] = fz;
+    if (forces) {
+        c.fx[g] = fx;
+        c.fy[g] = fy;
+        c.fz[g] = fz;
+    }
     c.mass[g] = m;
     c.inv_mass[g] = 1.0 / m;
     c.cut[g] = cu;
@@ -153,7 +159,6 @@ __device__ __forceinline__ void write_image(const AtomCols& c, const double (*sh
     c.img[g] = i0;
     c.img[cap + g] = i1;
     c.img[2 * cap + g] = i2;
-    c.origin[g] = (int32_t)parent;
     for (int q = 0; q < c.nplanes; q += 4) {
         double v[4];
 #pragma unroll
@@ -163,8 +168,7 @@ __device__ __forceinline__ void write_image(const AtomCols& c, const double (*sh
         for (int u = 0; u < 4; ++u)
             if (q + u < c.nplanes) c.planes[q + u][g] = v[u];
     }
-    root[g - nlocal] = (uint32_t)r;
-    chain[g - nlocal] = code;
+    return make_double3(x, y, z);
 }
 
 // A sorted record {x, y, z, cutoff} in one 256-bit load through the

@@ -144,7 +144,12 @@ __global__ void __launch_bounds__(kBlock) kb_cells(Span sp, BatchArgs A, int nei
         const BoxDev& D = A.dev[b];
         const BoxStep& S = A.step[b];
         const AtomCols& c = D.set[neighbor ? S.post : S.cur];
-        const uint32_t cell = cell_of(S.grid, c.x[i], c.y[i], c.z[i]);
+        double3 q;
+        if (neighbor && i >= S.nlocal)  // the border pass's ghosts get their columns here
+            q = make_ghost(c, S.nlocal, i - S.nlocal, D.ghost_root, D.ghost_chain, S.sc, false);
+        else
+            q = make_double3(c.x[i], c.y[i], c.z[i]);
+        const uint32_t cell = cell_of(S.grid, q.x, q.y, q.z);
         (neighbor ? D.atom_cell : D.sort_cell)[i] = cell;
         atomicAdd(&D.cell_counts[cell], 1u);
     });
@@ -326,9 +331,9 @@ __global__ void __launch_bounds__(kBlock) kb_border_images(Span sp, BatchArgs A,
         if (w == 0 && lane == 0) border_state_words(cats, S.nlocal, bs);
         const uint32_t tot = lane < kBorderCats ? bs[kBorderTotals + lane] : 0u;
         const uint32_t base_lane = (uint32_t)S.nlocal + warp_exclusive_sum(tot, lane);
-        border_warp_images(D.set[S.post], S.nlocal, D.cap, S.sc.off, S.sc.voff, cats, D.face_flags,
-                           D.boff, nullptr, 1, nw, w, lane, base_lane, bs, D.ghost_root,
-                           D.ghost_chain, D.send, D.fold_start, D.fold_list, sm[threadIdx.x / 32]);
+        border_warp_images(D.set[S.post], S.nlocal, D.cap, cats, D.face_flags, D.boff, nullptr, 1,
+                           nw, w, lane, base_lane, bs, D.ghost_root, D.ghost_chain, D.send,
+                           D.fold_start, D.fold_list, sm[threadIdx.x / 32]);
     });
 }
 void b_border_images(cudaStream_t st, const Span& sp, const BatchArgs& a) {

@@ -224,11 +224,13 @@ void launch_scatter_consume(cudaStream_t st, uint64_t n, const uint32_t* cell,
 }
 
 // The neighbor build's cells in one pass: the locals' cells from the sort
-// (local < nlocal), the others' from their positions; all counted.
+// (local < nlocal), the others' from their positions; all counted.  MAKE: the
+// ghosts of a border pass just queued get their columns here.
+template <bool MAKE>
 __global__ void __launch_bounds__(kBlock) k_cells_reuse(uint64_t nlocal, uint64_t n, AtomCols c,
                                                         Grid gr, const uint32_t* local_cell,
                                                         uint32_t* cell_out, uint32_t* counts,
-                                                        const uint32_t* n_dev) {
+                                                        const uint32_t* n_dev, GhostMake mk) {
     pdl_wait();  // launched with pdl_launch
     if (n_dev) {  // the count known only on the device (an upper bound in n)
         const uint64_t d = *n_dev;
@@ -240,7 +242,15 @@ __global__ void __launch_bounds__(kBlock) k_cells_reuse(uint64_t nlocal, uint64_
         const bool valid = i < n;
         uint32_t cell = 0;
         if (valid) {
-            cell = i < nlocal ? local_cell[i] : cell_of(gr, c.x[i], c.y[i], c.z[i]);
+            if (i < nlocal) {
+                cell = local_cell[i];
+            } else if (MAKE) {
+                const double3 q =
+                    make_ghost(c, nlocal, i - nlocal, mk.root, mk.chain, mk.sc, mk.forces != 0);
+                cell = cell_of(gr, q.x, q.y, q.z);
+            } else {
+                cell = cell_of(gr, c.x[i], c.y[i], c.z[i]);
+            }
             cell_out[i] = cell;
         }
         aggregated_count(counts, cell, valid);
@@ -249,11 +259,15 @@ __global__ void __launch_bounds__(kBlock) k_cells_reuse(uint64_t nlocal, uint64_
 
 void launch_cells_reuse(cudaStream_t st, uint64_t nlocal, uint64_t n, const AtomCols& c,
                         const Grid& gr, const uint32_t* local_cell, uint32_t* cell_out,
-                        uint32_t* counts, const uint32_t* n_dev) {
+                        uint32_t* counts, const uint32_t* n_dev, const GhostMake* make) {
     if (n == 0) return;
     note_launch();
-    pdl_launch(k_cells_reuse, grid_wave<k_cells_reuse>(n), kBlock, 0, st, nlocal, n, c, gr, local_cell,
-                                                                  cell_out, counts, n_dev);
+    if (make)
+        pdl_launch(k_cells_reuse<true>, grid_wave<k_cells_reuse<true>>(n), kBlock, 0, st, nlocal, n, c,
+                   gr, local_cell, cell_out, counts, n_dev, *make);
+    else
+        pdl_launch(k_cells_reuse<false>, grid_wave<k_cells_reuse<false>>(n), kBlock, 0, st, nlocal, n,
+                   c, gr, local_cell, cell_out, counts, n_dev, GhostMake{});
 }
 
 __device__ __forceinline__ void clear_pair_counters(DevFlags* clear) {

@@ -77,6 +77,9 @@ BorderCats build_border_cats() {
             need |= (uint8_t)(1u << c.sw[l]);
         }
         t.need[k] = need;
+        uint16_t code = (uint16_t)(c.n << 12);
+        for (int l = 0; l < c.n; ++l) code |= (uint16_t)(c.sw[l] << (3 * l));
+        t.code[k] = code;
         t.swap_of[k] = (uint8_t)c.sw[c.n - 1];
         t.parent[k] = -1;
         for (int q = 0; q < kBorderCats && c.n > 1; ++q)
@@ -153,10 +156,16 @@ __global__ void __launch_bounds__(kBlock) k_border_faces(uint64_t nlocal, AtomCo
 
 // Pass 2: one CTA per (category or all images, chunk of kScanChunk warp
 // tiles) scans the warp counts inside its chunk; ctot gets the chunk totals.
+// Clears the capacity word bs[10] that pass 3 may set.
 __global__ void __launch_bounds__(kBlock) k_border_cat_scan(const uint32_t* counts, uint32_t* offs,
                                                             uint64_t nw, uint32_t* ctot,
-                                                            uint64_t nchunks) {
+                                                            uint64_t nchunks, uint32_t* bs,
+                                                            uint32_t* host_bs) {
     pdl_wait();  // launched with pdl_launch
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        bs[10] = 0u;
+        if (host_bs) host_bs[10] = 0u;
+    }
     const uint64_t k = blockIdx.x / nchunks, ch = blockIdx.x % nchunks;
     const uint64_t w0 = ch * kScanChunk;
     const uint64_t n = nw - w0 < kScanChunk ? nw - w0 : kScanChunk;
@@ -164,15 +173,10 @@ __global__ void __launch_bounds__(kBlock) k_border_cat_scan(const uint32_t* coun
     if (threadIdx.x == 0) ctot[k * nchunks + ch] = total;
 }
 
-// Chunk totals -> exclusive chunk prefixes (in place) and category totals;
-// clears the capacity word bs[10] that pass 3 may set.
+// Chunk totals -> exclusive chunk prefixes (in place) and category totals.
 __global__ void __launch_bounds__(kBlock) k_border_chunk_prefix(uint32_t* ctot, uint64_t nchunks,
-                                                                uint32_t* bs, uint32_t* host_bs) {
+                                                                uint32_t* bs) {
     pdl_wait();  // launched with pdl_launch
-    if (threadIdx.x == 0) {
-        bs[10] = 0u;
-        if (host_bs) host_bs[10] = 0u;
-    }
     for (uint32_t k = threadIdx.x; k <= (uint32_t)kBorderCats; k += blockDim.x) {
         uint32_t acc = 0;
         for (uint64_t ch = 0; ch < nchunks; ++ch) {
@@ -185,29 +189,35 @@ __global__ void __launch_bounds__(kBlock) k_border_chunk_prefix(uint32_t* ctot, 
 }
 
 // Pass 3, one warp per 32 locals: every image of the warp's roots at its
-// final index, the swap send lists, ghost root/chain, and each root's fold
-// program (its images in fold order).
+// final index, the swap send lists, ghost root/chain/origin, and each root's
+// fold program (its images in fold order).  totals: the category totals (of a
+// single chunk, pass 2's; else those the prefix pass left in bs).
 __global__ void __launch_bounds__(kBlock) k_border_images(
-    uint64_t nlocal, uint64_t cap, AtomCols c, BorderPass bp, BorderCats cats, const uint8_t* face,
-    const uint32_t* offs, const uint32_t* cpre, uint64_t nchunks, uint64_t nw, uint32_t* bs,
-    uint32_t* root, uint32_t* chain, SendPtrs send, uint32_t* fold_start, uint32_t* fold_list,
-    uint32_t* host_bs) {
+    uint64_t nlocal, uint64_t cap, AtomCols c, BorderCats cats, const uint8_t* face,
+    const uint32_t* offs, const uint32_t* totals, const uint32_t* cpre, uint64_t nchunks,
+    uint64_t nw, uint32_t* bs, uint32_t* root, uint32_t* chain, SendPtrs send,
+    uint32_t* fold_start, uint32_t* fold_list, uint32_t* host_bs) {
     pdl_wait();  // launched with pdl_launch
     __shared__ BorderWarpSmem sm[kBlock / 32];
     const uint32_t lane = threadIdx.x & 31u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        border_state_words(cats, nlocal, bs);
-        if (host_bs)
-            for (int k = 0; k < 10; ++k) host_bs[k] = bs[k];
-    }
     // first ghost index of category `lane` (lanes below 26)
-    const uint32_t tot = lane < kBorderCats ? bs[kBorderTotals + lane] : 0u;
-    const uint32_t base_lane = (uint32_t)nlocal + warp_exclusive_sum(tot, lane);
+    const uint32_t tot = lane <= kBorderCats ? totals[lane] : 0u;
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        if (lane <= kBorderCats) bs[kBorderTotals + lane] = tot;
+        __syncwarp();
+        if (lane == 0) {
+            border_state_words(cats, nlocal, bs);
+            if (host_bs)
+                for (int k = 0; k < 10; ++k) host_bs[k] = bs[k];
+        }
+    }
+    const uint32_t base_lane =
+        (uint32_t)nlocal + warp_exclusive_sum(lane < kBorderCats ? tot : 0u, lane);
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x / 32);
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w < nw; w += nwarps)
-        border_warp_images(c, nlocal, cap, bp.shift, bp.vshift, cats, face, offs, cpre, nchunks,
-                           nw, w, lane, base_lane, bs, root, chain, send.p, fold_start, fold_list,
-                           sm[threadIdx.x / 32], host_bs);
+        border_warp_images(c, nlocal, cap, cats, face, offs, cpre, nchunks, nw, w, lane, base_lane,
+                           bs, root, chain, send.p, fold_start, fold_list, sm[threadIdx.x / 32],
+                           host_bs);
 }
 
 void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCols& c,
@@ -223,14 +233,36 @@ void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCo
     pdl_launch(k_border_faces, grid_wave<k_border_faces>(nw * 32), kBlock, 0, st, nlocal, c, bp, cats, face,
                                                                           counts, nw);
     note_launch();
-    pdl_launch(k_border_cat_scan, (unsigned)((kBorderCats + 1) * nchunks), kBlock, 0, st, counts, offs, nw,
-                                                                                ctot, nchunks);
+    pdl_launch(k_border_cat_scan, (unsigned)((kBorderCats + 1) * nchunks), kBlock, 0, st, counts,
+               offs, nw, ctot, nchunks, bs, host_bs);
+    // one chunk (up to 262,144 locals): its totals are the categories'
+    if (nchunks > 1) {
+        note_launch();
+        pdl_launch(k_border_chunk_prefix, 1, kBlock, 0, st, ctot, nchunks, bs);
+    }
+    const uint32_t* totals = nchunks > 1 ? bs + kBorderTotals : ctot;
+    const uint32_t* cpre = nchunks > 1 ? ctot : nullptr;
     note_launch();
-    pdl_launch(k_border_chunk_prefix, 1, kBlock, 0, st, ctot, nchunks, bs, host_bs);
+    pdl_launch(k_border_images, grid_wave<k_border_images>(nw * 32), kBlock, 0, st, nlocal, cap, c,
+               cats, face, offs, totals, cpre, nchunks, nw, bs, ghost_root, ghost_chain, send,
+               fold_start, fold_list, host_bs);
+}
+
+__global__ void __launch_bounds__(kBlock) k_make_ghosts(uint64_t nlocal, uint64_t nghost,
+                                                        AtomCols c, const uint32_t* root,
+                                                        const uint32_t* chain, SwapConst sc) {
+    pdl_wait();  // launched with pdl_launch
+    for (uint64_t gi = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; gi < nghost;
+         gi += (uint64_t)gridDim.x * blockDim.x)
+        make_ghost(c, nlocal, gi, root, chain, sc, true);
+}
+
+void launch_make_ghosts(cudaStream_t st, uint64_t nlocal, uint64_t nghost, const AtomCols& c,
+                        const uint32_t* root, const uint32_t* chain, const SwapConst& sc) {
+    if (nghost == 0) return;
     note_launch();
-    pdl_launch(k_border_images, grid_wave<k_border_images>(nw * 32), kBlock, 0, st, 
-        nlocal, cap, c, bp, cats, face, offs, ctot, nchunks, nw, bs, ghost_root, ghost_chain, send,
-        fold_start, fold_list, host_bs);
+    pdl_launch(k_make_ghosts, grid_wave<k_make_ghosts>(nghost), kBlock, 0, st, nlocal, nghost, c,
+               root, chain, sc);
 }
 
 __global__ void __launch_bounds__(kBlock) k_forward(uint64_t nlocal, uint64_t nghost, AtomCols c,

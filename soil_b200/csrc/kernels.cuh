@@ -227,10 +227,17 @@ void launch_scatter_consume(cudaStream_t st, uint64_t n, const uint32_t* cell,
                             const uint32_t* start, uint32_t* counts, uint32_t* out,
                             const uint32_t* n_dev = nullptr);
 // cell_out[i] = local_cell[i] (i < nlocal) or the cell of atom i, counted,
-// i in [0, n)
+// i in [0, n).  make (optional): the ghosts' columns are written first, in the
+// same pass.
+struct GhostMake {
+    const uint32_t* root = nullptr;
+    const uint32_t* chain = nullptr;
+    SwapConst sc;
+    int forces = 0;  // copy the roots' forces
+};
 void launch_cells_reuse(cudaStream_t st, uint64_t nlocal, uint64_t n, const AtomCols& c,
                         const Grid& gr, const uint32_t* local_cell, uint32_t* cell_out,
-                        uint32_t* counts, const uint32_t* n_dev = nullptr);
+                        uint32_t* counts, const uint32_t* n_dev, const GhostMake* make);
 // What the neighbor build's bin order carries per sorted slot: the atom, its
 // inverse asi[atom], the record sp = {x, y, z, cutoff} (plus the FP32
 // grid-relative copy spf when spf != nullptr) and the build positions of the
@@ -335,6 +342,7 @@ struct BorderCats {
     int8_t parent[kBorderCats];
     uint8_t swap_of[kBorderCats];
     uint8_t fold[kBorderCats];
+    uint16_t code[kBorderCats];  // the chain: swap ids, 3 bits each, its length from bit 12
     uint8_t swap_first[kNumSwaps];
     uint8_t swap_ncat[kNumSwaps];
 };
@@ -348,10 +356,10 @@ BorderPass border_pass(const BorderDim bds[3]);
 struct SendPtrs {
     uint32_t* p[kNumSwaps];
 };
-// borders + the reverse-comm fold program in three launches: face bits and
-// per-warp category counts of the locals, a scan per category, then every
-// image written from its root.  bs must be zero; ghosts beyond `cap` set
-// bs[10].  offs holds (kBorderCats + 1) * nw words and counts that plus
+// borders + the reverse-comm fold program: face bits and per-warp category
+// counts of the locals, a scan per category, then every image's place, root,
+// chain and origin (its columns are launch_make_ghosts' or the neighbor
+// build's binning pass').  bs must be zero; ghosts beyond `cap` set bs[10].  offs holds (kBorderCats + 1) * nw words and counts that plus
 // (kBorderCats + 1) * ceil(nw / 8192) (nw = ceil(nlocal / 32)).
 // cats: border_cats(), or border_cats_masked() for axes without periodicity.
 // host_bs (optional, host memory mapped for the device): the kernels also
@@ -362,6 +370,9 @@ void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCo
                     uint32_t* bs, uint32_t* ghost_root, uint32_t* ghost_chain,
                     const SendPtrs& send, uint32_t* fold_start, uint32_t* fold_list,
                     uint32_t* host_bs = nullptr);
+// The columns of ghosts [nlocal, nlocal + nghost) from their roots.
+void launch_make_ghosts(cudaStream_t st, uint64_t nlocal, uint64_t nghost, const AtomCols& c,
+                        const uint32_t* root, const uint32_t* chain, const SwapConst& sc);
 // forward_comm: every ghost from its root local atom through its swap chain
 void launch_forward(cudaStream_t st, uint64_t nlocal, uint64_t nghost, const AtomCols& c,
                     const uint32_t* ghost_root, const uint32_t* ghost_chain, const SwapConst& sc,

@@ -933,7 +933,7 @@ int phase_borders_defer(soil_sys* s, bool defer) {
     border_setup(s, bds);
     TRY(borders_reserve(s));
     const int mask = pbc_mask(s);
-    defer = defer && mask == 7;
+    defer = defer && mask == 7 && s->local_cells_valid;  // the build then bins only the ghosts
     uint32_t* hb = defer ? s->hword + kBorderStateWords : s->hword;
     const BorderPass bp = border_pass(bds);
     unsigned periodic_swaps = 0;
@@ -958,6 +958,7 @@ int phase_borders_defer(soil_sys* s, bool defer) {
             CK(cudaMemcpyAsync(hb, s->bstate.p, kBorderStateWords * 4, cudaMemcpyDeviceToHost,
                                s->st));
         if (defer) {
+            // the ghosts' columns are written by the neighbor build's binning
             for (int d = 0; d < 3; ++d) s->pending_bds[d] = bds[d];
             s->borders_pending = true;
             return SOIL_OK;
@@ -968,6 +969,9 @@ int phase_borders_defer(soil_sys* s, bool defer) {
         TRY(grow_atoms(s, (uint64_t)hb[3] + 1024, s->nlocal));  // hb[3]: atoms incl. all ghosts
     }
     TRY(borders_done(s, hb, bds));
+    launch_make_ghosts(s->st, s->nlocal, s->nghost, s->A, s->ghost_root.p, s->ghost_chain.p,
+                       swap_const(s));
+    TRY(check_launch(s));
     if (mask == 7) return SOIL_OK;
     // A swap with no neighbor (non-periodic axis) still packs the atoms at its
     // face, scanning the locals and the ghosts of the earlier axes
@@ -1085,6 +1089,18 @@ int borders_done(soil_sys* s, const uint32_t* hb, const BorderDim bds[3]) {
     for (int d = 0; d < 3; ++d)
         if ((mask & (1 << d)) && bds[d].thresh_lo > bds[d].thresh_hi) s->few_images = false;
     return SOIL_OK;
+}
+
+// The swap shifts of a border pass that is not read back yet.
+SwapConst swap_const_of(const BorderDim bds[3]) {
+    SwapConst sc;
+    for (int dim = 0; dim < 3; ++dim)
+        for (int sw = 0; sw < 2; ++sw)
+            for (int d = 0; d < 3; ++d) {
+                sc.off[2 * dim + sw][d] = bds[dim].shift[sw][d];
+                sc.voff[2 * dim + sw][d] = bds[dim].vshift[sw][d];
+            }
+    return sc;
 }
 
 SwapConst swap_const(const soil_sys* s) {
@@ -1405,9 +1421,16 @@ int phase_neighbor(soil_sys* s) {
     TRY(counts_zero(s, nc));
     const Grid gr = grid_of(s);
     const bool after_sort = s->local_cells_valid;
+    GhostMake make;  // the ghosts of a border pass still pending
+    if (pend) {
+        make.root = s->ghost_root.p;
+        make.chain = s->ghost_chain.p;
+        make.sc = swap_const_of(s->pending_bds);
+        make.forces = builtin_consumer(s) ? 0 : 1;  // it overwrites every force of the step
+    }
     if (after_sort)  // reuse the sort's local cells (neighbor.rs:1049-1066)
         launch_cells_reuse(s->st, nl, total, s->A, gr, s->sorted_local_cell.p, s->atom_cell.p,
-                           s->cell_counts.p, n_dev);
+                           s->cell_counts.p, n_dev, pend ? &make : nullptr);
     else
         launch_cells(s->st, 0, total, s->A, gr, s->atom_cell.p, s->cell_counts.p, n_dev);
     s->local_cells_valid = false;
