@@ -462,9 +462,11 @@ struct FillGuard {
     uint32_t* pub_total = nullptr;
     const DevFlags* flags = nullptr;
     DevFlags* pub_flags = nullptr;
+    const uint32_t* over = nullptr;  // when given, a ghost overflow keeps it shut too
 };
 __device__ __forceinline__ bool guard_open(const FillGuard& g) {
     if (!g.total) return true;
+    if (g.over && *g.over) return false;
     return (uint64_t)*g.total + 1 <= g.cap && *g.err == 0u;
 }
 __device__ __forceinline__ void guard_publish(const FillGuard& g) {
@@ -558,9 +560,13 @@ struct ForceCsr {
     const uint32_t* order;
     const double* pk;  // packed (x, y, z, r) records, current; NULL: the columns
 };
-// trip: the launch does nothing when *trip is set (LightStep).
+// trip: the launch does nothing when *trip is set (LightStep).  guard: nor
+// when the guard is shut (a consumer queued before the pair total is known).
+// few_images: no local has more than 7 images (small systems then take 8 lanes
+// per root).
 void launch_force_csr(cudaStream_t st, const ForceCsr& q, const AtomCols& c, const PlaneList& rev,
-                      bool fold, const uint32_t* trip = nullptr);
+                      bool fold, bool few_images, const uint32_t* trip = nullptr,
+                      const FillGuard* guard = nullptr);
 // order[b + k] for every block of kBlock roots: the block's roots sorted by
 // their entry count (their own and their images' in-list and row lengths),
 // ties in index order.

@@ -1064,6 +1064,7 @@ int borders_arrays(soil_sys* s) {
 
 // Swap records and ghost count from a finished pass (hb: its border state),
 // and room for the reverse-comm fold program.
+bool few_images_of(const soil_sys* s, const BorderDim bds[3]);
 int borders_done(soil_sys* s, const uint32_t* hb, const BorderDim bds[3]) {
     for (int dim = 0; dim < 3; ++dim) {
         const uint64_t recv_lo = hb[dim], n_lo = hb[4 + dim], n_hi = hb[7 + dim];
@@ -1082,13 +1083,17 @@ int borders_done(soil_sys* s, const uint32_t* hb, const BorderDim bds[3]) {
     s->last_nghost = s->nghost;
     s->border_gen += 1;
     s->nswaps = kNumSwaps;
-    // A local has images on both sides of a periodic dim only when the two
-    // face slabs overlap; otherwise it has at most 7 images.
-    const int mask = pbc_mask(s);
-    s->few_images = true;
-    for (int d = 0; d < 3; ++d)
-        if ((mask & (1 << d)) && bds[d].thresh_lo > bds[d].thresh_hi) s->few_images = false;
+    s->few_images = few_images_of(s, bds);
     return SOIL_OK;
+}
+
+// A local has images on both sides of a periodic dim only when the two face
+// slabs overlap; otherwise it has at most 7 images.
+bool few_images_of(const soil_sys* s, const BorderDim bds[3]) {
+    const int mask = pbc_mask(s);
+    for (int d = 0; d < 3; ++d)
+        if ((mask & (1 << d)) && bds[d].thresh_lo > bds[d].thresh_hi) return false;
+    return true;
 }
 
 // The swap shifts of a border pass that is not read back yet.
@@ -1300,7 +1305,7 @@ int launch_consumer(soil_sys* s, bool fold, const uint32_t* trip = nullptr) {
         zero_planes_of(s, SOIL_COL_REVERSE, rev.idx, &rev.n);
         ForceCsr q;
         TRY(csr_with_order(s, &q));
-        launch_force_csr(s->st, q, s->A, rev, fold, trip);
+        launch_force_csr(s->st, q, s->A, rev, fold, s->few_images, trip);
         return check_launch(s);
     }
     if (!seq_consumer(s) || variant == SOIL_FORCE_GATHER) {
@@ -1407,7 +1412,17 @@ float pair_eps(const soil_sys* s) {
     return (float)(1e-6 * (1.0 + s->cached_max_cutoff) + 4e-7 * M);
 }
 
+int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed);
 int phase_neighbor(soil_sys* s) {
+    bool consumed;
+    return phase_neighbor_with(s, false, &consumed);
+}
+
+// consumer_next: the built-in consumer (with its fold when newton) is all that
+// follows in this step, so it goes in before the host waits for the pair
+// total, guarded like pass 2; *consumed: it did and ran.
+int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
+    *consumed = false;
     if (s->state != FULL_REBUILD) return SOIL_OK;
     TRY(neighbor_plan(s));
     const uint64_t nl = s->nlocal;
@@ -1554,6 +1569,18 @@ int phase_neighbor(soil_sys* s) {
         CK(cudaEventRecord(s->ev_counts, s->st));
         if (with_in)
             launch_segsort_split(s->st, total, s->in_start.p, s->in_list.p, s->in_split.p, &guard);
+        if (consumer_next) {
+            timer_end(s, T_NEIGHBOR);
+            timer_begin(s, T_FORCE);
+            FillGuard open = guard;
+            open.over = pend ? s->bstate.p + 10 : nullptr;
+            PlaneList rev;
+            zero_planes_of(s, SOIL_COL_REVERSE, rev.idx, &rev.n);
+            launch_force_csr(s->st, csr_args(s), s->A, rev, s->newton,
+                             pend ? few_images_of(s, s->pending_bds) : s->few_images, nullptr, &open);
+            timer_end(s, T_FORCE);
+            *consumed = true;
+        }
     } else {
         CK(cudaMemcpyAsync(&s->hword[0], s->offsets.p + nl, 4, cudaMemcpyDeviceToHost, s->st));
         CK(cudaMemcpyAsync(s->hflags, s->dflags, sizeof(DevFlags), cudaMemcpyDeviceToHost, s->st));
@@ -1570,6 +1597,7 @@ int phase_neighbor(soil_sys* s) {
             TRY(grow_atoms(s, (uint64_t)hb[3] + 1024, s->nlocal));
             s->state = FULL_REBUILD;
             TRY(phase_borders_defer(s, false));
+            *consumed = false;
             return phase_neighbor(s);
         }
         TRY(borders_done(s, hb, s->pending_bds));
@@ -1581,6 +1609,7 @@ int phase_neighbor(soil_sys* s) {
     if (s->hflags->error)
         return fail(s->ctx, SOIL_ERR_INVALID, "neighbor stencil left the bin grid (atom outside the ghost layers)");
     if (!early || np + 1 > guard.cap) {  // the early pass did not run: again, into room for np
+        *consumed = false;
         TRY(ensure(s, s->indices, np + 1, 0, pair_room(np)));
         if (with_in) {
             TRY(ensure(s, s->in_list, np + 1, 0, pair_room(np)));
@@ -1600,6 +1629,14 @@ int phase_neighbor(soil_sys* s) {
     }
     // the grouped sequences are built when a consumer kernel first needs them
     return SOIL_OK;
+}
+
+// Whether the step's consumer is the plain CSR walk, which needs nothing of
+// the host once the lists are built (no packed records, no root order).
+bool consumer_goes_early(const soil_sys* s) {
+    if (!builtin_consumer(s) || force_variant() != SOIL_FORCE_CSR || packed_on()) return false;
+    const char* env = std::getenv("SOIL_ROOT_ORDER");
+    return !env || std::atoi(env) != 1;
 }
 
 int make_view(soil_sys* s, soil_dev_view* v) {
@@ -1868,14 +1905,17 @@ int step_rest(soil_sys* s, const StepPlan& p, bool last) {
     if (s->state == COMMUNICATE_ONLY && !p.fwd_fused) TRY(forward_comm(s, p.fused_zero));
     timer_end(s, T_FORWARD);
     timer_begin(s, T_NEIGHBOR);
-    TRY(phase_neighbor(s));
+    bool consumed = false;
+    TRY(phase_neighbor_with(s, consumer_goes_early(s), &consumed));
     timer_end(s, T_NEIGHBOR);
     // With newton, the grouped consumer folds ghost forces into their roots
     // in the same kernel (reverse_send_force's fold order); otherwise the
     // force and reverse-comm phases run apart.
     const bool fold_fused = consumer_folds(s);
-    timer_begin(s, T_FORCE);
-    if (fold_fused) {
+    if (!consumed) timer_begin(s, T_FORCE);
+    if (consumed) {
+        if (fold_fused) s->reverse_gen = s->border_gen;
+    } else if (fold_fused) {
         TRY(launch_consumer(s, true));
         s->reverse_gen = s->border_gen;
     } else {
