@@ -19,7 +19,10 @@
 //     evaluate G entries at a time and every lane adds the results in entry
 //     order (shuffles), so the sums are those of the one-thread walk.  Image
 //     forces go to shared memory and are folded by the group's first lane in
-//     fold_root's order.
+//     fold_root's order; with 8 lanes and at most 7 images per root, lane j
+//     keeps its j-th image's position and force sum in registers instead and
+//     the fold is a few shuffles (FEW: the roots at the box's corners, with
+//     seven images, set the time of a step).
 //   - Positions are exchanged as packed (x, y, z, r) records in two buffers
 //     used in turn: a step reads one while the next step's integration, by
 //     the same threads, writes the other.  One grid barrier per step, not
@@ -40,7 +43,7 @@
 //
 // Measured per light step against one thread per root walking the CSR with
 // its images in series, columns in global memory and two barriers a step:
-// 5.6 against 22 us on 1,000 atoms, 13 against 32 us on 65,537.
+// 3.2 against 22 us on 1,000 atoms, 11 against 32 us on 65,537.
 #include <cuda/atomic>
 
 #include "device_ops.cuh"
@@ -110,6 +113,39 @@ struct StepsSmem {
     uint8_t* eown;   // item of each entry: 0 the root, j its j-th image
 };
 
+// What only the integration needs of a thread's atom: in registers, or (PARK)
+// in shared memory where 1,024 threads leave 64 registers each.
+template <bool PARK>
+struct Parked {
+    double vx, vy, vz, h, lx, ly, lz;
+    __device__ __forceinline__ void bind(double*) {}
+    __device__ __forceinline__ Parked& get() { return *this; }
+    __device__ __forceinline__ void put(const Parked&) {}
+};
+template <>
+struct Parked<true> {
+    double* p;  // this thread's, one per kind every blockDim.x
+    __device__ __forceinline__ void bind(double* base) { p = base + threadIdx.x; }
+    __device__ __forceinline__ Parked<false> get() const {
+        const unsigned n = blockDim.x;
+        return {p[0], p[n], p[2 * n], p[3 * n], p[4 * n], p[5 * n], p[6 * n]};
+    }
+    __device__ __forceinline__ void put(const Parked<false>& v) {
+        const unsigned n = blockDim.x;
+        p[0] = v.vx;
+        p[n] = v.vy;
+        p[2 * n] = v.vz;
+    }
+    __device__ __forceinline__ void set(const Parked<false>& v) {
+        const unsigned n = blockDim.x;
+        put(v);
+        p[3 * n] = v.h;
+        p[4 * n] = v.lx;
+        p[5 * n] = v.ly;
+        p[6 * n] = v.lz;
+    }
+};
+
 __device__ StepsSmem carve(unsigned char* p, uint32_t e, uint32_t m) {
     StepsSmem s;
     s.fimg = reinterpret_cast<double*>(p);
@@ -125,6 +161,7 @@ __device__ StepsSmem carve(unsigned char* p, uint32_t e, uint32_t m) {
 
 constexpr size_t kBytesPerImage = 3 * 8 + 8 + 4 + 4 + 2 + 2;
 constexpr size_t kBytesPerEntry = 4 + 1;
+constexpr size_t kBytesParked = 7 * 8;
 
 // Position (or velocity) of an image: its root's plus its chain's offsets, in
 // chain order (forward_images).
@@ -143,12 +180,15 @@ __device__ __forceinline__ void shift_chain(uint32_t code, const double (*off)[3
 
 // FOLD: newton, with the reverse fold; else only locals receive and the
 // ghosts' forces are zero.
-template <int G, bool FOLD, int TMAX>
+template <int G, bool FOLD, int TMAX, bool FEW>
 __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ StepsArgs a) {
+    static_assert(!FEW || G == 8, "an item per lane");
+    constexpr bool kPark = TMAX > 256;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ Word s_seen;
     __shared__ int s_ok;
-    const StepsSmem sm = carve(smem_raw, a.ent_cap, a.img_cap);
+    const StepsSmem sm =
+        carve(smem_raw + (kPark ? blockDim.x * kBytesParked : 0), a.ent_cap, a.img_cap);
     const AtomCols& c = a.c;
     const uint64_t nl = a.nlocal;
     const uint32_t g = threadIdx.x & (G - 1);
@@ -180,6 +220,10 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
     const uint64_t at0 = __shfl_sync(0xffffffffu, at, 0, G);
     const uint32_t eb = (uint32_t)at0, ib = (uint32_t)(at0 >> 32);
     if (over) nimg = cnt = nin = nrow = npre = 0;
+    // FEW: this lane's image (lane 0: the root itself)
+    uint32_t my_gi = 0, my_code = 0, my_par = 0;
+    double my_rad = 0.0;
+    const bool has_item = valid && g <= nimg;
     const uint32_t ee = eb + cnt, e0 = eb + nin + nrow;
     for (uint32_t k = g; k < nin + nrow; k += G) {
         sm.ent[eb + k] = k < npre          ? a.fc.in_list[qs + k]
@@ -198,42 +242,62 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
             }
             k0 += n;
         }
-        if (g == 0) {
+        if (g == (FEW ? q + 1 : 0)) {
             for (int p = 0; p < a.fw.fwd.n; ++p)  // the first step's forward planes
                 c.planes[a.fw.fwd.idx[p]][nl + gi] = c.planes[a.fw.fwd.idx[p]][t];
-            sm.ig[ib + q] = gi;
-            sm.iend[ib + q] = k0;
-            sm.code[ib + q] = (uint16_t)a.fw.chain[gi];
-            sm.irad[ib + q] = a.fc.rad[nl + gi];
-            uint16_t par = kRootParent;
+            const uint32_t code = a.fw.chain[gi];
+            const double rad = a.fc.rad[nl + gi];
             const uint32_t o = (uint32_t)c.origin[nl + gi];
+            uint32_t par = kRootParent;
             if (o >= nl)  // an image one chain shorter of the same root
                 for (uint32_t r = 0; r < nimg; ++r)
-                    if (a.fc.fold_list[f0 + r] == o - (uint32_t)nl) par = (uint16_t)(ib + r);
-            sm.par[ib + q] = par;
+                    if (a.fc.fold_list[f0 + r] == o - (uint32_t)nl) par = FEW ? r + 1 : ib + r;
+            if (FEW) {
+                my_gi = gi;
+                my_code = code;
+                my_rad = rad;
+                my_par = par == kRootParent ? 0 : par;
+            } else {
+                sm.ig[ib + q] = gi;
+                sm.iend[ib + q] = k0;
+                sm.code[ib + q] = (uint16_t)code;
+                sm.irad[ib + q] = rad;
+                sm.par[ib + q] = (uint16_t)par;
+            }
         }
     }
     const uint32_t rounds = __reduce_max_sync(0xffffffffu, (cnt + G - 1) / G);
 
+    const uint32_t most_images = FEW ? __reduce_max_sync(0xffffffffu, nimg) : 0u;
+
     // ---- the group's atom ------------------------------------------------------
-    double x = 0, y = 0, z = 0, vx = 0, vy = 0, vz = 0, Rx = 0, Ry = 0, Rz = 0, h = 0, r = 0;
-    double lx = 0, ly = 0, lz = 0;
-    if (valid) {
-        h = 0.5 * a.dt * c.inv_mass[t];
-        x = c.x[t];
-        y = c.y[t];
-        z = c.z[t];
-        vx = c.vx[t];
-        vy = c.vy[t];
-        vz = c.vz[t];
-        Rx = c.fx[t];
-        Ry = c.fy[t];
-        Rz = c.fz[t];
-        r = a.fc.rad[t];
-        lx = a.ck.lbx[t];
-        ly = a.ck.lby[t];
-        lz = a.ck.lbz[t];
+    double x = 0, y = 0, z = 0, Rx = 0, Ry = 0, Rz = 0, r = 0;
+    Parked<kPark> parked;
+    parked.bind(reinterpret_cast<double*>(smem_raw));
+    {
+        Parked<false> w{};
+        if (valid) {
+            w.h = 0.5 * a.dt * c.inv_mass[t];
+            w.vx = c.vx[t];
+            w.vy = c.vy[t];
+            w.vz = c.vz[t];
+            w.lx = a.ck.lbx[t];
+            w.ly = a.ck.lby[t];
+            w.lz = a.ck.lbz[t];
+            x = c.x[t];
+            y = c.y[t];
+            z = c.z[t];
+            Rx = c.fx[t];
+            Ry = c.fy[t];
+            Rz = c.fz[t];
+            r = a.fc.rad[t];
+        }
+        if constexpr (kPark) parked.set(w);
+        else parked = w;
     }
+    if (g == 0) my_rad = r;
+    double ix = 0, iy = 0, iz = 0;  // FEW: this lane's item
+    double Ix = 0, Iy = 0, Iz = 0;  // FEW: its force
     __syncwarp();
 
     uint64_t done = 0;
@@ -242,18 +306,32 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
         // integrate (the previous step's final half-kick first), check, and
         // publish the new positions
         double* const rec = a.rec[step & 1];
-        initial_regs(h, a.dt, step > 0 || a.first_fused, Rx, Ry, Rz, vx, vy, vz, x, y, z);
-        const bool hit = valid && check_moved_at(a.ck, x, y, z, lx, ly, lz);
-        if (lead) put_pk(rec, t, x, y, z, r);
-        for (uint32_t q = g; q < nimg; q += G) {
-            double px = x, py = y, pz = z;
-            shift_chain(sm.code[ib + q], a.fw.sc.off, px, py, pz);
-            put_pk(rec, nl + sm.ig[ib + q], px, py, pz, sm.irad[ib + q]);
+        bool hit;
+        {
+            auto w = parked.get();
+            initial_regs(w.h, a.dt, step > 0 || a.first_fused, Rx, Ry, Rz, w.vx, w.vy, w.vz, x, y, z);
+            hit = valid && check_moved_at(a.ck, x, y, z, w.lx, w.ly, w.lz);
+            if constexpr (kPark) parked.put(w);
+            else parked = w;
+        }
+        if (FEW) {
+            ix = x;
+            iy = y;
+            iz = z;
+            shift_chain(my_code, a.fw.sc.off, ix, iy, iz);  // the root's chain is empty
+            if (has_item) put_pk(rec, g ? nl + my_gi : t, ix, iy, iz, my_rad);
+        } else {
+            if (lead) put_pk(rec, t, x, y, z, r);
+            for (uint32_t q = g; q < nimg; q += G) {
+                double px = x, py = y, pz = z;
+                shift_chain(sm.code[ib + q], a.fw.sc.off, px, py, pz);
+                put_pk(rec, nl + sm.ig[ib + q], px, py, pz, sm.irad[ib + q]);
+            }
         }
         if (a.rev.n && step > 0 && lead)  // forward planes a fold has changed
-            for (uint32_t q = 0; q < nimg; ++q)
+            for (uint32_t q = f0; q < f0 + nimg; ++q)
                 for (int p = 0; p < a.fw.fwd.n; ++p)
-                    c.planes[a.fw.fwd.idx[p]][nl + sm.ig[ib + q]] = c.planes[a.fw.fwd.idx[p]][t];
+                    c.planes[a.fw.fwd.idx[p]][nl + a.fc.fold_list[q]] = c.planes[a.fw.fwd.idx[p]][t];
         const int any = __syncthreads_or(hit);
         if (threadIdx.x == 0) {
             const Word add = 1u + (any ? kTripUnit : 0u) + (over ? kOverUnit : 0u);
@@ -281,7 +359,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
         // the consumer: G entries at a time, added in entry order
         double Fx = 0.0, Fy = 0.0, Fz = 0.0;
         uint32_t item = 0, iend = e0;
-        auto close = [&] {  // the item is complete
+        auto close = [&] {  // (not FEW) the item is complete
             if (item == 0) {
                 Rx = Fx;
                 Ry = Fy;
@@ -296,41 +374,68 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
             ++item;
             iend = item <= nimg ? sm.iend[ib + item - 1] : 0xffffffffu;
         };
+        // (the next entry's record loaded one trip ahead measured slower: 17.2
+        // against 15.4 us a step on 140,000 atoms)
         for (uint32_t rd = 0; rd < rounds; ++rd) {
             const uint32_t k = eb + rd * G + g;
             double fx = 0.0, fy = 0.0, fz = 0.0;
             bool touch = false;
+            uint32_t own = 0;
+            double4 q;
             if (k < ee) {
-                const double4 q = ld_pk(rec, sm.ent[k]);
-                const uint32_t own = sm.eown[k];
-                double px = x, py = y, pz = z, pr = r;
-                if (FOLD && own) {
-                    shift_chain(sm.code[ib + own - 1], a.fw.sc.off, px, py, pz);
-                    pr = sm.irad[ib + own - 1];
-                }
-                touch = pair_force(px, py, pz, pr, q.x, q.y, q.z, q.w, a.fc.K, fx, fy, fz);
+                own = FOLD ? sm.eown[k] : 0u;
+                q = ld_pk(rec, sm.ent[k]);
             }
+            double px = x, py = y, pz = z, pr = r;
+            if (FEW && FOLD) {
+                px = __shfl_sync(0xffffffffu, ix, own, 8);
+                py = __shfl_sync(0xffffffffu, iy, own, 8);
+                pz = __shfl_sync(0xffffffffu, iz, own, 8);
+                pr = __shfl_sync(0xffffffffu, my_rad, own, 8);
+            } else if (FOLD && own) {
+                shift_chain(sm.code[ib + own - 1], a.fw.sc.off, px, py, pz);
+                pr = sm.irad[ib + own - 1];
+            }
+            if (k < ee) touch = pair_force(px, py, pz, pr, q.x, q.y, q.z, q.w, a.fc.K, fx, fy, fz);
             const unsigned hits = __ballot_sync(0xffffffffu, touch) >> ((threadIdx.x & 31) & ~(G - 1));
 #pragma unroll
             for (int j = 0; j < G; ++j) {
                 const double ex = G > 1 ? __shfl_sync(0xffffffffu, fx, j, G) : fx;
                 const double ey = G > 1 ? __shfl_sync(0xffffffffu, fy, j, G) : fy;
                 const double ez = G > 1 ? __shfl_sync(0xffffffffu, fz, j, G) : fz;
-                const uint32_t kk = eb + rd * G + j;
-                if (kk < ee) {
-                    if (FOLD)
+                // FEW: each lane sums its own item (the shuffle is every lane's)
+                const uint32_t item_j = FEW && FOLD ? __shfl_sync(0xffffffffu, own, j, G) : g;
+                const bool add = ((hits >> j) & 1u) && item_j == g;
+                if (FOLD && !FEW) {
+                    const uint32_t kk = eb + rd * G + j;
+                    if (kk < ee)
                         while (kk >= iend) close();
-                    if ((hits >> j) & 1u) {
-                        Fx = Fx + ex;
-                        Fy = Fy + ey;
-                        Fz = Fz + ez;
-                    }
+                }
+                if (add) {
+                    Fx = Fx + ex;
+                    Fy = Fy + ey;
+                    Fz = Fz + ez;
                 }
             }
         }
-        if (FOLD) {
+        if (FEW && FOLD) {  // fold_root's order: image by image onto its parent's lane
+            for (uint32_t j = 1; j <= most_images; ++j) {
+                const double ex = __shfl_sync(0xffffffffu, Fx, j, 8);
+                const double ey = __shfl_sync(0xffffffffu, Fy, j, 8);
+                const double ez = __shfl_sync(0xffffffffu, Fz, j, 8);
+                const uint32_t p = __shfl_sync(0xffffffffu, my_par, j, 8);
+                if (j <= nimg && p == g) {
+                    Fx = Fx + ex;
+                    Fy = Fy + ey;
+                    Fz = Fz + ez;
+                }
+            }
+            Ix = Fx;
+            Iy = Fy;
+            Iz = Fz;
+        } else if (FOLD) {
             while (item <= nimg) close();
-            if (nimg && g == 0) {  // fold_root's order
+            if (nimg && g == 0)  // fold_root's order
                 for (uint32_t q = ib; q < ib + nimg; ++q) {
                     const double* f = sm.fimg + 3 * q;
                     const uint32_t p = sm.par[q];
@@ -344,43 +449,50 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
                         o[1] = o[1] + f[1];
                         o[2] = o[2] + f[2];
                     }
-                    for (int w = 0; w < a.rev.n; ++w) {
-                        double* pl = c.planes[a.rev.idx[w]];
-                        const uint64_t to = p == kRootParent ? t : nl + sm.ig[p];
-                        pl[to] = pl[to] + pl[nl + sm.ig[q]];
-                    }
+                }
+        } else {
+            Rx = Fx;
+            Ry = Fy;
+            Rz = Fz;
+        }
+        if (FOLD && G > 1) {  // the root's sum to the whole group
+            __syncwarp();
+            Rx = __shfl_sync(0xffffffffu, FEW ? Fx : Rx, 0, G);
+            Ry = __shfl_sync(0xffffffffu, FEW ? Fy : Ry, 0, G);
+            Rz = __shfl_sync(0xffffffffu, FEW ? Fz : Rz, 0, G);
+        }
+        if (FOLD && a.rev.n && lead)
+            for (uint32_t q = f0; q < f0 + nimg; ++q) {
+                const uint64_t gh = nl + a.fc.fold_list[q];
+                const uint32_t o = (uint32_t)c.origin[gh];
+                for (int w = 0; w < a.rev.n; ++w) {
+                    double* pl = c.planes[a.rev.idx[w]];
+                    pl[o] = pl[o] + pl[gh];
                 }
             }
-            if (G > 1) {
-                __syncwarp();
-                Rx = __shfl_sync(0xffffffffu, Rx, 0, G);
-                Ry = __shfl_sync(0xffffffffu, Ry, 0, G);
-                Rz = __shfl_sync(0xffffffffu, Rz, 0, G);
-            }
-        } else {
-            close();
-        }
         ++done;
     }
 
     // ---- the columns -----------------------------------------------------------
+    const auto w = parked.get();
     if (lead) {
         c.x[t] = x;
         c.y[t] = y;
         c.z[t] = z;
-        c.vx[t] = vx;
-        c.vy[t] = vy;
-        c.vz[t] = vz;
+        c.vx[t] = w.vx;
+        c.vy[t] = w.vy;
+        c.vz[t] = w.vz;
         c.fx[t] = Rx;
         c.fy[t] = Ry;
         c.fz[t] = Rz;
     }
     __syncwarp();
-    for (uint32_t q = g; q < nimg; q += G) {
-        const uint64_t gi = nl + sm.ig[ib + q];
-        double px = x, py = y, pz = z, ux = vx, uy = vy, uz = vz;
-        shift_chain(sm.code[ib + q], a.fw.sc.off, px, py, pz);
-        shift_chain(sm.code[ib + q], a.fw.sc.voff, ux, uy, uz);
+    for (uint32_t q = FEW ? g - 1 : g; q < nimg; q += G) {  // (FEW, lane 0: no image)
+        const uint64_t gi = nl + (FEW ? my_gi : sm.ig[ib + q]);
+        const uint32_t code = FEW ? my_code : sm.code[ib + q];
+        double px = x, py = y, pz = z, ux = w.vx, uy = w.vy, uz = w.vz;
+        shift_chain(code, a.fw.sc.off, px, py, pz);
+        shift_chain(code, a.fw.sc.voff, ux, uy, uz);
         c.x[gi] = px;
         c.y[gi] = py;
         c.z[gi] = pz;
@@ -388,9 +500,10 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
         c.vy[gi] = uy;
         c.vz[gi] = uz;
         if (done) {
-            c.fx[gi] = FOLD ? sm.fimg[3 * (ib + q)] : 0.0;
-            c.fy[gi] = FOLD ? sm.fimg[3 * (ib + q) + 1] : 0.0;
-            c.fz[gi] = FOLD ? sm.fimg[3 * (ib + q) + 2] : 0.0;
+            const double* f = FEW ? nullptr : sm.fimg + 3 * (ib + q);
+            c.fx[gi] = !FOLD ? 0.0 : FEW ? Ix : f[0];
+            c.fy[gi] = !FOLD ? 0.0 : FEW ? Iy : f[1];
+            c.fz[gi] = !FOLD ? 0.0 : FEW ? Iz : f[2];
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -402,9 +515,9 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
 
 namespace {
 
-template <int G, int TMAX>
+template <int G, int TMAX, bool FEW = false>
 const void* steps_kernel(bool fold) {
-    return fold ? (const void*)k_steps<G, true, TMAX> : (const void*)k_steps<G, false, TMAX>;
+    return fold ? (const void*)k_steps<G, true, TMAX, FEW> : (const void*)k_steps<G, false, TMAX, FEW>;
 }
 
 // Lanes per root: the widest group with the whole system in one CTA of at
@@ -432,22 +545,26 @@ bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, Ste
     uint64_t img = roots + roots / 2 + 64, ent;
     if (roomy) img = 3 * roots;
     if (img > most) img = most;
-    const uint64_t budget = 220 * 1024;
+    const uint64_t park = threads > 256 ? threads * kBytesParked : 0;
+    const uint64_t budget = 220 * 1024 - park;
     const uint64_t fit = (budget - img * kBytesPerImage) / kBytesPerEntry;
     const double mean = 2.0 * (double)npairs / (double)nlocal * (double)roots;
     ent = roomy ? fit : (uint64_t)(1.3 * mean) + 16 * roots / 8 + 256;
     if (ent > fit) ent = fit;
     p->ent_cap = (uint32_t)(ent & ~7ull);
     p->img_cap = (uint32_t)img;
-    p->smem = img * kBytesPerImage + ent * kBytesPerEntry + 16;
+    p->smem = park + img * kBytesPerImage + ent * kBytesPerEntry + 16;
     return true;
 }
 
-cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold) {
+cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold,
+                         bool few_images) {
     note_launch();
     const void* k;
-    if (p.group == 8 && p.threads <= 256) k = steps_kernel<8, 256>(fold);
-    else if (p.group == 8) k = steps_kernel<8, 1024>(fold);
+    if (p.group == 8 && p.threads <= 256)
+        k = few_images ? steps_kernel<8, 256, true>(fold) : steps_kernel<8, 256>(fold);
+    else if (p.group == 8)
+        k = few_images ? steps_kernel<8, 1024, true>(fold) : steps_kernel<8, 1024>(fold);
     else if (p.group == 4) k = steps_kernel<4, 1024>(fold);
     else if (p.group == 2) k = steps_kernel<2, 1024>(fold);
     else k = steps_kernel<1, 1024>(fold);

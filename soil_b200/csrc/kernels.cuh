@@ -607,8 +607,9 @@ struct StepsShape {
 // The shape for a system on `sms` SMs (roomy: with all the shared memory);
 // false when it has too many atoms for one resident launch.
 bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, StepsShape* p);
-// fold: newton.
-cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold);
+// fold: newton.  few_images: no root has more than 7 images.
+cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold,
+                         bool few_images);
 
 // ---- light steps without a consumer (k_flight.cu) -----------------------------
 constexpr uint32_t kFlightMaxSteps = 4096;  // one launch stays short when nothing trips

@@ -2101,7 +2101,7 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, boo
         a.img_cap = shape.img_cap;
         a.epoch = s->steps_epoch;
         s->hword[2] = s->hword[3] = 0;
-        CK(launch_steps(s->st, a, shape, s->newton));
+        CK(launch_steps(s->st, a, shape, s->newton, s->few_images));
         TRY(sync(s));
         if (s->hword[2] == SOIL_STEPS_OVERFLOW) {
             s->steps_epoch += 1;
