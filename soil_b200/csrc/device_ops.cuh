@@ -794,6 +794,30 @@ __device__ __forceinline__ void sorted_view(const AtomCols& c, uint64_t m, uint3
     }
 }
 
+// Atom a in sorted slot m: the bin order, its inverse, the sorted record and
+// (of a local) the build position.
+__device__ __forceinline__ void put_sorted(const SortedViews& v, uint32_t m, uint32_t a) {
+    v.sorted[m] = a;
+    sorted_view(v.c, m, a, v.asi, v.sp, v.spf, v.origin[0], v.origin[1], v.origin[2], v.bp,
+                v.atom_in_w != 0);
+}
+
+// First ghost slot of cell c: behind its locals.
+__device__ __forceinline__ uint32_t ghost_slots(const uint32_t* start, const uint32_t* sort_start,
+                                                uint32_t c) {
+    return start[c] + (sort_start[c + 1] - sort_start[c]);
+}
+
+// Ghost g of cell c to its rank among the cell's ghosts (tmp: unordered).
+__device__ __forceinline__ void rank_ghost(const SortedViews& v, uint32_t g, uint32_t c,
+                                           const uint32_t* start, const uint32_t* sort_start,
+                                           const uint32_t* tmp) {
+    const uint32_t b = ghost_slots(start, sort_start, c), e = start[c + 1];
+    uint32_t rank = 0;
+    for (uint32_t j = b; j < e; ++j) rank += tmp[j] < g;
+    put_sorted(v, b + rank, g);
+}
+
 // Restore ascending order of one segment (the stable counting sort's last
 // step) and return how many of its items are below `pivot`: segments of up
 // to 8 items (nearly all: bins and transposed lists hold a few atoms) are

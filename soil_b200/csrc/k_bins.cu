@@ -223,51 +223,47 @@ void launch_scatter_consume(cudaStream_t st, uint64_t n, const uint32_t* cell,
                                                                           out, n_dev);
 }
 
-// The neighbor build's cells in one pass: the locals' cells from the sort
-// (local < nlocal), the others' from their positions; all counted.  MAKE: the
-// ghosts of a border pass just queued get their columns here.
+// The ghosts' cells, counted (the locals' are the sort's, in bin order).
+// MAKE: the ghosts of a border pass just queued get their columns here.
 template <bool MAKE>
-__global__ void __launch_bounds__(kBlock) k_cells_reuse(uint64_t nlocal, uint64_t n, AtomCols c,
-                                                        Grid gr, const uint32_t* local_cell,
-                                                        uint32_t* cell_out, uint32_t* counts,
-                                                        const uint32_t* n_dev, GhostMake mk) {
+__global__ void __launch_bounds__(kBlock) k_ghost_cells(uint64_t nlocal, uint64_t n, AtomCols c,
+                                                        Grid gr, uint32_t* cell_out,
+                                                        uint32_t* counts, const uint32_t* n_dev,
+                                                        GhostMake mk) {
     pdl_wait();  // launched with pdl_launch
     if (n_dev) {  // the count known only on the device (an upper bound in n)
         const uint64_t d = *n_dev;
         n = d < n ? d : n;
     }
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
+    for (uint64_t i0 = nlocal + (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
         const uint64_t i = i0 + threadIdx.x;
         const bool valid = i < n;
         uint32_t cell = 0;
         if (valid) {
-            if (i < nlocal) {
-                cell = local_cell[i];
-            } else if (MAKE) {
-                const double3 q =
-                    make_ghost(c, nlocal, i - nlocal, mk.root, mk.chain, mk.sc, mk.forces != 0);
-                cell = cell_of(gr, q.x, q.y, q.z);
-            } else {
-                cell = cell_of(gr, c.x[i], c.y[i], c.z[i]);
-            }
+            double3 q;
+            if (MAKE)
+                q = make_ghost(c, nlocal, i - nlocal, mk.root, mk.chain, mk.sc, mk.forces != 0);
+            else
+                q = make_double3(c.x[i], c.y[i], c.z[i]);
+            cell = cell_of(gr, q.x, q.y, q.z);
             cell_out[i] = cell;
         }
         aggregated_count(counts, cell, valid);
     }
 }
 
-void launch_cells_reuse(cudaStream_t st, uint64_t nlocal, uint64_t n, const AtomCols& c,
-                        const Grid& gr, const uint32_t* local_cell, uint32_t* cell_out,
-                        uint32_t* counts, const uint32_t* n_dev, const GhostMake* make) {
-    if (n == 0) return;
+void launch_ghost_cells(cudaStream_t st, uint64_t nlocal, uint64_t n, const AtomCols& c,
+                        const Grid& gr, uint32_t* cell_out, uint32_t* counts,
+                        const uint32_t* n_dev, const GhostMake* make) {
+    if (n <= nlocal) return;
     note_launch();
     if (make)
-        pdl_launch(k_cells_reuse<true>, grid_wave<k_cells_reuse<true>>(n), kBlock, 0, st, nlocal, n, c,
-                   gr, local_cell, cell_out, counts, n_dev, *make);
+        pdl_launch(k_ghost_cells<true>, grid_wave<k_ghost_cells<true>>(n - nlocal), kBlock, 0, st,
+                   nlocal, n, c, gr, cell_out, counts, n_dev, *make);
     else
-        pdl_launch(k_cells_reuse<false>, grid_wave<k_cells_reuse<false>>(n), kBlock, 0, st, nlocal, n,
-                   c, gr, local_cell, cell_out, counts, n_dev, GhostMake{});
+        pdl_launch(k_ghost_cells<false>, grid_wave<k_ghost_cells<false>>(n - nlocal), kBlock, 0, st,
+                   nlocal, n, c, gr, cell_out, counts, n_dev, GhostMake{});
 }
 
 __device__ __forceinline__ void clear_pair_counters(DevFlags* clear) {
@@ -278,28 +274,20 @@ __device__ __forceinline__ void clear_pair_counters(DevFlags* clear) {
     }
 }
 
-// Atom a in sorted slot m: the bin order, its inverse, the sorted record and
-// (of a local) the build position.
-__device__ __forceinline__ void put_sorted(const SortedViews& v, uint32_t m, uint32_t a) {
-    v.sorted[m] = a;
-    sorted_view(v.c, m, a, v.asi, v.sp, v.spf, v.origin[0], v.origin[1], v.origin[2], v.bp,
-                v.atom_in_w != 0);
-}
-
 // The neighbor build's bins right after a spatial sort of the same grid:
 // the locals are already in cell order (local i is entry i - sort_start[c]
 // of its cell c), so they take their slots directly, in front of their
-// cell's ghosts; only the ghosts are scattered and ranked.
-// One pass over all atoms: local i (its cell's locals are consecutive in
-// bin order already) straight to its slot, with its sorted record and build
-// position; ghost g of cell c into the ghost part of c's slots (after its
-// locals), in no particular order: counts[c] still holds c's locals and
-// ghosts, and only ghosts take from it.  (Writing the records here reads the
-// columns in order; a pass of its own over the sorted slots gathered them:
-// 26.6 against 29.6 us for place, rank and views on 1,048,576 atoms, 91
-// against 97 on 4,194,304.)
+// cell's ghosts; only the ghosts are counted, scattered and ranked, and a
+// cell starts at its sort start plus the ghosts before it.
+// One pass over all atoms: local i straight to its slot, with its sorted
+// record and build position; ghost g of cell c into the ghost part of c's
+// slots, in no particular order, taking the counts back to zero.  (Writing
+// the records here reads the columns in order; a pass of its own over the
+// sorted slots gathered them: 26.6 against 29.6 us for place, rank and views on
+// 1,048,576 atoms, 91 against 97 on 4,194,304.)
 __global__ void __launch_bounds__(kBlock) k_place_bins(uint64_t nl, uint64_t n,
                                                        const uint32_t* n_dev,
+                                                       const uint32_t* local_cell,
                                                        const uint32_t* cell,
                                                        const uint32_t* start,
                                                        const uint32_t* sort_start,
@@ -313,56 +301,45 @@ __global__ void __launch_bounds__(kBlock) k_place_bins(uint64_t nl, uint64_t n,
     }
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = cell[i];
-        if (i < nl)
+        if (i < nl) {
+            const uint32_t c = local_cell[i];
             put_sorted(v, start[c] + ((uint32_t)i - sort_start[c]), (uint32_t)i);
-        else
-            tmp[start[c] + atomicSub(&counts[c], 1u) - 1u] = (uint32_t)i;
+        } else {
+            const uint32_t c = cell[i];
+            tmp[ghost_slots(start, sort_start, c) + atomicSub(&counts[c], 1u) - 1u] = (uint32_t)i;
+        }
     }
 }
 
 // Each ghost at its rank among its cell's ghosts (ascending index).
-// The cells' counts (read by nothing after k_place_bins) go back to zero on
-// the way, for the next counting pass.
 __global__ void __launch_bounds__(kBlock) k_ghost_rank(uint64_t nl, uint64_t n,
                                                        const uint32_t* n_dev,
                                                        const uint32_t* cell,
                                                        const uint32_t* start,
                                                        const uint32_t* sort_start,
-                                                       const uint32_t* tmp, uint32_t* counts,
-                                                       uint64_t nc, SortedViews v) {
+                                                       const uint32_t* tmp, SortedViews v) {
     pdl_wait();  // launched with pdl_launch
     if (n_dev) {
         const uint64_t d = *n_dev;
         n = d < n ? d : n;
     }
-    for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < nc;
-         c += (uint64_t)gridDim.x * blockDim.x)
-        counts[c] = 0u;
     for (uint64_t g = nl + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n;
-         g += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = cell[g];
-        const uint32_t gb = start[c] + (sort_start[c + 1] - sort_start[c]), ge = start[c + 1];
-        uint32_t rank = 0;
-        for (uint32_t j = gb; j < ge; ++j) rank += tmp[j] < (uint32_t)g;
-        put_sorted(v, gb + rank, (uint32_t)g);
-    }
+         g += (uint64_t)gridDim.x * blockDim.x)
+        rank_ghost(v, (uint32_t)g, cell[g], start, sort_start, tmp);
 }
 
-bool launch_place_bins(cudaStream_t st, uint64_t nl, uint64_t n, uint64_t nc,
-                       const uint32_t* n_dev, const uint32_t* cell, const uint32_t* start,
+void launch_place_bins(cudaStream_t st, uint64_t nl, uint64_t n, const uint32_t* n_dev,
+                       const uint32_t* local_cell, const uint32_t* cell, const uint32_t* start,
                        const uint32_t* sort_start, uint32_t* counts, uint32_t* tmp,
                        const SortedViews& v) {
-    if (n == 0) return false;
+    if (n == 0) return;
     note_launch();
-    pdl_launch(k_place_bins, grid_wave<k_place_bins>(n), kBlock, 0, st, nl, n, n_dev, cell, start,
-               sort_start, counts, tmp, v);
-    if (n == nl) return false;
+    pdl_launch(k_place_bins, grid_wave<k_place_bins>(n), kBlock, 0, st, nl, n, n_dev, local_cell, cell,
+               start, sort_start, counts, tmp, v);
+    if (n == nl) return;
     note_launch();
-    const uint64_t rank_items = n - nl > nc ? n - nl : nc;  // ghosts, or cells to clear
-    pdl_launch(k_ghost_rank, grid_wave<k_ghost_rank>(rank_items), kBlock, 0, st, nl, n, n_dev, cell,
-               start, sort_start, tmp, counts, nc, v);
-    return true;
+    pdl_launch(k_ghost_rank, grid_wave<k_ghost_rank>(n - nl), kBlock, 0, st, nl, n, n_dev, cell, start,
+               sort_start, tmp, v);
 }
 
 // One thread per segment, sorted in place (in registers for up to 8 items,

@@ -30,12 +30,15 @@ __device__ __forceinline__ void load8(const uint32_t* in, uint64_t base, uint64_
 }
 
 // out[base + k] = pre + v[0] + ... + v[k - 1] for the items below n.
+// With add, plus add[base + k].
 __device__ __forceinline__ void store8_scan(uint32_t* out, uint64_t base, uint64_t n,
-                                            const uint32_t (&v)[kScanItems], uint32_t pre) {
+                                            const uint32_t (&v)[kScanItems], uint32_t pre,
+                                            const uint32_t* add = nullptr) {
     uint32_t o[kScanItems];
+    if (add) load8(add, base, n, o);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        o[k] = pre;
+        o[k] = add ? o[k] + pre : pre;
         pre += v[k];
     }
     if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(out + base) & 15u) == 0) {
@@ -56,6 +59,7 @@ struct ScanJobs {
     uint64_t n[2];
     uint32_t* partial[2];
     uint64_t ntiles[2];
+    const uint32_t* add;  // (scan 0) added to every output, n + 1 words; may be null
 };
 
 // This block's scan: its fields picked by selects (a parameter array indexed
@@ -67,6 +71,7 @@ struct ScanJob {
     uint32_t* partial;
     uint64_t ntiles;
     uint64_t tile;  // this block's tile of it
+    const uint32_t* add;
 };
 
 __device__ __forceinline__ ScanJob scan_job(const ScanJobs& J) {
@@ -78,6 +83,7 @@ __device__ __forceinline__ ScanJob scan_job(const ScanJobs& J) {
     s.partial = second ? J.partial[1] : J.partial[0];
     s.ntiles = second ? J.ntiles[1] : J.ntiles[0];
     s.tile = second ? blockIdx.x - J.ntiles[0] : blockIdx.x;
+    s.add = second ? nullptr : J.add;
     return s;
 }
 
@@ -121,7 +127,8 @@ __global__ void __launch_bounds__(kBlock) k_scan_partials(uint32_t* partial, uin
 }
 
 __global__ void __launch_bounds__(kBlock) k_scan_down(const uint32_t* in, uint32_t* out, uint64_t n,
-                                                      const uint32_t* partial, uint64_t ntiles) {
+                                                      const uint32_t* partial, uint64_t ntiles,
+                                                      const uint32_t* add) {
     __shared__ uint32_t tot;
     const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
@@ -130,8 +137,8 @@ __global__ void __launch_bounds__(kBlock) k_scan_down(const uint32_t* in, uint32
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) s += v[k];
     const uint32_t pre = block_exclusive_scan(s, &tot) + partial[blockIdx.x];
-    store8_scan(out, base, n, v, pre);
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = partial[ntiles];
+    store8_scan(out, base, n, v, pre, add);
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = partial[ntiles] + (add ? add[n] : 0u);
 }
 
 // Pass 2 without the one-CTA pass over the tile sums: each CTA adds up the
@@ -158,8 +165,8 @@ __global__ void __launch_bounds__(kBlock) k_scan_down_carry(ScanJobs J) {
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) s += v[k];
     const uint32_t pre = block_exclusive_scan(s, &tot) + carry;
-    store8_scan(q.out, base, n, v, pre);
-    if (t + 1 == q.ntiles && threadIdx.x == 0) q.out[n] = carry + tot;
+    store8_scan(q.out, base, n, v, pre, q.add);
+    if (t + 1 == q.ntiles && threadIdx.x == 0) q.out[n] = carry + tot + (q.add ? q.add[n] : 0u);
 }
 
 // One launch without any wait between CTAs: a CTA of 1,024 threads takes a
@@ -220,8 +227,9 @@ __global__ void __launch_bounds__(kDirectThreads) k_scan_direct(ScanJobs J) {
     for (int k = 0; k < kScanItems; ++k) s += v[k];
     const uint32_t in_tile = cta_exclusive_1024(s, &tot);  // its barrier covers `before`
     const uint32_t carry = __reduce_add_sync(0xffffffffu, before[threadIdx.x & 31]);
-    store8_scan(q.out, base, q.n, v, carry + in_tile);
-    if (q.tile + 1 == q.ntiles && threadIdx.x == 0) q.out[q.n] = carry + tot;
+    store8_scan(q.out, base, q.n, v, carry + in_tile, q.add);
+    if (q.tile + 1 == q.ntiles && threadIdx.x == 0)
+        q.out[q.n] = carry + tot + (q.add ? q.add[q.n] : 0u);
 }
 
 uint64_t scan_temp_words(uint64_t n) { return (n + kScanTile - 1) / kScanTile + 2; }
@@ -238,19 +246,21 @@ static ScanJobs one_job(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t*
 }
 
 void exclusive_scan_u32(cudaStream_t st, const uint32_t* in, uint32_t* out, uint64_t n,
-                        uint32_t* temp, uint64_t direct_max) {
+                        uint32_t* temp, uint64_t direct_max, const uint32_t* add) {
     const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
     if (ntiles == 0) {
         cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
         return;
     }
     if (n <= direct_max) {
-        const ScanJobs J = one_job(in, out, n, nullptr, kDirectTile);
+        ScanJobs J = one_job(in, out, n, nullptr, kDirectTile);
+        J.add = add;
         note_launch();
         pdl_launch(k_scan_direct, (unsigned)J.ntiles[0], kDirectThreads, 0, st, J);
         return;
     }
-    const ScanJobs J = one_job(in, out, n, temp);
+    ScanJobs J = one_job(in, out, n, temp);
+    J.add = add;
     note_launch();
     pdl_launch(k_scan_reduce, (unsigned)ntiles, kBlock, 0, st, J);
     if (ntiles <= kScanCarryTiles) {
@@ -261,7 +271,7 @@ void exclusive_scan_u32(cudaStream_t st, const uint32_t* in, uint32_t* out, uint
     note_launch();
     k_scan_partials<<<1, kBlock, 0, st>>>(temp, ntiles);
     note_launch();
-    k_scan_down<<<(unsigned)ntiles, kBlock, 0, st>>>(in, out, n, temp, ntiles);
+    k_scan_down<<<(unsigned)ntiles, kBlock, 0, st>>>(in, out, n, temp, ntiles, add);
 }
 
 void exclusive_scan_u32_pair(cudaStream_t st, const uint32_t* in0, uint32_t* out0, uint64_t n0,

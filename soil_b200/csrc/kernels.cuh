@@ -185,14 +185,15 @@ void launch_interleave_w(cudaStream_t st, uint64_t n, int w, double* dst, const 
 
 // ---- scan (k_scan.cu) -----------------------------------------------------
 // Exclusive scan: out[0..n] with out[n] = total.  `temp` holds
-// scan_temp_words(n) u32.  Up to direct_max counts take one launch, whose last
+// scan_temp_words(n) u32; with add (n + 1 words), out[k] gets add[k] too (n > 0).  Up to direct_max counts take one launch, whose last
 // CTA reads all of them: 16 tiles of 8,192 counts, where it meets the
 // two-launch scan (3.0 us against 4.2 plus a launch on 13,000 counts, 4.8
 // against 4.7 plus a launch on 100,000).
 constexpr uint64_t kScanDirectMax = 16ull * 8192ull;
 uint64_t scan_temp_words(uint64_t n);
 void exclusive_scan_u32(cudaStream_t st, const uint32_t* in, uint32_t* out, uint64_t n,
-                        uint32_t* temp, uint64_t direct_max = kScanDirectMax);
+                        uint32_t* temp, uint64_t direct_max = kScanDirectMax,
+                        const uint32_t* add = nullptr);
 // Two independent scans in the same launches (when both are of the same
 // form; else one after the other).  temp holds scan_temp_words(n0) +
 // scan_temp_words(n1) u32.
@@ -226,18 +227,17 @@ void launch_scatter(cudaStream_t st, uint64_t n, const uint32_t* cell, uint32_t*
 void launch_scatter_consume(cudaStream_t st, uint64_t n, const uint32_t* cell,
                             const uint32_t* start, uint32_t* counts, uint32_t* out,
                             const uint32_t* n_dev = nullptr);
-// cell_out[i] = local_cell[i] (i < nlocal) or the cell of atom i, counted,
-// i in [0, n).  make (optional): the ghosts' columns are written first, in the
-// same pass.
+// cell_out[i] = the cell of ghost i, counted, i in [nlocal, n).  make
+// (optional): the ghosts' columns are written first, in the same pass.
 struct GhostMake {
     const uint32_t* root = nullptr;
     const uint32_t* chain = nullptr;
     SwapConst sc;
     int forces = 0;  // copy the roots' forces
 };
-void launch_cells_reuse(cudaStream_t st, uint64_t nlocal, uint64_t n, const AtomCols& c,
-                        const Grid& gr, const uint32_t* local_cell, uint32_t* cell_out,
-                        uint32_t* counts, const uint32_t* n_dev, const GhostMake* make);
+void launch_ghost_cells(cudaStream_t st, uint64_t nlocal, uint64_t n, const AtomCols& c,
+                        const Grid& gr, uint32_t* cell_out, uint32_t* counts,
+                        const uint32_t* n_dev, const GhostMake* make);
 // What the neighbor build's bin order carries per sorted slot: the atom, its
 // inverse asi[atom], the record sp = {x, y, z, cutoff} (plus the FP32
 // grid-relative copy spf when spf != nullptr) and the build positions of the
@@ -257,12 +257,11 @@ struct SortedViews {
 };
 // The neighbor build's bins and views just after a spatial sort on the same
 // grid: local i of cell c at start[c] + i - sort_start[c], then c's ghosts
-// [nl, n) in ascending order after its locals.  counts: the cells' local +
-// ghost counts (the ghosts' part is consumed); tmp: scratch of the atoms'
-// size.  Returns true when counts[0, nc) were put back to zero (there were
-// ghost slots to rank).
-bool launch_place_bins(cudaStream_t st, uint64_t nl, uint64_t n, uint64_t nc,
-                       const uint32_t* n_dev, const uint32_t* cell, const uint32_t* start,
+// [nl, n) in ascending order after its locals.  start: sort_start plus the
+// scan of counts, the cells' ghosts (consumed: all zero afterwards); tmp:
+// scratch of the atoms' size.
+void launch_place_bins(cudaStream_t st, uint64_t nl, uint64_t n, const uint32_t* n_dev,
+                       const uint32_t* local_cell, const uint32_t* cell, const uint32_t* start,
                        const uint32_t* sort_start, uint32_t* counts, uint32_t* tmp,
                        const SortedViews& v);
 // The views alone, of sorted slots [0, n)

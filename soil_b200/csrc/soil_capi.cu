@@ -317,9 +317,9 @@ uint64_t scan_direct_max() {
     return env ? std::strtoull(env, nullptr, 10) : kScanDirectMax;
 }
 
-int scan_counts(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n) {
+int scan_counts(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n, const uint32_t* add) {
     TRY(ensure(s, s->scan_tmp, scan_temp_words(n + 2)));
-    exclusive_scan_u32(s->st, in, out, n, s->scan_tmp.p, scan_direct_max());
+    exclusive_scan_u32(s->st, in, out, n, s->scan_tmp.p, scan_direct_max(), add);
     return SOIL_OK;
 }
 
@@ -1444,12 +1444,13 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
         make.forces = builtin_consumer(s) ? 0 : 1;  // it overwrites every force of the step
     }
     if (after_sort)  // reuse the sort's local cells (neighbor.rs:1049-1066)
-        launch_cells_reuse(s->st, nl, total, s->A, gr, s->sorted_local_cell.p, s->atom_cell.p,
-                           s->cell_counts.p, n_dev, pend ? &make : nullptr);
+        launch_ghost_cells(s->st, nl, total, s->A, gr, s->atom_cell.p, s->cell_counts.p, n_dev,
+                           pend ? &make : nullptr);
     else
         launch_cells(s->st, 0, total, s->A, gr, s->atom_cell.p, s->cell_counts.p, n_dev);
     s->local_cells_valid = false;
-    TRY(scan_counts(s, s->cell_counts.p, s->cell_start.p, nc));
+    TRY(scan_counts(s, s->cell_counts.p, s->cell_start.p, nc,
+                    after_sort ? s->sort_start.p : nullptr));
     SortedViews views;
     views.c = s->A;
     views.sorted = s->sorted_atoms.p;
@@ -1465,10 +1466,9 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
     views.clear = s->dflags;  // the counters of the pair passes
     if (after_sort) {
         // the locals are in bin order already: only the ghosts are sorted
-        const bool zeroed =
-            launch_place_bins(s->st, nl, total, nc, n_dev, s->atom_cell.p, s->cell_start.p,
-                              s->sort_start.p, s->cell_counts.p, s->ghost_tmp.p, views);
-        s->counts_clean = zeroed ? nc : 0;  // else the locals' counts remain
+        launch_place_bins(s->st, nl, total, n_dev, s->sorted_local_cell.p, s->atom_cell.p,
+                          s->cell_start.p, s->sort_start.p, s->cell_counts.p, s->ghost_tmp.p, views);
+        counts_consumed(s);
     } else {
         launch_scatter_consume(s->st, total, s->atom_cell.p, s->cell_start.p, s->cell_counts.p,
                                s->sorted_atoms.p, n_dev);
@@ -1486,7 +1486,7 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
         s->stencil_on_device = runs;
     }
     PairParams p;
-    p.atom_cell = s->atom_cell.p;
+    p.atom_cell = after_sort ? s->sorted_local_cell.p : s->atom_cell.p;
     p.atom_sorted_idx = s->asi.p;
     p.bin_start = s->cell_start.p;
     p.sorted_atoms = s->sorted_atoms.p;

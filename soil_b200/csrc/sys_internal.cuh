@@ -293,8 +293,9 @@ int counts_zero(soil_sys* s, uint64_t nc);
 std::vector<int32_t> stencil_runs(const std::vector<int32_t>& sten, bool newton);
 // Whether the pair scan preloads its ranges (SOIL_PAIRS_PRE=0: off; read at each call).
 int pairs_pre_ranges();
-// exclusive scan of in[0, n) into out[0, n]
-int scan_counts(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n);
+// exclusive scan of in[0, n) into out[0, n], plus add[0, n] when given
+int scan_counts(soil_sys* s, const uint32_t* in, uint32_t* out, uint64_t n,
+                const uint32_t* add = nullptr);
 Geom geom_of(const soil_sys* s);
 Grid grid_of(const soil_sys* s);
 void compute_bin_grid(soil_sys* s);
