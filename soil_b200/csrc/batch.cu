@@ -24,6 +24,7 @@
 #include <thread>
 
 #include "batch.cuh"
+#include "block_scan.cuh"
 #include "host_pool.h"
 #include "sys_internal.cuh"
 
@@ -57,6 +58,10 @@ struct SpanBuild {
         base.push_back((uint32_t)first);
         flag.push_back(f);
         start.push_back(start.back() + n);
+    }
+    // the tiles of a scan of n counts (an empty one still writes its total)
+    void add_scan(uint32_t bx, uint64_t n, int which) {
+        add(bx, n ? (n + kDirectTile - 1) / kDirectTile : 1, n, (uint8_t)which);
     }
     // like add, but leaves out empty ranges (element spans only)
     void add_nz(uint32_t bx, uint64_t n, uint64_t first, uint8_t f = 0) {
@@ -127,7 +132,7 @@ struct soil_batch {
     // system is batched; nghost and cells are refreshed where they change.
     struct Hot {
         uint64_t nlocal = 0, nghost = 0, cells = 0;
-        uint8_t newton = 0, cells_valid = 0;
+        uint8_t newton = 0;
     };
     std::vector<Hot> hot;
 };
@@ -271,6 +276,10 @@ int stage_commit(soil_batch* b, Stage& g) {
         sp.flag = (const uint8_t*)(g.d + o);
         sp.nseg = (uint32_t)n;
         sp.total = s.start.back();
+        // one row of elements per CTA while a wave holds them all, up to four
+        // above (a warp's segment lookup is then shared)
+        const uint64_t wave = 148ull * 8 * kBlock;
+        sp.items = (uint32_t)std::min<uint64_t>(4, std::max<uint64_t>(1, sp.total / wave));
     }
     if (off > first)
         BCK(cudaMemcpyAsync(g.d + first, g.h + first, off - first, cudaMemcpyHostToDevice, b->st));
@@ -353,7 +362,8 @@ void fill_dev(soil_batch* b, uint32_t k) {
     d.sorted_local_cell = s->sorted_local_cell.p;
     d.cell_counts = s->cell_counts.p;
     d.cell_start = s->cell_start.p;
-    d.cell_cursor = s->cell_cursor.p;
+    d.sort_start = s->sort_start.p;
+    d.bins = s->ghost_tmp.p;
     d.atom_cell = s->atom_cell.p;
     d.sorted_atoms = s->sorted_atoms.p;
     d.asi = s->asi.p;
@@ -365,8 +375,8 @@ void fill_dev(soil_batch* b, uint32_t k) {
     d.spf = s->spf.p;
     d.in_count = s->in_count.p;
     d.in_start = s->in_start.p;
-    d.in_cursor = s->in_cursor.p;
     d.in_list = s->in_list.p;
+    d.in_split = s->in_split.p;
     d.ghost_root = s->ghost_root.p;
     d.ghost_chain = s->ghost_chain.p;
     for (int q = 0; q < kNumSwaps; ++q) d.send[q] = s->send[q].p;
@@ -565,6 +575,12 @@ int grow_slots(soil_batch* b, uint32_t need) {
     return SOIL_OK;
 }
 
+// Bit 0: uniform cutoff, bit 1: FP32 filter (the pair passes' instances).
+int pair_kind(const soil_batch* b, uint32_t k) {
+    const BoxStep& t = b->h_step[k];
+    return (t.uniform ? 1 : 0) | (t.filter ? 2 : 0);
+}
+
 // The staged pair count serves the batch when SOIL_PAIRS_STAGED=1.
 bool pairs_staged_on() {
     const char* env = std::getenv("SOIL_PAIRS_STAGED");
@@ -683,6 +699,7 @@ int batch_step(soil_batch* b, bool last) {
         if (b->full_at_pbc[k]) s->nghost = 0;  // remove_ghost_atoms
         bool run, periodic;
         TRY(sort_plan(s, &run, &periodic));
+        if (run) TRY(counts_zero(s, s->total_cells));
         b->run[k] = run;
         b->periodic[k] = periodic;
         b->apply[k] = run && !periodic;
@@ -717,28 +734,32 @@ int batch_step(soil_batch* b, bool last) {
         Stage& g2 = b->stage[G_SORT];
         TRY(stage_begin(b, g2));
         TRY(put_tables(b, g2));
-        const int s_pbc = stage_add(g2), s_cells = stage_add(g2), s_loc = stage_add(g2),
-                  s_id = stage_add(g2), s_gather = stage_add(g2);
+        const int s_loc = stage_add(g2), s_scan = stage_add(g2), s_scatter = stage_add(g2),
+                  s_gather = stage_add(g2), s_seg = stage_add(g2), s_id = stage_add(g2);
         for (uint32_t k : M)
-            if (b->full_at_pbc[k]) g2.spans[s_pbc].add_nz(k, b->hot[k].nlocal, 0);
+            if (b->full_at_pbc[k] || b->run[k])
+                g2.spans[s_loc].add_nz(k, b->hot[k].nlocal, 0,
+                                       (uint8_t)((b->full_at_pbc[k] ? 1 : 0) | (b->run[k] ? 2 : 0)));
         for (uint32_t k : S) {
             const auto& h = b->hot[k];
-            g2.spans[s_cells].add(k, h.cells, 0);
-            g2.spans[s_loc].add_nz(k, h.nlocal, 0);
-            if (b->periodic[k]) g2.spans[s_id].add_nz(k, h.nlocal, 0);
+            g2.spans[s_scan].add_scan(k, h.cells, BA_CELLS);
+            g2.spans[s_scatter].add_nz(k, h.nlocal, 0, b->periodic[k]);
             if (b->apply[k]) g2.spans[s_gather].add_nz(k, h.nlocal, 0);
+            if (b->periodic[k]) {
+                g2.spans[s_seg].add_nz(k, h.cells, 0);
+                g2.spans[s_id].add_nz(k, h.nlocal, 0);
+            }
         }
         TRY(stage_commit(b, g2));
         tic(b);
-        b_pbc(st, g2.out[s_pbc], a);
-        b_zero_counts(st, g2.out[s_cells], a, BA_CELLS);
-        b_cells(st, g2.out[s_loc], a, false);
-        b_scan(st, g2.out[s_cells], a, BA_CELLS);
-        b_scatter(st, g2.out[s_loc], a, false);
-        b_segsort(st, g2.out[s_cells], a, BA_CELLS);
-        b_permute_cells(st, g2.out[s_loc], a);
+        b_pbc_cells(st, g2.out[s_loc], a);
+        b_scan(st, g2.out[s_scan], a);
+        b_scatter(st, g2.out[s_scatter], a);
+        b_sort_gather(st, g2.out[s_gather], a);
+        b_segsort(st, g2.out[s_seg], a);
+        b_permute_cells(st, g2.out[s_id], a);
         b_identity(st, g2.out[s_id], a);
-        b_perm_gather(st, g2.out[s_gather], a);
+        for (uint32_t k : S) counts_consumed(b->slot[k]);
         toc(b, BT_SORT);
         TRY(check_kernels(b));
     }
@@ -810,13 +831,16 @@ int batch_step(soil_batch* b, bool last) {
         TRY(for_boxes(b, R, [&](uint32_t k) -> int {
             soil_sys* s = b->slot[k];
             TRY(borders_done(s, b->h_bread + (size_t)k * kBorderStateWords, b->bds[k].data()));
+            if (!s->local_cells_valid)
+                return fail(b->ctx, SOIL_ERR_STATE, "batched rebuild without a spatial sort");
             TRY(neighbor_plan(s));
+            TRY(counts_zero(s, s->total_cells));
+            TRY(in_counts_zero(s));
             fill_dev(b, k);
             auto& h = b->hot[k];
             h.nghost = s->nghost;
             h.cells = s->total_cells;
             // local bins of this step's sort are reused once, by this build
-            h.cells_valid = s->local_cells_valid ? 1 : 0;
             s->local_cells_valid = false;
             return SOIL_OK;
         }));
@@ -826,9 +850,10 @@ int batch_step(soil_batch* b, bool last) {
     Stage& g4 = b->stage[G_NEIGHBOR];
     TRY(stage_begin(b, g4));
     TRY(put_tables(b, g4));
-    const int f_loc = stage_add(g4), s_fwd = stage_add(g4), n_cells = stage_add(g4),
-              n_copy = stage_add(g4), n_bin = stage_add(g4), n_all = stage_add(g4),
-              n_rows = stage_add(g4), n_tiles = stage_add(g4);
+    const int s_fwd = stage_add(g4), n_ghost = stage_add(g4), n_cells = stage_add(g4),
+              n_all = stage_add(g4), n_tiles = stage_add(g4), n_scan = stage_add(g4);
+    int n_rows[4];  // by cutoff kind and filter
+    for (int& r : n_rows) r = stage_add(g4);
     for (uint32_t k : M) {
         const auto& h = b->hot[k];
         if (!b->rebuild[k]) {
@@ -836,33 +861,28 @@ int batch_step(soil_batch* b, bool last) {
             continue;
         }
         const uint64_t nl = h.nlocal, ng = h.nghost;
-        g4.spans[f_loc].add_nz(k, nl, 0);
-        g4.spans[n_cells].add(k, h.cells, 0);
-        if (h.cells_valid) {
-            g4.spans[n_copy].add_nz(k, nl, 0);
-            g4.spans[n_bin].add_nz(k, ng, nl);
-        } else {
-            g4.spans[n_bin].add_nz(k, nl + ng, 0);
-        }
+        g4.spans[n_ghost].add_nz(k, ng, nl);
+        g4.spans[n_cells].add_scan(k, h.cells, BA_NEIGH_CELLS);
         g4.spans[n_all].add_nz(k, nl + ng, 0);
-        g4.spans[n_rows].add(k, nl, 0);
+        g4.spans[n_rows[pair_kind(b, k)]].add_nz(k, nl, 0);
         g4.spans[n_tiles].add_nz(k, (nl + 31) / 32, 0);
+        g4.spans[n_scan].add_scan(k, nl, BA_ROWS);
+        g4.spans[n_scan].add_scan(k, nl + ng, BA_IN);
     }
     TRY(stage_commit(b, g4));
     tic(b);
     b_forward(st, g4.out[s_fwd], a);
     if (!R.empty()) {
-        b_save_positions(st, g4.out[f_loc], a);
-        b_zero_counts(st, g4.out[n_cells], a, BA_NEIGH_CELLS);
-        b_copy_count_local_cells(st, g4.out[n_copy], a);
-        b_cells(st, g4.out[n_bin], a, true);
-        b_scan(st, g4.out[n_cells], a, BA_NEIGH_CELLS);
-        b_scatter(st, g4.out[n_all], a, true);
-        b_segsort(st, g4.out[n_cells], a, BA_NEIGH_CELLS);
-        b_sorted_views(st, g4.out[n_all], a);
+        b_ghost_cells(st, g4.out[n_ghost], a);
+        b_scan(st, g4.out[n_cells], a);
+        b_place_bins(st, g4.out[n_all], a);
+        b_ghost_rank(st, g4.out[n_ghost], a);
         if (pairs_staged_on()) b_pairs_staged(st, g4.out[n_tiles], a);
-        else b_pairs_rows(st, g4.out[f_loc], a);
-        b_scan(st, g4.out[n_rows], a, BA_ROWS);
+        else
+            for (int v = 0; v < 4; ++v)
+                b_pairs_rows(st, g4.out[n_rows[v]], a, (v & 1) != 0, (v & 2) != 0);
+        b_scan(st, g4.out[n_scan], a);
+        for (uint32_t k : R) counts_consumed(b->slot[k]);
         toc(b, BT_NEIGHBOR);
         TRY(check_kernels(b));
         BCK(cudaMemcpyAsync(b->h_totals, b->d_totals, (size_t)b->cap * 4, cudaMemcpyDeviceToHost, st));
@@ -877,10 +897,6 @@ int batch_step(soil_batch* b, bool last) {
                             "neighbor stencil left the bin grid (atom outside the ghost layers)");
             const uint64_t np = b->h_totals[k], total = s->nlocal + s->nghost;
             TRY(ensure(s, s->indices, np + 1, 0, pair_room(np)));
-            TRY(ensure(s, s->in_count, total + 1, 0, s->acap + 1));
-            s->in_zero = 0;  // the batch's count pass leaves the counts behind
-            TRY(ensure(s, s->in_start, total + 2, 0, s->acap + 2));
-            TRY(ensure(s, s->in_cursor, total + 1, 0, s->acap + 1));
             TRY(ensure(s, s->in_list, np + 1, 0, pair_room(np)));
             const int fv = force_variant();
             if (s->few_images && fv != SOIL_FORCE_GATHER && fv != SOIL_FORCE_CSR) {
@@ -896,7 +912,7 @@ int batch_step(soil_batch* b, bool last) {
             s->in_lists_valid = true;
             s->seq_valid = false;  // set once this step's sequences are enqueued
             s->order_valid = false;
-            s->split_valid = false;
+            s->split_valid = true;
             s->hflags->candidates = b->h_flags[k].candidates;
             s->hflags->rechecked = b->h_flags[k].rechecked;
             fill_dev(b, k);
@@ -909,33 +925,31 @@ int batch_step(soil_batch* b, bool last) {
     std::vector<uint32_t> grouped_now;  // rebuilding boxes that build grouped sequences
     TRY(stage_begin(b, g5));
     TRY(put_tables(b, g5));
-    const int r_loc = stage_add(g5), r_all = stage_add(g5), r_scan = stage_add(g5),
-              h_all = stage_add(g5), v_loc = stage_add(g5), l_loc = stage_add(g5),
-              q_all = stage_add(g5), q_grp = stage_add(g5), q_loc = stage_add(g5),
-              t_tiles = stage_add(g5), t_walk = stage_add(g5);
-    // Boxes whose locals have at most 7 images take the grouped consumer (its
-    // sequences built at each rebuild, reverse comm folded in); the others the
-    // per-atom gather and a reverse pass.
+    const int r_all = stage_add(g5), h_all = stage_add(g5), v_loc = stage_add(g5),
+              l_loc = stage_add(g5), c_loc = stage_add(g5), q_all = stage_add(g5),
+              q_grp = stage_add(g5), q_loc = stage_add(g5), t_tiles = stage_add(g5),
+              t_walk = stage_add(g5);
+    int r_rows[4];
+    for (int& r : r_rows) r = stage_add(g5);
+    // The consumer of the single system, which needs no preparation per build;
+    // SOIL_FORCE names another: the grouped kernels (for boxes whose locals have
+    // at most 7 images, their sequences built at each rebuild), or the per-atom
+    // gather with a reverse pass (102 + 41 against 133 us for the walk on 128
+    // boxes of 1.5 million atoms, 25 + 22 against 22 on 64 of 90,000).
     grouped_now.clear();
-    // The batch's consumer: the grouped kernels when SOIL_FORCE names one, else
-    // the per-atom gather with a reverse pass (measured fastest on the
-    // batched boxes, whose frequent rebuilds favour kernels without per-build
-    // preparation).
-    int variant = force_variant();
-    if (variant == SOIL_FORCE_CSR) variant = SOIL_FORCE_GATHER;
+    const int variant = force_variant();
     for (uint32_t k : M) {
         const auto& h = b->hot[k];
         const soil_sys* s = b->slot[k];
         const uint64_t nl = h.nlocal, total = nl + h.nghost;
-        const bool grouped = variant != SOIL_FORCE_GATHER && s->few_images &&
-                             (b->rebuild[k] || s->seq_valid);
+        const bool grouped = variant != SOIL_FORCE_GATHER && variant != SOIL_FORCE_CSR &&
+                             s->few_images && (b->rebuild[k] || s->seq_valid);
         if (b->rebuild[k]) {
-            g5.spans[r_loc].add_nz(k, nl, 0);
+            g5.spans[r_rows[pair_kind(b, k)]].add_nz(k, nl, 0);
             g5.spans[r_all].add_nz(k, total, 0);
-            g5.spans[r_scan].add(k, total, 0);
             if (grouped) {
                 g5.spans[q_all].add_nz(k, total, 0);
-                g5.spans[q_grp].add(k, nl, 0);
+                g5.spans[q_grp].add_scan(k, nl, BA_GRP);
                 g5.spans[q_loc].add_nz(k, nl, 0);
                 grouped_now.push_back(k);
             }
@@ -943,9 +957,11 @@ int batch_step(soil_batch* b, bool last) {
         if (grouped) {
             if (variant == SOIL_FORCE_WALK) g5.spans[t_walk].add_nz(k, nl, 0);
             else g5.spans[t_tiles].add_nz(k, (nl + 31) / 32, 0);
-        } else {
+        } else if (variant == SOIL_FORCE_GATHER) {
             g5.spans[h_all].add_nz(k, total, 0);
             if (h.newton && h.nghost) g5.spans[v_loc].add_nz(k, nl, 0);
+        } else {
+            g5.spans[c_loc].add_nz(k, nl, 0);
         }
         g5.spans[l_loc].add_nz(k, nl, 0);
     }
@@ -953,14 +969,12 @@ int batch_step(soil_batch* b, bool last) {
     TRY(stage_commit(b, g5));
     tic(b);
     if (!R.empty()) {
-        b_pairs_fill(st, g5.out[r_loc], a);
-        b_zero_counts(st, g5.out[r_scan], a, BA_IN);
-        b_in_count(st, g5.out[r_loc], a);
-        b_scan(st, g5.out[r_scan], a, BA_IN);
-        b_in_scatter(st, g5.out[r_loc], a);
-        b_segsort(st, g5.out[r_all], a, BA_IN);
+        for (int v = 0; v < 4; ++v)
+            b_pairs_fill(st, g5.out[r_rows[v]], a, (v & 1) != 0, (v & 2) != 0);
+        for (uint32_t k : R) b->slot[k]->in_zero = b->slot[k]->acap;  // every count taken back
+        b_in_sort(st, g5.out[r_all], a);
         b_seq_count(st, g5.out[q_all], a);
-        b_scan(st, g5.out[q_grp], a, BA_GRP);
+        b_scan(st, g5.out[q_grp], a);
         b_seq_fill(st, g5.out[q_loc], a);
         for (uint32_t k : grouped_now) b->slot[k]->seq_valid = true;
     }
@@ -968,6 +982,7 @@ int batch_step(soil_batch* b, bool last) {
     tic(b);
     b_force_grouped(st, g5.out[t_tiles], a);
     b_force_walk(st, g5.out[t_walk], a);
+    b_force_csr(st, g5.out[c_loc], a);
     b_harmonic(st, g5.out[h_all], a);
     toc(b, BT_FORCE);
     tic(b);
@@ -1004,7 +1019,6 @@ void rebuild_members(soil_batch* b) {
 
 int detach(soil_batch* b, uint32_t k) {
     soil_sys* s = b->slot[k];
-    s->counts_clean = 0;  // the batch's counting passes leave counts behind
     s->stencil_on_device.clear();
     s->pk_valid = false;  // the batch moved atoms without the packed records
     s->st = b->saved[k];
@@ -1117,6 +1131,9 @@ int soil_batch_add(soil_batch* b, soil_sys* s) {
         return fail(b->ctx, SOIL_ERR_INVALID,
                     "bin stencil of %zu cell runs exceeds the batched limit %d", runs.size() / 2,
                     kMaxStencil / 2);
+    // a box that keeps its lists brings the transposed ones with their splits
+    if (s->state == COMMUNICATE_ONLY && (!s->in_lists_valid || !s->split_valid))
+        TRY(build_in_lists(s));
     BCK(cudaStreamSynchronize(s->st));
     TRY(wait(b));
     uint32_t k = 0;
@@ -1133,7 +1150,6 @@ int soil_batch_add(soil_batch* b, soil_sys* s) {
     b->hot[k].nghost = s->nghost;
     b->hot[k].cells = s->total_cells;
     b->hot[k].newton = s->newton ? 1 : 0;
-    b->hot[k].cells_valid = 0;
     TRY(fill_step(b, k, false, nullptr));
     rebuild_members(b);
     return SOIL_OK;

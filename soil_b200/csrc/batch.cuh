@@ -34,7 +34,8 @@ struct BoxDev {
     uint32_t* sorted_local_cell;
     uint32_t* cell_counts;
     uint32_t* cell_start;
-    uint32_t* cell_cursor;
+    uint32_t* sort_start;  // the spatial sort's cell starts
+    uint32_t* bins;        // unordered bins (scratch)
     uint32_t* atom_cell;
     uint32_t* sorted_atoms;
     uint32_t* asi;
@@ -46,8 +47,8 @@ struct BoxDev {
     float4* spf;
     uint32_t* in_count;
     uint32_t* in_start;
-    uint32_t* in_cursor;
     uint32_t* in_list;
+    uint32_t* in_split;
     uint32_t* ghost_root;
     uint32_t* ghost_chain;
     uint32_t* send[kNumSwaps];
@@ -106,6 +107,7 @@ struct Span {
     const uint32_t* base;   // element offset inside the box
     const uint8_t* flag;    // per-segment switches (kernel specific)
     uint32_t nseg;
+    uint32_t items;  // consecutive rows of kBlock elements a CTA takes at a time
     uint64_t total;
 };
 
@@ -117,13 +119,13 @@ struct BatchArgs {
     uint32_t* totals;   // one per box (pair totals)
 };
 
-// Arrays a batched scan / zero / sort can target.
+// Arrays a batched scan can target (the segment's flag).
 enum BatchArray {
-    BA_CELLS = 0,     // cell_counts -> cell_start (+ cursor), segsort of sort_perm
-    BA_NEIGH_CELLS,   // cell_counts -> cell_start (+ cursor), segsort of sorted_atoms
-    BA_ROWS,          // rowcount -> offsets (total into totals[box])
-    BA_IN,            // in_count -> in_start (+ cursor), segsort of in_list
-    BA_GRP            // grp_cnt -> grp_start (grouped sequences)
+    BA_CELLS = 0,    // cell_counts -> sort_start
+    BA_NEIGH_CELLS,  // cell_counts (ghosts) + sort_start -> cell_start
+    BA_ROWS,         // rowcount -> offsets (total into totals[box])
+    BA_IN,           // in_count -> in_start
+    BA_GRP           // grp_cnt -> grp_start (grouped sequences)
 };
 
 // ---- launchers (k_batch.cu); every one enqueues a single kernel ------------
@@ -132,16 +134,21 @@ void b_initial(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_final(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_profile(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_zero_forces(cudaStream_t st, const Span& sp, const BatchArgs& a);
-void b_pbc(cudaStream_t st, const Span& sp, const BatchArgs& a);
-// zero the counts of `which` over each segment's element range
-void b_zero_counts(cudaStream_t st, const Span& sp, const BatchArgs& a, int which);
-// cells of positions (sort: locals into sort_cell; neighbor: any range into atom_cell)
-void b_cells(cudaStream_t st, const Span& sp, const BatchArgs& a, bool neighbor);
-void b_copy_count_local_cells(cudaStream_t st, const Span& sp, const BatchArgs& a);
-// one CTA per segment: exclusive scan of `which`, cursor copy, totals
-void b_scan(cudaStream_t st, const Span& sp, const BatchArgs& a, int which);
-void b_scatter(cudaStream_t st, const Span& sp, const BatchArgs& a, bool neighbor);
-void b_segsort(cudaStream_t st, const Span& sp, const BatchArgs& a, int which);
+// locals of a box: flag bit0 wraps them (pbc), bit1 bins and counts them (sort)
+void b_pbc_cells(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// ghosts: their columns from the border pass, their cells, counted
+void b_ghost_cells(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// exclusive scans; a segment's elements are its tiles of kDirectTile counts,
+// base the number of counts, flag the array (BatchArray)
+void b_scan(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// the locals scattered into their cells, taking the counts back to zero: into
+// bins, or (flag) sort_perm
+void b_scatter(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// the locals' columns to their ranks in bins, with perm and sorted_local_cell
+void b_sort_gather(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// periodic sorts (applied only if not the identity): sort_perm's cells put in
+// order, sorted_local_cell
+void b_segsort(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_permute_cells(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_identity(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_perm_gather(cudaStream_t st, const Span& sp, const BatchArgs& a);
@@ -151,15 +158,24 @@ void b_border_faces(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_border_cat_scan(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_border_images(cudaStream_t st, const Span& sp, const BatchArgs& a);
 void b_forward(cudaStream_t st, const Span& sp, const BatchArgs& a);
-void b_save_positions(cudaStream_t st, const Span& sp, const BatchArgs& a);
-void b_sorted_views(cudaStream_t st, const Span& sp, const BatchArgs& a);
-void b_pairs_rows(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// the neighbor build's bins and sorted records: all atoms placed, then the
+// ghosts (element range from nlocal on) ranked
+void b_place_bins(cudaStream_t st, const Span& sp, const BatchArgs& a);
+void b_ghost_rank(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// the pair count pass (uniform cutoff or not, FP32 filter or not: one span
+// each), counting the transposed lists' entries too
+void b_pairs_rows(cudaStream_t st, const Span& sp, const BatchArgs& a, bool uniform, bool fp32);
 // the pair count pass over warp tiles of 32 rows (element = tile of a box),
 // candidate records staged in shared memory (pairs_staged.cuh)
 void b_pairs_staged(cudaStream_t st, const Span& sp, const BatchArgs& a);
-void b_pairs_fill(cudaStream_t st, const Span& sp, const BatchArgs& a);
-void b_in_count(cudaStream_t st, const Span& sp, const BatchArgs& a);
-void b_in_scatter(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// rows into the CSR and into their partners' transposed lists
+void b_pairs_fill(cudaStream_t st, const Span& sp, const BatchArgs& a, bool uniform, bool fp32);
+// the transposed lists of all atoms ascending, with their splits
+void b_in_sort(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// the consumer: roots and their images over the CSR and its transpose, with
+// the reverse fold (element = local root)
+void b_force_csr(cudaStream_t st, const Span& sp, const BatchArgs& a);
+// the per-atom gather (element = local or ghost) and its reverse pass
 void b_harmonic(cudaStream_t st, const Span& sp, const BatchArgs& a);
 // grouped sequences: lengths over every atom (count) and the groups of the
 // locals (fill, after a BA_GRP scan); the consumer over warp tiles of 32

@@ -470,6 +470,54 @@ __device__ uint32_t row_scan(const PairParams& p, const Filter<UNIFORM, FP32>& t
     }
 }
 
+// Pass 2 of row i: into its CSR place, from its slots (or derived again when it
+// is longer than they are), and with the transposed lists into every partner's
+// list, the counts going back to 0.  Four entries at a time, their loads,
+// atomics and stores each issued together.
+template <bool UNIFORM, bool FP32>
+__device__ __forceinline__ void fill_row(const PairParams& p, const Filter<UNIFORM, FP32>& test,
+                                         uint64_t i, const uint32_t* rowcount,
+                                         const uint32_t* slots, const uint32_t* offsets,
+                                         uint32_t* indices) {
+    const uint32_t K = (uint32_t)p.row_slots;
+    const uint32_t cnt = rowcount[i];
+    // the row's first four slots, loaded with its length and offset (the
+    // slots of a row are 16-byte aligned; past cnt they are unused)
+    const uint4 head = *reinterpret_cast<const uint4*>(slots + i * K);
+    uint32_t* out = indices + offsets[i];
+    const bool slotted = cnt <= K;
+    if (!slotted) {
+        uint32_t rk = 0, cd = 0;
+        row_scan<UNIFORM, FP32, true>(p, test, i, out, 0xffffffffu, &rk, &cd, nullptr);
+    }
+    const uint32_t* src = slotted ? slots + i * K : out;
+    for (uint32_t k0 = 0; k0 < cnt; k0 += 4) {
+        uint32_t a[4], at[4];
+        if (k0 == 0 && slotted) {
+            a[0] = head.x;
+            a[1] = head.y;
+            a[2] = head.z;
+            a[3] = head.w;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k0 + u < cnt) a[u] = src[k0 + u];
+        }
+        if (slotted) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k0 + u < cnt) out[k0 + u] = a[u];
+        }
+        if (!p.in_list) continue;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k0 + u < cnt) at[u] = p.in_start[a[u]] + atomicSub(&p.in_count[a[u]], 1u) - 1u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k0 + u < cnt) p.in_list[at[u]] = (uint32_t)i;
+    }
+}
+
 // ---- per-atom bodies of the kernels ----------------------------------------
 
 // Atom i's packed record (x, y, z, its radius) in one 256-bit store: whole

@@ -305,11 +305,10 @@ __device__ __forceinline__ void csr_item_force(const ForceCsr& q, const Ld& ld, 
     sum_partners(ld, pa, q.K, nin + ix.nrow, ix, Fx, Fy, Fz);
 }
 
-// Root t and its images by one thread (CSR walk), then (FOLD) the fold.
-template <bool FOLD, class Ld>
-__device__ __forceinline__ void force_csr_root_ld(const ForceCsr& q, const Ld& ld,
-                                                  const AtomCols& c, const PlaneList& rev,
-                                                  uint64_t t) {
+// The forces on root t and on its images by one thread (CSR walk).
+template <class Ld>
+__device__ __forceinline__ void force_csr_items(const ForceCsr& q, const Ld& ld, const AtomCols& c,
+                                                uint64_t t) {
     const uint32_t f0 = q.fold_start[t], f1 = q.fold_start[t + 1];
     for (uint32_t f = f0 - 1; f + 1 <= f1; ++f) {  // the root (f = f0 - 1), then its images
         const uint64_t a = f + 1 == f0 ? t : q.nlocal + q.fold_list[f];
@@ -319,6 +318,14 @@ __device__ __forceinline__ void force_csr_root_ld(const ForceCsr& q, const Ld& l
         c.fy[a] = Fy;
         c.fz[a] = Fz;
     }
+}
+
+// ... then (FOLD) the fold.
+template <bool FOLD, class Ld>
+__device__ __forceinline__ void force_csr_root_ld(const ForceCsr& q, const Ld& ld,
+                                                  const AtomCols& c, const PlaneList& rev,
+                                                  uint64_t t) {
+    force_csr_items(q, ld, c, t);
     if (FOLD) fold_root(c, q.nlocal, t, q.fold_start, q.fold_list, rev);
 }
 

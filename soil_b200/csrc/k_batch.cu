@@ -17,8 +17,6 @@
 
 namespace soil {
 
-constexpr int kSpanItems = 4;
-
 // Segment holding flattened element g (the last segment whose start is <= g),
 // found by the 32 lanes of one warp together: each level probes 32 evenly
 // spaced starts, so 4,096 segments take three dependent loads.  Call with all
@@ -45,13 +43,14 @@ __device__ __forceinline__ uint32_t seg_of_warp(const Span& sp, uint64_t g) {
 // barrier) and its lanes walk forward from there.
 template <class F>
 __device__ __forceinline__ void for_span(const Span& sp, F f) {
-    const uint64_t chunk = (uint64_t)blockDim.x * kSpanItems;
+    pdl_wait();  // every span kernel is launched with pdl_launch
+    const uint64_t chunk = (uint64_t)blockDim.x * sp.items;
     const uint64_t warp0 = threadIdx.x & ~31u;
     for (uint64_t g0 = (uint64_t)blockIdx.x * chunk; g0 < sp.total;
          g0 += (uint64_t)gridDim.x * chunk) {
         const uint64_t gw = g0 + warp0 < sp.total ? g0 + warp0 : g0;
         uint32_t k = seg_of_warp(sp, gw);
-        for (int it = 0; it < kSpanItems; ++it) {
+        for (uint32_t it = 0; it < sp.items; ++it) {
             const uint64_t g = g0 + (uint64_t)it * blockDim.x + threadIdx.x;
             if (g >= sp.total) break;
             while (g >= sp.start[k + 1]) ++k;
@@ -60,12 +59,12 @@ __device__ __forceinline__ void for_span(const Span& sp, F f) {
     }
 }
 
-static unsigned span_grid(const Span& sp) { return grid_for((sp.total + kSpanItems - 1) / kSpanItems); }
+static unsigned span_grid(const Span& sp) { return grid_for((sp.total + sp.items - 1) / sp.items); }
 
 // One resident wave of span kernel K (grid_wave), never more than the span needs.
 template <auto K>
 static unsigned span_wave(const Span& sp) {
-    return grid_wave<K>((sp.total + kSpanItems - 1) / kSpanItems);
+    return grid_wave<K>((sp.total + sp.items - 1) / sp.items);
 }
 
 #define SPAN_KERNEL(name, ...)                                                        \
@@ -84,7 +83,7 @@ static unsigned span_wave(const Span& sp) {
     void fn(cudaStream_t st, const Span& sp, const BatchArgs& a) {   \
         if (sp.total == 0) return;                                   \
         note_launch();                                               \
-        kern<<<span_wave<kern>(sp), kBlock, 0, st>>>(sp, a);         \
+        pdl_launch(kern, span_wave<kern>(sp), kBlock, 0, st, sp, a); \
     }
 
 // ---- integrate --------------------------------------------------------------
@@ -121,149 +120,103 @@ SPAN_KERNEL(kb_zero_forces, {
 })
 SPAN_LAUNCH(b_zero_forces, kb_zero_forces)
 
-SPAN_KERNEL(kb_pbc, { pbc_atom(D.set[S.cur], i, S.geom, S.bvel[0], S.bvel[1], S.bvel[2]); })
-SPAN_LAUNCH(b_pbc, kb_pbc)
-
 // ---- bins -----------------------------------------------------------------
-__device__ __forceinline__ uint32_t* counts_of(const BoxDev& D, int which) {
-    if (which == BA_IN) return D.in_count;
-    return D.cell_counts;
-}
-
-__global__ void __launch_bounds__(kBlock) kb_zero_counts(Span sp, BatchArgs A, int which) {
-    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t) { counts_of(A.dev[b], which)[i] = 0u; });
-}
-void b_zero_counts(cudaStream_t st, const Span& sp, const BatchArgs& a, int which) {
-    if (sp.total == 0) return;
-    note_launch();
-    kb_zero_counts<<<span_wave<kb_zero_counts>(sp), kBlock, 0, st>>>(sp, a, which);
-}
-
-__global__ void __launch_bounds__(kBlock) kb_cells(Span sp, BatchArgs A, int neighbor) {
-    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t) {
+__global__ void __launch_bounds__(kBlock) kb_pbc_cells(Span sp, BatchArgs A) {
+    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t k) {
         const BoxDev& D = A.dev[b];
         const BoxStep& S = A.step[b];
-        const AtomCols& c = D.set[neighbor ? S.post : S.cur];
-        double3 q;
-        if (neighbor && i >= S.nlocal)  // the border pass's ghosts get their columns here
-            q = make_ghost(c, S.nlocal, i - S.nlocal, D.ghost_root, D.ghost_chain, S.sc, false);
-        else
-            q = make_double3(c.x[i], c.y[i], c.z[i]);
-        const uint32_t cell = cell_of(S.grid, q.x, q.y, q.z);
-        (neighbor ? D.atom_cell : D.sort_cell)[i] = cell;
-        atomicAdd(&D.cell_counts[cell], 1u);
+        const AtomCols& c = D.set[S.cur];
+        const uint8_t f = sp.flag[k];
+        double x, y, z;
+        if (f & 1) {
+            pbc_atom(c, i, S.geom, S.bvel[0], S.bvel[1], S.bvel[2], x, y, z);
+        } else {
+            x = c.x[i];
+            y = c.y[i];
+            z = c.z[i];
+        }
+        if (f & 2) {
+            const uint32_t cell = cell_of(S.grid, x, y, z);
+            D.sort_cell[i] = cell;
+            atomicAdd(&D.cell_counts[cell], 1u);
+        }
     });
 }
-void b_cells(cudaStream_t st, const Span& sp, const BatchArgs& a, bool neighbor) {
-    if (sp.total == 0) return;
-    note_launch();
-    kb_cells<<<span_wave<kb_cells>(sp), kBlock, 0, st>>>(sp, a, neighbor ? 1 : 0);
-}
+SPAN_LAUNCH(b_pbc_cells, kb_pbc_cells)
 
-SPAN_KERNEL(kb_copy_count_local_cells, {
-    const uint32_t cell = D.sorted_local_cell[i];
+SPAN_KERNEL(kb_ghost_cells, {
+    // the border pass's ghosts get their columns here; the consumer overwrites
+    // every force of the step
+    const double3 q = make_ghost(D.set[S.post], S.nlocal, i - S.nlocal, D.ghost_root,
+                                 D.ghost_chain, S.sc, false);
+    const uint32_t cell = cell_of(S.grid, q.x, q.y, q.z);
     D.atom_cell[i] = cell;
     atomicAdd(&D.cell_counts[cell], 1u);
 })
-SPAN_LAUNCH(b_copy_count_local_cells, kb_copy_count_local_cells)
+SPAN_LAUNCH(b_ghost_cells, kb_ghost_cells)
 
-// One CTA per segment: out = exclusive scan of in over the segment's n
-// elements (out[n] = total), optional cursor copy.  Each thread takes
-// kScanItems consecutive elements per pass (two 16-byte loads when the group
-// is whole; every array is its own allocation, so element 0 is 256-byte
-// aligned).  One CTA per segment lets the block scheduler balance boxes of
-// very different sizes; spans list the largest boxes first.
-constexpr int kScanItems = 8;
-
-__global__ void __launch_bounds__(kBlock) kb_scan(Span sp, BatchArgs A, int which) {
-    __shared__ uint32_t tot;
-    const uint32_t k = blockIdx.x;
+// One CTA per tile of a box's counts, no waits between them (scan_direct_tile).
+// (One CTA per box walked the tiles of the largest box in series: 43 us a scan
+// on 128 boxes of up to 65,536 atoms, 8.3 with a CTA per tile.)
+__global__ void __launch_bounds__(kDirectThreads) kb_scan(Span sp, BatchArgs A) {
+    pdl_wait();  // launched with pdl_launch
+    const uint32_t k = seg_of_warp(sp, blockIdx.x);
     const uint32_t b = sp.box[k];
     const BoxDev& D = A.dev[b];
-    const uint64_t n = sp.start[k + 1] - sp.start[k];
-    const uint32_t* in;
-    uint32_t *out, *cursor;
-    if (which == BA_ROWS) { in = D.rowcount; out = D.offsets; cursor = nullptr; }
-    else if (which == BA_IN) { in = D.in_count; out = D.in_start; cursor = D.in_cursor; }
-    else if (which == BA_GRP) { in = D.grp_cnt; out = D.grp_start; cursor = nullptr; }
-    else { in = D.cell_counts; out = D.cell_start; cursor = D.cell_cursor; }
-    uint32_t carry = 0;
-    for (uint64_t b0 = 0; b0 < n; b0 += (uint64_t)kBlock * kScanItems) {
-        const uint64_t t0 = b0 + (uint64_t)threadIdx.x * kScanItems;
-        uint32_t v[kScanItems];
-        const bool whole = t0 + kScanItems <= n;
-        if (whole) {
-            const uint4 p = *reinterpret_cast<const uint4*>(in + t0);
-            const uint4 q = *reinterpret_cast<const uint4*>(in + t0 + 4);
-            v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w;
-            v[4] = q.x; v[5] = q.y; v[6] = q.z; v[7] = q.w;
-        } else {
-            for (int j = 0; j < kScanItems; ++j) v[j] = t0 + j < n ? in[t0 + j] : 0u;
-        }
-        uint32_t sum = 0;
-        for (int j = 0; j < kScanItems; ++j) sum += v[j];
-        uint32_t run = block_exclusive_scan(sum, &tot) + carry;
-        for (int j = 0; j < kScanItems; ++j) {
-            const uint32_t x = v[j];
-            v[j] = run;
-            run += x;
-        }
-        if (whole) {
-            const uint4 p = make_uint4(v[0], v[1], v[2], v[3]);
-            const uint4 q = make_uint4(v[4], v[5], v[6], v[7]);
-            *reinterpret_cast<uint4*>(out + t0) = p;
-            *reinterpret_cast<uint4*>(out + t0 + 4) = q;
-            if (cursor) {
-                *reinterpret_cast<uint4*>(cursor + t0) = p;
-                *reinterpret_cast<uint4*>(cursor + t0 + 4) = q;
-            }
-        } else {
-            for (int j = 0; j < kScanItems; ++j)
-                if (t0 + j < n) {
-                    out[t0 + j] = v[j];
-                    if (cursor) cursor[t0 + j] = v[j];
-                }
-        }
-        carry += tot;
-        __syncthreads();
+    const uint64_t tile = blockIdx.x - sp.start[k], ntiles = sp.start[k + 1] - sp.start[k];
+    const uint64_t n = sp.base[k];
+    const int which = sp.flag[k];
+    const uint32_t* in = D.cell_counts;
+    const uint32_t* add = nullptr;
+    uint32_t* out = D.sort_start;
+    if (which == BA_NEIGH_CELLS) {
+        out = D.cell_start;
+        add = D.sort_start;
+    } else if (which == BA_ROWS) {
+        in = D.rowcount;
+        out = D.offsets;
+    } else if (which == BA_IN) {
+        in = D.in_count;
+        out = D.in_start;
+    } else if (which == BA_GRP) {
+        in = D.grp_cnt;
+        out = D.grp_start;
     }
-    if (threadIdx.x == 0) {
-        out[n] = carry;
-        if (which == BA_ROWS) A.totals[b] = carry;
-    }
+    const uint32_t total = scan_direct_tile(in, out, n, tile, ntiles, add);
+    if (which == BA_ROWS && tile + 1 == ntiles && threadIdx.x == 0) A.totals[b] = total;
 }
-void b_scan(cudaStream_t st, const Span& sp, const BatchArgs& a, int which) {
-    if (sp.nseg == 0) return;
-    note_launch();
-    kb_scan<<<sp.nseg, kBlock, 0, st>>>(sp, a, which);
-}
-
-__global__ void __launch_bounds__(kBlock) kb_scatter(Span sp, BatchArgs A, int neighbor) {
-    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t) {
-        const BoxDev& D = A.dev[b];
-        const uint32_t cell = (neighbor ? D.atom_cell : D.sort_cell)[i];
-        (neighbor ? D.sorted_atoms : D.sort_perm)[atomicAdd(&D.cell_cursor[cell], 1u)] = (uint32_t)i;
-    });
-}
-void b_scatter(cudaStream_t st, const Span& sp, const BatchArgs& a, bool neighbor) {
+void b_scan(cudaStream_t st, const Span& sp, const BatchArgs& a) {
     if (sp.total == 0) return;
     note_launch();
-    kb_scatter<<<span_wave<kb_scatter>(sp), kBlock, 0, st>>>(sp, a, neighbor ? 1 : 0);
+    pdl_launch(kb_scan, (unsigned)sp.total, kDirectThreads, 0, st, sp, a);
 }
 
-__global__ void __launch_bounds__(kBlock) kb_segsort(Span sp, BatchArgs A, int which) {
-    for_span(sp, [&](uint32_t b, uint64_t s, uint32_t) {
+__global__ void __launch_bounds__(kBlock) kb_scatter(Span sp, BatchArgs A) {
+    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t k) {
         const BoxDev& D = A.dev[b];
-        if (which == BA_IN) insertion_sort(D.in_list, D.in_start[s], D.in_start[s + 1]);
-        else insertion_sort(which == BA_NEIGH_CELLS ? D.sorted_atoms : D.sort_perm,
-                            D.cell_start[s], D.cell_start[s + 1]);
+        const uint32_t cell = D.sort_cell[i];
+        (sp.flag[k] ? D.sort_perm : D.bins)[D.sort_start[cell] + atomicSub(&D.cell_counts[cell], 1u) -
+                                            1u] = (uint32_t)i;
     });
 }
-void b_segsort(cudaStream_t st, const Span& sp, const BatchArgs& a, int which) {
-    if (sp.total == 0) return;
-    note_launch();
-    kb_segsort<<<span_wave<kb_segsort>(sp), kBlock, 0, st>>>(sp, a, which);
-}
+SPAN_LAUNCH(b_scatter, kb_scatter)
+
+// as k_sort_gather
+SPAN_KERNEL(kb_sort_gather, {
+    const uint32_t p = D.bins[i];
+    const uint32_t c = D.sort_cell[p];
+    const uint32_t first = D.sort_start[c];
+    const uint32_t end = D.sort_start[c + 1];
+    uint32_t to = first;
+    for (uint32_t j = first; j < end; ++j) to += D.bins[j] < p;
+    perm_gather_atom(D.set[S.cur], D.set[S.post], to, p, false);
+    D.sort_perm[to] = p;
+    D.sorted_local_cell[to] = c;
+})
+SPAN_LAUNCH(b_sort_gather, kb_sort_gather)
+
+SPAN_KERNEL(kb_segsort, { insertion_sort(D.sort_perm, D.sort_start[i], D.sort_start[i + 1]); })
+SPAN_LAUNCH(b_segsort, kb_segsort)
 
 SPAN_KERNEL(kb_permute_cells, { D.sorted_local_cell[i] = D.sort_cell[D.sort_perm[i]]; })
 SPAN_LAUNCH(b_permute_cells, kb_permute_cells)
@@ -281,6 +234,7 @@ SPAN_LAUNCH(b_perm_gather, kb_perm_gather)
 // f(box, warp tile index inside the box, segment).
 template <class F>
 __device__ __forceinline__ void for_warp_tiles(const Span& sp, F f) {
+    pdl_wait();  // every tile kernel is launched with pdl_launch
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x / 32);
     for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; g < sp.total;
          g += nwarps) {
@@ -302,11 +256,13 @@ __global__ void __launch_bounds__(kBlock) kb_border_faces(Span sp, BatchArgs A, 
 void b_border_faces(cudaStream_t st, const Span& sp, const BatchArgs& a) {
     if (sp.total == 0) return;
     note_launch();
-    kb_border_faces<<<grid_wave<kb_border_faces>(sp.total * 32), kBlock, 0, st>>>(sp, a, border_cats());
+    pdl_launch(kb_border_faces, grid_wave<kb_border_faces>(sp.total * 32), kBlock, 0, st, sp, a,
+               border_cats());
 }
 
 // one CTA per (box, category): exclusive scan of the warp counts
 __global__ void __launch_bounds__(kBlock) kb_border_cat_scan(Span sp, BatchArgs A) {
+    pdl_wait();  // launched with pdl_launch
     const uint32_t seg = blockIdx.x / (kBorderCats + 1), k = blockIdx.x % (kBorderCats + 1);
     const uint32_t b = sp.box[seg];
     const BoxDev& D = A.dev[b];
@@ -317,7 +273,7 @@ __global__ void __launch_bounds__(kBlock) kb_border_cat_scan(Span sp, BatchArgs 
 void b_border_cat_scan(cudaStream_t st, const Span& sp, const BatchArgs& a) {
     if (sp.nseg == 0) return;
     note_launch();
-    kb_border_cat_scan<<<sp.nseg * (kBorderCats + 1), kBlock, 0, st>>>(sp, a);
+    pdl_launch(kb_border_cat_scan, sp.nseg * (kBorderCats + 1), kBlock, 0, st, sp, a);
 }
 
 __global__ void __launch_bounds__(kBlock) kb_border_images(Span sp, BatchArgs A, BorderCats cats) {
@@ -339,7 +295,8 @@ __global__ void __launch_bounds__(kBlock) kb_border_images(Span sp, BatchArgs A,
 void b_border_images(cudaStream_t st, const Span& sp, const BatchArgs& a) {
     if (sp.total == 0) return;
     note_launch();
-    kb_border_images<<<grid_wave<kb_border_images>(sp.total * 32), kBlock, 0, st>>>(sp, a, border_cats());
+    pdl_launch(kb_border_images, grid_wave<kb_border_images>(sp.total * 32), kBlock, 0, st, sp, a,
+               border_cats());
 }
 
 SPAN_KERNEL(kb_forward, {
@@ -348,23 +305,44 @@ SPAN_KERNEL(kb_forward, {
 SPAN_LAUNCH(b_forward, kb_forward)
 
 // ---- neighbor build ---------------------------------------------------------
-SPAN_KERNEL(kb_save_positions, {
-    const AtomCols& c = D.set[S.post];
-    D.lbx[i] = c.x[i];
-    D.lby[i] = c.y[i];
-    D.lbz[i] = c.z[i];
-})
-SPAN_LAUNCH(b_save_positions, kb_save_positions)
+__device__ __forceinline__ SortedViews sorted_views(const BoxDev& D, const BoxStep& S) {
+    SortedViews v;
+    v.c = D.set[S.post];
+    v.sorted = D.sorted_atoms;
+    v.asi = D.asi;
+    v.sp = D.sp;
+    v.spf = S.filter ? D.spf : nullptr;
+    for (int d = 0; d < 3; ++d) v.origin[d] = S.geom.lo[d];
+    v.bp.x = D.lbx;
+    v.bp.y = D.lby;
+    v.bp.z = D.lbz;
+    v.bp.nlocal = S.nlocal;
+    v.atom_in_w = S.uniform;
+    v.clear = nullptr;
+    return v;
+}
 
-SPAN_KERNEL(kb_sorted_views, {
-    sorted_view(D.set[S.post], i, D.sorted_atoms[i], D.asi, D.sp, S.filter ? D.spf : nullptr,
-                S.geom.lo[0], S.geom.lo[1], S.geom.lo[2], BuildPos{}, S.uniform != 0);
+// as k_place_bins and k_ghost_rank
+SPAN_KERNEL(kb_place_bins, {
+    if (i < S.nlocal) {
+        const uint32_t c = D.sorted_local_cell[i];
+        put_sorted(sorted_views(D, S), D.cell_start[c] + ((uint32_t)i - D.sort_start[c]), (uint32_t)i);
+    } else {
+        const uint32_t c = D.atom_cell[i];
+        D.bins[ghost_slots(D.cell_start, D.sort_start, c) + atomicSub(&D.cell_counts[c], 1u) - 1u] =
+            (uint32_t)i;
+    }
 })
-SPAN_LAUNCH(b_sorted_views, kb_sorted_views)
+SPAN_LAUNCH(b_place_bins, kb_place_bins)
+
+SPAN_KERNEL(kb_ghost_rank, {
+    rank_ghost(sorted_views(D, S), (uint32_t)i, D.atom_cell[i], D.cell_start, D.sort_start, D.bins);
+})
+SPAN_LAUNCH(b_ghost_rank, kb_ghost_rank)
 
 __device__ __forceinline__ PairParams pair_params(const BoxDev& D, const BoxStep& S) {
     PairParams p;
-    p.atom_cell = D.atom_cell;
+    p.atom_cell = D.sorted_local_cell;  // read for rows, which are locals
     p.atom_sorted_idx = D.asi;
     p.bin_start = D.cell_start;
     p.sorted_atoms = D.sorted_atoms;
@@ -383,9 +361,9 @@ __device__ __forceinline__ PairParams pair_params(const BoxDev& D, const BoxStep
     p.sf_sq = S.sf_sq;
     p.sf = S.sf;
     p.eps32 = S.eps32;
-    p.in_count = nullptr;
-    p.in_start = nullptr;
-    p.in_list = nullptr;
+    p.in_count = D.in_count;
+    p.in_start = D.in_start;
+    p.in_list = D.in_list;
     p.pre_ranges = S.pre_ranges;
     return p;
 }
@@ -396,7 +374,8 @@ __device__ __forceinline__ void pairs_row(const PairParams& p, uint64_t i, uint3
                                           uint32_t& rk) {
     const Filter<UNIFORM, FP32> test(p);
     const uint32_t K = (uint32_t)p.row_slots;
-    rowcount[i] = row_scan<UNIFORM, FP32, true>(p, test, i, slots + i * K, K, &rk, &cd, flags);
+    rowcount[i] = row_scan<UNIFORM, FP32, true>(p, test, i, slots + i * K, K, &rk, &cd, flags,
+                                                p.in_count);
 }
 
 __device__ __forceinline__ void add_filter_stats(DevFlags* f, uint32_t cd, uint32_t rk) {
@@ -407,46 +386,42 @@ __device__ __forceinline__ void add_filter_stats(DevFlags* f, uint32_t cd, uint3
 // Pair count pass over the rows of every box in the span.  The candidate and
 // recheck statistics are summed per box inside each warp (lanes matched by
 // box) before one atomic per box and warp.
-__global__ void __launch_bounds__(kBlock) kb_pairs_rows(Span sp, BatchArgs A) {
-    const uint64_t chunk = (uint64_t)blockDim.x * kSpanItems;
-    const uint64_t warp0 = threadIdx.x & ~31u;
-    for (uint64_t g0 = (uint64_t)blockIdx.x * chunk; g0 < sp.total;
-         g0 += (uint64_t)gridDim.x * chunk) {
-        const uint64_t gw = g0 + warp0 < sp.total ? g0 + warp0 : g0;
-        uint32_t k = seg_of_warp(sp, gw);
-        uint32_t cur = 0xffffffffu, cd = 0, rk = 0;
-        for (int it = 0; it < kSpanItems; ++it) {
-            const uint64_t g = g0 + (uint64_t)it * blockDim.x + threadIdx.x;
-            if (g >= sp.total) break;
-            while (g >= sp.start[k + 1]) ++k;
-            const uint32_t b = sp.box[k];
-            const uint64_t i = (uint64_t)sp.base[k] + (g - sp.start[k]);
-            if (b != cur) {
-                if (cur != 0xffffffffu) add_filter_stats(A.flags + cur, cd, rk);
-                cur = b;
-                cd = 0;
-                rk = 0;
-            }
-            const BoxDev& D = A.dev[b];
-            const BoxStep& S = A.step[b];
-            const PairParams p = pair_params(D, S);
-            DevFlags* fl = A.flags + b;
-            if (S.uniform) {
-                if (S.filter) pairs_row<true, true>(p, i, D.rowcount, D.row_slots, fl, cd, rk);
-                else pairs_row<true, false>(p, i, D.rowcount, D.row_slots, fl, cd, rk);
-            } else {
-                if (S.filter) pairs_row<false, true>(p, i, D.rowcount, D.row_slots, fl, cd, rk);
-                else pairs_row<false, false>(p, i, D.rowcount, D.row_slots, fl, cd, rk);
-            }
+// (One kernel for every cutoff kind and filter took 106 registers: 109 us on
+// 128 boxes, 1.5 million atoms, against 108 with the transposed lists counted
+// too.)
+template <bool UNIFORM, bool FP32>
+__global__ void __launch_bounds__(kBlock, FP32 ? 3 : 4) kb_pairs_rows(Span sp, BatchArgs A) {
+    uint32_t cur = 0xffffffffu, cd = 0, rk = 0;
+    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t) {
+        if (b != cur) {
+            if (cur != 0xffffffffu) add_filter_stats(A.flags + cur, cd, rk);
+            cur = b;
+            cd = 0;
+            rk = 0;
         }
-        const unsigned peers = __match_any_sync(0xffffffffu, cur);
-        const uint32_t scd = __reduce_add_sync(peers, cd);
-        const uint32_t srk = __reduce_add_sync(peers, rk);
-        if (cur != 0xffffffffu && (int)(threadIdx.x & 31) == __ffs(peers) - 1)
-            add_filter_stats(A.flags + cur, scd, srk);
-    }
+        const BoxDev& D = A.dev[b];
+        pairs_row<UNIFORM, FP32>(pair_params(D, A.step[b]), i, D.rowcount, D.row_slots, A.flags + b,
+                                 cd, rk);
+    });
+    const unsigned peers = __match_any_sync(0xffffffffu, cur);
+    const uint32_t scd = __reduce_add_sync(peers, cd);
+    const uint32_t srk = __reduce_add_sync(peers, rk);
+    if (cur != 0xffffffffu && (int)(threadIdx.x & 31) == __ffs(peers) - 1)
+        add_filter_stats(A.flags + cur, scd, srk);
 }
-SPAN_LAUNCH(b_pairs_rows, kb_pairs_rows)
+
+// A span kernel's instance for the boxes of one cutoff kind and filter.
+#define PAIR_LAUNCH(fn, kern)                                                                      \
+    void fn(cudaStream_t st, const Span& sp, const BatchArgs& a, bool uniform, bool fp32) {        \
+        if (sp.total == 0) return;                                                                 \
+        note_launch();                                                                             \
+        auto go = [&](auto k, unsigned grid) { pdl_launch(k, grid, kBlock, 0, st, sp, a); };       \
+        if (uniform && fp32) go(kern<true, true>, span_wave<kern<true, true>>(sp));                \
+        else if (uniform) go(kern<true, false>, span_wave<kern<true, false>>(sp));                 \
+        else if (fp32) go(kern<false, true>, span_wave<kern<false, true>>(sp));                    \
+        else go(kern<false, false>, span_wave<kern<false, false>>(sp));                            \
+    }
+PAIR_LAUNCH(b_pairs_rows, kb_pairs_rows)
 
 // The staged pair count over warp tiles of every box (the single-system
 // kernel is k_pairs_staged); boxes whose stencil does not fit PairSegs scan
@@ -501,52 +476,55 @@ void b_pairs_staged(cudaStream_t st, const Span& sp, const BatchArgs& a) {
     const uint64_t per = kStageWarps;
     uint64_t blocks = (sp.total + per - 1) / per;
     if (blocks > 148ull * 8ull) blocks = 148ull * 8ull;
-    kb_pairs_staged<<<(unsigned)blocks, kStageWarps * 32, smem, st>>>(sp, a);
+    pdl_launch(kb_pairs_staged, (unsigned)blocks, kStageWarps * 32, smem, st, sp, a);
 }
 
+// Row i into its CSR place (from its slots, or derived again when longer) and
+// into every partner's transposed list, taking the counts back to zero.
 template <bool UNIFORM, bool FP32>
-__device__ __forceinline__ void fill_row(const PairParams& p, uint64_t i, const uint32_t* rowcount,
-                                         const uint32_t* slots, const uint32_t* offsets,
-                                         uint32_t* indices) {
-    const uint32_t K = (uint32_t)p.row_slots;
-    const uint32_t cnt = rowcount[i];
-    uint32_t* out = indices + offsets[i];
-    if (cnt <= K) {
-        const uint32_t* row = slots + i * K;
-        for (uint32_t q = 0; q < cnt; ++q) out[q] = row[q];
-    } else {
+__global__ void __launch_bounds__(kBlock) kb_pairs_fill(Span sp, BatchArgs A) {
+    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t) {
+        const BoxDev& D = A.dev[b];
+        const PairParams p = pair_params(D, A.step[b]);
         const Filter<UNIFORM, FP32> test(p);
-        uint32_t rk = 0, cd = 0;
-        row_scan<UNIFORM, FP32, true>(p, test, i, out, 0xffffffffu, &rk, &cd, nullptr);
-    }
+        fill_row<UNIFORM, FP32>(p, test, i, D.rowcount, D.row_slots, D.offsets, D.indices);
+    });
 }
+PAIR_LAUNCH(b_pairs_fill, kb_pairs_fill)
 
-SPAN_KERNEL(kb_pairs_fill, {
-    const PairParams p = pair_params(D, S);
-    if (S.uniform) {
-        if (S.filter) fill_row<true, true>(p, i, D.rowcount, D.row_slots, D.offsets, D.indices);
-        else fill_row<true, false>(p, i, D.rowcount, D.row_slots, D.offsets, D.indices);
-    } else {
-        if (S.filter) fill_row<false, true>(p, i, D.rowcount, D.row_slots, D.offsets, D.indices);
-        else fill_row<false, false>(p, i, D.rowcount, D.row_slots, D.offsets, D.indices);
-    }
+SPAN_KERNEL(kb_in_sort, {
+    D.in_split[i] = sort_segment(D.in_list, D.in_start[i], D.in_start[i + 1], (uint32_t)i);
 })
-SPAN_LAUNCH(b_pairs_fill, kb_pairs_fill)
-
-SPAN_KERNEL(kb_in_count, {
-    for (uint32_t q = D.offsets[i]; q < D.offsets[i + 1]; ++q) atomicAdd(&D.in_count[D.indices[q]], 1u);
-})
-SPAN_LAUNCH(b_in_count, kb_in_count)
-
-SPAN_KERNEL(kb_in_scatter, {
-    for (uint32_t q = D.offsets[i]; q < D.offsets[i + 1]; ++q)
-        D.in_list[atomicAdd(&D.in_cursor[D.indices[q]], 1u)] = (uint32_t)i;
-})
-SPAN_LAUNCH(b_in_scatter, kb_in_scatter)
+SPAN_LAUNCH(b_in_sort, kb_in_sort)
 
 // ---- force and reverse comm ---------------------------------------------------
-// Register-capped like the single-system force kernel (5 blocks per SM) and
-// launched as one resident wave.
+// The single system's walk (k_force_csr): one thread per root, its images
+// after it, then the fold.  (At 64 registers, four CTAs per SM, the boxes'
+// pointers spill: 159 against 133 us on 1.5 million atoms in 128 boxes.)
+__global__ void __launch_bounds__(kBlock, 3) kb_force_csr(Span sp, BatchArgs A) {
+    for_span(sp, [&](uint32_t b, uint64_t i, uint32_t) {
+        const BoxDev& D = A.dev[b];
+        const BoxStep& S = A.step[b];
+        const AtomCols& c = D.set[S.post];
+        ForceCsr q;
+        q.rad = c.planes[D.radius_plane];
+        q.K = S.K;
+        q.nlocal = S.nlocal;
+        q.newton = S.newton;
+        q.offsets = D.offsets;
+        q.indices = D.indices;
+        q.in_start = D.in_start;
+        q.in_list = D.in_list;
+        q.in_split = D.in_split;
+        q.fold_start = D.fold_start;
+        q.fold_list = D.fold_list;
+        force_csr_items(q, ColLd{c.x, c.y, c.z, q.rad}, c, i);
+        if (S.newton) fold_root(c, S.nlocal, i, D.fold_start, D.fold_list, D.rev);
+    });
+}
+SPAN_LAUNCH(b_force_csr, kb_force_csr)
+
+// The per-atom gather (SOIL_FORCE=gather) with its reverse pass.
 __global__ void __launch_bounds__(kBlock, 5) kb_harmonic(Span sp, BatchArgs A) {
     for_span(sp, [&](uint32_t b, uint64_t i, uint32_t) {
         const BoxDev& D = A.dev[b];
@@ -556,12 +534,7 @@ __global__ void __launch_bounds__(kBlock, 5) kb_harmonic(Span sp, BatchArgs A) {
                       D.indices, D.in_start, D.in_list);
     });
 }
-void b_harmonic(cudaStream_t st, const Span& sp, const BatchArgs& a) {
-    if (sp.total == 0) return;
-    note_launch();
-    const unsigned g = span_grid(sp);
-    kb_harmonic<<<g < 148u * 5u ? g : 148u * 5u, kBlock, 0, st>>>(sp, a);
-}
+SPAN_LAUNCH(b_harmonic, kb_harmonic)
 
 SPAN_KERNEL(kb_reverse, { fold_root(D.set[S.post], S.nlocal, i, D.fold_start, D.fold_list, D.rev); })
 SPAN_LAUNCH(b_reverse, kb_reverse)
@@ -629,7 +602,7 @@ void b_force_walk(cudaStream_t st, const Span& sp, const BatchArgs& a) {
     if (sp.total == 0) return;
     note_launch();
     const unsigned g = span_grid(sp);
-    kb_force_walk<<<g < 148u * 4u ? g : 148u * 4u, kBlock, 0, st>>>(sp, a);
+    pdl_launch(kb_force_walk, g < 148u * 4u ? g : 148u * 4u, kBlock, 0, st, sp, a);
 }
 
 void b_force_grouped(cudaStream_t st, const Span& sp, const BatchArgs& a) {
@@ -637,7 +610,7 @@ void b_force_grouped(cudaStream_t st, const Span& sp, const BatchArgs& a) {
     note_launch();
     uint64_t blocks = (sp.total + kBlock / 32 - 1) / (kBlock / 32);
     if (blocks > 148ull * 3ull) blocks = 148ull * 3ull;  // one resident wave
-    kb_force_grouped<<<(unsigned)blocks, kBlock, 0, st>>>(sp, a);
+    pdl_launch(kb_force_grouped, (unsigned)blocks, kBlock, 0, st, sp, a);
 }
 
 }  // namespace soil

@@ -11,46 +11,6 @@
 
 namespace soil {
 
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kBlock * kScanItems;
-
-// A thread's 8 consecutive items [base, base + 8) (zero past n): two 16-byte
-// loads when the group is whole and aligned, else one by one.
-__device__ __forceinline__ void load8(const uint32_t* in, uint64_t base, uint64_t n,
-                                      uint32_t (&v)[kScanItems]) {
-    if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(in + base) & 15u) == 0) {
-        const uint4 a = *reinterpret_cast<const uint4*>(in + base);
-        const uint4 b = *reinterpret_cast<const uint4*>(in + base + 4);
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) v[k] = (base + k < n) ? in[base + k] : 0u;
-}
-
-// out[base + k] = pre + v[0] + ... + v[k - 1] for the items below n.
-// With add, plus add[base + k].
-__device__ __forceinline__ void store8_scan(uint32_t* out, uint64_t base, uint64_t n,
-                                            const uint32_t (&v)[kScanItems], uint32_t pre,
-                                            const uint32_t* add = nullptr) {
-    uint32_t o[kScanItems];
-    if (add) load8(add, base, n, o);
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        o[k] = add ? o[k] + pre : pre;
-        pre += v[k];
-    }
-    if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(out + base) & 15u) == 0) {
-        *reinterpret_cast<uint4*>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<uint4*>(out + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + k < n) out[base + k] = o[k];
-}
-
 // Up to two independent scans in one launch: blocks [0, tiles0) take tiles of
 // scan 0, the rest tiles of scan 1 (each with its own partials).
 struct ScanJobs {
@@ -176,60 +136,10 @@ __global__ void __launch_bounds__(kBlock) k_scan_down_carry(ScanJobs J) {
 // ticket, the publication of the tile's sum and the wait for the
 // predecessor's, each a trip through L2): 3.0 against 4.1 us on 13,000 counts,
 // 4.5 against 4.9 on 70,000, and one launch for two scans.
-constexpr int kDirectThreads = 1024;
-constexpr uint64_t kDirectTile = (uint64_t)kDirectThreads * kScanItems;
-
-__device__ __forceinline__ uint32_t cta_exclusive_1024(uint32_t v, uint32_t* total) {
-    __shared__ uint32_t w[32];
-    static_assert(kDirectThreads == 32 * 32, "one warp scans the warps' sums");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    if (lane == 31) w[warp] = inc;
-    __syncthreads();
-    uint32_t x = w[lane], xi = x;  // every warp scans the sums: one barrier fewer
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, xi, o);
-        if (lane >= o) xi += t;
-    }
-    *total = __shfl_sync(0xffffffffu, xi, 31);
-    return __shfl_sync(0xffffffffu, xi - x, warp) + inc - v;
-}
-
 __global__ void __launch_bounds__(kDirectThreads) k_scan_direct(ScanJobs J) {
     pdl_wait();  // launched with pdl_launch
-    __shared__ uint32_t before[32];
     const ScanJob q = scan_job(J);
-    const uint64_t base = q.tile * kDirectTile + (uint64_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    load8(q.in, base, q.n, v);
-    uint32_t c = 0;  // this thread's share of the counts before the tile
-    const uint64_t first = q.tile * kDirectTile;
-    if ((reinterpret_cast<uintptr_t>(q.in) & 15u) == 0) {
-        const uint4* in4 = reinterpret_cast<const uint4*>(q.in);
-#pragma unroll 8
-        for (uint64_t k = threadIdx.x; k < first / 4; k += kDirectThreads) {
-            const uint4 a = in4[k];
-            c += a.x + a.y + a.z + a.w;
-        }
-    } else {
-        for (uint64_t k = threadIdx.x; k < first; k += kDirectThreads) c += q.in[k];
-    }
-    c = __reduce_add_sync(0xffffffffu, c);
-    if ((threadIdx.x & 31) == 0) before[threadIdx.x >> 5] = c;
-    uint32_t s = 0, tot;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) s += v[k];
-    const uint32_t in_tile = cta_exclusive_1024(s, &tot);  // its barrier covers `before`
-    const uint32_t carry = __reduce_add_sync(0xffffffffu, before[threadIdx.x & 31]);
-    store8_scan(q.out, base, q.n, v, carry + in_tile, q.add);
-    if (q.tile + 1 == q.ntiles && threadIdx.x == 0)
-        q.out[q.n] = carry + tot + (q.add ? q.add[q.n] : 0u);
+    scan_direct_tile(q.in, q.out, q.n, q.tile, q.ntiles, q.add);
 }
 
 uint64_t scan_temp_words(uint64_t n) { return (n + kScanTile - 1) / kScanTile + 2; }

@@ -358,6 +358,20 @@ int counts_zero(soil_sys* s, uint64_t nc) {
     return SOIL_OK;
 }
 
+// in_count[0, acap) zero, with in_start and in_split, before a pair count of any
+// number of ghosts that the capacity holds.
+int in_counts_zero(soil_sys* s) {
+    TRY(ensure(s, s->in_count, s->acap + 1));
+    TRY(ensure(s, s->in_start, s->acap + 2));
+    TRY(ensure(s, s->in_split, s->acap + 1));
+    const uint64_t have = s->in_zero_at == s->in_count.p ? s->in_zero : 0;
+    if (have < s->acap)
+        CK(cudaMemsetAsync(s->in_count.p + have, 0, (s->acap - have) * 4, s->st));
+    s->in_zero_at = s->in_count.p;
+    s->in_zero = 0;  // counted into now; zero again once pass 2 has consumed it
+    return SOIL_OK;
+}
+
 // After a consuming scatter over every counted atom: all counts are zero.
 void counts_consumed(soil_sys* s) { s->counts_clean = s->cell_counts.cap; }
 
@@ -830,7 +844,6 @@ int sort_plan(soil_sys* s, bool* run, bool* periodic) {
     TRY(ensure(s, s->ghost_tmp, s->acap));
     TRY(ensure(s, s->cell_counts, nc + 1, 0, 2 * nc + 64));
     TRY(ensure(s, s->cell_start, nc + 2, 0, 2 * nc + 64));
-    TRY(ensure(s, s->cell_cursor, nc + 1, 0, 2 * nc + 64));
     TRY(ensure(s, s->scan_tmp, scan_temp_words(nc + s->acap + 2), 0,
                scan_temp_words(2 * nc + s->acap + 64)));
     TRY(ensure(s, s->sort_start, nc + 2, 0, 2 * nc + 64));
@@ -1356,7 +1369,6 @@ int neighbor_plan(soil_sys* s) {
     TRY(ensure(s, s->row_slots, (uint64_t)nl * kRowSlots + 1));
     TRY(ensure(s, s->cell_counts, nc + 1, 0, 2 * nc + 64));
     TRY(ensure(s, s->cell_start, nc + 2, 0, 2 * nc + 64));
-    TRY(ensure(s, s->cell_cursor, nc + 1, 0, 2 * nc + 64));
     TRY(ensure(s, s->scan_tmp, scan_temp_words(nc + s->acap + 2), 0,
                scan_temp_words(2 * nc + s->acap + 64)));
     TRY(ensure(s, s->ghost_tmp, s->acap));
@@ -2396,7 +2408,7 @@ int soil_sys_destroy(soil_sys* s) {
     };
     fr(s->lbx); fr(s->lby); fr(s->lbz);
     fr(s->sort_cell); fr(s->sort_perm); fr(s->sorted_local_cell); fr(s->sort_start); fr(s->ghost_tmp);
-    fr(s->cell_counts); fr(s->cell_start); fr(s->cell_cursor);
+    fr(s->cell_counts); fr(s->cell_start);
     fr(s->atom_cell); fr(s->sorted_atoms); fr(s->asi); fr(s->rowcount); fr(s->offsets); fr(s->indices);
     fr(s->row_slots); fr(s->sp); fr(s->spf);
     fr(s->sel_flag); fr(s->sel_pos); fr(s->sel_out); fr(s->sel_cnt); fr(s->ext);

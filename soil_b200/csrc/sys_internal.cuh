@@ -127,7 +127,7 @@ struct soil_sys {
     DArr<uint32_t> sort_cell, sort_perm, sorted_local_cell;
     DArr<uint32_t> sort_start;  // the spatial sort's cell starts (its locals' bins)
     DArr<uint32_t> ghost_tmp;   // the neighbor build's unordered ghost slots
-    DArr<uint32_t> cell_counts, cell_start, cell_cursor;
+    DArr<uint32_t> cell_counts, cell_start;
     // cell_counts[0, counts_clean) is known to be zero (the consuming scatters
     // leave it so); counts_at: the allocation that holds
     uint64_t counts_clean = 0;
@@ -287,6 +287,9 @@ int sync(soil_sys* s);
 int check_launch(soil_sys* s);
 // cell_counts[0, nc) zero before a counting pass
 int counts_zero(soil_sys* s, uint64_t nc);
+void counts_consumed(soil_sys* s);
+int in_counts_zero(soil_sys* s);
+int build_in_lists(soil_sys* s);
 // The pair scan's stencil: offsets (ascending) merged into runs of consecutive
 // cells, as (offset, cells) pairs; without newton the own cell (offset 0),
 // which the scan takes first, is left out.

@@ -223,3 +223,53 @@ def test_batch_rejects_unsupported(ctx):
     batch.close()
     s.close()
     m.close()
+
+
+def test_boxes_of_several_scan_tiles_and_kinds(ctx):
+    """Boxes whose rows, cells and incoming lists take one tile of the scans or
+    several, with a uniform cutoff or not and either filter, in one batch."""
+    ws = []
+    for i, n in enumerate((300, 8192, 8193, 20011)):
+        make = W.mono if i % 2 else W.poly
+        ws.append(make("tiles", 220 + i, n, 0.4, 1e-4, 0, harmonic_k=1e3,
+                       shear_rate=0.1 if i < 2 else 0.0,
+                       filter=abi.SOIL_FILTER_FP32_RECHECK if i >= 2 else abi.SOIL_FILTER_FP64))
+        ws[-1].vel *= 5.0
+    alone = [system.from_workload(ctx, w) for w in ws]
+    mixed = [system.from_workload(ctx, w) for w in ws]
+    batch = system.Batch(ctx)
+    for s in mixed:
+        batch.add(s)
+    for n in (1, 7, 12):
+        batch.step(n)
+        for s in alone:
+            s.step(n)
+    for k, (a, b) in enumerate(zip(alone, mixed)):
+        assert_same(a, b, f"box {k}")
+    batch.close()
+    for s in alone + mixed:
+        s.close()
+
+
+def test_box_that_got_its_consumer_after_its_lists(ctx):
+    """A box built without a consumer, given one and batched while it keeps
+    its lists: the transposed lists are made when it joins."""
+    w = W.poly("late", 230, 3000, 0.45, 1e-5, 0)
+    pair_ = []
+    for _ in range(2):
+        s = system.System(ctx, w.box, w.cfg, w.dt)
+        rc = s.register_column("radius", 1, abi.SOIL_COL_FORWARD)
+        s.add_atoms(w.tag, w.pos, w.vel, w.mass, w.cutoff, columns=[w.radius])
+        s.setup()
+        s.step(3)
+        s.set_harmonic(1e3, rc)
+        pair_.append(s)
+    alone, member = pair_
+    batch = system.Batch(ctx)
+    batch.add(member)
+    batch.step(9)
+    alone.step(9)
+    assert_same(alone, member, "late consumer")
+    batch.close()
+    alone.close()
+    member.close()
