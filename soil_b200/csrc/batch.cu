@@ -144,8 +144,7 @@ enum { G_INTEGRATE, G_SORT, G_SORT_APPLY, G_BORDERS, G_NEIGHBOR, G_FORCE };
 int balloc(soil_batch* b, void** p, uint64_t bytes) {
     if (bytes == 0) bytes = 16;
     TRY(ctx_reserve(b->ctx, bytes));
-    if (cudaMallocFromPoolAsync(p, bytes, b->ctx->pool, b->st) != cudaSuccess) {
-        cudaGetLastError();
+    if (pool_alloc(b->ctx, b->st, p, bytes) != cudaSuccess) {
         ctx_release(b->ctx, bytes);
         return fail(b->ctx, SOIL_ERR_OOM, "device allocation of %llu bytes failed",
                     (unsigned long long)bytes);

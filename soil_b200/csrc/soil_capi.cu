@@ -71,14 +71,91 @@ void ctx_release(soil_ctx* ctx, uint64_t bytes) {
     ctx->frees += 1;
 }
 
+constexpr size_t kHostBlockBytes = 512, kHostSlabBytes = 64 << 10, kKeptStreams = 64;
+constexpr uint64_t kKeptSlabBytes = 512ull << 20;
+
+// The kept slabs back to the pool; false when there are none.
+bool kept_slabs_release(soil_ctx* ctx, cudaStream_t st) {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    if (ctx->slabs.empty()) return false;
+    for (const auto& b : ctx->slabs) cudaFreeAsync(b.second, st);
+    ctx->slabs.clear();
+    ctx->slab_bytes = 0;
+    return true;
+}
+
+// Stream-ordered from the context's pool: no device-wide synchronisation, and
+// freed memory stays in the pool for the next growth.
+cudaError_t pool_alloc(soil_ctx* ctx, cudaStream_t st, void** p, uint64_t bytes) {
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e == cudaErrorMemoryAllocation && kept_slabs_release(ctx, st)) {
+        e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    return e;
+}
+
+namespace {
+
+// A slab some system left, of at least `size` bytes, or else of at least
+// `least`; its size goes to *got (0: none).
+char* kept_slab(soil_ctx* ctx, uint64_t size, uint64_t least, uint64_t* got) {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    auto it = ctx->slabs.lower_bound(size);
+    if (it == ctx->slabs.end()) it = ctx->slabs.lower_bound(least);
+    *got = 0;
+    if (it == ctx->slabs.end()) return nullptr;
+    char* p = it->second;
+    *got = it->first;
+    ctx->slab_bytes -= it->first;
+    ctx->slabs.erase(it);
+    return p;
+}
+
+uint64_t arena_round(uint64_t bytes) { return (std::max<uint64_t>(bytes, 1) + 255) / 256 * 256; }
+
+cudaError_t arena_alloc(soil_sys* s, void** p, uint64_t bytes) {
+    Arena& a = s->arena;
+    // a returned block that is not much larger (its tail stays unused)
+    const auto it = a.free.lower_bound(bytes);
+    if (it != a.free.end() && it->first <= bytes + bytes / 2 + 4096) {
+        *p = it->second;
+        a.free.erase(it);
+        return cudaSuccess;
+    }
+    for (size_t k = a.slabs.size(); k-- > 0;) {
+        Arena::Slab& b = a.slabs[k];
+        if (b.size - b.used >= bytes) {
+            *p = b.p + b.used;
+            b.used += bytes;
+            return cudaSuccess;
+        }
+    }
+    uint64_t size = std::max(bytes, std::min<uint64_t>(std::max<uint64_t>(a.total, 1u << 20), 32u << 20));
+    uint64_t kept;
+    void* q = kept_slab(s->ctx, size, bytes, &kept);
+    if (kept) size = kept;
+    cudaError_t e = q ? cudaSuccess : pool_alloc(s->ctx, s->st, &q, size);
+    if (e != cudaSuccess && size > bytes) {
+        size = bytes;
+        e = pool_alloc(s->ctx, s->st, &q, size);
+    }
+    if (e != cudaSuccess) return e;
+    a.slabs.push_back({(char*)q, size, bytes});
+    a.total += size;
+    *p = q;
+    return cudaSuccess;
+}
+
+}  // namespace
+
 int dev_alloc(soil_sys* s, void** p, uint64_t bytes) {
     if (bytes == 0) bytes = 16;
     TRY(ctx_reserve(s->ctx, bytes));
-    // stream-ordered from the context's pool: no device-wide synchronisation,
-    // and freed memory stays in the pool for the next growth
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, s->ctx->pool, s->st);
+    const uint64_t r = arena_round(bytes);
+    const cudaError_t e = r > kArenaMax ? pool_alloc(s->ctx, s->st, p, bytes) : arena_alloc(s, p, r);
     if (e != cudaSuccess) {
-        cudaGetLastError();
         ctx_release(s->ctx, bytes);
         return fail(s->ctx, SOIL_ERR_OOM, "cudaMallocAsync(%llu): %s", (unsigned long long)bytes,
                     cudaGetErrorString(e));
@@ -89,9 +166,75 @@ int dev_alloc(soil_sys* s, void** p, uint64_t bytes) {
 // Frees in stream order after every use already enqueued on the system's stream.
 void dev_free(soil_sys* s, void* p, uint64_t bytes) {
     if (!p) return;
-    cudaFreeAsync(p, s->st);
     if (bytes == 0) bytes = 16;
+    const uint64_t r = arena_round(bytes);
+    if (r > kArenaMax) cudaFreeAsync(p, s->st);
+    else s->arena.free.emplace(r, (char*)p);
     ctx_release(s->ctx, bytes);
+}
+
+// The slabs back to the context (or its pool), once every array is gone and the
+// stream has drained.
+void arena_free(soil_sys* s) {
+    std::lock_guard<std::mutex> g(s->ctx->mu);
+    for (const Arena::Slab& b : s->arena.slabs) {
+        if (s->ctx->slab_bytes + b.size <= kKeptSlabBytes) {
+            s->ctx->slabs.emplace(b.size, b.p);
+            s->ctx->slab_bytes += b.size;
+        } else {
+            cudaFreeAsync(b.p, s->st);
+        }
+    }
+    s->arena = Arena{};
+}
+
+// ---- what systems take from their context and give back -----------------------
+int host_block_take(soil_ctx* ctx, HostBlock* b) {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    if (ctx->host_free.empty()) {
+        uint8_t *h = nullptr, *d = nullptr;
+        if (cudaHostAlloc((void**)&h, kHostSlabBytes, cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer((void**)&d, h, 0) != cudaSuccess) {
+            cudaGetLastError();
+            if (h) cudaFreeHost(h);
+            return SOIL_ERR_OOM;
+        }
+        ctx->host_slabs.push_back(h);
+        for (size_t k = 0; k + kHostBlockBytes <= kHostSlabBytes; k += kHostBlockBytes)
+            ctx->host_free.push_back({h + k, d + k});
+    }
+    *b = ctx->host_free.back();
+    ctx->host_free.pop_back();
+    std::memset(b->h, 0, kHostBlockBytes);
+    return SOIL_OK;
+}
+
+void host_block_give(soil_ctx* ctx, const HostBlock& b) {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    ctx->host_free.push_back(b);
+}
+
+cudaError_t stream_take(soil_ctx* ctx, cudaStream_t* st) {
+    {
+        std::lock_guard<std::mutex> g(ctx->mu);
+        if (!ctx->streams.empty()) {
+            *st = ctx->streams.back();
+            ctx->streams.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+}
+
+void stream_give(soil_ctx* ctx, cudaStream_t st) {
+    {
+        std::lock_guard<std::mutex> g(ctx->mu);
+        if (ctx->streams.size() < kKeptStreams) {
+            ctx->streams.push_back(st);
+            return;
+        }
+    }
+    cudaStreamDestroy(st);
 }
 
 // ---- per-atom columns -------------------------------------------------------
@@ -2315,6 +2458,11 @@ int soil_ctx_create(int device, uint64_t hbm_budget_bytes, soil_ctx** out) {
 }
 
 int soil_ctx_destroy(soil_ctx* ctx) {
+    if (ctx) {
+        kept_slabs_release(ctx, ctx->streams.empty() ? nullptr : ctx->streams[0]);
+        for (cudaStream_t st : ctx->streams) cudaStreamDestroy(st);
+        for (uint8_t* h : ctx->host_slabs) cudaFreeHost(h);
+    }
     // the pool's memory goes back once the last outstanding free has run
     if (ctx && ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
@@ -2355,7 +2503,7 @@ int soil_sys_create(soil_ctx* ctx, const soil_box* box, const soil_neigh_cfg* cf
     soil_sys* s = new (std::nothrow) soil_sys();
     if (!s) return SOIL_ERR_OOM;
     s->ctx = ctx;
-    if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) {
+    if (stream_take(ctx, &s->st) != cudaSuccess) {
         cudaGetLastError();
         delete s;
         return fail(ctx, SOIL_ERR_CUDA, "cudaStreamCreate failed");
@@ -2379,17 +2527,16 @@ int soil_sys_create(soil_ctx* ctx, const soil_box* box, const soil_neigh_cfg* cf
     s->newton = cfg->newton != 0;
     s->additive_skin = cfg->additive_skin;
     s->filter = cfg->filter;
-    int r;
-    if ((r = dev_alloc(s, (void**)&s->dflags, sizeof(DevFlags))) != SOIL_OK ||
-        cudaHostAlloc((void**)&s->hflags, sizeof(DevFlags), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostAlloc((void**)&s->hword, kHostWords * 4, cudaHostAllocMapped) !=
-            cudaSuccess ||
-        cudaHostGetDevicePointer((void**)&s->hflags_dev, s->hflags, 0) != cudaSuccess ||
-        cudaHostGetDevicePointer((void**)&s->hword_dev, s->hword, 0) != cudaSuccess) {
-        cudaGetLastError();
+    static_assert(sizeof(DevFlags) <= 64 && 64 + kHostWords * 4 <= kHostBlockBytes, "host block");
+    const int r = dev_alloc(s, (void**)&s->dflags, sizeof(DevFlags));
+    if (r != SOIL_OK || host_block_take(ctx, &s->host) != SOIL_OK) {
         soil_sys_destroy(s);
         return r != SOIL_OK ? r : fail(ctx, SOIL_ERR_OOM, "pinned allocation failed");
     }
+    s->hflags = (DevFlags*)s->host.h;
+    s->hflags_dev = (DevFlags*)s->host.d;
+    s->hword = (uint32_t*)(s->host.h + 64);
+    s->hword_dev = (uint32_t*)(s->host.d + 64);
     cudaMemsetAsync(s->dflags, 0, sizeof(DevFlags), s->st);
     *out = s;
     return SOIL_OK;
@@ -2428,9 +2575,9 @@ int soil_sys_destroy(soil_sys* s) {
     for (cudaEvent_t e : s->ev_pool) cudaEventDestroy(e);
     if (s->ev_counts) cudaEventDestroy(s->ev_counts);
     if (s->dflags) dev_free(s, s->dflags, sizeof(DevFlags));
-    if (s->hflags) cudaFreeHost(s->hflags);
-    if (s->hword) cudaFreeHost(s->hword);
-    if (s->st) cudaStreamDestroy(s->st);
+    arena_free(s);
+    if (s->host.h) host_block_give(s->ctx, s->host);
+    if (s->st) stream_give(s->ctx, s->st);
     delete s;
     return SOIL_OK;
 }
@@ -2700,8 +2847,8 @@ int soil_sys_get_atoms(soil_sys* s, uint64_t first, uint64_t n, uint32_t* tag, d
     auto get3 = [&](double* dst, double* a, double* b, double* c) -> int {
         if (!dst) return SOIL_OK;
         launch_interleave3(s->st, n, s->stage.p, a + f, b + f, c + f);
+        // (the next use of the staging array follows this copy in the stream)
         CK(cudaMemcpyAsync(dst, s->stage.p, n * 24, cudaMemcpyDeviceToHost, s->st));
-        CK(cudaStreamSynchronize(s->st));
         return SOIL_OK;
     };
     TRY(get3(pos3, s->A.x, s->A.y, s->A.z));

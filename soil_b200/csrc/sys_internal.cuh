@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cfloat>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -12,6 +13,12 @@
 
 using namespace soil;
 
+// A system's block of pinned host memory, as the host and the device address it.
+struct HostBlock {
+    uint8_t* h = nullptr;
+    uint8_t* d = nullptr;
+};
+
 struct soil_ctx {
     int device = 0;
     uint64_t budget = 0;
@@ -19,7 +26,17 @@ struct soil_ctx {
     std::string err;
     uint64_t allocs = 0, frees = 0;
     cudaMemPool_t pool = nullptr;  // stream-ordered device memory of every system and batch
-    mutable std::mutex mu;  // guards in_use, the counters and err
+    // What systems that are gone leave for the next ones, once their stream has
+    // drained: pinned blocks (cut from slabs of 64 KB, so as many as systems
+    // lived at once), at most kKeptStreams streams, and at most kKeptSlabBytes
+    // of device slabs, which also go back when an allocation fails.  All of it
+    // goes back with the context.
+    std::vector<uint8_t*> host_slabs;
+    std::vector<HostBlock> host_free;
+    std::vector<cudaStream_t> streams;
+    std::multimap<uint64_t, char*> slabs;  // by size
+    uint64_t slab_bytes = 0;
+    mutable std::mutex mu;  // guards in_use, the counters, err and the lists above
 };
 
 namespace soil_host {
@@ -32,6 +49,23 @@ struct ColMeta {
     unsigned flags;
     int plane0;
 };
+
+// Device memory of one system: its arrays are cut from a few slabs of the
+// context's pool, each twice as large as all before it, because a driver call
+// per array costs microseconds (milliseconds once many streams share the
+// pool: the first step of 128 boxes spent a second in 8,000 of them).  What
+// an array gives back serves the system's next arrays, in the order of its one
+// stream.  Arrays above kArenaMax come from the pool directly.
+struct Arena {
+    struct Slab {
+        char* p;
+        uint64_t size, used;
+    };
+    std::vector<Slab> slabs;
+    std::multimap<uint64_t, char*> free;  // by size
+    uint64_t total = 0;
+};
+constexpr uint64_t kArenaMax = 8ull << 20;
 
 template <class T>
 struct DArr {
@@ -55,6 +89,8 @@ using soil_host::SwapHost;
 struct soil_sys {
     soil_ctx* ctx = nullptr;
     cudaStream_t st = nullptr;
+    soil_host::Arena arena;
+    HostBlock host;  // hflags and hword
     double dt = 1.0;
 
     // ---- Domain (domain.rs:105-142), one rank ----
@@ -241,6 +277,7 @@ int fail(soil_ctx* ctx, int status, const char* fmt, ...);
 
 int ctx_reserve(soil_ctx* ctx, uint64_t bytes);
 void ctx_release(soil_ctx* ctx, uint64_t bytes);
+cudaError_t pool_alloc(soil_ctx* ctx, cudaStream_t st, void** p, uint64_t bytes);
 int dev_alloc(soil_sys* s, void** p, uint64_t bytes);
 void dev_free(soil_sys* s, void* p, uint64_t bytes);
 
