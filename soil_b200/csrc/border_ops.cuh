@@ -102,12 +102,15 @@ __device__ __forceinline__ uint32_t image_index(const BorderWarpSmem& sm, int k,
 // category k (nlocal + the totals of the categories before it).  offs holds
 // offsets inside the tile's scan chunk; cpre (NULL: a single chunk) the
 // chunks' prefixes.  sm: this warp's scratch.  host_bs (optional): the host's
-// copy of bs, which gets the capacity word too.
+// copy of bs, which gets the capacity word too.  multi (optional): the roots
+// with two images or more, in no particular order, counted in
+// bs[kBorderMulti].
 __device__ __forceinline__ void border_warp_images(
     const AtomCols& c, uint64_t nlocal, uint64_t cap, const BorderCats& cats, const uint8_t* face,
     const uint32_t* offs, const uint32_t* cpre, uint64_t nchunks, uint64_t nw, uint64_t w, uint32_t lane,
     uint32_t base_lane, uint32_t* bs, uint32_t* root, uint32_t* chain, uint32_t* const* send,
-    uint32_t* fold_start, uint32_t* fold_list, BorderWarpSmem& sm, uint32_t* host_bs = nullptr) {
+    uint32_t* fold_start, uint32_t* fold_list, BorderWarpSmem& sm, uint32_t* host_bs = nullptr,
+    uint32_t* multi = nullptr) {
     const unsigned below = (1u << lane) - 1u;
     const uint64_t r = w * 32 + lane;
     const uint32_t bits = r < nlocal ? face[r] : 0u;
@@ -147,6 +150,13 @@ __device__ __forceinline__ void border_warp_images(
     const uint32_t fs = fold0 + warp_exclusive_sum(own, lane);
     if (r < nlocal) fold_start[r] = fs;
     if (r + 1 == nlocal) fold_start[nlocal] = fs + own;
+    if (multi) {
+        const unsigned many = __ballot_sync(0xffffffffu, own >= 2);
+        uint32_t at = 0;
+        if (many && lane == 0) at = atomicAdd(&bs[kBorderMulti], (uint32_t)__popc(many));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (own >= 2) multi[at + __popc(many & below)] = (uint32_t)r;
+    }
     if (bits) {
         for (uint32_t mk = mine_cats; mk; mk &= mk - 1) {
             const int k = __ffs(mk) - 1;

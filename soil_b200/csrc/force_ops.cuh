@@ -338,6 +338,127 @@ __device__ __forceinline__ void force_csr_root(const ForceCsr& q, const AtomCols
     else force_csr_root_ld<FOLD>(q, ColLd{c.x, c.y, c.z, q.rad}, c, rev, t);
 }
 
+// The same forces by 8 lanes per root (all 32 lanes of a warp call; t: the
+// root of the lane's group, valid: it has one), for roots with at most 7
+// images.  Lane j
+// holds item j of the group (0: the root, j: its j-th image in fold order); the
+// items' entries are numbered through, 8 evaluated at a time, and every lane
+// adds the results in entry order, keeping its own item's sum; the fold moves
+// the images' sums to their parents' lanes in fold order.  Same operations in
+// the same order as force_csr_root.  What bounds it is one chain of dependent
+// loads (fold list, list bounds, entry, partner) instead of one per image.
+template <bool FOLD>
+__device__ __forceinline__ void force_group_root(const ForceCsr& q, const AtomCols& c,
+                                                 const PlaneList& rev, uint64_t t, bool valid) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t g = threadIdx.x & 7u;
+    const uint32_t f0 = valid ? q.fold_start[t] : 0u;
+    const uint32_t nimg = valid ? q.fold_start[t + 1] - f0 : 0u;
+    // this lane's item
+    uint64_t a = t;
+    uint32_t gi = 0, qs = 0, nin = 0, npre = 0, rs = 0, nrow = 0, org = 0;
+    double4 pa = make_double4(0.0, 0.0, 0.0, 0.0);
+    const bool mine = valid && g <= nimg;
+    if (mine) {
+        if (g) {
+            gi = q.fold_list[f0 + g - 1];
+            a = q.nlocal + gi;
+            org = (uint32_t)c.origin[a];
+        }
+        if (g == 0 || q.newton) {
+            qs = q.in_start[a];
+            nin = q.in_start[a + 1] - qs;
+        }
+        if (g == 0) {
+            npre = q.in_split[a];
+            rs = q.offsets[t];
+            nrow = q.offsets[t + 1] - rs;
+        }
+        pa = make_double4(c.x[a], c.y[a], c.z[a], q.rad[a]);
+    }
+    // items numbered through: this lane's are entries [from, to)
+    const uint32_t n = nin + nrow;
+    uint32_t to = n;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kAll, to, o, 8);
+        if (g >= (uint32_t)o) to += v;
+    }
+    const uint32_t total = __shfl_sync(kAll, to, 7, 8);
+    uint32_t ends[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ends[j] = __shfl_sync(kAll, to, j, 8);
+    const uint32_t rounds = __reduce_max_sync(kAll, (total + 7) / 8);
+    double Fx = 0.0, Fy = 0.0, Fz = 0.0;     // this lane's item
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t k = r * 8 + g;
+        int item = 0;
+#pragma unroll
+        for (int j = 0; j < 7; ++j) item += k >= ends[j];
+        // the item's lists and position from its lane
+        const uint32_t iqs = __shfl_sync(kAll, qs, item, 8), inpre = __shfl_sync(kAll, npre, 0, 8);
+        const uint32_t irs = __shfl_sync(kAll, rs, 0, 8), inrow = __shfl_sync(kAll, nrow, 0, 8);
+        const uint32_t base = __shfl_sync(kAll, to - n, item, 8);
+        const double px = __shfl_sync(kAll, pa.x, item, 8), py = __shfl_sync(kAll, pa.y, item, 8);
+        const double pz = __shfl_sync(kAll, pa.z, item, 8), pr = __shfl_sync(kAll, pa.w, item, 8);
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        bool touch = false;
+        if (k < total) {
+            const uint32_t e = k - base;
+            uint32_t o;
+            if (item) o = q.in_list[iqs + e];
+            else if (e < inpre) o = q.in_list[iqs + e];
+            else if (e < inpre + inrow) o = q.indices[irs + (e - inpre)];
+            else o = q.in_list[iqs + (e - inrow)];
+            touch = pair_force(px, py, pz, pr, c.x[o], c.y[o], c.z[o], q.rad[o], q.K, fx, fy, fz);
+        }
+        const unsigned hits = __ballot_sync(kAll, touch) >> ((threadIdx.x & 31u) & ~7u);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double ex = __shfl_sync(kAll, fx, j, 8), ey = __shfl_sync(kAll, fy, j, 8);
+            const double ez = __shfl_sync(kAll, fz, j, 8);
+            const uint32_t kk = r * 8 + j;
+            if (((hits >> j) & 1u) && kk >= to - n && kk < to) {
+                Fx = Fx + ex;
+                Fy = Fy + ey;
+                Fz = Fz + ez;
+            }
+        }
+    }
+    if (FOLD) {  // fold_root's order
+        uint32_t par = 0;  // this image's parent item
+        if (mine && g && org >= q.nlocal) par = 0xffu;
+#pragma unroll
+        for (int j = 1; j < 8; ++j) {
+            const uint32_t gj = __shfl_sync(kAll, gi, j, 8);
+            if (par && (uint32_t)j <= nimg && org == q.nlocal + gj) par = (uint32_t)j;
+        }
+        const uint32_t most = __reduce_max_sync(kAll, nimg);
+        for (uint32_t j = 1; j <= most; ++j) {
+            const double ex = __shfl_sync(kAll, Fx, j, 8), ey = __shfl_sync(kAll, Fy, j, 8);
+            const double ez = __shfl_sync(kAll, Fz, j, 8);
+            const uint32_t p = __shfl_sync(kAll, par, j, 8);
+            if (j <= nimg && p == g) {
+                Fx = Fx + ex;
+                Fy = Fy + ey;
+                Fz = Fz + ez;
+            }
+        }
+        if (valid && g == 0)
+            for (uint32_t f = f0; f < f0 + nimg && rev.n; ++f) {
+                const uint64_t gh = q.nlocal + q.fold_list[f];
+                const uint32_t o = (uint32_t)c.origin[gh];
+                for (int k = 0; k < rev.n; ++k)
+                    c.planes[rev.idx[k]][o] = c.planes[rev.idx[k]][o] + c.planes[rev.idx[k]][gh];
+            }
+    }
+    if (mine) {
+        c.fx[a] = Fx;
+        c.fy[a] = Fy;
+        c.fz[a] = Fz;
+    }
+}
+
 // Entry k of a group's sequence.
 struct SeqIdx {
     const uint32_t* seq;

@@ -116,6 +116,24 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_csr(ForceCsr q, AtomCols c,
     pdl_wait();  // launched with pdl_launch
     if (trip && *trip) return;  // the step rebuilds: its forces come later
     if (!guard_open(guard)) return;
+    if (q.multi) {
+        // The roots with two images or more (edges and corners of the box) by 8
+        // lanes each, spread from the last block on (the first ones may have
+        // one block of roots more); every other root and its image, if it has
+        // one, by its thread below.  A corner root's eight items in series on
+        // one thread set the kernel's time on systems of a few waves: 20.2
+        // against 16.5 us on 200,003 atoms, 41.1 against 39.4 on 600,011.
+        const uint64_t n = *q.nmulti;
+        const uint64_t warp = (uint64_t)(gridDim.x - 1 - blockIdx.x) * (kBlock / 32) + threadIdx.x / 32;
+        for (uint64_t k = warp * 4; k < n; k += (uint64_t)gridDim.x * (kBlock / 32) * 4) {
+            const uint64_t at = k + (threadIdx.x & 31) / 8;
+            force_group_root<FOLD>(q, c, rev, at < n ? q.multi[at] : 0, at < n);
+        }
+        for (uint64_t t = (uint64_t)blockIdx.x * kBlock + threadIdx.x; t < q.nlocal;
+             t += (uint64_t)gridDim.x * kBlock)
+            if (q.fold_start[t + 1] - q.fold_start[t] < 2) force_csr_root<FOLD, PK>(q, c, rev, t);
+        return;
+    }
     // grid-stride over whole blocks of kBlock roots, so a block's order
     // permutes its own roots
     for (uint64_t b = (uint64_t)blockIdx.x * kBlock; b < q.nlocal; b += (uint64_t)gridDim.x * kBlock) {
@@ -124,134 +142,22 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_csr(ForceCsr q, AtomCols c,
     }
 }
 
-// The same forces by 8 lanes per root, for systems whose roots do not fill the
-// chip with one thread each and whose roots have at most 7 images.  Lane j
-// holds item j of the group (0: the root, j: its j-th image in fold order); the
-// items' entries are numbered through, 8 evaluated at a time, and every lane
-// adds the results in entry order, keeping its own item's sum; the fold moves
-// the images' sums to their parents' lanes in fold order.  Same operations in
-// the same order as force_csr_root.  What bounds it is one chain of dependent
-// loads (fold list, list bounds, entry, partner) instead of one per image.
+// 8 lanes per root for a system whose roots do not fill the chip with one
+// thread each.
 template <bool FOLD>
 __global__ void __launch_bounds__(kBlock, 4) k_force_group(ForceCsr q, AtomCols c, PlaneList rev,
                                                            const uint32_t* trip, FillGuard guard) {
     pdl_wait();  // launched with pdl_launch
     if (trip && *trip) return;  // the step rebuilds: its forces come later
     if (!guard_open(guard)) return;
-    constexpr unsigned kAll = 0xffffffffu;
-    const uint32_t g = threadIdx.x & 7u;
     const uint64_t t = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) / 8;
-    const bool valid = t < q.nlocal;
-    const uint32_t f0 = valid ? q.fold_start[t] : 0u;
-    const uint32_t nimg = valid ? q.fold_start[t + 1] - f0 : 0u;
-    // this lane's item
-    uint64_t a = t;
-    uint32_t gi = 0, qs = 0, nin = 0, npre = 0, rs = 0, nrow = 0, org = 0;
-    double4 pa = make_double4(0.0, 0.0, 0.0, 0.0);
-    const bool mine = valid && g <= nimg;
-    if (mine) {
-        if (g) {
-            gi = q.fold_list[f0 + g - 1];
-            a = q.nlocal + gi;
-            org = (uint32_t)c.origin[a];
-        }
-        if (g == 0 || q.newton) {
-            qs = q.in_start[a];
-            nin = q.in_start[a + 1] - qs;
-        }
-        if (g == 0) {
-            npre = q.in_split[a];
-            rs = q.offsets[t];
-            nrow = q.offsets[t + 1] - rs;
-        }
-        pa = make_double4(c.x[a], c.y[a], c.z[a], q.rad[a]);
-    }
-    // items numbered through: this lane's are entries [from, to)
-    const uint32_t n = nin + nrow;
-    uint32_t to = n;
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(kAll, to, o, 8);
-        if (g >= (uint32_t)o) to += v;
-    }
-    const uint32_t total = __shfl_sync(kAll, to, 7, 8);
-    uint32_t ends[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ends[j] = __shfl_sync(kAll, to, j, 8);
-    const uint32_t rounds = __reduce_max_sync(kAll, (total + 7) / 8);
-    double Fx = 0.0, Fy = 0.0, Fz = 0.0;     // this lane's item
-    for (uint32_t r = 0; r < rounds; ++r) {
-        const uint32_t k = r * 8 + g;
-        int item = 0;
-#pragma unroll
-        for (int j = 0; j < 7; ++j) item += k >= ends[j];
-        // the item's lists and position from its lane
-        const uint32_t iqs = __shfl_sync(kAll, qs, item, 8), inpre = __shfl_sync(kAll, npre, 0, 8);
-        const uint32_t irs = __shfl_sync(kAll, rs, 0, 8), inrow = __shfl_sync(kAll, nrow, 0, 8);
-        const uint32_t base = __shfl_sync(kAll, to - n, item, 8);
-        const double px = __shfl_sync(kAll, pa.x, item, 8), py = __shfl_sync(kAll, pa.y, item, 8);
-        const double pz = __shfl_sync(kAll, pa.z, item, 8), pr = __shfl_sync(kAll, pa.w, item, 8);
-        double fx = 0.0, fy = 0.0, fz = 0.0;
-        bool touch = false;
-        if (k < total) {
-            const uint32_t e = k - base;
-            uint32_t o;
-            if (item) o = q.in_list[iqs + e];
-            else if (e < inpre) o = q.in_list[iqs + e];
-            else if (e < inpre + inrow) o = q.indices[irs + (e - inpre)];
-            else o = q.in_list[iqs + (e - inrow)];
-            touch = pair_force(px, py, pz, pr, c.x[o], c.y[o], c.z[o], q.rad[o], q.K, fx, fy, fz);
-        }
-        const unsigned hits = __ballot_sync(kAll, touch) >> ((threadIdx.x & 31u) & ~7u);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const double ex = __shfl_sync(kAll, fx, j, 8), ey = __shfl_sync(kAll, fy, j, 8);
-            const double ez = __shfl_sync(kAll, fz, j, 8);
-            const uint32_t kk = r * 8 + j;
-            if (((hits >> j) & 1u) && kk >= to - n && kk < to) {
-                Fx = Fx + ex;
-                Fy = Fy + ey;
-                Fz = Fz + ez;
-            }
-        }
-    }
-    if (FOLD) {  // fold_root's order
-        uint32_t par = 0;  // this image's parent item
-        if (mine && g && org >= q.nlocal) par = 0xffu;
-#pragma unroll
-        for (int j = 1; j < 8; ++j) {
-            const uint32_t gj = __shfl_sync(kAll, gi, j, 8);
-            if (par && (uint32_t)j <= nimg && org == q.nlocal + gj) par = (uint32_t)j;
-        }
-        const uint32_t most = __reduce_max_sync(kAll, nimg);
-        for (uint32_t j = 1; j <= most; ++j) {
-            const double ex = __shfl_sync(kAll, Fx, j, 8), ey = __shfl_sync(kAll, Fy, j, 8);
-            const double ez = __shfl_sync(kAll, Fz, j, 8);
-            const uint32_t p = __shfl_sync(kAll, par, j, 8);
-            if (j <= nimg && p == g) {
-                Fx = Fx + ex;
-                Fy = Fy + ey;
-                Fz = Fz + ez;
-            }
-        }
-        if (valid && g == 0)
-            for (uint32_t f = f0; f < f0 + nimg && rev.n; ++f) {
-                const uint64_t gh = q.nlocal + q.fold_list[f];
-                const uint32_t o = (uint32_t)c.origin[gh];
-                for (int k = 0; k < rev.n; ++k)
-                    c.planes[rev.idx[k]][o] = c.planes[rev.idx[k]][o] + c.planes[rev.idx[k]][gh];
-            }
-    }
-    if (mine) {
-        c.fx[a] = Fx;
-        c.fy[a] = Fy;
-        c.fz[a] = Fz;
-    }
+    force_group_root<FOLD>(q, c, rev, t, t < q.nlocal);
 }
 
-// Largest system that takes 8 lanes per root: one resident wave of them
-// (on 8,009 sheared atoms 5 against 12.5 us).
-constexpr uint64_t kForceGroupRoots = 148ull * 4 * kBlock / 8;
+// Largest system that takes 8 lanes per root: two resident waves of them (5.3
+// against 12.5 us with one thread each on 8,009 atoms, 9.7 against 13.1 on
+// 24,001, 11.8 against 12.6 on 37,800).
+constexpr uint64_t kForceGroupRoots = 2 * 148ull * 4 * kBlock / 8;
 
 // Entries of root t's walk: its and its images' in-lists and its row.
 __device__ __forceinline__ uint32_t csr_work(const ForceCsr& q, uint64_t t) {
@@ -296,11 +202,13 @@ void launch_root_order(cudaStream_t st, const ForceCsr& q, uint32_t* order) {
     k_root_order<<<(unsigned)((q.nlocal + kBlock - 1) / kBlock), kBlock, 0, st>>>(q, order);
 }
 
-void launch_force_csr(cudaStream_t st, const ForceCsr& q, const AtomCols& c, const PlaneList& rev,
+void launch_force_csr(cudaStream_t st, const ForceCsr& q0, const AtomCols& c, const PlaneList& rev,
                       bool fold, bool few_images, const uint32_t* trip, const FillGuard* guard) {
-    if (q.nlocal == 0) return;
+    if (q0.nlocal == 0) return;
     note_launch();
     const FillGuard gd = guard ? *guard : FillGuard{};
+    ForceCsr q = q0;
+    if (q.order) q.multi = nullptr;  // an order of whole blocks of roots
     if (q.nlocal <= kForceGroupRoots && few_images && !q.pk && !q.order) {
         const unsigned blocks = (unsigned)((q.nlocal * 8 + kBlock - 1) / kBlock);
         if (fold) pdl_launch(k_force_group<true>, blocks, kBlock, 0, st, q, c, rev, trip, gd);

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kBlock) k_border_faces(uint64_t nlocal, AtomCo
 
 // Pass 2: one CTA per (category or all images, chunk of kScanChunk warp
 // tiles) scans the warp counts inside its chunk; ctot gets the chunk totals.
-// Clears the capacity word bs[10] that pass 3 may set.
+// Clears the capacity word bs[10] and the count bs[kBorderMulti] of pass 3.
 __global__ void __launch_bounds__(kBlock) k_border_cat_scan(const uint32_t* counts, uint32_t* offs,
                                                             uint64_t nw, uint32_t* ctot,
                                                             uint64_t nchunks, uint32_t* bs,
@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(kBlock) k_border_cat_scan(const uint32_t* coun
     pdl_wait();  // launched with pdl_launch
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         bs[10] = 0u;
+        bs[kBorderMulti] = 0u;
         if (host_bs) host_bs[10] = 0u;
     }
     const uint64_t k = blockIdx.x / nchunks, ch = blockIdx.x % nchunks;
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(kBlock) k_border_images(
     uint64_t nlocal, uint64_t cap, AtomCols c, BorderCats cats, const uint8_t* face,
     const uint32_t* offs, const uint32_t* totals, const uint32_t* cpre, uint64_t nchunks,
     uint64_t nw, uint32_t* bs, uint32_t* root, uint32_t* chain, SendPtrs send,
-    uint32_t* fold_start, uint32_t* fold_list, uint32_t* host_bs) {
+    uint32_t* fold_start, uint32_t* fold_list, uint32_t* multi, uint32_t* host_bs) {
     pdl_wait();  // launched with pdl_launch
     __shared__ BorderWarpSmem sm[kBlock / 32];
     const uint32_t lane = threadIdx.x & 31u;
@@ -217,14 +218,14 @@ __global__ void __launch_bounds__(kBlock) k_border_images(
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w < nw; w += nwarps)
         border_warp_images(c, nlocal, cap, cats, face, offs, cpre, nchunks, nw, w, lane, base_lane,
                            bs, root, chain, send.p, fold_start, fold_list, sm[threadIdx.x / 32],
-                           host_bs);
+                           host_bs, multi);
 }
 
 void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCols& c,
                     const BorderCats& cats, const BorderPass& bp, uint8_t* face, uint32_t* counts,
                     uint32_t* offs, uint32_t* bs, uint32_t* ghost_root, uint32_t* ghost_chain,
                     const SendPtrs& send, uint32_t* fold_start, uint32_t* fold_list,
-                    uint32_t* host_bs) {
+                    uint32_t* multi, uint32_t* host_bs) {
     if (nlocal == 0) return;
     const uint64_t nw = (nlocal + 31) / 32;
     const uint64_t nchunks = (nw + kScanChunk - 1) / kScanChunk;
@@ -245,7 +246,7 @@ void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCo
     note_launch();
     pdl_launch(k_border_images, grid_wave<k_border_images>(nw * 32), kBlock, 0, st, nlocal, cap, c,
                cats, face, offs, totals, cpre, nchunks, nw, bs, ghost_root, ghost_chain, send,
-               fold_start, fold_list, host_bs);
+               fold_start, fold_list, multi, host_bs);
 }
 
 __global__ void __launch_bounds__(kBlock) k_make_ghosts(uint64_t nlocal, uint64_t nghost,

@@ -310,11 +310,12 @@ struct BorderDim {
 };
 // Border state words of one borders pass (device memory, read back once):
 //   [0..3] scan_end of dim d, [4..6] lo-swap totals, [7..9] hi-swap totals,
-//   [10] overflow flag, [16 + k] image count of chain category k (k < 26),
-//   [42] all images.
+//   [10] overflow flag, [11] roots with two images or more (k_border_images'
+//   list), [16 + k] image count of chain category k (k < 26), [42] all images.
 constexpr int kBorderStateWords = 48;
 constexpr int kBorderCats = 26;
 constexpr int kBorderTotals = 16;
+constexpr int kBorderMulti = 11;
 
 // Geometry of one borders pass: face thresholds per dim, image shifts per
 // swap id (2*dim + side, side 0 = the lo swap).
@@ -361,14 +362,15 @@ struct SendPtrs {
 // build's binning pass').  bs must be zero; ghosts beyond `cap` set bs[10].  offs holds (kBorderCats + 1) * nw words and counts that plus
 // (kBorderCats + 1) * ceil(nw / 8192) (nw = ceil(nlocal / 32)).
 // cats: border_cats(), or border_cats_masked() for axes without periodicity.
-// host_bs (optional, host memory mapped for the device): the kernels also
-// write bs[0, 11) there, so no copy is needed after them.
+// multi: the roots with two images or more, unordered, counted in
+// bs[kBorderMulti].  host_bs (optional, host memory mapped for the device): the
+// kernels also write bs[0, 11) there, so no copy is needed after them.
 void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCols& c,
                     const BorderCats& cats, const BorderPass& bp, uint8_t* face, uint32_t* counts,
                     uint32_t* offs,
                     uint32_t* bs, uint32_t* ghost_root, uint32_t* ghost_chain,
                     const SendPtrs& send, uint32_t* fold_start, uint32_t* fold_list,
-                    uint32_t* host_bs = nullptr);
+                    uint32_t* multi, uint32_t* host_bs = nullptr);
 // The columns of ghosts [nlocal, nlocal + nghost) from their roots.
 void launch_make_ghosts(cudaStream_t st, uint64_t nlocal, uint64_t nghost, const AtomCols& c,
                         const uint32_t* root, const uint32_t* chain, const SwapConst& sc);
@@ -558,6 +560,10 @@ struct ForceCsr {
     // order[b + k].  Threads of a warp then walk groups of similar length.
     const uint32_t* order;
     const double* pk;  // packed (x, y, z, r) records, current; NULL: the columns
+    // the roots with two images or more and their count (border pass); NULL:
+    // not known, or a root may have more than 7 images
+    const uint32_t* multi;
+    const uint32_t* nmulti;
 };
 // trip: the launch does nothing when *trip is set (LightStep).  guard: nor
 // when the guard is shut (a consumer queued before the pair total is known).

@@ -1107,7 +1107,7 @@ int phase_borders_defer(soil_sys* s, bool defer) {
         const bool direct = defer && s->nlocal > 0;
         launch_borders(s->st, s->nlocal, s->acap, s->A, cats, bp, s->face_flags.p, s->bcount.p,
                        s->boff.p, s->bstate.p, s->ghost_root.p, s->ghost_chain.p, send,
-                       s->fold_start.p, s->fold_list.p,
+                       s->fold_start.p, s->fold_list.p, s->multi_roots.p,
                        direct ? s->hword_dev + kBorderStateWords : nullptr);
         TRY(check_launch(s));
         if (!direct)
@@ -1125,6 +1125,7 @@ int phase_borders_defer(soil_sys* s, bool defer) {
         TRY(grow_atoms(s, (uint64_t)hb[3] + 1024, s->nlocal));  // hb[3]: atoms incl. all ghosts
     }
     TRY(borders_done(s, hb, bds));
+    s->multi_gen = s->border_gen;
     launch_make_ghosts(s->st, s->nlocal, s->nghost, s->A, s->ghost_root.p, s->ghost_chain.p,
                        swap_const(s));
     TRY(check_launch(s));
@@ -1215,6 +1216,7 @@ int borders_arrays(soil_sys* s) {
     TRY(ensure(s, s->face_flags, cap + 1));
     TRY(ensure(s, s->fold_start, s->nlocal + 2));
     TRY(ensure(s, s->fold_list, cap + 1));
+    TRY(ensure(s, s->multi_roots, cap + 1));
     return SOIL_OK;
 }
 
@@ -1397,7 +1399,7 @@ ForceArgs consumer_args(const soil_sys* s) {
     return p;
 }
 
-ForceCsr csr_args(const soil_sys* s) {
+ForceCsr csr_args(const soil_sys* s, bool few_images) {
     ForceCsr q;
     q.order = nullptr;
     q.rad = s->A.planes[s->cols[s->radius_col].plane0];
@@ -1412,6 +1414,8 @@ ForceCsr csr_args(const soil_sys* s) {
     q.fold_start = s->fold_start.p;
     q.fold_list = s->fold_list.p;
     q.pk = s->pk_valid ? s->pk.p : nullptr;
+    q.multi = few_images ? s->multi_roots.p : nullptr;
+    q.nmulti = few_images ? s->bstate.p + kBorderMulti : nullptr;
     return q;
 }
 
@@ -1427,7 +1431,7 @@ int csr_with_order(soil_sys* s, ForceCsr* q) {
         TRY(check_launch(s));
         s->split_valid = true;
     }
-    *q = csr_args(s);
+    *q = csr_args(s, s->few_images && s->multi_gen == s->border_gen);
     const char* env = std::getenv("SOIL_ROOT_ORDER");
     if (!env || std::atoi(env) != 1) return SOIL_OK;
     if (!s->order_valid) {
@@ -1731,8 +1735,9 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
             open.over = pend ? s->bstate.p + 10 : nullptr;
             PlaneList rev;
             zero_planes_of(s, SOIL_COL_REVERSE, rev.idx, &rev.n);
-            launch_force_csr(s->st, csr_args(s), s->A, rev, s->newton,
-                             pend ? few_images_of(s, s->pending_bds) : s->few_images, nullptr, &open);
+            const bool few = pend ? few_images_of(s, s->pending_bds) : s->few_images;
+            const bool listed = few && (pend || s->multi_gen == s->border_gen);
+            launch_force_csr(s->st, csr_args(s, listed), s->A, rev, s->newton, few, nullptr, &open);
             timer_end(s, T_FORCE);
             *consumed = true;
         }
@@ -1756,6 +1761,7 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
             return phase_neighbor(s);
         }
         TRY(borders_done(s, hb, s->pending_bds));
+        s->multi_gen = s->border_gen;
         total = s->nlocal + s->nghost;
     }
     const uint64_t np = s->hword[0];
@@ -2565,7 +2571,7 @@ int soil_sys_destroy(soil_sys* s) {
     fr(s->seq_cnt); fr(s->grp_cnt); fr(s->grp_start); fr(s->seq); fr(s->seq_owner);
     fr(s->rstate); fr(s->rec); fr(s->root_order); fr(s->pk);
     fr(s->ghost_root); fr(s->ghost_chain);
-    fr(s->fold_start); fr(s->fold_list);
+    fr(s->fold_start); fr(s->fold_list); fr(s->multi_roots);
     for (auto& a : s->send) fr(a);
     fr(s->bstate);
     fr(s->bcount); fr(s->boff);

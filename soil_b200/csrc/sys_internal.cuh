@@ -143,7 +143,8 @@ struct soil_sys {
     DArr<uint32_t> fold_roots, fold_nroots;  // locals with images (reverse comm), their count
     // border passes so far, the pass fold_roots belongs to, and the pass the
     // last reverse comm folded
-    uint64_t border_gen = 0, fold_roots_gen = ~0ull, reverse_gen = ~0ull;
+    // (multi_gen: the pass multi_roots belongs to; a batch's passes make none)
+    uint64_t border_gen = 0, fold_roots_gen = ~0ull, reverse_gen = ~0ull, multi_gen = ~0ull;
     double shear_rate = 0.0;
     uint64_t deform_step = 0;
     double harmonic_k = 0.0;
@@ -215,6 +216,7 @@ struct soil_sys {
     bool order_valid = false;
     DArr<uint32_t> ghost_root, ghost_chain;
     DArr<uint32_t> fold_start, fold_list;  // reverse-comm fold program (written by borders)
+    DArr<uint32_t> multi_roots;  // locals with two images or more (written by borders)
     DArr<uint32_t> send[kNumSwaps];
     DArr<uint32_t> bstate;
     DArr<uint32_t> bcount, boff;  // per-warp chain-category counts / offsets of borders

@@ -11,7 +11,7 @@ from soil_b200 import system, workloads as W
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [20, 31, 200, 1000, 18943, 18944, 18945])
+@pytest.mark.parametrize("n", [20, 31, 200, 1000, 18945, 37888, 37889, 60000])
 @pytest.mark.parametrize("newton", [1, 0])
 @pytest.mark.parametrize("rate", [0.0, 0.3])
 def test_rebuild_step_forces_match_oracle(ctx, n, newton, rate):
