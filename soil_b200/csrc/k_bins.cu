@@ -145,46 +145,6 @@ void launch_cells(cudaStream_t st, uint64_t first, uint64_t n, const AtomCols& c
     k_cells<<<grid_wave<k_cells>(n), kBlock, 0, st>>>(first, n, c, gr, cell_out, counts, n_dev);
 }
 
-__global__ void __launch_bounds__(kBlock) k_count_cells(uint64_t n, const uint32_t* cell,
-                                                        uint32_t* counts) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
-        const uint64_t i = i0 + threadIdx.x;
-        const bool valid = i < n;
-        aggregated_count(counts, valid ? cell[i] : 0u, valid);
-    }
-}
-
-void launch_count_cells(cudaStream_t st, uint64_t n, const uint32_t* cell, uint32_t* counts) {
-    if (n == 0) return;
-    note_launch();
-    k_count_cells<<<grid_wave<k_count_cells>(n), kBlock, 0, st>>>(n, cell, counts);
-}
-
-__global__ void __launch_bounds__(kBlock) k_scatter(uint64_t n, const uint32_t* cell,
-                                                    uint32_t* cursor, uint32_t* out) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
-        const uint64_t i = i0 + threadIdx.x;
-        const bool valid = i < n;
-        const uint32_t key = valid ? cell[i] : 0xffffffffu;
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        const int lane = threadIdx.x & 31;
-        const int leader = __ffs(peers) - 1;
-        uint32_t base = 0;
-        if (valid && lane == leader) base = atomicAdd(&cursor[key], (uint32_t)__popc(peers));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (valid) out[base + __popc(peers & lanemask_lt())] = (uint32_t)i;
-    }
-}
-
-void launch_scatter(cudaStream_t st, uint64_t n, const uint32_t* cell, uint32_t* cursor,
-                    uint32_t* out) {
-    if (n == 0) return;
-    note_launch();
-    k_scatter<<<grid_wave<k_scatter>(n), kBlock, 0, st>>>(n, cell, cursor, out);
-}
-
 // The scatter that consumes the counts: out[start[c] + --counts[c]] = i
 // (warp-aggregated), so every count is zero again afterwards and the next
 // counting pass needs no clearing; the order inside a cell is restored by

@@ -217,11 +217,6 @@ void launch_initial_pbc(cudaStream_t st, uint64_t n, const AtomCols& c, double d
 // device (n an upper bound), for launches queued before the host knows it.
 void launch_cells(cudaStream_t st, uint64_t first, uint64_t n, const AtomCols& c, const Grid& gr,
                   uint32_t* cell_out, uint32_t* counts, const uint32_t* n_dev = nullptr);
-// counts[cell[i]]++ for i in [0, n) (cells already known)
-void launch_count_cells(cudaStream_t st, uint64_t n, const uint32_t* cell, uint32_t* counts);
-// out[cursor[cell[i]]++] = i (unordered within a cell)
-void launch_scatter(cudaStream_t st, uint64_t n, const uint32_t* cell, uint32_t* cursor,
-                    uint32_t* out);
 // out[start[c] + --counts[c]] = i for c = cell[i] (unordered within a cell);
 // leaves every count at zero
 void launch_scatter_consume(cudaStream_t st, uint64_t n, const uint32_t* cell,
