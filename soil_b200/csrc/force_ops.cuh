@@ -282,12 +282,12 @@ struct CsrIdx {
 // reference's summation order, from the transposed list and the CSR: in-list
 // rows below a (ascending; in_split[a] of them), a's own row, the in-list
 // rows above a; each entry evaluated as f(a, partner) (the negation argument
-// at the top of k_force.cu).  Ghosts receive only with newton and have no row.
+// at the top of k_force.cu).  pa: a's own record.  Ghosts receive only with newton and have no row.
 template <class Ld>
 __device__ __forceinline__ void csr_item_force(const ForceCsr& q, const Ld& ld, uint64_t a,
-                                               double& Fx, double& Fy, double& Fz) {
+                                               const double4& pa, double& Fx, double& Fy,
+                                               double& Fz) {
     const bool local = a < q.nlocal;
-    const double4 pa = ld(a);
     Fx = 0.0;
     Fy = 0.0;
     Fz = 0.0;
@@ -313,7 +313,7 @@ __device__ __forceinline__ void force_csr_items(const ForceCsr& q, const Ld& ld,
     for (uint32_t f = f0 - 1; f + 1 <= f1; ++f) {  // the root (f = f0 - 1), then its images
         const uint64_t a = f + 1 == f0 ? t : q.nlocal + q.fold_list[f];
         double Fx, Fy, Fz;
-        csr_item_force(q, ld, a, Fx, Fy, Fz);
+        csr_item_force(q, ld, a, ld(a), Fx, Fy, Fz);
         c.fx[a] = Fx;
         c.fy[a] = Fy;
         c.fz[a] = Fz;
@@ -347,9 +347,17 @@ __device__ __forceinline__ void force_csr_root(const ForceCsr& q, const AtomCols
 // the images' sums to their parents' lanes in fold order.  Same operations in
 // the same order as force_csr_root.  What bounds it is one chain of dependent
 // loads (fold list, list bounds, entry, partner) instead of one per image.
+// Returns the lane's item, its force as written.
+struct GroupItem {
+    uint64_t a;   // its atom
+    uint32_t gi;  // an image: its ghost index
+    bool mine;    // there is one
+    double x, y, z, Fx, Fy, Fz;
+};
 template <bool FOLD>
-__device__ __forceinline__ void force_group_root(const ForceCsr& q, const AtomCols& c,
-                                                 const PlaneList& rev, uint64_t t, bool valid) {
+__device__ __forceinline__ GroupItem force_group_root(const ForceCsr& q, const AtomCols& c,
+                                                      const PlaneList& rev, uint64_t t,
+                                                      bool valid) {
     constexpr unsigned kAll = 0xffffffffu;
     const uint32_t g = threadIdx.x & 7u;
     const uint32_t f0 = valid ? q.fold_start[t] : 0u;
@@ -456,6 +464,74 @@ __device__ __forceinline__ void force_group_root(const ForceCsr& q, const AtomCo
         c.fx[a] = Fx;
         c.fy[a] = Fy;
         c.fz[a] = Fz;
+    }
+    return {a, gi, mine, pa.x, pa.y, pa.z, Fx, Fy, Fz};
+}
+
+// One local of a step that goes on after its forces (ForceStep): its final
+// half-kick and, in mode kStepOn, the next step's integration with its check
+// (the registers then hold the new position and velocity).
+__device__ __forceinline__ bool step_local(const ForceStep& p, const AtomCols& c, uint64_t t,
+                                           double Fx, double Fy, double Fz, double& x, double& y,
+                                           double& z, double& vx, double& vy, double& vz) {
+    bool hit = false;
+    vx = vy = vz = 0.0;
+    if (p.mode != kStepForces) {
+        const double h = 0.5 * p.dt * c.inv_mass[t];
+        vx = c.vx[t];
+        vy = c.vy[t];
+        vz = c.vz[t];
+        if (p.mode == kStepOn) {
+            const double lx = p.ck.lbx[t], ly = p.ck.lby[t], lz = p.ck.lbz[t];
+            initial_regs(h, p.dt, true, Fx, Fy, Fz, vx, vy, vz, x, y, z);
+            hit = check_moved_at(p.ck, x, y, z, lx, ly, lz);
+        } else {  // final_atom
+            vx = vx + h * Fx;
+            vy = vy + h * Fy;
+            vz = vz + h * Fz;
+        }
+        c.vx[t] = vx;
+        c.vy[t] = vy;
+        c.vz[t] = vz;
+    }
+    if (p.x) {
+        p.x[t] = x;
+        p.y[t] = y;
+        p.z[t] = z;
+    }
+    return hit;
+}
+
+// ... and one of its images (ghost gi), from the local's new position and
+// velocity (forward_images) or, in the other modes, where it is.
+__device__ __forceinline__ void step_image(const ForceStep& p, const AtomCols& c, uint64_t nlocal,
+                                           uint32_t gi, double x, double y, double z, double vx,
+                                           double vy, double vz) {
+    const uint64_t g = nlocal + gi;
+    if (p.mode == kStepOn) {
+        const uint32_t code = p.chain[gi];
+        const uint32_t len = code >> 12;
+        for (uint32_t k = 0; k < len; ++k) {
+            const int w = (code >> (3 * k)) & 7;
+            x = x + p.sc.off[w][0];
+            y = y + p.sc.off[w][1];
+            z = z + p.sc.off[w][2];
+            vx = vx + p.sc.voff[w][0];
+            vy = vy + p.sc.voff[w][1];
+            vz = vz + p.sc.voff[w][2];
+        }
+        c.vx[g] = vx;
+        c.vy[g] = vy;
+        c.vz[g] = vz;
+    } else if (p.x) {
+        x = c.x[g];
+        y = c.y[g];
+        z = c.z[g];
+    }
+    if (p.x) {
+        p.x[g] = x;
+        p.y[g] = y;
+        p.z[g] = z;
     }
 }
 

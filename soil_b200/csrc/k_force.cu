@@ -142,6 +142,90 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_csr(ForceCsr q, AtomCols c,
     }
 }
 
+// k_force_csr of a step inside a stretch, then each root's half-kicks, its next
+// position and those of its images.  The walk is bound by its instructions and
+// the latency of its gathers, the integration pass by memory bandwidth, so as
+// one launch they overlap, and the forces just summed need no second read: a
+// step on 4,194,304 atoms 244 us against 208 + 93 + 10 for the three launches,
+// on 200,003 atoms 20.8 against 16.5 + 4.2 + 3.7.
+__global__ void __launch_bounds__(kBlock, 4) k_force_step(ForceCsr q, AtomCols c, ForceStep p) {
+    pdl_wait();  // launched with pdl_launch
+    const unsigned long long w = *(volatile unsigned long long*)p.word;
+    const bool head = p.head && *p.head;
+    const bool skip = head || (w >= p.first && w <= p.number);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (head) *(volatile unsigned long long*)p.word = p.number;
+        *(volatile uint32_t*)p.answer = (uint32_t)(2 * p.number) | (skip ? 1u : 0u);
+    }
+    if (skip) return;
+    constexpr unsigned kAll = 0xffffffffu;
+    const PlaneList none{};
+    bool hit = false;
+    {  // as in k_force_csr
+        const uint64_t n = *q.nmulti;
+        const uint64_t warp = (uint64_t)(gridDim.x - 1 - blockIdx.x) * (kBlock / 32) + threadIdx.x / 32;
+        for (uint64_t k = warp * 4; k < n; k += (uint64_t)gridDim.x * (kBlock / 32) * 4) {
+            const uint64_t at = k + (threadIdx.x & 31) / 8;
+            const GroupItem it =
+                force_group_root<true>(q, c, none, at < n ? q.multi[at] : 0, at < n);
+            const bool root = it.mine && (threadIdx.x & 7) == 0;
+            double x = it.x, y = it.y, z = it.z, vx = 0.0, vy = 0.0, vz = 0.0;
+            if (root) hit |= step_local(p, c, it.a, it.Fx, it.Fy, it.Fz, x, y, z, vx, vy, vz);
+            x = __shfl_sync(kAll, x, 0, 8);
+            y = __shfl_sync(kAll, y, 0, 8);
+            z = __shfl_sync(kAll, z, 0, 8);
+            vx = __shfl_sync(kAll, vx, 0, 8);
+            vy = __shfl_sync(kAll, vy, 0, 8);
+            vz = __shfl_sync(kAll, vz, 0, 8);
+            if (it.mine && !root) step_image(p, c, q.nlocal, it.gi, x, y, z, vx, vy, vz);
+        }
+    }
+    const ColLd ld{c.x, c.y, c.z, q.rad};
+    for (uint64_t t = (uint64_t)blockIdx.x * kBlock + threadIdx.x; t < q.nlocal;
+         t += (uint64_t)gridDim.x * kBlock) {
+        const uint32_t f0 = q.fold_start[t], nimg = q.fold_start[t + 1] - f0;
+        if (nimg >= 2) continue;
+        const uint32_t gi = nimg ? q.fold_list[f0] : 0u;
+        double Fx = 0.0, Fy = 0.0, Fz = 0.0, x = 0.0, y = 0.0, z = 0.0;
+        for (uint32_t j = 0; j <= nimg; ++j) {  // the root, then its image
+            const uint64_t a = j ? q.nlocal + gi : t;
+            const double4 pa = ld(a);
+            double fx, fy, fz;
+            csr_item_force(q, ld, a, pa, fx, fy, fz);
+            if (j == 0) {
+                Fx = fx;
+                Fy = fy;
+                Fz = fz;
+                x = pa.x;
+                y = pa.y;
+                z = pa.z;
+            } else {  // fold_root
+                c.fx[a] = fx;
+                c.fy[a] = fy;
+                c.fz[a] = fz;
+                Fx = Fx + fx;
+                Fy = Fy + fy;
+                Fz = Fz + fz;
+            }
+        }
+        c.fx[t] = Fx;
+        c.fy[t] = Fy;
+        c.fz[t] = Fz;
+        double vx, vy, vz;
+        hit |= step_local(p, c, t, Fx, Fy, Fz, x, y, z, vx, vy, vz);
+        if (nimg) step_image(p, c, q.nlocal, gi, x, y, z, vx, vy, vz);
+    }
+    const unsigned any = __ballot_sync(kAll, hit);
+    if (any && (threadIdx.x & 31) == 0) *(volatile unsigned long long*)p.word = p.number + 1;
+}
+
+void launch_force_step(cudaStream_t st, const ForceCsr& q, const AtomCols& c, const ForceStep& p) {
+    note_launch();
+    const unsigned full = 148u * 4u;  // as k_force_csr
+    const unsigned need = (unsigned)((q.nlocal + kBlock - 1) / kBlock);
+    pdl_launch(k_force_step, need < full ? need : full, kBlock, 0, st, q, c, p);
+}
+
 // 8 lanes per root for a system whose roots do not fill the chip with one
 // thread each.
 template <bool FOLD>
@@ -153,11 +237,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_group(ForceCsr q, AtomCols 
     const uint64_t t = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) / 8;
     force_group_root<FOLD>(q, c, rev, t, t < q.nlocal);
 }
-
-// Largest system that takes 8 lanes per root: two resident waves of them (5.3
-// against 12.5 us with one thread each on 8,009 atoms, 9.7 against 13.1 on
-// 24,001, 11.8 against 12.6 on 37,800).
-constexpr uint64_t kForceGroupRoots = 2 * 148ull * 4 * kBlock / 8;
 
 // Entries of root t's walk: its and its images' in-lists and its row.
 __device__ __forceinline__ uint32_t csr_work(const ForceCsr& q, uint64_t t) {

@@ -136,6 +136,23 @@ void launch_final(cudaStream_t st, uint64_t n, const AtomCols& c, double dt) {
     pdl_launch(k_final, grid_wave<k_final>(n), kBlock, 0, st, n, c, dt);
 }
 
+__global__ void __launch_bounds__(kBlock) k_copy_positions(uint64_t n, AtomCols from, AtomCols to) {
+    pdl_wait();  // launched with pdl_launch
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const double x = from.x[i], y = from.y[i], z = from.z[i];
+        to.x[i] = x;
+        to.y[i] = y;
+        to.z[i] = z;
+    }
+}
+
+void launch_copy_positions(cudaStream_t st, uint64_t n, const AtomCols& from, const AtomCols& to) {
+    if (n == 0) return;
+    note_launch();
+    pdl_launch(k_copy_positions, grid_wave<k_copy_positions>(n), kBlock, 0, st, n, from, to);
+}
+
 __global__ void __launch_bounds__(kBlock) k_zero(uint64_t n, AtomCols c, PlaneList zp) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {

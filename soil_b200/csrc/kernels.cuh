@@ -560,6 +560,40 @@ struct ForceCsr {
     const uint32_t* multi;
     const uint32_t* nmulti;
 };
+// Largest system that takes 8 lanes per root: two resident waves of them (5.3
+// against 12.5 us with one thread each on 8,009 atoms, 9.7 against 13.1 on
+// 24,001, 11.8 against 12.6 on 37,800).
+constexpr uint64_t kForceGroupRoots = 2 * 148ull * 4 * kBlock / 8;
+
+// What a step's consumer launch does after its forces (k_force_step): nothing
+// more, the final half-kick, or that and the next step's integration,
+// displacement check and forward comm.
+enum { kStepForces = 0, kStepFinal = 1, kStepOn = 2 };
+struct ForceStep {
+    int mode;
+    // kStepOn: the next positions' columns (not the ones the launch reads: other
+    // roots still read those); else the columns to copy the positions to, or NULL
+    double* x;
+    double* y;
+    double* z;
+    double dt;
+    CheckArgs ck;  // its trip words are not used
+    const uint32_t* chain;
+    SwapConst sc;
+    // Steps of one stretch are numbered on from `first`, this one `number`; a
+    // step whose check trips, and every later one of its stretch, does nothing:
+    // *word = the number of the tripped step (older numbers: another stretch's).
+    // head: the first step's trip word, whose integration ran by itself.
+    const uint32_t* head;
+    unsigned long long* word;
+    unsigned long long first, number;
+    // the launch hands the host 2 * number, plus 1 when it does nothing
+    uint32_t* answer;
+};
+// Newton, at most 7 images per root, q.multi given, no packed records.
+void launch_force_step(cudaStream_t st, const ForceCsr& q, const AtomCols& c, const ForceStep& p);
+// to's positions = from's, atoms [0, n)
+void launch_copy_positions(cudaStream_t st, uint64_t n, const AtomCols& from, const AtomCols& to);
 // trip: the launch does nothing when *trip is set (LightStep).  guard: nor
 // when the guard is shut (a consumer queued before the pair total is known).
 // few_images: no local has more than 7 images (small systems then take 8 lanes

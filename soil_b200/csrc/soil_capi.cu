@@ -2293,9 +2293,10 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, boo
     return SOIL_OK;
 }
 
-// The host's copy of a light step's answer, once the device has written it.
-int light_answer(soil_sys* s, uint32_t tag, bool* tripped) {
-    const volatile uint32_t* w = s->hword + kHostAnswer;
+// The host's copy of a light step's answer (host word `at`), once the device
+// has written it.
+int light_answer(soil_sys* s, int at, uint32_t tag, bool* tripped) {
+    const volatile uint32_t* w = s->hword + at;
     for (uint64_t k = 0;; ++k) {
         uint32_t v = *w;
         if ((v & ~1u) != tag && k % 4096 == 4095) {
@@ -2314,15 +2315,8 @@ int light_answer(soil_sys* s, uint32_t tag, bool* tripped) {
     }
 }
 
-// One light step (light_limit >= 1) of a system with the CSR consumer, phase
-// by phase: forward comm and the consumer go in behind the integration pass
-// and do nothing if its check tripped; the host reads the answer while they
-// run, so the stream never waits for it.
-int light_step(soil_sys* s, bool last) {
-    StepPlan p = plan_step(s);
-    TRY(light_words(s));
-    if (!s->in_lists_valid) TRY(build_in_lists(s));
-    TRY(pk_ready(s));  // before the pass moves the atoms
+// The integration pass of a light step: its words, its check's trip word.
+int light_integrate(soil_sys* s, const StepPlan& p, LightStep* out) {
     LightStep w;
     w.trip = s->rstate.p + 10 + s->light_gen % 2;
     w.next = s->rstate.p + 10 + (s->light_gen + 1) % 2;
@@ -2330,7 +2324,6 @@ int light_step(soil_sys* s, bool last) {
     s->light_gen += 1;
     w.tag = 2u * s->light_gen;
     s->hword[kHostAnswer] = w.tag - 2u;
-    timer_begin(s, T_INTEGRATE);
     if (s->pending_final)
         launch_final_initial(s->st, s->nlocal, s->A, s->dt, p.fused_zero, s->lbx.p, s->lby.p,
                              s->lbz.p, s->nlocal, displacement_threshold_sq(s), s->pbc_box,
@@ -2341,6 +2334,22 @@ int light_step(soil_sys* s, bool last) {
                        nullptr, &w);
     s->pending_final = false;
     TRY(check_launch(s));
+    *out = w;
+    return SOIL_OK;
+}
+
+// One light step (light_limit >= 1) of a system with the CSR consumer, phase
+// by phase: forward comm and the consumer go in behind the integration pass
+// and do nothing if its check tripped; the host reads the answer while they
+// run, so the stream never waits for it.
+int light_step(soil_sys* s, bool last) {
+    StepPlan p = plan_step(s);
+    TRY(light_words(s));
+    if (!s->in_lists_valid) TRY(build_in_lists(s));
+    TRY(pk_ready(s));  // before the pass moves the atoms
+    LightStep w;
+    timer_begin(s, T_INTEGRATE);
+    TRY(light_integrate(s, p, &w));
     timer_end(s, T_INTEGRATE);
     const size_t spans = s->spans.size();
     timer_begin(s, T_FORWARD);
@@ -2350,7 +2359,7 @@ int light_step(soil_sys* s, bool last) {
     TRY(launch_consumer(s, s->newton, w.trip));
     timer_end(s, T_FORCE);
     bool tripped = false;
-    TRY(light_answer(s, w.tag, &tripped));
+    TRY(light_answer(s, kHostAnswer, w.tag, &tripped));
     if (tripped) {
         while (s->spans.size() > spans) {  // the empty launches are no phase
             s->ev_pool.push_back(s->spans.back().a);
@@ -2369,6 +2378,90 @@ int light_step(soil_sys* s, bool last) {
         TRY(check_launch(s));
         timer_end(s, T_FINAL);
     }
+    return SOIL_OK;
+}
+
+// Light steps that may run as one launch each (k_force_step): the CSR consumer
+// with newton from the columns, its roots' images listed, no phase timers, and
+// no #[reverse] planes (a fold would change what forward comm copies).  Smaller
+// systems that the resident launch refused keep 8 lanes per root in launches
+// of their own.
+uint64_t stretch_limit(const soil_sys* s, uint64_t want) {
+    if (s->nlocal <= kForceGroupRoots) return 0;
+    if (s->timing_mask || !s->newton || !s->few_images || s->multi_gen != s->border_gen) return 0;
+    if (force_variant() != SOIL_FORCE_CSR || packed_on()) return 0;
+    const char* env = std::getenv("SOIL_ROOT_ORDER");
+    if (env && std::atoi(env) == 1) return 0;
+    int idx[kMaxPlanes], nr;
+    zero_planes_of(s, SOIL_COL_REVERSE, idx, &nr);
+    return nr > 0 ? 0 : light_limit(s, want);
+}
+
+// `count` (at least two) light steps of a system that stretch_limit allows,
+// one launch each: the first step's integration and forward comm, then every
+// step's forces with the next step's integration and forward comm, the
+// positions alternating between the two column sets and back in the first at
+// the end.  Two steps are queued at any time; one whose check trips, and the
+// one behind it, do nothing.  last: with the final half-kick of the last step.
+// Answers as flight_steps.
+int stretch_steps(soil_sys* s, uint64_t count, bool last, uint64_t* done, bool* tripped,
+                  StepPlan* plan) {
+    *plan = plan_step(s);
+    TRY(light_words(s));
+    if (!s->in_lists_valid) TRY(build_in_lists(s));
+    TRY(pk_ready(s));  // none
+    ForceCsr q;
+    TRY(csr_with_order(s, &q));
+    LightStep w;
+    TRY(light_integrate(s, *plan, &w));
+    TRY(forward_comm(s, plan->fused_zero, &w));
+    AtomCols other = s->A;
+    other.x = s->B.x;
+    other.y = s->B.y;
+    other.z = s->B.z;
+    ForceStep p;
+    p.dt = s->dt;
+    p.ck = make_check(s->lbx.p, s->lby.p, s->lbz.p, s->nlocal, displacement_threshold_sq(s),
+                      s->pbc_box, s->dflags, pbc_mask(s));
+    p.chain = s->ghost_chain.p;
+    p.sc = swap_const(s);
+    p.word = reinterpret_cast<unsigned long long*>(s->rstate.p + 12);
+    p.first = s->chain_gen + 1;
+    s->chain_gen += count;
+    const auto answer = [&](uint64_t j) {
+        const uint64_t number = p.first + j;
+        return light_answer(s, kHostAnswer + 1 + (int)(number % 2), (uint32_t)(2 * number), tripped);
+    };
+    *tripped = false;
+    *done = 0;
+    for (uint64_t j = 0; j < count && !*tripped; ++j) {
+        const AtomCols& at = j % 2 ? other : s->A;
+        const AtomCols& to = j % 2 ? s->A : other;
+        p.mode = j + 1 < count ? kStepOn : last ? kStepFinal : kStepForces;
+        const bool move = p.mode == kStepOn || j % 2;
+        p.x = move ? to.x : nullptr;
+        p.y = move ? to.y : nullptr;
+        p.z = move ? to.z : nullptr;
+        p.head = j ? nullptr : w.trip;
+        p.number = p.first + j;
+        p.answer = s->hword_dev + kHostAnswer + 1 + p.number % 2;
+        launch_force_step(s->st, q, at, p);
+        TRY(check_launch(s));
+        if (j == 0) continue;
+        TRY(answer(j - 1));
+        if (!*tripped) *done = j;
+    }
+    if (!*tripped) {
+        TRY(answer(count - 1));
+        if (!*tripped) *done = count;
+    }
+    if (*tripped && *done % 2)
+        launch_copy_positions(s->st, s->nlocal + s->nghost, other, s->A);
+    TRY(check_launch(s));
+    s->reverse_gen = s->border_gen;
+    light_steps_done(s, *done, *tripped);
+    if (!*tripped && last) s->pending_final = false;
+    plan->tripped = true;
     return SOIL_OK;
 }
 
@@ -2394,6 +2487,19 @@ int step_many(soil_sys* s, uint64_t n) {
                 launch_final(s->st, s->nlocal, s->A, s->dt);
                 s->pending_final = false;
                 TRY(check_launch(s));
+            }
+            continue;
+        }
+        const uint64_t stretch = builtin_consumer(s) ? stretch_limit(s, n - k) : 0;
+        if (stretch >= 2) {
+            uint64_t done = 0;
+            bool tripped = false;
+            StepPlan p;
+            TRY(stretch_steps(s, stretch, k + stretch == n, &done, &tripped, &p));
+            k += done;
+            if (tripped) {
+                TRY(step_rest(s, p, k + 1 == n));
+                k += 1;
             }
             continue;
         }

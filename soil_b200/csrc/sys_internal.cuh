@@ -204,10 +204,12 @@ struct soil_sys {
     bool few_images = false;  // no local has images on both sides of a dim (<= 7 images)
     // light steps: the resident launch's three barrier words (u32 0-5), the
     // end-step words of the flights (8, 9, used in turn) and the trip words of
-    // the light steps launched phase by phase (10, 11, used in turn)
+    // the light steps launched phase by phase (10, 11, used in turn) and the
+    // stretches' tripped step (12-13, a u64)
     DArr<uint32_t> rstate;
     uint64_t flights = 0;
     uint32_t light_gen = 0;  // light steps launched phase by phase so far
+    uint64_t chain_gen = 0;  // numbers given to the steps of stretches so far
     uint64_t steps_epoch = 0;    // grid barriers of the resident launches so far
     bool steps_roomy = false;    // a resident launch needed all the shared memory
     uint64_t steps_refused_gen = ~0ull;  // border pass whose lists did not fit one

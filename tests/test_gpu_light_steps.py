@@ -116,3 +116,45 @@ def test_resident_steps_crowded_corner(ctx):
     assert_same_state(g, o)
     assert_same_lists(g, o)
     g.close()
+
+
+# Stretches of one launch a step (systems past one resident launch): calls of
+# every length around the two column sets they alternate between, ends before
+# a periodic sort, checks that trip after odd and even numbers of steps, and
+# axes without images.
+@pytest.mark.parametrize("sort_every", [0, 3, 8])
+@pytest.mark.parametrize("speed,open_axes", [(0.3, 0), (40.0, 0), (40.0, 1), (15.0, 2)])
+def test_stretches_match_one_launch_per_phase(ctx, sort_every, speed, open_axes):
+    w = W.poly("stretch", 181 + sort_every, 151777, 0.45, 1e-4, 0, harmonic_k=1e3,
+               sort_every=sort_every)
+    w.vel *= speed
+    calls = [1, 2, 3, 1, 4, 5, 2, 30]
+
+    def boundary(s):
+        if open_axes:
+            s.set_boundary([abi.SOIL_BOUNDARY_FIXED] * open_axes
+                           + [abi.SOIL_BOUNDARY_PERIODIC] * (3 - open_axes))
+
+    out = []
+    for mode in ("2", "0"):
+        os.environ["SOIL_RESIDENT_STEPS"] = mode
+        try:
+            g = system.System(ctx, w.box, w.cfg, w.dt)
+            boundary(g)
+            rc = g.register_column("radius", 1, abi.SOIL_COL_FORWARD)
+            g.add_atoms(w.tag, w.pos, w.vel, w.mass, w.cutoff, columns=[w.radius])
+            g.set_harmonic(w.harmonic_k, rc)
+            g.setup()
+            for n in calls:
+                g.step(n)
+        finally:
+            del os.environ["SOIL_RESIDENT_STEPS"]
+        out.append(g)
+    assert_same_state(*out, f"sort_every={sort_every} speed={speed} open={open_axes}")
+    assert_same_lists(*out)
+    a, b = out[0].counts(), out[1].counts()
+    assert (a.rebuilds, a.sorts) == (b.rebuilds, b.sorts)
+    if speed == 40.0:
+        assert a.rebuilds > 2
+    for g in out:
+        g.close()
