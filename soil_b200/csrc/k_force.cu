@@ -146,8 +146,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_csr(ForceCsr q, AtomCols c,
 // position and those of its images.  The walk is bound by its instructions and
 // the latency of its gathers, the integration pass by memory bandwidth, so as
 // one launch they overlap, and the forces just summed need no second read: a
-// step on 4,194,304 atoms 244 us against 208 + 93 + 10 for the three launches,
-// on 200,003 atoms 20.8 against 16.5 + 4.2 + 3.7.
+// step on 4,194,304 atoms 234 us against 208 + 93 + 10 for the three launches,
+// on 200,003 atoms 20.7 against 16.5 + 4.2 + 3.7.
 __global__ void __launch_bounds__(kBlock, 4) k_force_step(ForceCsr q, AtomCols c, ForceStep p) {
     pdl_wait();  // launched with pdl_launch
     const unsigned long long w = *(volatile unsigned long long*)p.word;
