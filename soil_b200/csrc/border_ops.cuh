@@ -57,22 +57,26 @@ __device__ __forceinline__ void border_warp_counts(const AtomCols& c, uint64_t n
     if (lane == kBorderCats) counts[kBorderCats * nw + w] = images;
 }
 
-// Per-dim border state in the format the host reads (bs[0..9]) from the
-// category totals bs[kBorderTotals + k].
-__device__ __forceinline__ void border_state_words(const BorderCats& cats, uint64_t nlocal,
-                                                   uint32_t* bs) {
-    bs[0] = (uint32_t)nlocal;
-    for (int d = 0; d < 3; ++d) {
-        uint32_t n[2] = {0, 0};
-        for (int side = 0; side < 2; ++side) {
-            const int s = 2 * d + side;
-            for (int q = 0; q < cats.swap_ncat[s]; ++q)
-                n[side] += bs[kBorderTotals + cats.swap_first[s] + q];
-        }
-        bs[4 + d] = n[0];
-        bs[7 + d] = n[1];
-        bs[d + 1] = bs[d] + n[0] + n[1];
-    }
+// Per-dim border state in the format the host reads (bs[0..9]; and its own
+// copy, when given), by one warp: base_lane as for border_warp_images (on lane
+// 26 the end of all ghosts).  A swap's categories follow one another, so its
+// ghosts are those from its first category's base to the next swap's.  (One
+// lane adding up the totals from memory was what a small system's border pass
+// waited for: k_border_images 9.3 us on 8,009 atoms.)
+__device__ __forceinline__ void border_state_words(const BorderCats& cats, uint32_t base_lane,
+                                                   uint32_t lane, uint32_t* bs,
+                                                   uint32_t* host_bs) {
+    // word 0: nlocal; 1-3: the end of dim d; 4-6, 7-9: ghosts of its lo / hi swap
+    const int d = lane == 0 ? 0 : (int)(lane - 1) % 3;
+    const int from = lane < 7 ? 2 * d : 2 * d + 1;
+    const int to = lane == 0 ? 0 : lane < 4 ? 2 * d + 2 : lane < 7 ? 2 * d + 1 : 2 * d + 2;
+    const int first = cats.swap_first[from], last = to < kNumSwaps ? cats.swap_first[to] : kBorderCats;
+    const uint32_t lo = __shfl_sync(0xffffffffu, base_lane, first);
+    const uint32_t hi = __shfl_sync(0xffffffffu, base_lane, last);
+    if (lane >= 10) return;
+    const uint32_t v = lane < 4 ? hi : hi - lo;
+    bs[lane] = v;
+    if (host_bs) host_bs[lane] = v;
 }
 
 // Warp tiles per scan chunk: the category scans run one CTA per (category,

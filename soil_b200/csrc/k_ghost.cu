@@ -203,17 +203,12 @@ __global__ void __launch_bounds__(kBlock) k_border_images(
     const uint32_t lane = threadIdx.x & 31u;
     // first ghost index of category `lane` (lanes below 26)
     const uint32_t tot = lane <= kBorderCats ? totals[lane] : 0u;
-    if (blockIdx.x == 0 && threadIdx.x < 32) {
-        if (lane <= kBorderCats) bs[kBorderTotals + lane] = tot;
-        __syncwarp();
-        if (lane == 0) {
-            border_state_words(cats, nlocal, bs);
-            if (host_bs)
-                for (int k = 0; k < 10; ++k) host_bs[k] = bs[k];
-        }
-    }
     const uint32_t base_lane =
         (uint32_t)nlocal + warp_exclusive_sum(lane < kBorderCats ? tot : 0u, lane);
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        if (lane <= kBorderCats) bs[kBorderTotals + lane] = tot;
+        border_state_words(cats, base_lane, lane, bs, host_bs);
+    }
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x / 32);
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w < nw; w += nwarps)
         border_warp_images(c, nlocal, cap, cats, face, offs, cpre, nchunks, nw, w, lane, base_lane,
