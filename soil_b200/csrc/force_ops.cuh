@@ -289,7 +289,7 @@ struct CsrIdx {
 // rows below a (ascending; in_split[a] of them), a's own row, the in-list
 // rows above a; each entry evaluated as f(a, partner) (the negation argument
 // at the top of k_force.cu).  pa: a's own record.  Ghosts receive only with newton and have no row.
-template <class Ld>
+template <bool SORT = false, class Ld>
 __device__ __forceinline__ void csr_item_force(const ForceCsr& q, const Ld& ld, uint64_t a,
                                                const double4& pa, double& Fx, double& Fy,
                                                double& Fz) {
@@ -299,10 +299,16 @@ __device__ __forceinline__ void csr_item_force(const ForceCsr& q, const Ld& ld, 
     Fz = 0.0;
     CsrIdx ix{q.in_list, q.indices, 0, 0, 0, 0};
     uint32_t nin = 0;
-    if (q.newton || local) {
+    if (SORT || q.newton || local) {
         ix.qs = q.in_start[a];
         nin = q.in_start[a + 1] - ix.qs;
-        ix.npre = q.in_split[a];
+        if (SORT) {
+            ix.npre = sort_segment(q.unsorted, ix.qs, ix.qs + nin, (uint32_t)a);
+            q.split_out[a] = ix.npre;
+            if (!q.newton && !local) nin = 0;
+        } else {
+            ix.npre = q.in_split[a];
+        }
     }
     if (local) {
         ix.rs = q.offsets[a];
@@ -312,14 +318,14 @@ __device__ __forceinline__ void csr_item_force(const ForceCsr& q, const Ld& ld, 
 }
 
 // The forces on root t and on its images by one thread (CSR walk).
-template <class Ld>
+template <bool SORT = false, class Ld>
 __device__ __forceinline__ void force_csr_items(const ForceCsr& q, const Ld& ld, const AtomCols& c,
                                                 uint64_t t) {
     const uint32_t f0 = q.fold_start[t], f1 = q.fold_start[t + 1];
     for (uint32_t f = f0 - 1; f + 1 <= f1; ++f) {  // the root (f = f0 - 1), then its images
         const uint64_t a = f + 1 == f0 ? t : q.nlocal + q.fold_list[f];
         double Fx, Fy, Fz;
-        csr_item_force(q, ld, a, ld(a), Fx, Fy, Fz);
+        csr_item_force<SORT>(q, ld, a, ld(a), Fx, Fy, Fz);
         c.fx[a] = Fx;
         c.fy[a] = Fy;
         c.fz[a] = Fz;
@@ -327,21 +333,21 @@ __device__ __forceinline__ void force_csr_items(const ForceCsr& q, const Ld& ld,
 }
 
 // ... then (FOLD) the fold.
-template <bool FOLD, class Ld>
+template <bool FOLD, bool SORT = false, class Ld>
 __device__ __forceinline__ void force_csr_root_ld(const ForceCsr& q, const Ld& ld,
                                                   const AtomCols& c, const PlaneList& rev,
                                                   uint64_t t) {
-    force_csr_items(q, ld, c, t);
+    force_csr_items<SORT>(q, ld, c, t);
     if (FOLD) fold_root(c, q.nlocal, t, q.fold_start, q.fold_list, rev);
 }
 
 // PK: the partners' records from q.pk (which must then be set), else from
 // the columns.
-template <bool FOLD, bool PK>
+template <bool FOLD, bool PK, bool SORT = false>
 __device__ __forceinline__ void force_csr_root(const ForceCsr& q, const AtomCols& c,
                                                const PlaneList& rev, uint64_t t) {
     if constexpr (PK) force_csr_root_ld<FOLD>(q, PkLd{q.pk}, c, rev, t);
-    else force_csr_root_ld<FOLD>(q, ColLd{c.x, c.y, c.z, q.rad}, c, rev, t);
+    else force_csr_root_ld<FOLD, SORT>(q, ColLd{c.x, c.y, c.z, q.rad}, c, rev, t);
 }
 
 // The same forces by 8 lanes per root (all 32 lanes of a warp call; t: the
@@ -360,7 +366,7 @@ struct GroupItem {
     bool mine;    // there is one
     double x, y, z, Fx, Fy, Fz;
 };
-template <bool FOLD>
+template <bool FOLD, bool SORT = false>
 __device__ __forceinline__ GroupItem force_group_root(const ForceCsr& q, const AtomCols& c,
                                                       const PlaneList& rev, uint64_t t,
                                                       bool valid) {
@@ -379,17 +385,23 @@ __device__ __forceinline__ GroupItem force_group_root(const ForceCsr& q, const A
             a = q.nlocal + gi;
             org = (uint32_t)c.origin[a];
         }
-        if (g == 0 || q.newton) {
+        if (SORT || g == 0 || q.newton) {
             qs = q.in_start[a];
             nin = q.in_start[a + 1] - qs;
         }
+        if (SORT) {
+            npre = sort_segment(q.unsorted, qs, qs + nin, (uint32_t)a);
+            q.split_out[a] = npre;
+            if (g && !q.newton) nin = 0;
+        }
         if (g == 0) {
-            npre = q.in_split[a];
+            if (!SORT) npre = q.in_split[a];
             rs = q.offsets[t];
             nrow = q.offsets[t + 1] - rs;
         }
         pa = make_double4(c.x[a], c.y[a], c.z[a], q.rad[a]);
     }
+    if (SORT) __syncwarp();  // the lists are read by other lanes
     // items numbered through: this lane's are entries [from, to)
     const uint32_t n = nin + nrow;
     uint32_t to = n;

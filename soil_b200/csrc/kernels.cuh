@@ -559,6 +559,11 @@ struct ForceCsr {
     // not known, or a root may have more than 7 images
     const uint32_t* multi;
     const uint32_t* nmulti;
+    // set when the in-lists are not sorted yet: the walk of a root and its
+    // images sorts theirs first and writes their splits (in_list and in_split,
+    // writable; no packed records)
+    uint32_t* unsorted;
+    uint32_t* split_out;
 };
 // Largest system that takes 8 lanes per root: two resident waves of them (5.3
 // against 12.5 us with one thread each on 8,009 atoms, 9.7 against 13.1 on

@@ -1416,6 +1416,7 @@ ForceCsr csr_args(const soil_sys* s, bool few_images) {
     q.pk = s->pk_valid ? s->pk.p : nullptr;
     q.multi = few_images ? s->multi_roots.p : nullptr;
     q.nmulti = few_images ? s->bstate.p + kBorderMulti : nullptr;
+    q.unsorted = q.split_out = nullptr;
     return q;
 }
 
@@ -1726,7 +1727,7 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
         launch_pair_fill(s->st, p, s->rowcount.p, s->row_slots.p, s->offsets.p, s->indices.p,
                          guard);
         CK(cudaEventRecord(s->ev_counts, s->st));
-        if (with_in)
+        if (with_in && !consumer_next)  // else the consumer sorts them
             launch_segsort_split(s->st, total, s->in_start.p, s->in_list.p, s->in_split.p, &guard);
         if (consumer_next) {
             timer_end(s, T_NEIGHBOR);
@@ -1737,7 +1738,10 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
             zero_planes_of(s, SOIL_COL_REVERSE, rev.idx, &rev.n);
             const bool few = pend ? few_images_of(s, s->pending_bds) : s->few_images;
             const bool listed = few && (pend || s->multi_gen == s->border_gen);
-            launch_force_csr(s->st, csr_args(s, listed), s->A, rev, s->newton, few, nullptr, &open);
+            ForceCsr q = csr_args(s, listed);
+            q.unsorted = s->in_list.p;
+            q.split_out = s->in_split.p;
+            launch_force_csr(s->st, q, s->A, rev, s->newton, few, nullptr, &open);
             timer_end(s, T_FORCE);
             *consumed = true;
         }
