@@ -518,6 +518,34 @@ __device__ __forceinline__ void fill_row(const PairParams& p, const Filter<UNIFO
     }
 }
 
+// fill_row by G lanes (g: this one; the group's lanes are converged): an entry
+// each, so a row costs one trip for its slots and one for its partners' counts.
+template <int G, bool UNIFORM, bool FP32>
+__device__ __forceinline__ void fill_row_group(const PairParams& p,
+                                               const Filter<UNIFORM, FP32>& test, uint64_t i,
+                                               uint32_t g, const uint32_t* rowcount,
+                                               const uint32_t* slots, const uint32_t* offsets,
+                                               uint32_t* indices) {
+    const uint32_t K = (uint32_t)p.row_slots;
+    const uint32_t cnt = rowcount[i];
+    uint32_t a = slots[i * K + g];  // past cnt unused
+    uint32_t* out = indices + offsets[i];
+    const bool slotted = cnt <= K;
+    if (!slotted) {  // one lane's work, and its in-list entries too
+        if (g) return;
+        uint32_t rk = 0, cd = 0;
+        row_scan<UNIFORM, FP32, true>(p, test, i, out, 0xffffffffu, &rk, &cd, nullptr);
+    }
+    const uint32_t step = slotted ? (uint32_t)G : 1u;
+    const uint32_t* src = slotted ? slots + i * K : out;
+    for (uint32_t k = g; k < cnt; k += step) {
+        if (k != g || !slotted) a = src[k];
+        if (slotted) out[k] = a;
+        if (p.in_list)
+            p.in_list[p.in_start[a] + atomicSub(&p.in_count[a], 1u) - 1u] = (uint32_t)i;
+    }
+}
+
 // ---- per-atom bodies of the kernels ----------------------------------------
 
 // Atom i's packed record (x, y, z, its radius) in one 256-bit store: whole

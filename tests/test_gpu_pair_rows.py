@@ -70,3 +70,18 @@ def test_scans_of_every_form(ctx, n, limit):
     finally:
         if limit:
             os.environ.pop("SOIL_SCAN1P_MAX") if old is None else os.environ.update(SOIL_SCAN1P_MAX=old)
+
+
+# Pass 2 by 8 lanes per row up to 65,536 rows, and rows longer than their slots
+# in it; the consumer of the step sorts the transposed lists.
+@pytest.mark.parametrize("n,phi", [(3, 0.3), (7, 0.45), (33, 3.0), (3000, 6.0), (65536, 0.4),
+                                   (65537, 0.4)])
+@pytest.mark.parametrize("newton", [1, 0])
+def test_rows_filled_by_lanes(ctx, n, phi, newton):
+    w = W.poly("fill", 200, n, phi, 1e-5, 0, harmonic_k=1e2, newton=newton)
+    g, o = system.from_workload(ctx, w), oracle.from_workload(w)
+    g.step(3)
+    o.step(3)
+    assert_same_state(g, o, f"n={n} phi={phi}")
+    assert_same_lists(g, o)
+    g.close()
