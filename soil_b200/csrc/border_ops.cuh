@@ -80,8 +80,72 @@ __device__ __forceinline__ void border_state_words(const BorderCats& cats, uint3
 }
 
 // Warp tiles per scan chunk: the category scans run one CTA per (category,
-// chunk); chunk prefixes (cpre[k * nchunks + chunk]) are added back here.
+// chunk); chunk prefixes (cpre[k * nchunks + chunk]; NULL: a single chunk) are
+// added back here.
 constexpr uint64_t kScanChunk = 8192;
+struct ScannedOffs {
+    const uint32_t* offs;
+    const uint32_t* cpre;
+    uint64_t nchunks, nw, w;
+    __device__ __forceinline__ uint32_t operator()(uint32_t k) const {
+        return offs[k * nw + w] + (cpre ? cpre[k * nchunks + w / kScanChunk] : 0u);
+    }
+};
+
+// A pass of few tiles needs no scan launch: each CTA of pass 2 sums the
+// counts before its own tiles itself.
+struct BorderCtaOffs {
+    uint32_t before[kBorderCats + 1];               // in the tiles before this CTA's
+    uint32_t total[kBorderCats + 1];                // in all tiles
+    uint32_t tile[kBorderCats + 1][kBlock / 32];    // in each of its tiles
+};
+// (all threads; a barrier follows)
+__device__ __forceinline__ void border_cta_offs(const uint32_t* counts, uint64_t nw, uint64_t first,
+                                                BorderCtaOffs& sm) {
+    constexpr uint32_t kWarps = kBlock / 32, kCats = (kBorderCats + kWarps) / kWarps;
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x / 32;
+    uint32_t before[kCats] = {}, total[kCats] = {};
+    for (uint64_t t0 = 0; t0 < nw; t0 += 256) {  // every load of 256 tiles in flight
+        uint32_t v[kCats][8];
+#pragma unroll
+        for (int q = 0; q < (int)kCats; ++q)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const uint64_t t = t0 + u * 32 + lane;
+                const uint32_t k = w + q * kWarps;
+                v[q][u] = t < nw && k <= (uint32_t)kBorderCats ? counts[k * nw + t] : 0u;
+            }
+#pragma unroll
+        for (int q = 0; q < (int)kCats; ++q)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const uint64_t t = t0 + u * 32 + lane;
+                total[q] += v[q][u];
+                before[q] += t < first ? v[q][u] : 0u;
+                if (t >= first && t < first + kWarps && w + q * kWarps <= (uint32_t)kBorderCats)
+                    sm.tile[w + q * kWarps][t - first] = v[q][u];
+            }
+    }
+#pragma unroll
+    for (int q = 0; q < (int)kCats; ++q) {
+        const uint32_t k = w + q * kWarps;
+        const uint32_t b = __reduce_add_sync(0xffffffffu, before[q]);
+        const uint32_t n = __reduce_add_sync(0xffffffffu, total[q]);
+        if (lane == 0 && k <= (uint32_t)kBorderCats) {
+            sm.before[k] = b;
+            sm.total[k] = n;
+        }
+    }
+}
+struct CtaOffs {
+    const BorderCtaOffs& sm;
+    uint32_t wib;
+    __device__ __forceinline__ uint32_t operator()(uint32_t k) const {
+        uint32_t v = sm.before[k];
+        for (uint32_t t = 0; t < wib; ++t) v += sm.tile[k][t];
+        return v;
+    }
+};
 
 // Shared-memory scratch of one warp in pass 2: per category its members among
 // the tile's lanes and the ghost index of the first, and the first ghost index
@@ -103,35 +167,29 @@ __device__ __forceinline__ uint32_t image_index(const BorderWarpSmem& sm, int k,
 }
 
 // Pass 2 for warp tile w.  base_lane: on lane k < 26 the first ghost index of
-// category k (nlocal + the totals of the categories before it).  offs holds
-// offsets inside the tile's scan chunk; cpre (NULL: a single chunk) the
-// chunks' prefixes.  sm: this warp's scratch.  host_bs (optional): the host's
+// category k (nlocal + the totals of the categories before it).  off(k): the
+// members of category k (k = 26: images) in the tiles before.  sm: this warp's scratch.  host_bs (optional): the host's
 // copy of bs, which gets the capacity word too.  multi (optional): the roots
 // with two images or more, in no particular order, counted in
 // bs[kBorderMulti].
+template <class Off>
 __device__ __forceinline__ void border_warp_images(
     const AtomCols& c, uint64_t nlocal, uint64_t cap, const BorderCats& cats, const uint8_t* face,
-    const uint32_t* offs, const uint32_t* cpre, uint64_t nchunks, uint64_t nw, uint64_t w, uint32_t lane,
-    uint32_t base_lane, uint32_t* bs, uint32_t* root, uint32_t* chain, uint32_t* const* send,
+    const Off& off, uint64_t w, uint32_t lane, uint32_t base_lane, uint32_t* bs, uint32_t* root, uint32_t* chain, uint32_t* const* send,
     uint32_t* fold_start, uint32_t* fold_list, BorderWarpSmem& sm, uint32_t* host_bs = nullptr,
     uint32_t* multi = nullptr) {
     const unsigned below = (1u << lane) - 1u;
     const uint64_t r = w * 32 + lane;
     const uint32_t bits = r < nlocal ? face[r] : 0u;
-    const uint64_t cw = w / kScanChunk;
     const uint32_t any = __reduce_or_sync(0xffffffffu, bits);
     if (!any) {  // no images: empty fold programs
-        const uint32_t fold0 =
-            offs[kBorderCats * nw + w] + (cpre ? cpre[kBorderCats * nchunks + cw] : 0u);
+        const uint32_t fold0 = off(kBorderCats);
         if (r < nlocal) fold_start[r] = fold0;
         if (r + 1 == nlocal) fold_start[nlocal] = fold0;
         return;
     }
     // lane k <= 26: offset of this tile's members of category k (k = 26: images)
-    const uint32_t off_lane =
-        lane <= (uint32_t)kBorderCats
-            ? offs[lane * nw + w] + (cpre ? cpre[lane * nchunks + cw] : 0u)
-            : 0u;
+    const uint32_t off_lane = lane <= (uint32_t)kBorderCats ? off(lane) : 0u;
     const uint32_t fold0 = __shfl_sync(0xffffffffu, off_lane, kBorderCats);
     const uint32_t rv =
         __shfl_sync(0xffffffffu, base_lane, lane < (uint32_t)kNumSwaps ? cats.swap_first[lane] : 0);

@@ -287,8 +287,8 @@ __global__ void __launch_bounds__(kBlock) kb_border_images(Span sp, BatchArgs A,
         const uint32_t tot = lane < kBorderCats ? bs[kBorderTotals + lane] : 0u;
         const uint32_t base_lane = (uint32_t)S.nlocal + warp_exclusive_sum(tot, lane);
         if (w == 0) border_state_words(cats, base_lane, lane, bs, nullptr);
-        border_warp_images(D.set[S.post], S.nlocal, D.cap, cats, D.face_flags, D.boff, nullptr, 1,
-                           nw, w, lane, base_lane, bs, D.ghost_root, D.ghost_chain, D.send,
+        border_warp_images(D.set[S.post], S.nlocal, D.cap, cats, D.face_flags,
+                           ScannedOffs{D.boff, nullptr, 1, nw, w}, w, lane, base_lane, bs, D.ghost_root, D.ghost_chain, D.send,
                            D.fold_start, D.fold_list, sm[threadIdx.x / 32]);
     });
 }

@@ -142,11 +142,17 @@ BorderPass border_pass(const BorderDim bds[3]) {
 
 // Pass 1, one warp per 32 locals: face bits, and per category the number of
 // member roots of the warp (counts[k * nw + w]); counts[26 * nw + w] = all
-// images of the warp's roots.
+// images of the warp's roots.  Clears the capacity word bs[10] and the count
+// bs[kBorderMulti] of pass 3.
 __global__ void __launch_bounds__(kBlock) k_border_faces(uint64_t nlocal, AtomCols c, BorderPass bp,
                                                          BorderCats cats, uint8_t* face,
-                                                         uint32_t* counts, uint64_t nw) {
+                                                         uint32_t* counts, uint64_t nw,
+                                                         uint32_t* bs) {
     pdl_wait();  // launched with pdl_launch
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        bs[10] = 0u;
+        bs[kBorderMulti] = 0u;
+    }
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x / 32);
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w < nw; w += nwarps)
@@ -156,17 +162,10 @@ __global__ void __launch_bounds__(kBlock) k_border_faces(uint64_t nlocal, AtomCo
 
 // Pass 2: one CTA per (category or all images, chunk of kScanChunk warp
 // tiles) scans the warp counts inside its chunk; ctot gets the chunk totals.
-// Clears the capacity word bs[10] and the count bs[kBorderMulti] of pass 3.
 __global__ void __launch_bounds__(kBlock) k_border_cat_scan(const uint32_t* counts, uint32_t* offs,
                                                             uint64_t nw, uint32_t* ctot,
-                                                            uint64_t nchunks, uint32_t* bs,
-                                                            uint32_t* host_bs) {
+                                                            uint64_t nchunks) {
     pdl_wait();  // launched with pdl_launch
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        bs[10] = 0u;
-        bs[kBorderMulti] = 0u;
-        if (host_bs) host_bs[10] = 0u;
-    }
     const uint64_t k = blockIdx.x / nchunks, ch = blockIdx.x % nchunks;
     const uint64_t w0 = ch * kScanChunk;
     const uint64_t n = nw - w0 < kScanChunk ? nw - w0 : kScanChunk;
@@ -192,29 +191,49 @@ __global__ void __launch_bounds__(kBlock) k_border_chunk_prefix(uint32_t* ctot, 
 // Pass 3, one warp per 32 locals: every image of the warp's roots at its
 // final index, the swap send lists, ghost root/chain/origin, and each root's
 // fold program (its images in fold order).  totals: the category totals (of a
-// single chunk, pass 2's; else those the prefix pass left in bs).
+// single chunk, pass 2's; else those the prefix pass left in bs).  FEW: no
+// pass 2 ran, each CTA adds up the counts itself (its warps take one tile each).
+template <bool FEW>
 __global__ void __launch_bounds__(kBlock) k_border_images(
     uint64_t nlocal, uint64_t cap, AtomCols c, BorderCats cats, const uint8_t* face,
-    const uint32_t* offs, const uint32_t* totals, const uint32_t* cpre, uint64_t nchunks,
-    uint64_t nw, uint32_t* bs, uint32_t* root, uint32_t* chain, SendPtrs send,
+    const uint32_t* counts, const uint32_t* offs, const uint32_t* totals, const uint32_t* cpre,
+    uint64_t nchunks, uint64_t nw, uint32_t* bs, uint32_t* root, uint32_t* chain, SendPtrs send,
     uint32_t* fold_start, uint32_t* fold_list, uint32_t* multi, uint32_t* host_bs) {
     pdl_wait();  // launched with pdl_launch
     __shared__ BorderWarpSmem sm[kBlock / 32];
     const uint32_t lane = threadIdx.x & 31u;
+    __shared__ BorderCtaOffs few[1];  // FEW
+    const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if (FEW) {
+        border_cta_offs(counts, nw, (uint64_t)blockIdx.x * (kBlock / 32), few[0]);
+        __syncthreads();
+    }
     // first ghost index of category `lane` (lanes below 26)
-    const uint32_t tot = lane <= kBorderCats ? totals[lane] : 0u;
+    const uint32_t tot = lane <= kBorderCats ? (FEW ? few[0].total[lane] : totals[lane]) : 0u;
     const uint32_t base_lane =
         (uint32_t)nlocal + warp_exclusive_sum(lane < kBorderCats ? tot : 0u, lane);
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         if (lane <= kBorderCats) bs[kBorderTotals + lane] = tot;
         border_state_words(cats, base_lane, lane, bs, host_bs);
     }
+    if (FEW) {
+        if (w0 < nw)
+            border_warp_images(c, nlocal, cap, cats, face, CtaOffs{few[0], threadIdx.x / 32}, w0,
+                               lane, base_lane, bs, root, chain, send.p, fold_start, fold_list,
+                               sm[threadIdx.x / 32], host_bs, multi);
+        return;
+    }
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x / 32);
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w < nw; w += nwarps)
-        border_warp_images(c, nlocal, cap, cats, face, offs, cpre, nchunks, nw, w, lane, base_lane,
-                           bs, root, chain, send.p, fold_start, fold_list, sm[threadIdx.x / 32],
-                           host_bs, multi);
+    for (uint64_t w = w0; w < nw; w += nwarps)
+        border_warp_images(c, nlocal, cap, cats, face, ScannedOffs{offs, cpre, nchunks, nw, w}, w,
+                           lane, base_lane, bs, root, chain, send.p, fold_start, fold_list,
+                           sm[threadIdx.x / 32], host_bs, multi);
 }
+
+// Tiles up to which pass 3 sums the counts itself (32,768 locals): with and
+// without pass 2, 3.7 + 7.2 / 7.2 us on 8,009 locals, 3.9 + 10.2 / 10.2 on
+// 32,768, and a launch less in a chain that the host bounds.
+constexpr uint64_t kFewTiles = 1024;
 
 void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCols& c,
                     const BorderCats& cats, const BorderPass& bp, uint8_t* face, uint32_t* counts,
@@ -227,10 +246,16 @@ void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCo
     uint32_t* ctot = counts + (kBorderCats + 1) * nw;  // chunk totals, then prefixes
     note_launch();
     pdl_launch(k_border_faces, grid_wave<k_border_faces>(nw * 32), kBlock, 0, st, nlocal, c, bp, cats, face,
-                                                                          counts, nw);
+                                                                          counts, nw, bs);
     note_launch();
+    if (nw <= kFewTiles) {
+        pdl_launch(k_border_images<true>, (unsigned)((nw * 32 + kBlock - 1) / kBlock), kBlock, 0, st,
+                   nlocal, cap, c, cats, face, counts, nullptr, nullptr, nullptr, 1, nw, bs,
+                   ghost_root, ghost_chain, send, fold_start, fold_list, multi, host_bs);
+        return;
+    }
     pdl_launch(k_border_cat_scan, (unsigned)((kBorderCats + 1) * nchunks), kBlock, 0, st, counts,
-               offs, nw, ctot, nchunks, bs, host_bs);
+               offs, nw, ctot, nchunks);
     // one chunk (up to 262,144 locals): its totals are the categories'
     if (nchunks > 1) {
         note_launch();
@@ -239,8 +264,8 @@ void launch_borders(cudaStream_t st, uint64_t nlocal, uint64_t cap, const AtomCo
     const uint32_t* totals = nchunks > 1 ? bs + kBorderTotals : ctot;
     const uint32_t* cpre = nchunks > 1 ? ctot : nullptr;
     note_launch();
-    pdl_launch(k_border_images, grid_wave<k_border_images>(nw * 32), kBlock, 0, st, nlocal, cap, c,
-               cats, face, offs, totals, cpre, nchunks, nw, bs, ghost_root, ghost_chain, send,
+    pdl_launch(k_border_images<false>, grid_wave<k_border_images<false>>(nw * 32), kBlock, 0, st,
+               nlocal, cap, c, cats, face, counts, offs, totals, cpre, nchunks, nw, bs, ghost_root, ghost_chain, send,
                fold_start, fold_list, multi, host_bs);
 }
 

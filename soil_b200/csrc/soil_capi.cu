@@ -1105,6 +1105,7 @@ int phase_borders_defer(soil_sys* s, bool defer) {
         // A deferred pass with locals writes the words the host reads straight
         // into its (mapped) copy: no copy in the stream after the pass.
         const bool direct = defer && s->nlocal > 0;
+        if (direct) hb[10] = 0u;
         launch_borders(s->st, s->nlocal, s->acap, s->A, cats, bp, s->face_flags.p, s->bcount.p,
                        s->boff.p, s->bstate.p, s->ghost_root.p, s->ghost_chain.p, send,
                        s->fold_start.p, s->fold_list.p, s->multi_roots.p,

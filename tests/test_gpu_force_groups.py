@@ -2,6 +2,7 @@
 lanes per root: forces (ghosts' included) equal the CPU oracle's at the sizes
 around its line, with roots of 0 to 26 images, and when the early launch finds
 its arrays too small or the ghosts outgrow theirs."""
+import numpy as np
 import pytest
 
 import oracle
@@ -40,4 +41,20 @@ def test_lists_and_ghosts_that_outgrow_their_arrays(ctx):
         seen = max(seen, g.counts().npairs)
     assert seen > 2 * 4000
     assert_same_lists(g, o)
+    g.close()
+
+
+# The border pass with and without a scan of its own (up to 1,024 tiles of 32
+# locals without), around its tiles' and CTAs' edges.
+@pytest.mark.parametrize("n", [3, 8, 33, 255, 257, 8192, 8193, 32768, 32769])
+def test_border_pass_of_few_and_many_tiles(ctx, n):
+    w = W.poly("border-tiles", 210, n, 0.3, 1e-4, 0, harmonic_k=1e2)
+    g, o = system.from_workload(ctx, w), oracle.from_workload(w)
+    g.step(2)
+    o.step(2)
+    assert_same_state(g, o, f"n={n}")
+    assert_same_lists(g, o)
+    for a, b in zip(g.swaps(), o.swaps()):
+        assert a["recv_start"] == b["recv_start"] and a["recv_count"] == b["recv_count"]
+        np.testing.assert_array_equal(a["send"], b["send"])
     g.close()
