@@ -137,15 +137,17 @@ constexpr double kTwoAtATime = 1.25;  // mean atoms per cell
 template <bool UNIFORM, bool FP32, int NR>
 static void launch_rows_t(cudaStream_t st, const PairParams& p, uint32_t* rowcount,
                           uint32_t* slots, DevFlags* flags) {
-    const bool pre = p.pre_ranges && p.nstencil < NR;
+    const bool pre = p.pre_ranges && p.nstencil < NR;  // never for NR = 0 (long stencils)
     const int g = !pre ? 1 : p.nlocal <= kRows8Lanes ? 8 : p.nlocal <= kRows4Lanes ? 4 : 1;
     const unsigned blocks = (unsigned)((p.nlocal * (uint64_t)g + kBlock - 1) / kBlock);
     auto launch = [&](auto k, unsigned grid) {
         pdl_launch(k, grid, kBlock, 0, st, p, rowcount, slots, flags);
     };
-    if (g == 8) launch(k_pairs_group<8, UNIFORM, FP32, NR>, blocks);
-    else if (g == 4) launch(k_pairs_group<4, UNIFORM, FP32, NR>, blocks);
-    else if (p.cell_atoms >= kTwoAtATime)
+    if constexpr (NR > 0) {
+        if (g == 8) return launch(k_pairs_group<8, UNIFORM, FP32, NR>, blocks);
+        if (g == 4) return launch(k_pairs_group<4, UNIFORM, FP32, NR>, blocks);
+    }
+    if (p.cell_atoms >= kTwoAtATime)
         launch(k_pairs_rows<UNIFORM, FP32, 2, NR>, grid_wave<k_pairs_rows<UNIFORM, FP32, 2, NR>>(p.nlocal));
     else
         launch(k_pairs_rows<UNIFORM, FP32, 1, NR>, grid_wave<k_pairs_rows<UNIFORM, FP32, 1, NR>>(p.nlocal));
@@ -158,8 +160,10 @@ static void launch_pairs_t(cudaStream_t st, const PairParams& p, uint32_t* rowco
     note_launch();
     if (!g && p.nstencil < kPreRanges)
         launch_rows_t<UNIFORM, FP32, kPreRanges>(st, p, rowcount, slots, flags);
-    else if (!g)
+    else if (!g && p.nstencil < kPreRangesFull)
         launch_rows_t<UNIFORM, FP32, kPreRangesFull>(st, p, rowcount, slots, flags);
+    else if (!g)
+        launch_rows_t<UNIFORM, FP32, 0>(st, p, rowcount, slots, flags);
     else if (p.nlocal <= kFillGroupRows)
         pdl_launch(k_pairs_fill_group<UNIFORM, FP32>,
                    (unsigned)((p.nlocal * kFillLanes + kBlock - 1) / kBlock), kBlock, 0, st, p,

@@ -85,3 +85,33 @@ def test_rows_filled_by_lanes(ctx, n, phi, newton):
     assert_same_state(g, o, f"n={n} phi={phi}")
     assert_same_lists(g, o)
     g.close()
+
+
+# Stencils of every length: a box sheared until its full stencil has more runs
+# than a row keeps in registers.
+@pytest.mark.parametrize("n", [33, 3001, 40001])
+@pytest.mark.parametrize("newton", [1, 0])
+@pytest.mark.parametrize("kind", ["poly", "mono-fp32"])
+def test_rows_of_strongly_tilted_boxes(ctx, n, newton, kind):
+    make = W.poly if kind == "poly" else W.mono
+    kw = dict(filter=abi.SOIL_FILTER_FP32_RECHECK) if kind.endswith("fp32") else {}
+    w = make("tilted", 220, n, 0.4, 1e-4, 0, harmonic_k=1e2, shear_rate=150.0, newton=newton, **kw)
+    g, o = system.from_workload(ctx, w), oracle.from_workload(w)
+    for _ in range(3):
+        g.step(10)
+        o.step(10)
+        assert_same_state(g, o, f"{kind} n={n}")
+        assert_same_lists(g, o)
+    stats = []
+    for pre in ("1", "0"):
+        os.environ["SOIL_PAIRS_PRE"] = pre
+        try:
+            h = system.from_workload(ctx, w)
+            h.step(30)
+            c = h.counts()
+            stats.append((c.npairs, c.filter_candidates, c.filter_rechecked))
+            h.close()
+        finally:
+            del os.environ["SOIL_PAIRS_PRE"]
+    assert stats[0] == stats[1]
+    g.close()
