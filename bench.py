@@ -61,6 +61,9 @@ from soil_b200 import abi, dist, workloads  # noqa: E402
 #              + forward columns (16 B per f64) per ghost
 #   reverse:   R send index (4) + R ghost F (24) + RMW owner F (48) per ghost
 #   final:     80 B/local
+# systems with a consumer that run whole stretches in one launch (148 CTAs of 1,024)
+STEPS_MAX_ROOTS = 148 * 1024
+
 BYTES_PER_UNIT = {
     "integrate": lambda c, fw: 156 * c.nlocal + (56 + 16 * fw) * c.nghost,
     "final": lambda c, fw: 80 * c.nlocal,
@@ -310,14 +313,13 @@ def run_soil(args, world, rank, local):
     light = {abi.TIMER_NAMES[t]: ms0[t] / max(iv0[t], 1) for t in range(abi.SOIL_NUM_TIMERS)
              if abi.TIMER_NAMES[t] in BYTES_PER_UNIT}
     dominant = max(light, key=light.get)
-    # Systems up to 2^20 atoms run their communicate-only steps resident
-    # (k_steps, one launch for many steps) unless SOIL_RESIDENT_STEPS=0; phase
-    # timers would force the launch-per-phase path, so they stay off there and
-    # the roofline comes from the light-step time of the rebuild probe.
-    # A workload that rebuilds on every step has no communicate-only stretch
-    # to run resident, and keeps its phase timer.
-    resident = (w.n <= 2 ** 20 and os.environ.get("SOIL_RESIDENT_STEPS", "2") != "0"
-                and not all_rebuilds)
+    # Communicate-only steps run without phases of their own (a stretch per
+    # launch up to STEPS_MAX_ROOTS atoms or without a consumer, else a step per
+    # launch) unless SOIL_RESIDENT_STEPS=0; phase timers would force the
+    # launch-per-phase path, so they stay off there and the roofline comes from
+    # the light-step time of the rebuild probe.  A workload that rebuilds on
+    # every step has none of these steps, and keeps its phase timer.
+    resident = os.environ.get("SOIL_RESIDENT_STEPS", "2") != "0" and not all_rebuilds
     s.set_timing(0 if resident else 1 << abi.TIMER_NAMES.index(dominant))
 
     c0 = s.counts()
@@ -369,17 +371,26 @@ def run_soil(args, world, rank, local):
     s.set_timing(0)
     probe = rebuild_probe(s, stream)
     if resident and probe["ms_per_light_step"]:
-        # one k_steps launch runs many light steps: algorithmic bytes of a
-        # light step (integration pass + consumer) over the light-step time
+        # algorithmic bytes of a light step over the light-step time: those of
+        # the integration pass and the consumer; as one launch per step (no
+        # second read of the forces) the consumer's, then per local R v,
+        # inv_mass, build position, W v, x, per ghost R chain, W v, x
+        light_kernel = ("k_flight_find + k_flight_apply" if not w.harmonic_k
+                        else "k_steps" if w.n <= STEPS_MAX_ROOTS else "k_force_step")
         step_bytes = BYTES_PER_UNIT["integrate"](c1, fwd_width) + (
             BYTES_PER_UNIT["force"](c1, fwd_width) if w.harmonic_k else 0)
+        if light_kernel == "k_force_step":
+            step_bytes = (BYTES_PER_UNIT["force"](c1, fwd_width) + 104 * c1.nlocal
+                          + 52 * c1.nghost)
         ach = step_bytes / (probe["ms_per_light_step"] * 1e-3) / 1e9
-        roofline = {"bound": "hbm", "kernel": "k_steps", "phase": "light step (resident)",
+        tr = load_traffic(light_kernel, args.config)
+        roofline = {"bound": "hbm", "kernel": light_kernel, "phase": "light step (resident)",
                     "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                    "peak_source": peak_kind, "traffic": None,
+                    "peak_source": peak_kind,
+                    "traffic": tr["dram_bytes_per_atom"] * (c1.nlocal + c1.nghost) if tr else None,
                     "algorithmic_bytes_per_step": step_bytes,
                     "ms_per_light_step": probe["ms_per_light_step"],
-                    "what": "light-step time from the rebuild probe (chunks of resident steps)"}
+                    "what": "light-step time from the rebuild probe (chunks of steps)"}
     del s
 
     e2e = None

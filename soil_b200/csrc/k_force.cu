@@ -8,13 +8,19 @@
 // a (ascending i), then +f(a,j) for its own row, then (full lists only) -f
 // from later rows.
 //
-// Two kernels reproduce that sum bit for bit:
+// These kernels reproduce that sum bit for bit:
+//
+//  k_force_csr  the default: one thread per local root walks its and its
+//               images' transposed lists and rows (8 lanes per root on small
+//               systems, k_force_group, and for roots with several images),
+//               then folds; k_force_step also ends the step and begins the
+//               next one.
 //
 //  k_harmonic   one thread per atom walks the CSR and its transpose
-//               (harmonic_atom); used by the batched engine and by systems
-//               whose locals can have more than 7 ghost images.
+//               (harmonic_atom), with a reverse pass of its own
+//               (SOIL_FORCE=gather).
 //
-//  k_force_seq  the single-system consumer.  At every rebuild each atom's
+//  k_force_seq  (SOIL_FORCE=tiles2, tiles4) at every rebuild each atom's
 //               contributions are merged into one partner sequence in the
 //               reference's order (k_seq_fill).  IEEE negation is exact, so
 //               f(i,j) = -f(j,i) bit for bit (d -> -d flips the sign of every
