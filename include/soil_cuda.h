@@ -181,14 +181,18 @@ typedef struct soil_batch soil_batch;
 
 /* ---- lifecycle ---------------------------------------------------------- */
 int soil_abi_version(void);
-/* Create a context on CUDA device `device`; hbm_budget_bytes = 0 means no cap. */
+/* Create a context on CUDA device `device`; hbm_budget_bytes = 0 means no cap.
+ * The cap bounds the device memory that the arrays of the context's systems and
+ * batches take (soil_ctx_bytes_in_use).  A context without a cap holds some
+ * memory beyond that: its systems cut their arrays from slabs, and up to 512 MB
+ * of slabs stay for later systems; those go back when an allocation fails. */
 int soil_ctx_create(int device, uint64_t hbm_budget_bytes, soil_ctx** out);
 /* Destroy the systems, batches and servers of a context before the context:
  * their device memory comes from the context's stream-ordered pool, which is
  * released here (memory still allocated from it is returned when freed). */
 int soil_ctx_destroy(soil_ctx* ctx);
 const char* soil_last_error(const soil_ctx* ctx);
-/* Device bytes currently held by all systems of the context. */
+/* Device bytes of the arrays that all systems and batches of the context hold. */
 int soil_ctx_bytes_in_use(const soil_ctx* ctx, uint64_t* out);
 /* Device allocations and frees the context has made so far (no reference
  * counterpart: lets a host check that steady-state steps allocate nothing). */

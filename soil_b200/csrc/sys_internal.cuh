@@ -55,7 +55,8 @@ struct ColMeta {
 // per array costs microseconds (milliseconds once many streams share the
 // pool: the first step of 128 boxes spent a second in 8,000 of them).  What
 // an array gives back serves the system's next arrays, in the order of its one
-// stream.  Arrays above kArenaMax come from the pool directly.
+// stream.  Arrays above kArenaMax, and every array of a context with a budget,
+// come from the pool directly.
 struct Arena {
     struct Slab {
         char* p;
