@@ -72,15 +72,13 @@ void ctx_release(soil_ctx* ctx, uint64_t bytes) {
 }
 
 constexpr size_t kHostBlockBytes = 512, kHostSlabBytes = 64 << 10, kKeptStreams = 64;
-constexpr uint64_t kKeptSlabBytes = 512ull << 20;
 
 // The kept slabs back to the pool; false when there are none.
 bool kept_slabs_release(soil_ctx* ctx, cudaStream_t st) {
     std::lock_guard<std::mutex> g(ctx->mu);
-    if (ctx->slabs.empty()) return false;
-    for (const auto& b : ctx->slabs) cudaFreeAsync(b.second, st);
-    ctx->slabs.clear();
-    ctx->slab_bytes = 0;
+    if (ctx->kept.slabs.empty()) return false;
+    for (const auto& b : ctx->kept.slabs) cudaFreeAsync(b.second, st);
+    ctx->kept = KeptSlabs{};
     return true;
 }
 
@@ -98,54 +96,26 @@ cudaError_t pool_alloc(soil_ctx* ctx, cudaStream_t st, void** p, uint64_t bytes)
 
 namespace {
 
-// A slab some system left, of at least `size` bytes, or else of at least
-// `least`; its size goes to *got (0: none).
-char* kept_slab(soil_ctx* ctx, uint64_t size, uint64_t least, uint64_t* got) {
-    std::lock_guard<std::mutex> g(ctx->mu);
-    auto it = ctx->slabs.lower_bound(size);
-    if (it == ctx->slabs.end()) it = ctx->slabs.lower_bound(least);
-    *got = 0;
-    if (it == ctx->slabs.end()) return nullptr;
-    char* p = it->second;
-    *got = it->first;
-    ctx->slab_bytes -= it->first;
-    ctx->slabs.erase(it);
-    return p;
-}
-
 uint64_t arena_round(uint64_t bytes) { return (std::max<uint64_t>(bytes, 1) + 255) / 256 * 256; }
 
 cudaError_t arena_alloc(soil_sys* s, void** p, uint64_t bytes) {
     Arena& a = s->arena;
-    // a returned block that is not much larger (its tail stays unused)
-    const auto it = a.free.lower_bound(bytes);
-    if (it != a.free.end() && it->first <= bytes + bytes / 2 + 4096) {
-        *p = it->second;
-        a.free.erase(it);
-        return cudaSuccess;
+    *p = a.take(bytes);
+    if (*p) return cudaSuccess;
+    uint64_t size = a.next_slab(bytes), kept = 0;
+    void* q;
+    {
+        std::lock_guard<std::mutex> g(s->ctx->mu);
+        q = s->ctx->kept.take(size, bytes, &kept);
     }
-    for (size_t k = a.slabs.size(); k-- > 0;) {
-        Arena::Slab& b = a.slabs[k];
-        if (b.size - b.used >= bytes) {
-            *p = b.p + b.used;
-            b.used += bytes;
-            return cudaSuccess;
-        }
-    }
-    uint64_t size = std::max(bytes, std::min<uint64_t>(std::max<uint64_t>(a.total, 1u << 20), 32u << 20));
-    uint64_t kept;
-    void* q = kept_slab(s->ctx, size, bytes, &kept);
     if (kept) size = kept;
     cudaError_t e = q ? cudaSuccess : pool_alloc(s->ctx, s->st, &q, size);
     if (e != cudaSuccess && size > bytes) {
         size = bytes;
         e = pool_alloc(s->ctx, s->st, &q, size);
     }
-    if (e != cudaSuccess) return e;
-    a.slabs.push_back({(char*)q, size, bytes});
-    a.total += size;
-    *p = q;
-    return cudaSuccess;
+    if (e == cudaSuccess) *p = a.add((char*)q, size, bytes);
+    return e;
 }
 
 }  // namespace
@@ -179,7 +149,7 @@ void dev_free(soil_sys* s, void* p, uint64_t bytes) {
     if (bytes == 0) bytes = 16;
     const uint64_t r = arena_round(bytes);
     if (from_pool(s->ctx, r)) cudaFreeAsync(p, s->st);
-    else s->arena.free.emplace(r, (char*)p);
+    else s->arena.give((char*)p, r);
     ctx_release(s->ctx, bytes);
 }
 
@@ -187,14 +157,8 @@ void dev_free(soil_sys* s, void* p, uint64_t bytes) {
 // stream has drained.
 void arena_free(soil_sys* s) {
     std::lock_guard<std::mutex> g(s->ctx->mu);
-    for (const Arena::Slab& b : s->arena.slabs) {
-        if (s->ctx->slab_bytes + b.size <= kKeptSlabBytes) {
-            s->ctx->slabs.emplace(b.size, b.p);
-            s->ctx->slab_bytes += b.size;
-        } else {
-            cudaFreeAsync(b.p, s->st);
-        }
-    }
+    for (const Arena::Slab& b : s->arena.slabs)
+        if (!s->ctx->kept.give(b.p, b.size)) cudaFreeAsync(b.p, s->st);
     s->arena = Arena{};
 }
 

@@ -4,11 +4,11 @@
 #pragma once
 
 #include <cfloat>
-#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
 
+#include "arena.cuh"
 #include "kernels.cuh"
 
 using namespace soil;
@@ -34,8 +34,7 @@ struct soil_ctx {
     std::vector<uint8_t*> host_slabs;
     std::vector<HostBlock> host_free;
     std::vector<cudaStream_t> streams;
-    std::multimap<uint64_t, char*> slabs;  // by size
-    uint64_t slab_bytes = 0;
+    soil_host::KeptSlabs kept;
     mutable std::mutex mu;  // guards in_use, the counters, err and the lists above
 };
 
@@ -49,24 +48,6 @@ struct ColMeta {
     unsigned flags;
     int plane0;
 };
-
-// Device memory of one system: its arrays are cut from a few slabs of the
-// context's pool, each twice as large as all before it, because a driver call
-// per array costs microseconds (milliseconds once many streams share the
-// pool: the first step of 128 boxes spent a second in 8,000 of them).  What
-// an array gives back serves the system's next arrays, in the order of its one
-// stream.  Arrays above kArenaMax, and every array of a context with a budget,
-// come from the pool directly.
-struct Arena {
-    struct Slab {
-        char* p;
-        uint64_t size, used;
-    };
-    std::vector<Slab> slabs;
-    std::multimap<uint64_t, char*> free;  // by size
-    uint64_t total = 0;
-};
-constexpr uint64_t kArenaMax = 8ull << 20;
 
 template <class T>
 struct DArr {
