@@ -75,13 +75,14 @@ struct KeptSlabs {
         bytes += size;
         return true;
     }
-    // One of at least `size` bytes, or else of at least `least`; its size goes to
-    // *got (0: none).
+    // One of at least `size` bytes, or else of at least `least`, but of no more
+    // than twice `size`: a system of 1 MB does not hold 32.  Its size goes to *got
+    // (0: none).
     char* take(uint64_t size, uint64_t least, uint64_t* got) {
         auto it = slabs.lower_bound(size);
-        if (it == slabs.end()) it = slabs.lower_bound(least);
+        if (it == slabs.end() || it->first > 2 * size) it = slabs.lower_bound(least);
         *got = 0;
-        if (it == slabs.end()) return nullptr;
+        if (it == slabs.end() || it->first > 2 * size) return nullptr;
         char* p = it->second;
         *got = it->first;
         bytes -= it->first;

@@ -55,3 +55,26 @@ def test_arrays_never_overlap_and_nothing_is_lost(lib, seed):
         at = p + n
         assert any(b <= p and p + n <= b + s for b, s in slabs)
     lib.arena_delete(a)
+
+
+def test_kept_slabs_go_to_systems_of_their_size(lib):
+    """A kept slab serves a system that wants at least half of it, smaller ones
+    when there is none; more than 512 MB are not kept."""
+    k = lib.kept_new()
+    for n in (32, 2, 1, 1):
+        assert lib.kept_give(k, n * MB, n * MB)
+    assert lib.kept_take(k, 1 * MB, 4096) == 1 * MB
+    assert lib.kept_take(k, 1 * MB, 4096) == 1 * MB
+    assert lib.kept_take(k, 1 * MB, 4096) == 2 * MB
+    assert lib.kept_take(k, 1 * MB, 4096) == 0  # only the 32 MB slab is left
+    assert lib.kept_take(k, 15 * MB, 4096) == 0
+    assert lib.kept_give(k, MB, MB)
+    assert lib.kept_take(k, 8 * MB, 8 * MB) == 0
+    assert lib.kept_take(k, 8 * MB, 4096) == 1 * MB  # none of 8 to 16: the smaller one
+    assert lib.kept_take(k, 16 * MB, 16 * MB) == 32 * MB
+    assert lib.kept_bytes(k) == 0
+    for _ in range(16):
+        assert lib.kept_give(k, 32 * MB, 32 * MB)
+    assert not lib.kept_give(k, MB, MB)
+    assert lib.kept_bytes(k) == 512 * MB
+    lib.kept_delete(k)
