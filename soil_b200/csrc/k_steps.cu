@@ -531,7 +531,7 @@ int steps_group(uint64_t nlocal, uint64_t sms) {
 }  // namespace
 
 bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, StepsShape* p) {
-    if (nlocal == 0 || nlocal > sms * 1024) return false;
+    if (nlocal == 0 || nlocal > steps_max_roots(sms)) return false;
     p->group = steps_group(nlocal, sms);
     const uint64_t lanes = nlocal * (uint64_t)p->group;
     uint64_t threads = ((lanes + sms - 1) / sms + 31) / 32 * 32;
@@ -559,7 +559,6 @@ bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, Ste
 
 cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold,
                          bool few_images) {
-    note_launch();
     const void* k;
     if (p.group == 8 && p.threads <= 256)
         k = few_images ? steps_kernel<8, 256, true>(fold) : steps_kernel<8, 256>(fold);
@@ -573,7 +572,9 @@ cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& 
     if (e != cudaSuccess) return e;
     StepsArgs arg = a;
     void* params[] = {&arg};
-    return cudaLaunchCooperativeKernel(k, dim3(p.grid), dim3(p.threads), params, p.smem, st);
+    e = cudaLaunchCooperativeKernel(k, dim3(p.grid), dim3(p.threads), params, p.smem, st);
+    if (e == cudaSuccess) note_launch();
+    return e;
 }
 
 }  // namespace soil

@@ -643,6 +643,8 @@ struct StepsShape {
     uint32_t ent_cap, img_cap;
     size_t smem;
 };
+// Largest system of one resident launch on `sms` SMs.
+constexpr uint64_t steps_max_roots(uint64_t sms) { return sms * 1024; }
 // The shape for a system on `sms` SMs (roomy: with all the shared memory);
 // false when it has too many atoms for one resident launch.
 bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, StepsShape* p);

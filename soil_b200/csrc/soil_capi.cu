@@ -2118,12 +2118,13 @@ uint64_t light_limit(const soil_sys* s, uint64_t want) {
 }
 
 // Those that may run as one stretch on the device (k_steps, k_flight): no
-// phase timers, and a system with a consumer fits one resident launch and has
-// no radii that change with every fold.
+// phase timers, and a system with a consumer (SOIL_RESIDENT_STEPS=0: never) fits
+// one resident launch, one root per thread of a CTA of 1,024 per SM, and has no
+// radii that change with every fold.
 uint64_t resident_limit(const soil_sys* s, uint64_t want) {
     if (s->timing_mask) return 0;
     if (builtin_consumer(s)) {
-        if (s->nlocal > kStepsMaxRoots || s->steps_refused_gen == s->border_gen) return 0;
+        if (s->nlocal > steps_max_roots(s->ctx->sms) || s->steps_refused_gen == s->border_gen) return 0;
         int idx[kMaxPlanes], nr;
         zero_planes_of(s, SOIL_COL_REVERSE, idx, &nr);
         for (int k = 0; k < nr; ++k)
@@ -2204,8 +2205,9 @@ int steps_records(soil_sys* s, double* rec[2]) {
 // Up to `max` communicate-only steps in one launch; *done of them complete.
 // *tripped: the next step's integration pass also ran and its displacement
 // check tripped (that step continues on the host from decide_rebuild, with
-// *plan).  *refused: nothing ran, the lists do not fit the launch (or there
-// is no memory for its records); resident_limit says so until they change.
+// *plan).  *refused: nothing ran, the lists do not fit the launch (or it does not
+// fit the device, or there is no memory for its records); resident_limit says so
+// until the lists change.
 int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, bool* refused,
                    StepPlan* plan) {
     *done = 0;
@@ -2235,13 +2237,21 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, boo
     a.out = s->hword_dev;
     for (;;) {
         StepsShape shape;
-        if (!steps_shape(s->nlocal, s->npairs, kStepsSms, s->steps_roomy, &shape))
+        if (!steps_shape(s->nlocal, s->npairs, s->ctx->sms, s->steps_roomy, &shape))
             return fail(s->ctx, SOIL_ERR_STATE, "resident steps: too many atoms");
         a.ent_cap = shape.ent_cap;
         a.img_cap = shape.img_cap;
         a.epoch = s->steps_epoch;
         s->hword[2] = s->hword[3] = 0;
-        CK(launch_steps(s->st, a, shape, s->newton, s->few_images));
+        const cudaError_t e = launch_steps(s->st, a, shape, s->newton, s->few_images);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            // fewer SMs than the device has are this process's to use
+            cudaGetLastError();
+            s->steps_refused_gen = s->border_gen;
+            *refused = true;
+            return SOIL_OK;
+        }
+        CK(e);
         TRY(sync(s));
         if (s->hword[2] == SOIL_STEPS_OVERFLOW) {
             s->steps_epoch += 1;
@@ -2529,6 +2539,7 @@ int soil_ctx_create(int device, uint64_t hbm_budget_bytes, soil_ctx** out) {
     soil_ctx* c = new (std::nothrow) soil_ctx();
     if (!c) return SOIL_ERR_OOM;
     c->device = device;
+    c->sms = (uint64_t)prop.multiProcessorCount;
     c->budget = hbm_budget_bytes;
     // Device arrays come from a stream-ordered pool of this context that keeps
     // freed memory (the budget counts what is in use); growth of a system's

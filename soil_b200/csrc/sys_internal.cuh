@@ -21,6 +21,7 @@ struct HostBlock {
 
 struct soil_ctx {
     int device = 0;
+    uint64_t sms = 0;  // the device's multiprocessors
     uint64_t budget = 0;
     uint64_t in_use = 0;
     std::string err;
@@ -341,9 +342,5 @@ constexpr int kHostWords = kHostAnswer + 8;
 // pass bound by HBM).
 constexpr uint64_t kSortGatherMax = 2000000;
 constexpr int kRowSlotsPerAtom = 16;
-// Systems with a consumer take the resident light steps (SOIL_RESIDENT_STEPS=0:
-// never) up to one root per thread of one CTA of 1,024 per SM.
-constexpr uint64_t kStepsSms = 148;
-constexpr uint64_t kStepsMaxRoots = kStepsSms * 1024;
 
 }  // namespace soil_host

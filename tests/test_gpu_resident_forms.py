@@ -1,0 +1,51 @@
+"""Which form light steps take, seen by the kernel launches they issue."""
+import ctypes as C
+
+import pytest
+
+import oracle
+from helpers import assert_same_lists, assert_same_state
+from internal_hooks import build_internal
+from soil_b200 import abi, system, workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _launches(g, n):
+    lib = abi.load_library()
+    l0 = lib.soil_kernel_launches()
+    g.step(n)
+    return lib.soil_kernel_launches() - l0
+
+
+@pytest.fixture(scope="module")
+def hook(tmp_path_factory):
+    lib = build_internal(tmp_path_factory.mktemp("hook"), "ctx_hook")
+    lib.ctx_get_sms.restype = C.c_uint64
+    lib.ctx_get_sms.argtypes = [C.c_void_p]
+    lib.ctx_set_sms.argtypes = [C.c_void_p, C.c_uint64]
+    return lib
+
+
+# 37 SMs hold up to 37,888 roots: 9,000 (4 lanes each) and 37,888 (1) take the
+# resident launch, 37,889 one launch a step.  A shape for 40,000 SMs asks for
+# more CTAs than any device holds at once: the launch is refused, and small and
+# large systems go on without it.
+@pytest.mark.parametrize("sms,n,resident", [(37, 9000, True), (37, 37888, True), (37, 37889, False),
+                                            (40000, 37800, False), (40000, 60000, False)])
+def test_resident_launch_is_shaped_for_the_device(hook, sms, n, resident):
+    import torch
+    c = system.Context(0)
+    assert hook.ctx_get_sms(c.h) == torch.cuda.get_device_properties(0).multi_processor_count
+    hook.ctx_set_sms(c.h, sms)
+    w = W.poly("forms-sms", 322, n, 0.45, 1e-5, 0, harmonic_k=1e3)
+    g, o = system.from_workload(c, w), oracle.from_workload(w)
+    g.step(1)
+    launches = _launches(g, 12)
+    assert g.counts().rebuilds == 1
+    assert launches <= 2 if resident else launches >= 12, launches
+    o.step(13)
+    assert_same_state(g, o)
+    assert_same_lists(g, o)
+    g.close()
+    c.close()
