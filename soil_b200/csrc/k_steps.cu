@@ -37,9 +37,11 @@
 // per-atom operations in the same order as the launch-per-phase path, so
 // results are bit-identical.  A CTA whose entries or images do not fit its
 // shared memory says so at the first barrier, and every CTA leaves with
-// nothing written.  Barrier waits are bounded: a CTA whose wait runs out
-// records SOIL_STEPS_ERR_BARRIER and returns; the cooperative launch
-// guarantees co-residency, so the bound is a guard, never the expected exit.
+// nothing written; the host learns what the CTA that has most needs, and
+// launches again with room for that or not at all.  Barrier waits are bounded:
+// a CTA whose wait runs out records SOIL_STEPS_ERR_BARRIER and returns; the
+// cooperative launch guarantees co-residency, so the bound is a guard, never
+// the expected exit.
 //
 // Measured per light step against one thread per root walking the CSR with
 // its images in series, columns in global memory and two barriers a step:
@@ -159,10 +161,6 @@ __device__ StepsSmem carve(unsigned char* p, uint32_t e, uint32_t m) {
     return s;
 }
 
-constexpr size_t kBytesPerImage = 3 * 8 + 8 + 4 + 4 + 2 + 2;
-constexpr size_t kBytesPerEntry = 4 + 1;
-constexpr size_t kBytesParked = 7 * 8;
-
 // Position (or velocity) of an image: its root's plus its chain's offsets, in
 // chain order (forward_images).
 __device__ __forceinline__ void shift_chain(uint32_t code, const double (*off)[3], double& x,
@@ -183,7 +181,7 @@ __device__ __forceinline__ void shift_chain(uint32_t code, const double (*off)[3
 template <int G, bool FOLD, int TMAX, bool FEW>
 __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ StepsArgs a) {
     static_assert(!FEW || G == 8, "an item per lane");
-    constexpr bool kPark = TMAX > 256;
+    constexpr bool kPark = TMAX > (int)kStepsParkAbove;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ Word s_seen;
     __shared__ int s_ok;
@@ -216,6 +214,10 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
     uint64_t tot;
     const uint64_t at = cta_exclusive_pair(lead ? ((uint64_t)nimg << 32) | cnt : 0u, &tot);
     const bool over = (uint32_t)tot > a.ent_cap || (uint32_t)(tot >> 32) > a.img_cap;
+    if (threadIdx.x == 0) {  // read by CTA 0 after the first barrier
+        atomicMax(a.need, (uint32_t)tot);
+        atomicMax(a.need + 1, (uint32_t)(tot >> 32));
+    }
     // the first lane's prefix is its whole group's (the other lanes' counts are 0)
     const uint64_t at0 = __shfl_sync(0xffffffffu, at, 0, G);
     const uint32_t eb = (uint32_t)at0, ib = (uint32_t)(at0 >> 32);
@@ -348,8 +350,10 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
         __syncthreads();
         const Word seen = s_seen;
         if (!s_ok || seen >= kOverUnit) {  // nothing is written
-            if (blockIdx.x == 0 && threadIdx.x == 0)
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                for (int k = 0; k < 2; ++k) a.out[4 + k] = atomicExch(a.need + k, 0u);
                 a.out[2] = s_ok ? SOIL_STEPS_OVERFLOW : SOIL_STEPS_ERR_BARRIER;
+            }
             return;
         }
         if (seen >= kTripUnit) {
@@ -510,6 +514,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_steps(const __grid_constant__ Steps
         a.out[0] = (uint32_t)done;
         a.out[1] = stop ? 1u : 0u;
         a.out[2] = 0u;
+        for (int k = 0; k < 2; ++k) a.out[4 + k] = atomicExch(a.need + k, 0u);
     }
 }
 
@@ -520,47 +525,12 @@ const void* steps_kernel(bool fold) {
     return fold ? (const void*)k_steps<G, true, TMAX, FEW> : (const void*)k_steps<G, false, TMAX, FEW>;
 }
 
-// Lanes per root: the widest group with the whole system in one CTA of at
-// most 1,024 threads per SM.
-int steps_group(uint64_t nlocal, uint64_t sms) {
-    for (int g = 8; g > 1; g /= 2)
-        if (nlocal * (uint64_t)g <= sms * 1024) return g;
-    return 1;
-}
-
 }  // namespace
-
-bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, StepsShape* p) {
-    if (nlocal == 0 || nlocal > steps_max_roots(sms)) return false;
-    p->group = steps_group(nlocal, sms);
-    const uint64_t lanes = nlocal * (uint64_t)p->group;
-    uint64_t threads = ((lanes + sms - 1) / sms + 31) / 32 * 32;
-    if (threads < 64) threads = 64;
-    p->threads = (int)threads;
-    const uint64_t roots = threads / (uint64_t)p->group;
-    p->grid = (int)((nlocal + roots - 1) / roots);
-    // room for 1.3 times the mean entries per root and 1.5 images per root (a
-    // CTA on a face has a little over one); `roomy`: all the shared memory
-    const uint64_t most = 26 * roots;
-    uint64_t img = roots + roots / 2 + 64, ent;
-    if (roomy) img = 3 * roots;
-    if (img > most) img = most;
-    const uint64_t park = threads > 256 ? threads * kBytesParked : 0;
-    const uint64_t budget = 220 * 1024 - park;
-    const uint64_t fit = (budget - img * kBytesPerImage) / kBytesPerEntry;
-    const double mean = 2.0 * (double)npairs / (double)nlocal * (double)roots;
-    ent = roomy ? fit : (uint64_t)(1.3 * mean) + 16 * roots / 8 + 256;
-    if (ent > fit) ent = fit;
-    p->ent_cap = (uint32_t)(ent & ~7ull);
-    p->img_cap = (uint32_t)img;
-    p->smem = park + img * kBytesPerImage + ent * kBytesPerEntry + 16;
-    return true;
-}
 
 cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold,
                          bool few_images) {
     const void* k;
-    if (p.group == 8 && p.threads <= 256)
+    if (p.group == 8 && p.threads <= (int)kStepsParkAbove)
         k = few_images ? steps_kernel<8, 256, true>(fold) : steps_kernel<8, 256>(fold);
     else if (p.group == 8)
         k = few_images ? steps_kernel<8, 1024, true>(fold) : steps_kernel<8, 1024>(fold);

@@ -5,6 +5,7 @@
 #include <atomic>
 
 #include "soil_internal.cuh"
+#include "steps_shape.cuh"
 
 namespace soil {
 
@@ -633,21 +634,10 @@ struct StepsArgs {
     uint64_t max_steps;
     unsigned long long* bar;  // 3 barrier words; the one of barrier `epoch` is zero at launch
     uint64_t epoch;           // grid barriers passed by earlier launches
-    uint32_t* out;  // host memory mapped for the device: steps completed; 1 if the next
-                    // step's check tripped; status; status of any CTA's wait
+    uint32_t* need;  // zero at launch and after it: most entries, most images of a CTA
+    uint32_t* out;   // host memory mapped for the device: steps completed; 1 if the next
+                     // step's check tripped; status; status of any CTA's wait; need[0, 2)
 };
-// Launch shape of k_steps: lanes per root, threads per CTA, CTAs (one per SM),
-// and the shared memory for ent_cap entries and img_cap images.
-struct StepsShape {
-    int group, threads, grid;
-    uint32_t ent_cap, img_cap;
-    size_t smem;
-};
-// Largest system of one resident launch on `sms` SMs.
-constexpr uint64_t steps_max_roots(uint64_t sms) { return sms * 1024; }
-// The shape for a system on `sms` SMs (roomy: with all the shared memory);
-// false when it has too many atoms for one resident launch.
-bool steps_shape(uint64_t nlocal, uint64_t npairs, uint64_t sms, bool roomy, StepsShape* p);
 // fold: newton.  few_images: no root has more than 7 images.
 cudaError_t launch_steps(cudaStream_t st, const StepsArgs& a, const StepsShape& p, bool fold,
                          bool few_images);

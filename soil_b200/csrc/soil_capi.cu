@@ -2124,7 +2124,7 @@ uint64_t light_limit(const soil_sys* s, uint64_t want) {
 uint64_t resident_limit(const soil_sys* s, uint64_t want) {
     if (s->timing_mask) return 0;
     if (builtin_consumer(s)) {
-        if (s->nlocal > steps_max_roots(s->ctx->sms) || s->steps_refused_gen == s->border_gen) return 0;
+        if (s->nlocal > steps_max_roots(s->ctx->sms) || s->border_gen < s->steps_retry_gen) return 0;
         int idx[kMaxPlanes], nr;
         zero_planes_of(s, SOIL_COL_REVERSE, idx, &nr);
         for (int k = 0; k < nr; ++k)
@@ -2207,7 +2207,7 @@ int steps_records(soil_sys* s, double* rec[2]) {
 // check tripped (that step continues on the host from decide_rebuild, with
 // *plan).  *refused: nothing ran, the lists do not fit the launch (or it does not
 // fit the device, or there is no memory for its records); resident_limit says so
-// until the lists change.
+// until the lists change, or longer.
 int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, bool* refused,
                    StepPlan* plan) {
     *done = 0;
@@ -2218,11 +2218,14 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, boo
     std::memset(&a, 0, sizeof(a));
     TRY(csr_with_order(s, &a.fc));
     TRY(light_words(s));
-    if (steps_records(s, a.rec) != SOIL_OK) {
-        s->steps_refused_gen = s->border_gen;
+    const auto refuse = [&]() -> int {
+        s->steps_need = StepsNeed{};
+        s->steps_backoff = std::min<uint64_t>(64, std::max<uint64_t>(1, 2 * s->steps_backoff));
+        s->steps_retry_gen = s->border_gen + s->steps_backoff;
         *refused = true;
         return SOIL_OK;
-    }
+    };
+    if (steps_records(s, a.rec) != SOIL_OK) return refuse();
     s->pk_valid = false;  // the columns move without the packed records
     a.c = s->A;
     a.nlocal = s->nlocal;
@@ -2234,11 +2237,18 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, boo
     if (s->newton) zero_planes_of(s, SOIL_COL_REVERSE, a.rev.idx, &a.rev.n);
     a.max_steps = std::min<uint64_t>(max, 0x7fffffffull);
     a.bar = reinterpret_cast<unsigned long long*>(s->rstate.p);
+    a.need = s->rstate.p + 6;
     a.out = s->hword_dev;
-    for (;;) {
+    // Room as the last launch's lists needed it; lists that do not fit say what
+    // they need, and get it or no launch.
+    StepsNeed need = s->steps_need;
+    for (bool known = false;;) {
         StepsShape shape;
-        if (!steps_shape(s->nlocal, s->npairs, s->ctx->sms, s->steps_roomy, &shape))
-            return fail(s->ctx, SOIL_ERR_STATE, "resident steps: too many atoms");
+        if (!steps_shape(s->nlocal, s->npairs, s->ctx->sms, need, &shape)) {
+            if (known || !need.ent) return refuse();
+            need = StepsNeed{};  // another system's by now: atoms have left
+            continue;
+        }
         a.ent_cap = shape.ent_cap;
         a.img_cap = shape.img_cap;
         a.epoch = s->steps_epoch;
@@ -2247,23 +2257,15 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, boo
         if (e == cudaErrorCooperativeLaunchTooLarge) {
             // fewer SMs than the device has are this process's to use
             cudaGetLastError();
-            s->steps_refused_gen = s->border_gen;
-            *refused = true;
-            return SOIL_OK;
+            return refuse();
         }
         CK(e);
         TRY(sync(s));
-        if (s->hword[2] == SOIL_STEPS_OVERFLOW) {
-            s->steps_epoch += 1;
-            if (s->steps_roomy) {
-                s->steps_refused_gen = s->border_gen;
-                *refused = true;
-                return SOIL_OK;
-            }
-            s->steps_roomy = true;  // from now on, for this system
-            continue;
-        }
-        break;
+        if (s->hword[2] != SOIL_STEPS_OVERFLOW) break;
+        s->steps_epoch += 1;
+        if (known) return refuse();
+        need = {s->hword[4], s->hword[5]};
+        known = true;
     }
     if (s->hword[2] || s->hword[3]) {
         CK(cudaMemsetAsync(s->rstate.p, 0, s->rstate.cap * 4, s->st));
@@ -2275,6 +2277,8 @@ int resident_steps(soil_sys* s, uint64_t max, uint64_t* done, bool* tripped, boo
     if (*done > a.max_steps || (!*tripped && *done != a.max_steps))
         return fail(s->ctx, SOIL_ERR_CUDA, "resident steps: inconsistent step count");
     s->steps_epoch += *done + (*tripped ? 1 : 0);
+    s->steps_need = {s->hword[4], s->hword[5]};
+    s->steps_backoff = 0;
     light_steps_done(s, *done, *tripped);
     plan->check = true;
     plan->fwd_fused = true;

@@ -185,17 +185,20 @@ struct soil_sys {
     DArr<uint8_t> seq_owner;
     bool seq_valid = false;
     bool few_images = false;  // no local has images on both sides of a dim (<= 7 images)
-    // light steps: the resident launch's three barrier words (u32 0-5), the
-    // end-step words of the flights (8, 9, used in turn) and the trip words of
-    // the light steps launched phase by phase (10, 11, used in turn) and the
-    // stretches' tripped step (12-13, a u64)
+    // light steps: the resident launch's three barrier words (u32 0-5) and what
+    // its lists need (6, 7), the end-step words of the flights (8, 9, used in
+    // turn), the trip words of the light steps launched phase by phase (10, 11,
+    // used in turn) and the stretches' tripped step (12-13, a u64)
     DArr<uint32_t> rstate;
     uint64_t flights = 0;
     uint32_t light_gen = 0;  // light steps launched phase by phase so far
     uint64_t chain_gen = 0;  // numbers given to the steps of stretches so far
     uint64_t steps_epoch = 0;    // grid barriers of the resident launches so far
-    bool steps_roomy = false;    // a resident launch needed all the shared memory
-    uint64_t steps_refused_gen = ~0ull;  // border pass whose lists did not fit one
+    StepsNeed steps_need;        // of the last resident launch
+    // The border pass from which a resident launch is tried again after one that
+    // was refused, and the passes between: twice as many with each refusal in a
+    // row, so that lists which never fit cost few launches.
+    uint64_t steps_retry_gen = 0, steps_backoff = 0;
     DArr<double4> rec;  // their second record buffer, where the row slots are too small
     DArr<uint32_t> root_order;  // CSR-walk consumer: roots by work per block (rebuilt with the lists)
     bool order_valid = false;

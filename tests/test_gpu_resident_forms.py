@@ -49,3 +49,39 @@ def test_resident_launch_is_shaped_for_the_device(hook, sms, n, resident):
     assert_same_lists(g, o)
     g.close()
     c.close()
+
+
+def _crowded(n, crowd, side):
+    """A packing with `crowd` more atoms in a cube of `side` at its centre."""
+    w = W.poly("forms", 320, n, 0.45, 1e-7, 0, harmonic_k=1e1)
+    w.pos[:crowd] = 0.5 * w.L + (w.pos[:crowd] / w.L - 0.5) * side
+    return w
+
+
+# (9,000: 8 lanes per root, 64 roots a CTA; 150,000: 1 lane, 1,024 roots, where
+# shared memory is shortest)
+@pytest.mark.parametrize("n,crowd,side", [(9000, 200, 2.5), (150000, 300, 3.0)])
+def test_lists_that_need_more_room_stay_resident(ctx, n, crowd, side):
+    w = _crowded(n, crowd, side)
+    g, o = system.from_workload(ctx, w), oracle.from_workload(w)
+    g.step(1)
+    first = _launches(g, 12)  # the launch that did not fit, the one that did, the last half-kick
+    again = _launches(g, 12)
+    assert g.counts().rebuilds == 1
+    o.step(25)
+    assert_same_state(g, o)
+    assert_same_lists(g, o)
+    assert first <= 4 and again <= 2, (first, again)
+    g.close()
+
+
+def test_lists_that_never_fit_step_by_launches(ctx):
+    w = _crowded(9000, 3000, 2.0)
+    g, o = system.from_workload(ctx, w), oracle.from_workload(w)
+    g.step(1)
+    assert _launches(g, 12) >= 24 and _launches(g, 12) >= 24
+    assert g.counts().rebuilds == 1
+    o.step(25)
+    assert_same_state(g, o)
+    assert_same_lists(g, o)
+    g.close()
