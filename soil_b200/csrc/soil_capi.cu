@@ -2118,12 +2118,13 @@ uint64_t light_limit(const soil_sys* s, uint64_t want) {
 }
 
 // Those that may run as one stretch on the device (k_steps, k_flight): no
-// phase timers, and a system with a consumer (SOIL_RESIDENT_STEPS=0: never) fits
-// one resident launch, one root per thread of a CTA of 1,024 per SM, and has no
-// radii that change with every fold.
+// phase timers, and a system with a consumer (SOIL_RESIDENT_STEPS=0: never) runs
+// the CSR walk, fits one resident launch, one root per thread of a CTA of 1,024
+// per SM, and has no radii that change with every fold.
 uint64_t resident_limit(const soil_sys* s, uint64_t want) {
     if (s->timing_mask) return 0;
     if (builtin_consumer(s)) {
+        if (force_variant() != SOIL_FORCE_CSR) return 0;  // k_steps is a CSR walk
         if (s->nlocal > steps_max_roots(s->ctx->sms) || s->border_gen < s->steps_retry_gen) return 0;
         int idx[kMaxPlanes], nr;
         zero_planes_of(s, SOIL_COL_REVERSE, idx, &nr);

@@ -1,5 +1,6 @@
 """Which form light steps take, seen by the kernel launches they issue."""
 import ctypes as C
+import os
 
 import pytest
 
@@ -84,4 +85,28 @@ def test_lists_that_never_fit_step_by_launches(ctx):
     o.step(25)
     assert_same_state(g, o)
     assert_same_lists(g, o)
+    g.close()
+
+
+@pytest.mark.parametrize("force,resident", [("csr", True), ("walk", False), ("tiles4", False),
+                                            ("tiles2", False), ("gather", False)])
+def test_light_steps_run_the_kernel_soil_force_names(ctx, force, resident):
+    """Only the CSR walk has a resident form; the others launch in every step."""
+    w = W.poly("forms-force", 321, 4000, 0.45, 1e-5, 0, harmonic_k=1e3)
+    o = oracle.from_workload(w)
+    old = os.environ.get("SOIL_FORCE")
+    os.environ["SOIL_FORCE"] = force
+    try:
+        g = system.from_workload(ctx, w)
+        g.step(1)
+        launches = _launches(g, 40)
+    finally:
+        if old is None:
+            del os.environ["SOIL_FORCE"]
+        else:
+            os.environ["SOIL_FORCE"] = old
+    assert g.counts().rebuilds == 1
+    assert launches <= 4 if resident else launches >= 80, launches
+    o.step(41)
+    assert_same_state(g, o, force)
     g.close()
