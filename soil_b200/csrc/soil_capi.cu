@@ -404,6 +404,26 @@ void timer_end(soil_sys* s, int t) {
     s->open_timer = -1;
 }
 
+// The spans from the `keep`th on are no phases: their launches did nothing.
+void timer_drop(soil_sys* s, size_t keep) {
+    while (s->spans.size() > keep) {
+        s->ev_pool.push_back(s->spans.back().a);
+        s->ev_pool.push_back(s->spans.back().b);
+        s->spans.pop_back();
+    }
+}
+
+// Span `at`, the last one, goes on.
+void timer_reopen(soil_sys* s, size_t at) {
+    if (at >= s->spans.size()) return;  // not timed
+    const soil_sys::TimedSpan sp = s->spans.back();
+    s->spans.pop_back();
+    s->ev_pool.push_back(sp.b);
+    s->open_timer = sp.timer;
+    s->open_ev = sp.a;
+    s->open_launches = launches_so_far() - sp.launches;
+}
+
 // Fold completed spans into the sums (the stream must be idle).
 void resolve_timers(soil_sys* s) {
     for (auto& sp : s->spans) {
@@ -1698,6 +1718,14 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
     guard.flags = s->dflags;
     guard.pub_flags = s->hflags_dev;
     const bool early = s->indices.p && (!with_in || s->in_list.p) && nl > 0;
+    size_t build_span = s->spans.size(), force_span = build_span;
+    // The early consumer did nothing, and the build goes on.
+    const auto not_consumed = [&] {
+        if (!*consumed) return;
+        *consumed = false;
+        timer_drop(s, force_span);
+        timer_reopen(s, build_span);
+    };
     if (early) {
         launch_pair_fill(s->st, p, s->rowcount.p, s->row_slots.p, s->offsets.p, s->indices.p,
                          guard);
@@ -1706,6 +1734,7 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
             launch_segsort_split(s->st, total, s->in_start.p, s->in_list.p, s->in_split.p, &guard);
         if (consumer_next) {
             timer_end(s, T_NEIGHBOR);
+            force_span = s->spans.size();
             timer_begin(s, T_FORCE);
             FillGuard open = guard;
             open.over = pend ? s->bstate.p + 10 : nullptr;
@@ -1735,8 +1764,8 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
             // this build with the host reading the ghost counts first.
             TRY(grow_atoms(s, (uint64_t)hb[3] + 1024, s->nlocal));
             s->state = FULL_REBUILD;
+            not_consumed();
             TRY(phase_borders_defer(s, false));
-            *consumed = false;
             return phase_neighbor(s);
         }
         TRY(borders_done(s, hb, s->pending_bds));
@@ -1749,7 +1778,7 @@ int phase_neighbor_with(soil_sys* s, bool consumer_next, bool* consumed) {
     if (s->hflags->error)
         return fail(s->ctx, SOIL_ERR_INVALID, "neighbor stencil left the bin grid (atom outside the ghost layers)");
     if (!early || np + 1 > guard.cap) {  // the early pass did not run: again, into room for np
-        *consumed = false;
+        not_consumed();
         TRY(ensure(s, s->indices, np + 1, 0, pair_room(np)));
         if (with_in) {
             TRY(ensure(s, s->in_list, np + 1, 0, pair_room(np)));
@@ -2355,11 +2384,7 @@ int light_step(soil_sys* s, bool last) {
     bool tripped = false;
     TRY(light_answer(s, kHostAnswer, w.tag, &tripped));
     if (tripped) {
-        while (s->spans.size() > spans) {  // the empty launches are no phase
-            s->ev_pool.push_back(s->spans.back().a);
-            s->ev_pool.push_back(s->spans.back().b);
-            s->spans.pop_back();
-        }
+        timer_drop(s, spans);
         p.tripped = true;
         return step_rest(s, p, last);
     }
