@@ -21,6 +21,9 @@ Printed JSON keys beyond the base contract:
                          measured past the timed region until >= 3 rebuilds
   ms_per_step_at_rebuild_rate, neighbor_builds_per_s
                          the two mixed at the rebuild rate seen there
+  ms_per_rebuild_cycle   (no consumer) a rebuild with the stretch of steps before
+                         it, which costs the same whatever its length: no cost
+                         per light or rebuild step, no HBM fraction
   roofline               dominant kernel: algorithmic bytes / mean launch time
   cpu_baseline           the CPU oracle on a bounded sample of the same system
   e2e                    the same metric through the C ABI from pinned host
@@ -188,7 +191,18 @@ def make_workload(name, filt, natoms=None):
     return w, desc
 
 
-def rebuild_probe(s, stream, min_rebuilds=3, chunk=25, max_steps=800):
+def phase_roofline(kernel, phase, alg_bytes, ms, launches, peak, peak_kind, traffic):
+    """The HBM roofline of a timed phase; None when nothing of it was timed."""
+    if not launches or not ms:
+        return None
+    achieved = alg_bytes / (ms / launches * 1e-3) / 1e9
+    return {"bound": "hbm", "kernel": kernel, "phase": phase, "achieved": achieved, "peak": peak,
+            "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind, "traffic": traffic,
+            "algorithmic_bytes_per_launch": alg_bytes, "mean_launch_ms": ms / launches,
+            "launches": int(launches)}
+
+
+def rebuild_probe(s, stream, min_rebuilds=3, chunk=25, max_steps=800, stretches=False):
     """Light and rebuild step costs of a system past the timed region.
 
     Steps it in calls of about `chunk` steps (lengths varied), each timed with
@@ -197,7 +211,9 @@ def rebuild_probe(s, stream, min_rebuilds=3, chunk=25, max_steps=800):
     chunk_ms = L * steps + X * rebuilds + C over the chunks (least squares):
     L is the light (communicate-only) step, L + X the rebuild step, C the
     per-call cost (each call ends with the final half-kick, as every
-    soil_step call does)."""
+    soil_step call does).  stretches: the steps between two rebuilds cost the
+    same whatever their number (systems without a consumer), so the fit is
+    chunk_ms = B * rebuilds + C, B a rebuild and the stretch before it."""
     import torch
     rows = []
     steps = rebuilds = 0
@@ -228,6 +244,14 @@ def rebuild_probe(s, stream, min_rebuilds=3, chunk=25, max_steps=800):
     t = np.array([ms for _, _, ms in rows])
     out = {"steps": steps, "rebuilds": rebuilds, "chunk_steps": list(lengths),
            "rebuild_rate": rebuilds / steps}
+    if stretches:
+        out.update(ms_per_light_step=None, ms_per_rebuild_step=None, ms_per_rebuild_cycle=None,
+                   ms_per_step_at_rebuild_rate=float(t.sum() / steps),
+                   neighbor_builds_per_s=float(rebuilds / (t.sum() * 1e-3)))
+        if np.linalg.matrix_rank(A[:, 1:]) == 2:
+            (cycle, _), *_ = np.linalg.lstsq(A[:, 1:], t, rcond=None)
+            out["ms_per_rebuild_cycle"] = float(cycle)
+        return out
     if rebuilds and np.linalg.matrix_rank(A) == 3:
         (light, extra, _), *_ = np.linalg.lstsq(A, t, rcond=None)
         out.update(ms_per_light_step=float(light), ms_per_rebuild_step=float(light + extra))
@@ -318,8 +342,10 @@ def run_soil(args, world, rank, local):
     # launch) unless SOIL_RESIDENT_STEPS=0; phase timers would force the
     # launch-per-phase path, so they stay off there and the roofline comes from
     # the light-step time of the rebuild probe.  A workload that rebuilds on
-    # every step has none of these steps, and keeps its phase timer.
-    resident = os.environ.get("SOIL_RESIDENT_STEPS", "2") != "0" and not all_rebuilds
+    # every step has none of these steps, and keeps its phase timer; so does one
+    # whose consumer is not the CSR walk (SOIL_FORCE).
+    resident = (os.environ.get("SOIL_RESIDENT_STEPS", "2") != "0" and not all_rebuilds
+                and (not w.harmonic_k or phase_kernel(lib, "force") == "k_force_csr"))
     s.set_timing(0 if resident else 1 << abi.TIMER_NAMES.index(dominant))
 
     c0 = s.counts()
@@ -349,36 +375,32 @@ def run_soil(args, world, rank, local):
     value = world * w.n * args.steps / (ms_max * 1e-3)
     rebuilds = int(c1.rebuilds - c0.rebuilds)
     peak, peak_kind = load_peaks()
-    per_launch_ms = ms_dom[k] / max(launches_dom[k], 1)
     alg_bytes = BYTES_PER_UNIT[dominant](c1, fwd_width)
-    achieved = alg_bytes / (per_launch_ms * 1e-3) / 1e9
     kname = phase_kernel(lib, dominant)
     tr = load_traffic(kname, args.config)
     traffic = None
     if tr:
         traffic = tr["dram_bytes_per_atom"] * (c1.nlocal if dominant in ("integrate", "final")
                                                else c1.nlocal + c1.nghost)
-    roofline = {"bound": "hbm", "kernel": kname, "phase": dominant,
-                "achieved": achieved, "peak": peak,
-                "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
-                "traffic": traffic, "algorithmic_bytes_per_launch": alg_bytes,
-                "mean_launch_ms": per_launch_ms, "launches": int(launches_dom[k])}
+    roofline = phase_roofline(kname, dominant, alg_bytes, ms_dom[k], launches_dom[k], peak,
+                              peak_kind, traffic)
 
     # per-phase breakdown (warm-up steps) for the record
     phases = {abi.TIMER_NAMES[t]: round(ms0[t], 4) for t in range(abi.SOIL_NUM_TIMERS) if iv0[t]}
     # the rebuild half of the metric: light and rebuild steps past the timed
     # region, until at least three rebuilds
     s.set_timing(0)
-    probe = rebuild_probe(s, stream)
+    flights = resident and not w.harmonic_k
+    probe = (rebuild_probe(s, stream, min_rebuilds=20, stretches=True) if flights
+             else rebuild_probe(s, stream))
     if resident and probe["ms_per_light_step"]:
         # algorithmic bytes of a light step over the light-step time: those of
         # the integration pass and the consumer; as one launch per step (no
         # second read of the forces) the consumer's, then per local R v,
         # inv_mass, build position, W v, x, per ghost R chain, W v, x
-        light_kernel = ("k_flight_find + k_flight_apply" if not w.harmonic_k
-                        else "k_steps" if w.n <= STEPS_MAX_ROOTS else "k_force_step")
-        step_bytes = BYTES_PER_UNIT["integrate"](c1, fwd_width) + (
-            BYTES_PER_UNIT["force"](c1, fwd_width) if w.harmonic_k else 0)
+        light_kernel = "k_steps" if w.n <= STEPS_MAX_ROOTS else "k_force_step"
+        step_bytes = (BYTES_PER_UNIT["integrate"](c1, fwd_width)
+                      + BYTES_PER_UNIT["force"](c1, fwd_width))
         if light_kernel == "k_force_step":
             step_bytes = (BYTES_PER_UNIT["force"](c1, fwd_width) + 104 * c1.nlocal
                           + 52 * c1.nghost)
@@ -420,6 +442,7 @@ def run_soil(args, world, rank, local):
             "ms_per_light_step": probe["ms_per_light_step"],
             "ms_per_rebuild_step": probe["ms_per_rebuild_step"],
             "ms_per_step_at_rebuild_rate": probe["ms_per_step_at_rebuild_rate"],
+            "ms_per_rebuild_cycle": probe.get("ms_per_rebuild_cycle"),
             "rebuild_probe": {k: probe[k] for k in ("steps", "rebuilds", "chunk_steps",
                                                     "rebuild_rate")},
             "roofline": roofline,
@@ -556,19 +579,18 @@ def run_batched(args, world, rank, local):
     total_atoms = dist.sum_over_ranks(natoms, world)
     value = total_atoms * args.steps / (ms_max * 1e-3)
 
-    # roofline of the consumer kernel (one launch per step over every box):
-    # R pos+radius of every atom, W force, R offsets, R each pair twice
-    force_ms = tim["force"][0] / max(tim["force"][1], 1)
-    force_bytes = sum(64 * (c.nlocal + c.nghost) + 8 * c.npairs for c in cs)
+    # roofline of the consumer kernel (one launch per step over every box); the
+    # walk folds the ghosts' forces itself, the gather leaves them to a pass
+    kname = phase_kernel(lib, "force")
+    if kname == "k_harmonic":
+        force_bytes = sum(64 * (c.nlocal + c.nghost) + 8 * c.npairs for c in cs)
+    else:
+        force_bytes = sum(BYTES_PER_UNIT["force"](c, 1) for c in cs)
     peak, peak_kind = load_peaks()
-    achieved = force_bytes / (force_ms * 1e-3) / 1e9
-    tr = load_traffic("batched_force", "c4")
-    roofline = {"bound": "hbm", "kernel": "kb_harmonic (all boxes, one launch)",
-                "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "peak_source": peak_kind,
-                "traffic": tr["dram_bytes_per_launch"] if tr else None,
-                "algorithmic_bytes_per_launch": force_bytes, "mean_launch_ms": force_ms,
-                "launches": tim["force"][1]}
+    tr = load_traffic("batched " + kname, "c4")
+    roofline = phase_roofline("kb" + kname[1:] + " (all boxes, one launch)", "force", force_bytes,
+                              tim["force"][0], tim["force"][1], peak, peak_kind,
+                              tr["dram_bytes_per_launch"] if tr else None)
     stages = {k: round(v[0] / max(v[1], 1), 4) for k, v in tim.items()}
     host = {k: round(v / args.steps, 4) for k, v in batch.get_host_timing().items()}
     cb = None
