@@ -154,11 +154,16 @@ void dev_free(soil_sys* s, void* p, uint64_t bytes) {
 }
 
 // The slabs back to the context (or its pool), once every array is gone and the
-// stream has drained.
+// stream has drained.  A system whose columns come from the pool by themselves
+// leaves none: its slab of small arrays saves the next one little, and between
+// the columns it would keep the pool from handing out the room of all of them
+// again (the second of two systems of 1,048,576 atoms then mapped 32 MB more, 0.4
+// ms, and much longer while others use the machine).
 void arena_free(soil_sys* s) {
     std::lock_guard<std::mutex> g(s->ctx->mu);
+    const bool keep = s->acap * 8 <= kArenaMax;
     for (const Arena::Slab& b : s->arena.slabs)
-        if (!s->ctx->kept.give(b.p, b.size)) cudaFreeAsync(b.p, s->st);
+        if (!keep || !s->ctx->kept.give(b.p, b.size)) cudaFreeAsync(b.p, s->st);
     s->arena = Arena{};
 }
 
