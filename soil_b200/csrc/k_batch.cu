@@ -2,11 +2,11 @@
 //
 // Three launch shapes:
 //   element spans   blocks walk the flattened element range in chunks of
-//                   kBlock * kSpanItems, locate the chunk's segment once and
-//                   advance per element (boxes hold hundreds of atoms or more);
-//   segment per CTA exclusive scans, one CTA per box;
-//   tile spans      border tiles, one CTA per tile (the tile's CTA-wide scan
-//                   ranks its ghosts in order).
+//                   Span::items rows of kBlock elements; a warp locates the
+//                   chunk's segment once and its lanes advance per element
+//                   (boxes hold hundreds of atoms or more);
+//   scan tiles      one CTA per 8,192 counts of a box (scan_direct_tile);
+//   tile spans      border and staged pair tiles, one warp per 32 locals.
 // Every element calls the same device function as the single-system kernels.
 #include "batch.cuh"
 #include "block_scan.cuh"

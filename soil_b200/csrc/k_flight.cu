@@ -16,9 +16,10 @@
 //
 // Bit-identical to one integration pass and forward comm per step.  A step
 // costs its arithmetic instead of a pass over the columns and a grid barrier:
-// on 32,768 atoms in free flight (some ten steps between rebuilds) a light step
-// went from 8.1 us in a cooperative launch with one grid barrier per step to
-// under 1 us, and 200 steps with their 20 rebuilds from 3.78 to 2.16 ms.
+// on 32,768 atoms in free flight (some ten steps between rebuilds) a stretch
+// takes 6.1 + 8.0 us (the second launch with its wait for the first), where a
+// step took 8.1 us in a cooperative launch with one grid barrier per step, and
+// 200 steps with their 20 rebuilds went from 3.78 to 2.16 ms.
 #include "device_ops.cuh"
 #include "kernels.cuh"
 

@@ -339,10 +339,11 @@ SwapConst swap_const(const soil_sys* s);
 // a light step's displacement check.
 constexpr int kHostAnswer = 2 * kBorderStateWords;
 constexpr int kHostWords = kHostAnswer + 8;
-// Largest system whose spatial sort ranks and gathers in one pass; above, a
-// segment sort and a gather are faster (46.9 against 49.5 us on 1,048,576
-// atoms, 176 against 167 on 4,194,304, where the rank's loads come on top of a
-// pass bound by HBM).
+// Largest system whose spatial sort ranks and gathers in one pass: faster than a
+// segment sort and a gather on 1,048,576 atoms (46.9 against 49.5 us), slower on
+// 4,194,304 (176 against 167, where the rank's loads come on top of a pass bound
+// by HBM).  A whole sheared step gains 2 to 3 us up to 2,000,003 atoms (647 of
+// 649), 1 on 2,500,009 and 3,000,017, nothing on 4,194,304.
 constexpr uint64_t kSortGatherMax = 2000000;
 constexpr int kRowSlotsPerAtom = 16;
 
