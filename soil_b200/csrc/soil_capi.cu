@@ -2018,6 +2018,24 @@ int step_integrate(soil_sys* s, StepPlan* out) {
     return SOIL_OK;
 }
 
+// A step's forces and reverse comm; consumed: the consumer ran already.  With
+// newton, the grouped consumer folds ghost forces into their roots in the same
+// kernel (reverse_send_force's fold order); otherwise the force and reverse-comm
+// phases run apart.
+int step_forces(soil_sys* s, bool consumed) {
+    const bool fold_fused = consumer_folds(s);
+    if (!consumed) {
+        timer_begin(s, T_FORCE);
+        TRY(fold_fused ? launch_consumer(s, true) : phase_force(s));
+        timer_end(s, T_FORCE);
+    }
+    if (fold_fused) s->reverse_gen = s->border_gen;
+    timer_begin(s, T_REVERSE);
+    if (!fold_fused && reverse_needed(s)) TRY(phase_reverse_comm(s));
+    timer_end(s, T_REVERSE);
+    return SOIL_OK;
+}
+
 // The rest of a timestep after its integration pass: decide_rebuild, the
 // rebuild phases when due, forward comm, the consumer, reverse comm and the
 // final half-kick (applied now when `last`, else deferred into the next
@@ -2082,23 +2100,7 @@ int step_rest(soil_sys* s, const StepPlan& p, bool last) {
     bool consumed = false;
     TRY(phase_neighbor_with(s, consumer_goes_early(s), &consumed));
     timer_end(s, T_NEIGHBOR);
-    // With newton, the grouped consumer folds ghost forces into their roots
-    // in the same kernel (reverse_send_force's fold order); otherwise the
-    // force and reverse-comm phases run apart.
-    const bool fold_fused = consumer_folds(s);
-    if (!consumed) timer_begin(s, T_FORCE);
-    if (consumed) {
-        if (fold_fused) s->reverse_gen = s->border_gen;
-    } else if (fold_fused) {
-        TRY(launch_consumer(s, true));
-        s->reverse_gen = s->border_gen;
-    } else {
-        TRY(phase_force(s));
-    }
-    timer_end(s, T_FORCE);
-    timer_begin(s, T_REVERSE);
-    if (!fold_fused && reverse_needed(s)) TRY(phase_reverse_comm(s));
-    timer_end(s, T_REVERSE);
+    TRY(step_forces(s, consumed));
     if (last) {
         timer_begin(s, T_FINAL);
         TRY(phase_final(s));
@@ -2366,10 +2368,11 @@ int light_integrate(soil_sys* s, const StepPlan& p, LightStep* out) {
     return SOIL_OK;
 }
 
-// One light step (light_limit >= 1) of a system with the CSR consumer, phase
-// by phase: forward comm and the consumer go in behind the integration pass
-// and do nothing if its check tripped; the host reads the answer while they
-// run, so the stream never waits for it.
+// One light step (light_limit >= 1) of a system with a consumer, phase by phase:
+// forward comm goes in behind the integration pass and does nothing if its check
+// tripped; so does the CSR consumer, and the host reads the answer while they
+// run, so the stream never waits for it.  Another consumer (SOIL_FORCE) goes in
+// once the answer is there.
 int light_step(soil_sys* s, bool last) {
     StepPlan p = plan_step(s);
     TRY(light_words(s));
@@ -2383,9 +2386,12 @@ int light_step(soil_sys* s, bool last) {
     timer_begin(s, T_FORWARD);
     TRY(forward_comm(s, p.fused_zero, &w));
     timer_end(s, T_FORWARD);
-    timer_begin(s, T_FORCE);
-    TRY(launch_consumer(s, s->newton, w.trip));
-    timer_end(s, T_FORCE);
+    const bool early = force_variant() == SOIL_FORCE_CSR;
+    if (early) {
+        timer_begin(s, T_FORCE);
+        TRY(launch_consumer(s, s->newton, w.trip));
+        timer_end(s, T_FORCE);
+    }
     bool tripped = false;
     TRY(light_answer(s, kHostAnswer, w.tag, &tripped));
     if (tripped) {
@@ -2393,7 +2399,8 @@ int light_step(soil_sys* s, bool last) {
         p.tripped = true;
         return step_rest(s, p, last);
     }
-    if (s->newton) s->reverse_gen = s->border_gen;
+    if (!early) TRY(step_forces(s, false));
+    else if (s->newton) s->reverse_gen = s->border_gen;
     light_steps_done(s, 1, false);
     if (last) {
         timer_begin(s, T_FINAL);
@@ -2527,7 +2534,7 @@ int step_many(soil_sys* s, uint64_t n) {
             }
             continue;
         }
-        if (builtin_consumer(s) && force_variant() == SOIL_FORCE_CSR && light_limit(s, 1) >= 1)
+        if (builtin_consumer(s) && light_limit(s, 1) >= 1)
             TRY(light_step(s, k + 1 == n));
         else
             TRY(full_step(s, k + 1 == n));

@@ -110,3 +110,41 @@ def test_light_steps_run_the_kernel_soil_force_names(ctx, force, resident):
     o.step(41)
     assert_same_state(g, o, force)
     g.close()
+
+
+@pytest.mark.parametrize("force", ["walk", "tiles2", "gather"])
+@pytest.mark.parametrize("newton,reverse", [(1, 0), (1, 1), (0, 0)])
+def test_named_kernels_step_alike_with_and_without_the_host(ctx, force, newton, reverse):
+    """Light steps whose check's answer the host reads while forward comm runs
+    give the bits of one launch per phase, #[reverse] columns included."""
+    w = W.poly("forms-named", 323, 6000, 0.5, 1e-3, 0, harmonic_k=1e3, newton=newton)
+    w.vel *= 2.0
+    out = []
+    keys = ("SOIL_FORCE", "SOIL_RESIDENT_STEPS")
+    old = {k: os.environ.get(k) for k in keys}
+    try:
+        for mode in ("2", "0"):
+            os.environ.update(dict(zip(keys, (force, mode))))
+            g = system.System(ctx, w.box, w.cfg, w.dt)
+            rc = g.register_column("radius", 1, abi.SOIL_COL_FORWARD)
+            cols = [w.radius]
+            if reverse:
+                g.register_column("acc", 1, abi.SOIL_COL_REVERSE)
+                cols.append(1.0 + w.pos[:, 0])
+            g.add_atoms(w.tag, w.pos, w.vel, w.mass, w.cutoff, columns=cols)
+            g.set_harmonic(w.harmonic_k, rc)
+            g.setup()
+            for n in (1, 2, 1, 25):
+                g.step(n)
+            out.append(g)
+    finally:
+        for k, v in old.items():
+            if v is None:
+                os.environ.pop(k, None)
+            else:
+                os.environ[k] = v
+    assert_same_state(*out, force)
+    assert_same_lists(*out)
+    assert 2 < out[0].counts().rebuilds < 29
+    for g in out:
+        g.close()
