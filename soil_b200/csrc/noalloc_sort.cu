@@ -71,7 +71,11 @@ __global__ void __launch_bounds__(kBlock) k_noalloc_cells(uint64_t n, const doub
 __global__ void __launch_bounds__(kBlock) k_noalloc_scatter(uint64_t n, const uint32_t* start,
                                                             uint32_t* cell, uint32_t* counts,
                                                             uint32_t* out) {
-    pdl_wait();  // launched with pdl_launch
+    // The wait alone: the segment sort starts when this kernel has completed.
+    // Released earlier, its few CTAs pile up on the SMs that free up first, and
+    // with many atoms per cell each is a long serial sort (131 against 89 us a call
+    // on 2,000,000 atoms, 30 per cell).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t v = cell[i], c = v & kCellMask;
